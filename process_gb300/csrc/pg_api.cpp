@@ -1949,13 +1949,9 @@ void simulate_seq_impl(const pg_placed* pl, const pg_seq_cfg* c, uint64_t seed, 
     auto smp_d = upload(P, samples, st);
     auto leaf_d = upload(P, leaf_tin, st);
     auto ins_d = upload(P, ins_thr, st);
-    // guide table of the insert CDF: first index whose threshold exceeds g * 2^23
-    std::vector<uint16_t> guide(256);
-    for (uint32_t g = 0; g < 256; ++g) {
-      const uint32_t v = g << 23;
-      const uint32_t k = uint32_t(std::upper_bound(ins_thr.begin(), ins_thr.end(), v) - ins_thr.begin());
-      guide[g] = uint16_t(std::min<uint32_t>(k, uint32_t(ins_thr.size()) - 1));
-    }
+    std::vector<uint32_t> guide(pg::SEQ_GUIDE, 0);
+    if (ins_thr.size() <= pg::SEQ_GUIDE_INS)
+      for (uint32_t g = 0; g < pg::SEQ_GUIDE; ++g) guide[g] = pg::insert_guide(ins_thr.data(), uint32_t(ins_thr.size()), g);
     auto guide_d = upload(P, guide, st);
     DBuf<pg::SeqRec> recs(P, pl->M);
     DBuf<uint32_t> pair_cnt(P, uint64_t(n_tiles) * samples.size()), rlo(P, n_tiles), rhi(P, n_tiles);

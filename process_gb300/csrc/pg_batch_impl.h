@@ -64,7 +64,7 @@ struct pg_batch {
   DBuf<uint64_t> c_pairs;
   DBuf<pg::SeqSample> samples;
   DBuf<uint32_t> leaf_tin, etin, etout, ins_cdf, counter, alt, depth;
-  DBuf<uint16_t> ins_guide;
+  DBuf<uint32_t> ins_guide;
   DBuf<pg::SeqRec> recs;
   uint64_t rec_cap = 0;
   cudaGraphExec_t graph = nullptr;
@@ -246,7 +246,7 @@ void batch_layout(pg_batch* b) {
   std::vector<uint32_t> t_start, t_len, t_end, t_inst, c_first, c_ntiles, c_depth, c_nstarts, c_id, blk_slot,
       blk_index, leaf_tin, etin, etout, ins_cdf, item_off{0}, cnt_off{0};
   std::vector<uint64_t> c_pairs;
-  std::vector<uint16_t> guide_all;
+  std::vector<uint32_t> guide_all;
   std::vector<pg::SeqSample> samples;
   b->sinst.assign(B, pg::SeqInst{});
   b->stride.assign(B, 0);
@@ -337,13 +337,10 @@ void batch_layout(pg_batch* b) {
     prm.has_cna = 0;
     // insert tables: positions into the concatenated arrays, patched below
     prm.ins_cdf = reinterpret_cast<const uint32_t*>(uintptr_t(ins_cdf.size()));
-    prm.ins_guide = reinterpret_cast<const uint16_t*>(uintptr_t(guide_all.size()));
+    prm.ins_guide = reinterpret_cast<const uint32_t*>(uintptr_t(guide_all.size()));
     ins_cdf.insert(ins_cdf.end(), thr.begin(), thr.end());
-    for (uint32_t g = 0; g < 256; ++g) {
-      const uint32_t v = g << 23;
-      const uint32_t k = uint32_t(std::upper_bound(thr.begin(), thr.end(), v) - thr.begin());
-      guide_all.push_back(uint16_t(std::min<uint32_t>(k, uint32_t(thr.size()) - 1)));
-    }
+    for (uint32_t g = 0; g < pg::SEQ_GUIDE; ++g)
+      guide_all.push_back(thr.size() <= pg::SEQ_GUIDE_INS ? pg::insert_guide(thr.data(), uint32_t(thr.size()), g) : 0u);
     // counts and work items
     S.pair_off = pair_total;
     pair_total += uint64_t(S.n_samples) * n_tiles;

@@ -191,6 +191,24 @@ struct SeqRec {            // 16 B, one per placed mutation, sorted by locus
 // tiles are sized so that their fragment count rarely exceeds one batch
 constexpr uint32_t SEQ_FRAGS_PER_BATCH = 1280;
 
+// The insert-size lookup of a 31-bit word v: entry g = v >> 21 of the guide
+// covers the words of one cell and holds k, the first index whose threshold
+// exceeds the cell's first word (bits 0-9), the last word of the cell that
+// still gets k, relative to the cell's first (bits 10-30), and whether later
+// words need a walk over the thresholds (bit 31; else they get k + 1).  Tables
+// of at most SEQ_GUIDE_INS thresholds have a guide: 1024 cells leave about
+// one word in a hundred of a normal-shaped table to the walk (256 left one in
+// thirty, so that most warps had a lane in it).
+constexpr uint32_t SEQ_GUIDE = 1024, SEQ_GUIDE_INS = 1024;
+inline uint32_t insert_guide(const uint32_t* thr, uint32_t n, uint32_t g) {
+  const uint32_t first = g << 21, next = first + (1u << 21);   // cells end at 2^31 at the latest
+  uint32_t lo = 0, hi = n;
+  while (lo < hi) { const uint32_t mid = (lo + hi) / 2; if (thr[mid] <= first) lo = mid + 1; else hi = mid; }
+  if (lo >= n || thr[lo] >= next) return (lo < n ? lo : n - 1) | 0x7ffffc00u;
+  const bool walk = lo + 1 >= n || thr[lo + 1] < next;
+  return lo | (thr[lo] - first - 1u) << 10 | (walk ? 0x80000000u : 0u);
+}
+
 struct SeqTiles {
   uint32_t n_tiles;        // over all selected chromosomes
   const uint32_t* start;   // first start position of the tile (absolute)
@@ -224,7 +242,7 @@ struct SeqParams {
   uint32_t span;           // max fragment span past the start (read_len or max insert)
   uint32_t ins_min, n_ins; // insert size = ins_min + index in the CDF table
   const uint32_t* ins_cdf;
-  const uint16_t* ins_guide; // 256 entries: first index whose threshold exceeds g * 2^23
+  const uint32_t* ins_guide; // SEQ_GUIDE entries (see insert_guide), 16-byte aligned
   uint32_t err_thr;        // substitution error iff u < err_thr
   uint32_t err_t1, err_t2; // the erroneous base: the first of the three others iff u < err_t1,
                            //   the second iff err_t1 <= u < err_t2, else the third

@@ -49,10 +49,9 @@ __host__ __device__ inline RoundKeys round_keys(uint32_t k0, uint32_t k1) {
 __device__ __forceinline__ U4 philox(const RoundKeys& rk, uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3) {
 #pragma unroll
   for (int i = 0; i < 10; ++i) {
-    const uint32_t lo0 = 0xD2511F53u * c0, hi0 = __umulhi(0xD2511F53u, c0);
-    const uint32_t lo1 = 0xCD9E8D57u * c2, hi1 = __umulhi(0xCD9E8D57u, c2);
-    const uint32_t n0 = hi1 ^ c1 ^ rk.k0[i], n2 = hi0 ^ c3 ^ rk.k1[i];
-    c0 = n0; c1 = lo1; c2 = n2; c3 = lo0;
+    const uint64_t p0 = uint64_t(0xD2511F53u) * c0, p1 = uint64_t(0xCD9E8D57u) * c2;
+    const uint32_t n0 = uint32_t(p1 >> 32) ^ c1 ^ rk.k0[i], n2 = uint32_t(p0 >> 32) ^ c3 ^ rk.k1[i];
+    c0 = n0; c1 = uint32_t(p1); c2 = n2; c3 = uint32_t(p0);
   }
   return {c0, c1, c2, c3};
 }

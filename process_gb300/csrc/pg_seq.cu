@@ -30,15 +30,25 @@
 //     Indels are not affected by substitution errors.
 //
 // Kernel layout (one CTA per (tile, sample); fragments in batches):
-//   phase A  every thread generates fragments (one Philox block each) and
-//            writes its two mates to shared memory; mates are bucketed by
-//            start position (16 bp buckets, counting sort);
-//   phase B  work items (mutation record, start bucket) scan the mates of one
-//            bucket that may cover the record and count depth and alt in
-//            registers, one shared-memory atomic per item.
-// Both phases keep every lane busy whatever the number of mutations a read
-// covers.  Windows with more records than shared memory holds run a per-read
-// loop on the global arrays instead.
+//   phase A  every thread generates fragments (one Philox block each); their
+//            two mates go to shared memory in the order of their start
+//            buckets (16 bp, counting sort);
+//   phase B  four lanes share a mutation record and visit the mates of the
+//            buckets that may cover it, counting depth and alt in registers.
+// Windows with more records than shared memory holds run a per-read loop on
+// the global arrays instead.
+//
+// Bound by instruction issue (62% of the slots, 11 warp instructions per
+// fragment) and by shared-memory wavefronts (72%), not by HBM.  At 155 Mbp,
+// 100x paired, four samples with copy-number events (2.07e8 fragments) the
+// launch takes 2.88 ms.  The form with evenly split candidate runs (a thread
+// walks 17 or so candidates across record borders), a lineage walk and two
+// table lookups per draw took 4.53 ms at 18.6 warp instructions per fragment.
+// Lanes per record in phase B, same launch: 32 3.50 ms, 16 3.37, 8 3.01,
+// 4 2.92 (2.89 with two candidates per step), 2 2.87: fewer lanes amortise a
+// record's set-up over more records per warp; four keeps more warps busy
+// where windows hold few records.  One batch per tile in CTAs of 512 threads
+// took 3.25 ms.
 #include <type_traits>
 
 #include "pg_common.cuh"
@@ -51,10 +61,12 @@ namespace pg {
 constexpr int SEQ_THREADS = 256;
 constexpr uint32_t SEQ_CAP = 512;        // mutation records staged per CTA
 constexpr uint32_t SEQ_MCAP = 2 * SEQ_FRAGS_PER_BATCH;   // mates per batch
+constexpr uint32_t SEQ_REC_LANES = 4;    // lanes that share a record in phase B
 constexpr uint32_t SEQ_BW = 16;          // start bucket width (bp)
 constexpr uint32_t SEQ_NBK = 1024;       // start buckets per window (window <= 16 kbp)
-constexpr uint32_t SEQ_INS_CAP = 1024;   // insert-size CDF entries staged in shared memory
-constexpr uint32_t SEQ_GUIDE = 256;      // guide table of the insert-size CDF
+static_assert(SEQ_NBK == 4 * SEQ_THREADS, "the bucket scan takes four buckets per thread");
+static_assert(SEQ_GUIDE == 4 * SEQ_THREADS, "the insert table is staged by one 16-byte load per thread");
+static_assert(SEQ_MCAP < 65536, "bucket offsets and a batch's counts are 16-bit");
 
 __global__ void k_seq_records(PlaceOut s, uint32_t n, const uint32_t* __restrict__ edge_tin,
                               const uint32_t* __restrict__ edge_tout, SeqRec* __restrict__ recs) {
@@ -258,9 +270,9 @@ __global__ void __launch_bounds__(SPLIT_THREADS) k_tile_split_level(
 __device__ __forceinline__ uint32_t mate_word(uint32_t w, uint32_t mate) {
   return mate ? w * 0x85EBCA6Bu + 0x27D4EB2Fu : w;
 }
-__device__ __forceinline__ uint32_t err_word(uint32_t wm, uint32_t locus) {
-  return (wm ^ (locus * 0x9E3779B1u)) * 0xC2B2AE35u;
-}
+constexpr uint32_t ERR_LOCUS = 0x9E3779B1u;
+__device__ __forceinline__ uint32_t err_word_at(uint32_t wm, uint32_t lc) { return (wm ^ lc) * 0xC2B2AE35u; }
+__device__ __forceinline__ uint32_t err_word(uint32_t wm, uint32_t locus) { return err_word_at(wm, locus * ERR_LOCUS); }
 // which of the three other bases an error word below err_thr picks
 __device__ __forceinline__ uint32_t err_third(const SeqParams& prm, uint32_t e) {
   return e < prm.err_t1 ? 0u : (e < prm.err_t2 ? 1u : 2u);
@@ -321,34 +333,49 @@ struct Fragment {
 
 // The copy-number draw tables of one (tile, sample) staged in shared memory:
 // the tile's parts with their thresholds and, per part, the option
-// thresholds of its atom and each option's covering instances there.
-constexpr uint32_t SEQ_CN_PARTS = 4, SEQ_CN_OPTS = 8;
+// thresholds of its atom (unused ones past any 31-bit word) and each option's
+// covering instances there.  The instances of all (part, option) pairs are
+// numbered through as local ids (the instance of id l: linst[l]), so that a
+// fragment's instance draw needs no lookup and a record can hold the set of
+// instances that carry it as a bit mask over the ids.
+constexpr uint32_t SEQ_CN_PARTS = 4, SEQ_CN_OPTS = 8, SEQ_CN_IDS = 16;
 struct CnCache {
+  uint4 othr[SEQ_CN_PARTS][SEQ_CN_OPTS / 4];   // option thresholds
+  uint4 opt[SEQ_CN_PARTS][SEQ_CN_OPTS];        // covering instances, leaves, first leaf, first local id
   uint32_t pstart[SEQ_CN_PARTS], plen[SEQ_CN_PARTS], pthr[SEQ_CN_PARTS];
-  uint32_t othr[SEQ_CN_PARTS][SEQ_CN_OPTS], oioff[SEQ_CN_PARTS][SEQ_CN_OPTS], oicnt[SEQ_CN_PARTS][SEQ_CN_OPTS];
-  uint32_t onl[SEQ_CN_OPTS], oloff[SEQ_CN_OPTS];
-  uint32_t n_parts, n_opt;
+  uint32_t linst[SEQ_CN_IDS];
+  uint32_t n_parts, n_opt, n_ids;
 };
 
+// one warp fills the cache; n_ids exceeds SEQ_CN_IDS when the local ids do
+// not fit (linst is then incomplete and the cache is not used)
 __device__ __forceinline__ void fill_cn_cache(CnCache& c, const SeqParams& prm, const SeqSample& sm, uint32_t t,
-                                              uint32_t s, uint32_t tid) {
+                                              uint32_t s, uint32_t lane) {
   const uint32_t pb = prm.part_off[t], pn = prm.part_off[t + 1] - pb, no = sm.n_opt;
-  if (tid == 0) { c.n_parts = pn; c.n_opt = no; }
-  if (tid < pn) {
-    c.pstart[tid] = prm.part_start[pb + tid];
-    c.plen[tid] = prm.part_len[pb + tid];
-    c.pthr[tid] = prm.part_cdf[uint64_t(s) * prm.n_parts + pb + tid];
+  if (lane < pn) {
+    c.pstart[lane] = prm.part_start[pb + lane];
+    c.plen[lane] = prm.part_len[pb + lane];
+    c.pthr[lane] = prm.part_cdf[uint64_t(s) * prm.n_parts + pb + lane];
   }
-  if (tid < no) { c.onl[tid] = prm.opt_nleaf[sm.opt_off + tid]; c.oloff[tid] = prm.opt_leaf_off[sm.opt_off + tid]; }
-  if (tid < pn * no) {
-    const uint32_t p = tid / no, o = tid % no;
+  const uint32_t p = lane / SEQ_CN_OPTS, o = lane % SEQ_CN_OPTS;   // SEQ_CN_PARTS x SEQ_CN_OPTS = 32 lanes
+  const bool mine = p < pn && o < no;
+  uint32_t thr = 0xffffffffu, icnt = 0, ioff = 0, nl = 0, lo = 0;
+  if (mine) {
     const uint32_t atom = prm.part_atom[pb + p];
-    c.othr[p][o] = prm.opt_cdf[sm.opt_cdf_off + atom * no + o];
+    thr = prm.opt_cdf[sm.opt_cdf_off + atom * no + o];
     const uint32_t ai = atom * prm.n_classes + prm.opt_class[sm.opt_off + o];
-    c.oioff[p][o] = prm.atom_ioff[ai];
-    c.oicnt[p][o] = prm.atom_icnt[ai];
+    ioff = prm.atom_ioff[ai];
+    icnt = prm.atom_icnt[ai];
+    nl = prm.opt_nleaf[sm.opt_off + o];
+    lo = prm.opt_leaf_off[sm.opt_off + o];
   }
+  const uint32_t incl = warp_incl_scan(icnt), id0 = incl - icnt;
+  reinterpret_cast<uint32_t*>(c.othr[p])[o] = thr;
+  c.opt[p][o] = make_uint4(icnt, nl, lo, id0);
+  for (uint32_t i = 0; i < icnt && id0 + i < SEQ_CN_IDS; ++i) c.linst[id0 + i] = prm.gc.inst_list[ioff + i];
+  if (lane == 31) { c.n_parts = pn; c.n_opt = no; c.n_ids = incl; }
 }
+static_assert(SEQ_CN_PARTS * SEQ_CN_OPTS == 32 && SEQ_CN_OPTS == 8, "one lane per (part, option)");
 
 // cdf_lookup for tables of at most NMAX (a power of two) thresholds: the
 // count of thresholds <= u >> 1 by binary lifting, without a data-dependent
@@ -370,8 +397,9 @@ __device__ __forceinline__ uint32_t part_offset(uint32_t u, uint32_t lo, uint32_
 }
 
 // CN selects the copy-number path at compile time (0: no copy-number
-// events, 1: the tile's tables in shared memory, 2: the tables in global
-// memory) or, -1, at run time from prm.has_cna and cc.
+// events, 1: the tile's tables in shared memory, and inst is the mate tag of
+// the drawn local id (see ReadSmem), 2: the tables in global memory) or, -1, at run time from prm.has_cna
+// (0 or 2).
 // (KeyT: Key, or the precomputed RoundKeys of the same key)
 __device__ __forceinline__ U4 pair_block(const Key& key, uint32_t j, uint32_t t, uint32_t s) {
   return philox(key.k0, key.k1, j, t, s, TAG_PAIR);
@@ -384,12 +412,11 @@ template <bool INS_SMEM, int CN = -1, class KeyT>
 __device__ __forceinline__ Fragment make_fragment(const KeyT& key, uint32_t j, uint32_t t, uint32_t s, uint32_t start,
                                                   uint32_t len, uint32_t ce, const SeqSample& sm,
                                                   const uint32_t* __restrict__ leaf_tin, const SeqParams& prm,
-                                                  const uint32_t* ins, const uint16_t* guide,
-                                                  const CnCache* cc = nullptr) {
+                                                  const uint32_t* guide, const CnCache* cc = nullptr) {
   const U4 r = pair_block(key, j, t, s);
   Fragment f;
   const uint32_t R = prm.read_len;
-  const int path = CN >= 0 ? CN : (!prm.has_cna ? 0 : (cc ? 1 : 2));
+  const int path = CN >= 0 ? CN : (!prm.has_cna ? 0 : 2);
   if (path == 0) {
     f.p0 = start + __umulhi(r.x, len);
     const bool normal = sm.all_normal || r.y < sm.normal_thr;
@@ -404,10 +431,17 @@ __device__ __forceinline__ Fragment make_fragment(const KeyT& key, uint32_t j, u
     } else {
       f.p0 = cc->pstart[0] + __umulhi(r.x, cc->plen[0]);
     }
-    const uint32_t o = cdf_lookup_small<SEQ_CN_OPTS>(cc->othr[part], cc->n_opt, r.y);
-    const uint32_t nl = cc->onl[o], icnt = cc->oicnt[part][o];
-    f.inst = icnt ? uint32_t(__ldg(prm.gc.inst_list + cc->oioff[part][o] + __umulhi(r.w, icnt))) : 0xffffu;
-    f.cell = nl ? __ldg(prm.cls_leaf_tin + cc->oloff[o] + __umulhi(r.w * icnt, nl)) : prm.normal_tin;
+    // the option: the number of thresholds at or below the 31-bit word
+    const uint32_t v = r.y >> 1, no = cc->n_opt;
+    const uint4 h = cc->othr[part][0];
+    uint32_t o = uint32_t(h.x <= v) + uint32_t(h.y <= v) + uint32_t(h.z <= v) + uint32_t(h.w <= v);
+    if (no > 4) {
+      const uint4 g = cc->othr[part][1];
+      o += uint32_t(g.x <= v) + uint32_t(g.y <= v) + uint32_t(g.z <= v) + uint32_t(g.w <= v);
+    }
+    const uint4 op = cc->opt[part][min(o, no - 1)];   // {covering instances, leaves, first leaf, first id}
+    f.inst = op.x ? 0x10000u << ((op.w + __umulhi(r.w, op.x)) & 15u) : 0x8000u;
+    f.cell = op.y ? __ldg(prm.cls_leaf_tin + op.z + __umulhi(r.w * op.x, op.y)) : prm.normal_tin;
   } else {
     const uint32_t pb = __ldg(prm.part_off + t), pn = __ldg(prm.part_off + t + 1) - pb;
     uint32_t part = pb;
@@ -433,9 +467,12 @@ __device__ __forceinline__ Fragment make_fragment(const KeyT& key, uint32_t j, u
   if (prm.paired) {
     uint32_t k;
     if (INS_SMEM) {
-      const uint32_t v = r.z >> 1;
-      k = guide[v >> 23];
-      while (k + 1 < prm.n_ins && ins[k] <= v) ++k;
+      // one lookup, but where several thresholds share the word's cell
+      const uint32_t g = guide[r.z >> 22];
+      const bool past = (g & 0x7ffffc00u) < ((r.z << 9) & 0x7ffffc00u);
+      k = (g & 1023u) + (past ? 1u : 0u);
+      if (past && int32_t(g) < 0)
+        while (__ldg(prm.ins_cdf + k) <= (r.z >> 1)) ++k;   // the last threshold is 2^31, past every word
     } else {
       k = cdf_lookup(prm.ins_cdf, prm.n_ins, r.z);
     }
@@ -448,40 +485,45 @@ __device__ __forceinline__ Fragment make_fragment(const KeyT& key, uint32_t j, u
 
 // shared memory of one read CTA
 struct ReadSmem {
-  uint32_t s_locus[SEQ_CAP], s_tin[SEQ_CAP], s_tout[SEQ_CAP], s_info[SEQ_CAP];
-  uint32_t s_alt[SEQ_CAP], s_dep[SEQ_CAP];
+  // records of the window: offset in the window << 16 | kind, tin, tout - tin,
+  // and the mask of the local ids that carry the record << 16 (or, where the
+  // instances have no local ids, the record's info word); their first and
+  // last-plus-one candidate buckets
+  uint4 s_rec[SEQ_CAP];
+  uint32_t s_bnd[SEQ_CAP];
+  uint2 s_cnt[SEQ_CAP];          // depth, alt
   // mates of the batch in start-bucket order
-  uint32_t s_mpi[SEQ_MCAP];      // start offset in the window | allele instance << 16 (a dropped
-                                 //   fragment: offset 0xffff, instance 0xffff)
   uint2 s_mcw[SEQ_MCAP];         // source cell (Euler index), the mate's error word
-  uint32_t s_boff[SEQ_NBK + 4];  // bucket counts, then offsets
-  uint32_t s_ins[SEQ_INS_CAP];
-  uint16_t s_guide[SEQ_GUIDE];
-  uint16_t s_wstart[SEQ_CAP];    // first candidate mate (sorted position) of each record
-  uint32_t s_wpre[SEQ_CAP];      // prefix of the records' candidate counts
-  uint32_t s_scan[8];
-  uint32_t s_wtot;
+  uint32_t s_mpi[SEQ_MCAP];      // start offset in the window | local id's bit (or the instance) << 16 (a
+                                 //   dropped fragment: offset with bit 15 set)
+  uint4 s_hist[SEQ_NBK / 4];     // mates per start bucket; all zero between batches
+  uint16_t s_boff[SEQ_NBK + 4];  // first mate of each bucket
+  uint4 s_guide[SEQ_GUIDE / 4];
+  uint32_t s_scan[SEQ_THREADS / 32];
   CnCache s_cn;
 };
 
 // One work item: the n_pairs fragments of tile t (window [start, ...),
 // records [lo, lo + nw) of g_recs) for sample s, counted into the rows
 // g_alt_row / g_dep_row (indexed by record).  Called by every thread of the
-// CTA with the same arguments.
+// CTA with the same arguments; s_hist is all zero on entry and on return.
+//
+// The fragments go through in batches.  Phase A draws them, a histogram's
+// atomics giving each mate its rank in its 16 bp start bucket, and places the
+// mates in bucket order.  Phase B takes one record per warp: its candidate
+// mates (those starting in the buckets of [L - R + 1, L]) are one contiguous
+// run, visited 32 at a time with the record's terms the same in every lane.
+// Instruction issue bounds the kernel, so what a visit needs is prepared per
+// record: "the mate's instance carries the mutation" is one bit of the
+// record's mask, and the error thresholds of an indel are 0.
 template <class KeyT>
 __device__ __forceinline__ void read_tile(ReadSmem& sh, const SeqRec* __restrict__ g_recs, uint32_t t, uint32_t s,
                                           uint32_t n_pairs, uint32_t lo, uint32_t nw, uint32_t start, uint32_t len,
                                           uint32_t ce, const SeqSample& sm, const uint32_t* __restrict__ leaf_tin,
                                           const SeqParams& prm, const KeyT& key, uint32_t* __restrict__ g_alt_row,
                                           uint32_t* __restrict__ g_dep_row) {
-  auto& s_locus = sh.s_locus; auto& s_tin = sh.s_tin; auto& s_tout = sh.s_tout; auto& s_info = sh.s_info;
-  auto& s_alt = sh.s_alt; auto& s_dep = sh.s_dep;
-  auto& s_mpi = sh.s_mpi; auto& s_mcw = sh.s_mcw;
-  auto& s_boff = sh.s_boff; auto& s_ins = sh.s_ins; auto& s_guide = sh.s_guide;
-  auto& s_wstart = sh.s_wstart; auto& s_wpre = sh.s_wpre; auto& s_scan = sh.s_scan;
-  uint32_t& s_wtot = sh.s_wtot;
-  CnCache& s_cn = sh.s_cn;
-  const uint32_t tid = threadIdx.x;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  constexpr uint32_t WARPS = SEQ_THREADS / 32;
   if (nw == 0 || n_pairs == 0) return;       // nothing to count in this window
   const uint32_t R = prm.read_len;
   const uint32_t wlen = len - 1 + prm.span;   // the window is [start, start + wlen)
@@ -489,12 +531,12 @@ __device__ __forceinline__ void read_tile(ReadSmem& sh, const SeqRec* __restrict
   uint32_t* galt = g_alt_row + lo;
   uint32_t* gdep = g_dep_row + lo;
   const SeqRec* grec = g_recs + lo;
-  const bool ins_smem = prm.paired && prm.n_ins <= SEQ_INS_CAP;
+  const bool ins_smem = prm.paired && prm.n_ins <= SEQ_GUIDE_INS;
 
   if (nw > SEQ_CAP || nbk > SEQ_NBK || wlen >= 32768u) {
     // dense or long window: per-read loop over the global records
     for (uint32_t j = tid; j < n_pairs; j += SEQ_THREADS) {
-      const Fragment f = make_fragment<false>(key, j, t, s, start, len, ce, sm, leaf_tin, prm, nullptr, nullptr);
+      const Fragment f = make_fragment<false>(key, j, t, s, start, len, ce, sm, leaf_tin, prm, nullptr);
       if (f.inst == 0xffffu) continue;   // dropped: no covering instance
       for (uint32_t mate = 0; mate < (prm.paired ? 2u : 1u); ++mate) {
         const uint32_t a = mate ? f.p1 : f.p0;
@@ -510,52 +552,74 @@ __device__ __forceinline__ void read_tile(ReadSmem& sh, const SeqRec* __restrict
     return;
   }
 
-  for (uint32_t i = tid; i < nw; i += SEQ_THREADS) {
-    const SeqRec r = grec[i];
-    s_locus[i] = r.locus; s_tin[i] = r.tin; s_tout[i] = r.tout; s_info[i] = r.info;
-    s_alt[i] = 0; s_dep[i] = 0;
-  }
-  if (ins_smem) {
-    for (uint32_t i = tid; i < prm.n_ins; i += SEQ_THREADS) s_ins[i] = prm.ins_cdf[i];
-    for (uint32_t g = tid; g < SEQ_GUIDE; g += SEQ_THREADS) s_guide[g] = prm.ins_guide[g];
-  }
   // copy-number draws from shared memory when the tile's tables fit
-  // (the first barrier of the batch loop publishes them)
-  const bool cn_smem = prm.has_cna && prm.part_off[t + 1] - prm.part_off[t] <= SEQ_CN_PARTS &&
+  const bool cn_fits = prm.has_cna && prm.part_off[t + 1] - prm.part_off[t] <= SEQ_CN_PARTS &&
                        sm.n_opt <= SEQ_CN_OPTS;
-  if (cn_smem) fill_cn_cache(s_cn, prm, sm, t, s, tid);
-  const CnCache* cc = cn_smem ? &s_cn : nullptr;
+  // (the first records are on their way meanwhile)
+  SeqRec r{};
+  if (tid / 4 < nw) r = grec[tid / 4];
+  if (cn_fits && warp == 0) fill_cn_cache(sh.s_cn, prm, sm, t, s, lane);
+  if (ins_smem) sh.s_guide[tid] = __ldg(reinterpret_cast<const uint4*>(prm.ins_guide) + tid);
+  __syncthreads();
+  const int cn = !prm.has_cna ? 0 : (cn_fits && sh.s_cn.n_ids <= SEQ_CN_IDS ? 1 : 2);
+  // the records, four threads each (they share the walk over the local ids)
+  const uint32_t n_ids = cn == 1 ? sh.s_cn.n_ids : 0u;
+  for (uint32_t i0 = 0; i0 < nw; i0 += SEQ_THREADS / 4) {
+    const uint32_t i = i0 + tid / 4, sub = tid % 4;
+    if (i0 > 0 && i < nw) r = grec[i];
+    const uint32_t x = r.info & 0xffffu;
+    const uint64_t km = (uint64_t(r.tin) << 16) | ((r.info >> 16) & 0x7fffu);
+    uint32_t m = cn == 0 && x < SEQ_CN_IDS ? 1u << x : 0u;
+    if (i < nw)
+      for (uint32_t l = sub; l < n_ids; l += 4) {
+        // a copy has a larger instance number than its source, and instances
+        // 0 and 1 have no source
+        const uint32_t y = sh.s_cn.linst[l];
+        if (y == x || (y > max(x, 1u) && inst_carries(prm, y, x, km))) m |= 1u << l;
+      }
+    m |= __shfl_xor_sync(0xffffffffu, m, 1);
+    m |= __shfl_xor_sync(0xffffffffu, m, 2);
+    if (i < nw && sub == 0) {
+      const uint32_t off = r.locus - start;
+      sh.s_rec[i] = make_uint4((off << 16) | (r.info >> 31), r.tin, r.tout - r.tin, cn == 2 ? r.info : m << 16);
+      sh.s_bnd[i] = (off + 1 >= R ? off + 1 - R : 0u) / SEQ_BW | (min(off / SEQ_BW, nbk - 1) + 1) << 16;
+      sh.s_cnt[i] = make_uint2(0u, 0u);
+    }
+  }
 
-  const uint32_t per_batch = SEQ_MCAP / 2;
-
-  constexpr uint32_t FPT = SEQ_MCAP / 2 / SEQ_THREADS;   // fragments per thread and batch
+  constexpr uint32_t per_batch = SEQ_MCAP / 2;
+  constexpr uint32_t FPT = per_batch / SEQ_THREADS;   // fragments per thread and batch
+  uint32_t* hist = reinterpret_cast<uint32_t*>(sh.s_hist);
+  const bool paired = prm.paired != 0;
   for (uint32_t b0 = 0; b0 < n_pairs; b0 += per_batch) {
     const uint32_t nb_pairs = min(per_batch, n_pairs - b0);
-    for (uint32_t b = tid; b <= nbk; b += SEQ_THREADS) s_boff[b] = 0;
-    __syncthreads();
     // phase A: fragments stay in registers (mate offsets, both < 2^15, and
     // bucket ranks, both < 2^16, packed in pairs); each mate takes its rank
-    // within its start bucket from the histogram's atomic
+    // within its start bucket from the histogram's atomic.  (No barrier
+    // since the last batch's phase B: what this writes, the histogram, was
+    // cleared by the last scan.)
     uint32_t o01[FPT], ca[FPT], fi[FPT], fw[FPT], rk01[FPT];
     // one instance of the draw code per (copy-number path, insert table)
     // pair, chosen once per tile: the unrolled loop holds only that path
-    auto gen = [&](auto cn, auto ins_tag) {
+    auto gen = [&](auto cn_tag, auto ins_tag) {
 #pragma unroll
       for (uint32_t q = 0; q < FPT; ++q) {
         const uint32_t k = tid + q * SEQ_THREADS;
         if (k < nb_pairs) {
-          const Fragment f = make_fragment<decltype(ins_tag)::value, decltype(cn)::value>(
-              key, b0 + k, t, s, start, len, ce, sm, leaf_tin, prm, ins_smem ? s_ins : nullptr,
-              ins_smem ? s_guide : nullptr, cc);
+          const Fragment f = make_fragment<decltype(ins_tag)::value, decltype(cn_tag)::value>(
+              key, b0 + k, t, s, start, len, ce, sm, leaf_tin, prm, reinterpret_cast<const uint32_t*>(sh.s_guide),
+              &sh.s_cn);
           ca[q] = f.cell;
-          fi[q] = f.inst;
+          if constexpr (decltype(cn_tag)::value == 0) fi[q] = 0x10000u << (f.inst & 15u);
+          else if constexpr (decltype(cn_tag)::value == 1) fi[q] = f.inst;
+          else fi[q] = f.inst == 0xffffu ? 0x8000u : f.inst << 16;
           fw[q] = f.w;
           const uint32_t o0 = f.p0 - start;
-          uint32_t rk = atomicAdd(s_boff + o0 / SEQ_BW, 1u);
+          uint32_t rk = atomicAdd(hist + o0 / SEQ_BW, 1u);
           uint32_t o1 = 0;
-          if (prm.paired) {
+          if (paired) {
             o1 = f.p1 - start;
-            rk |= atomicAdd(s_boff + o1 / SEQ_BW, 1u) << 16;
+            rk |= atomicAdd(hist + o1 / SEQ_BW, 1u) << 16;
           }
           o01[q] = o0 | (o1 << 16);
           rk01[q] = rk;
@@ -567,19 +631,25 @@ __device__ __forceinline__ void read_tile(ReadSmem& sh, const SeqRec* __restrict
     using T2 = std::integral_constant<int, 2>;
     using YES = std::true_type;
     using NO = std::false_type;
-    if (!prm.has_cna) { if (ins_smem) gen(T0{}, YES{}); else gen(T0{}, NO{}); }
-    else if (cc) { if (ins_smem) gen(T1{}, YES{}); else gen(T1{}, NO{}); }
+    if (cn == 0) { if (ins_smem) gen(T0{}, YES{}); else gen(T0{}, NO{}); }
+    else if (cn == 1) { if (ins_smem) gen(T1{}, YES{}); else gen(T1{}, NO{}); }
     else { if (ins_smem) gen(T2{}, YES{}); else gen(T2{}, NO{}); }
     __syncthreads();
-    // bucket offsets (exclusive scan of at most 1024 counts)
+    // bucket offsets: exclusive scan of the 1024 counts, four per thread,
+    // the counts cleared for the next batch
     {
-      uint32_t v[4];
+      const uint4 c = sh.s_hist[tid];
+      sh.s_hist[tid] = make_uint4(0u, 0u, 0u, 0u);
+      const uint32_t c1 = c.x + c.y, c2 = c1 + c.z, c3 = c2 + c.w;
+      const uint32_t incl = warp_incl_scan(c3);
+      if (lane == 31) sh.s_scan[warp] = incl;
+      __syncthreads();
+      uint32_t base = incl - c3;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) { const uint32_t b = tid * 4 + q; v[q] = b < nbk ? s_boff[b] : 0u; }
-      const uint32_t tot = block_excl_scan4(v, s_scan);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) { const uint32_t b = tid * 4 + q; if (b < nbk) s_boff[b] = v[q]; }
-      if (tid == 0) s_boff[nbk] = tot;
+      for (uint32_t w = 0; w < WARPS - 1; ++w) base += w < warp ? sh.s_scan[w] : 0u;
+      const uint32_t a0 = base, a1 = base + c.x, a2 = base + c1, a3 = base + c2;
+      *reinterpret_cast<uint2*>(sh.s_boff + 4 * tid) = make_uint2(a0 | (a1 << 16), a2 | (a3 << 16));
+      if (tid == SEQ_THREADS - 1) sh.s_boff[SEQ_NBK] = uint16_t(base + c3);
     }
     __syncthreads();
     // scatter the mates in start-bucket order
@@ -588,86 +658,69 @@ __device__ __forceinline__ void read_tile(ReadSmem& sh, const SeqRec* __restrict
       const uint32_t k = tid + q * SEQ_THREADS;
       if (k < nb_pairs) {
         const uint32_t o0 = o01[q] & 0xffffu, o1 = o01[q] >> 16;
-        const uint32_t x0 = s_boff[o0 / SEQ_BW] + (rk01[q] & 0xffffu);
-        // a dropped fragment's mates carry the start offset 0xffff: past every locus
-        const uint32_t oo0 = fi[q] == 0xffffu ? 0xffffu : o0, oo1 = fi[q] == 0xffffu ? 0xffffu : o1;
-        s_mpi[x0] = oo0 | (fi[q] << 16); s_mcw[x0] = make_uint2(ca[q], fw[q]);
-        if (prm.paired) {
-          const uint32_t x1 = s_boff[o1 / SEQ_BW] + (rk01[q] >> 16);
-          s_mpi[x1] = oo1 | (fi[q] << 16); s_mcw[x1] = make_uint2(ca[q], mate_word(fw[q], 1u));
+        const uint32_t x0 = sh.s_boff[o0 / SEQ_BW] + (rk01[q] & 0xffffu);
+        sh.s_mpi[x0] = o0 | fi[q]; sh.s_mcw[x0] = make_uint2(ca[q], fw[q]);
+        if (paired) {
+          const uint32_t x1 = sh.s_boff[o1 / SEQ_BW] + (rk01[q] >> 16);
+          sh.s_mpi[x1] = o1 | fi[q]; sh.s_mcw[x1] = make_uint2(ca[q], mate_word(fw[q], 1u));
         }
       }
     }
     __syncthreads();
-    // phase B: a record's candidate mates (those starting in the buckets of
-    // [L-R+1, L]) are one contiguous run of the bucket-sorted mates; the runs
-    // of all records are concatenated and split evenly over the threads
-    {
-      uint32_t v[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const uint32_t i = tid * 4 + q;
-        uint32_t cnt = 0;
+    // phase B: SEQ_REC_LANES lanes per record
+    const uint32_t err_thr = prm.err_thr, err_t1 = prm.err_t1, R16 = R << 16, lc0 = start * ERR_LOCUS;
+    auto visits = [&](auto ids_tag) {
+      constexpr bool IDS = decltype(ids_tag)::value;
+      for (uint32_t i0 = 0; i0 < nw; i0 += SEQ_THREADS / SEQ_REC_LANES) {
+        const uint32_t i = i0 + tid / SEQ_REC_LANES;
+        uint32_t acc = 0;                    // depth | alt << 16 (a batch holds 2560 mates)
         if (i < nw) {
-          const uint32_t off = s_locus[i] - start;
-          const uint32_t blo = (off + 1 >= R ? off + 1 - R : 0u) / SEQ_BW;
-          const uint32_t bhi = min(off / SEQ_BW, nbk - 1);
-          s_wstart[i] = uint16_t(s_boff[blo]);
-          cnt = s_boff[bhi + 1] - s_boff[blo];
-        }
-        v[q] = cnt;
-      }
-      const uint32_t tot = block_excl_scan4(v, s_scan);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) { const uint32_t i = tid * 4 + q; if (i < SEQ_CAP) s_wpre[i] = v[q]; }
-      if (tid == 0) s_wtot = tot;
-    }
-    __syncthreads();
-    {
-      const uint32_t W = s_wtot;
-      const uint32_t k0 = uint32_t(uint64_t(W) * tid / SEQ_THREADS);
-      const uint32_t k1 = uint32_t(uint64_t(W) * (tid + 1) / SEQ_THREADS);
-      if (k0 < k1) {
-        uint32_t i = 0, hi = nw;                              // record holding work item k0
-        while (hi - i > 1) { const uint32_t mid = (i + hi) >> 1; if (s_wpre[mid] <= k0) i = mid; else hi = mid; }
-        uint32_t next = i + 1 < nw ? s_wpre[i + 1] : W;
-        uint32_t L = s_locus[i], off = L - start, tin = s_tin[i], tout = s_tout[i], info = s_info[i];
-        uint32_t base = s_wstart[i] - s_wpre[i];
-        uint32_t dep = 0, alt = 0;
-        for (uint32_t k = k0; k < k1;) {
-          while (k >= next) {                                 // the run of the next record starts
-            if (dep) { atomicAdd(s_dep + i, dep); if (alt) atomicAdd(s_alt + i, alt); }
-            dep = 0; alt = 0;
-            ++i;
-            next = i + 1 < nw ? s_wpre[i + 1] : W;
-            L = s_locus[i]; off = L - start; tin = s_tin[i]; tout = s_tout[i]; info = s_info[i];
-            base = s_wstart[i] - s_wpre[i];
+          const uint4 r = sh.s_rec[i];
+          const uint32_t bnd = sh.s_bnd[i], e = sh.s_boff[bnd >> 16];
+          const uint32_t off16 = r.x & 0xffff0000u, lc = (r.x >> 16) * ERR_LOCUS + lc0;
+          const uint32_t thr = (r.x & 1u) ? 0u : err_thr, t1 = (r.x & 1u) ? 0u : err_t1;
+#pragma unroll 2
+          for (uint32_t k = sh.s_boff[bnd & 0xffffu] + tid % SEQ_REC_LANES; k < e; k += SEQ_REC_LANES) {
+            const uint32_t pi = sh.s_mpi[k];
+            const uint2 cw = sh.s_mcw[k];
+            // the mate covers L when its start o is in (L - R, L] (unsigned: o > off wraps)
+            const bool cov = off16 - pi * 0x10000u < R16;
+            // the cell is in the edge's subtree when tin <= cell < tout
+            bool carried = cw.x - r.y < r.z;
+            if constexpr (IDS) {
+              carried = carried && (pi & r.w) != 0u;   // (r.w has no bits below 16)
+            } else {
+              const uint32_t y = pi >> 16, x = r.w & 0xffffu;
+              if (carried && y > max(x, 1u))
+                carried = inst_carries(prm, y, x, (uint64_t(r.y) << 16) | ((r.w >> 16) & 0x7fffu));
+              else
+                carried = carried && y == x;
+            }
+            // carried: the alt base unless an error hits it; else an error of
+            // the first third shows it (an indel has neither)
+            const bool ob = (err_word_at(cw.y, lc) < (carried ? thr : t1)) != carried;
+            const uint32_t one = ob ? 0x10001u : 1u;
+            if (cov) acc += one;
           }
-          // two visits of the same record at a time when the run allows it
-          const uint32_t nv = (k + 1 < next && k + 1 < k1) ? 2u : 1u;
-          const uint32_t x = base + k, x1 = nv == 2u ? x + 1u : x;
-          const uint32_t pi = s_mpi[x], pj = s_mpi[x1];
-          const uint2 cw = s_mcw[x], cv = s_mcw[x1];
-          // the mate covers L when its start o is in (L - R, L] (unsigned: o > off wraps)
-          const bool cov = off - (pi & 0xffffu) < R;
-          const bool cov1 = nv == 2u && off - (pj & 0xffffu) < R;
-          const bool ob = observed(prm, tin, tout, info, cw.x, pi >> 16, cw.y, L);
-          const bool ob1 = observed(prm, tin, tout, info, cv.x, pj >> 16, cv.y, L);
-          dep += (cov ? 1u : 0u) + (cov1 ? 1u : 0u);
-          alt += ((cov & ob) ? 1u : 0u) + ((cov1 & ob1) ? 1u : 0u);
-          k += nv;
         }
-        if (dep) { atomicAdd(s_dep + i, dep); if (alt) atomicAdd(s_alt + i, alt); }
+#pragma unroll
+        for (uint32_t o = SEQ_REC_LANES / 2; o >= 1; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (acc && tid % SEQ_REC_LANES == 0) {
+          uint2 c = sh.s_cnt[i];
+          c.x += acc & 0xffffu;
+          c.y += acc >> 16;
+          sh.s_cnt[i] = c;
+        }
       }
-    }
-    __syncthreads();
+    };
+    if (cn == 2) visits(NO{}); else visits(YES{});
   }
+  __syncthreads();
   for (uint32_t i = tid; i < nw; i += SEQ_THREADS) {
-    const uint32_t d = s_dep[i];
-    if (d) {
-      atomicAdd(gdep + i, d);
-      const uint32_t a = s_alt[i];
-      if (a) atomicAdd(galt + i, a);
+    const uint2 c = sh.s_cnt[i];
+    if (c.x) {
+      atomicAdd(gdep + i, c.x);
+      if (c.y) atomicAdd(galt + i, c.y);
     }
   }
 }
@@ -679,8 +732,9 @@ __global__ void __launch_bounds__(SEQ_THREADS, 4) k_reads(const SeqRec* __restri
                                                           const uint32_t* __restrict__ leaf_tin, SeqParams prm,
                                                           RoundKeys key, uint64_t n_recs, uint32_t* __restrict__ g_alt,
                                                           uint32_t* __restrict__ g_dep) {
-  __shared__ ReadSmem sh;
+  __shared__ __align__(16) ReadSmem sh;
   const uint32_t t = blockIdx.x, s = blockIdx.y;
+  sh.s_hist[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
   const uint32_t lo = tiles.rec_lo[t];
   const SeqSample sm = samples[s];
   read_tile(sh, g_recs, t, s, pair_cnt[uint64_t(s) * tiles.n_tiles + t], lo, tiles.rec_hi[t] - lo, tiles.start[t],
@@ -782,7 +836,7 @@ __global__ void k_sam_reads(const SeqRec* __restrict__ recs, uint32_t n_recs, co
   const uint64_t base = out_off[uint64_t(s) * n_chunk + k];
   const uint32_t mates = prm.paired ? 2u : 1u;
   for (uint32_t j = threadIdx.x; j < n_pairs; j += blockDim.x) {
-    const Fragment f = make_fragment<false>(key, j, t, s, start, len, ce, sm, leaf_tin, prm, nullptr, nullptr);
+    const Fragment f = make_fragment<false>(key, j, t, s, start, len, ce, sm, leaf_tin, prm, nullptr);
     for (uint32_t m = 0; m < mates; ++m) {
       const uint64_t r = (base + j) * mates + m;
       SamRead& o = out[r];
@@ -861,7 +915,7 @@ __global__ void k_tile_counts_b(SeqBatch b) {
 static_assert(sizeof(SeqParams) % 4 == 0 && sizeof(SeqParams) / 4 <= SEQ_THREADS, "SeqParams staging");
 
 __global__ void __launch_bounds__(SEQ_THREADS, 4) k_reads_batch(SeqBatch b, const SeqRec* __restrict__ g_recs) {
-  __shared__ ReadSmem sh;
+  __shared__ __align__(16) ReadSmem sh;
   __shared__ SeqParams s_prm;        // the item's instance parameters, staged once per instance change
   __shared__ SeqSample s_sm;
   __shared__ Key s_key;
@@ -869,6 +923,7 @@ __global__ void __launch_bounds__(SEQ_THREADS, 4) k_reads_batch(SeqBatch b, cons
   __shared__ const SeqRec* s_recs;
   __shared__ uint64_t s_row;
   uint32_t cur = 0xffffffffu;        // instance whose parameters s_prm holds
+  sh.s_hist[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
   for (;;) {
     if (threadIdx.x == 0) {
       // decode the next work item once for the CTA
