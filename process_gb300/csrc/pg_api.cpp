@@ -1799,9 +1799,8 @@ void simulate_seq_impl(const pg_placed* pl, const pg_seq_cfg* c, uint64_t seed, 
     // ---- tiles
     // tiles are laid out on the device from the per-chromosome table
     std::vector<uint32_t> c_ntiles, c_nstarts, c_id, c_first, c_depth, c_start, c_end;
-    std::vector<uint64_t> c_pairs, heap_base;   // per chromosome: its split tree's heap (2^(depth + 1) entries)
-    uint64_t heap_total = 0;
-    uint32_t max_depth = 0;
+    std::vector<uint64_t> c_pairs;
+    uint32_t max_tiles = 0;
     uint32_t n_tiles = 0;
     const double mates = paired ? 2.0 : 1.0;
     uint64_t frags_per_sample = 0;
@@ -1819,9 +1818,7 @@ void simulate_seq_impl(const pg_placed* pl, const pg_seq_cfg* c, uint64_t seed, 
       c_first.push_back(n_tiles); c_depth.push_back(D);
       c_start.push_back(e->chr_off[ci]); c_end.push_back(e->chr_off[ci] + L);
       frags_per_sample += pairs;
-      heap_base.push_back(heap_total);
-      heap_total += uint64_t(2) << D;
-      max_depth = std::max(max_depth, D);
+      max_tiles = std::max(max_tiles, nt);
       require(uint64_t(n_tiles) + nt < (uint64_t(1) << 31), "too many tiles");
       n_tiles += nt;
     }
@@ -1942,7 +1939,6 @@ void simulate_seq_impl(const pg_placed* pl, const pg_seq_cfg* c, uint64_t seed, 
       pg::seq_make_tiles(uint32_t(c_first.size()), cf.p, cn.p, cs.p, cns.p, cen.p, T, n_tiles, ts_d.p, tl_d.p,
                          te_d.p, st);
     }
-    auto hb_d = upload(P, heap_base, st);
     auto cnt_d = upload(P, c_ntiles, st), cns_d = upload(P, c_nstarts, st), cid_d = upload(P, c_id, st);
     auto cf_d = upload(P, c_first, st), cd_d = upload(P, c_depth, st);
     auto cp_d = upload(P, c_pairs, st);
@@ -1980,9 +1976,8 @@ void simulate_seq_impl(const pg_placed* pl, const pg_seq_cfg* c, uint64_t seed, 
       ocls_d = upload(P, opt_class, st); oloff_d = upload(P, opt_leaf_off, st); onl_d = upload(P, opt_nleaf, st);
       cltin_d = upload(P, cls_leaf_tin, st); ocdf_d = upload(P, opt_cdf, st);
     }
-    DBuf<uint32_t> heap(P, heap_total * samples.size());
-    pg::seq_tile_counts(uint32_t(samples.size()), uint32_t(c_id.size()), max_depth, cf_d.p, cnt_d.p, cd_d.p, cns_d.p,
-                        cid_d.p, cp_d.p, hb_d.p, heap_total, heap.p, T, n_tiles, pl->has_cna ? mcum_d.p : nullptr,
+    pg::seq_tile_counts(uint32_t(samples.size()), uint32_t(c_id.size()), max_tiles, cf_d.p, cnt_d.p, cd_d.p, cns_d.p,
+                        cid_d.p, cp_d.p, T, n_tiles, pl->has_cna ? mcum_d.p : nullptr,
                         pl->has_cna ? mtot_d.p : nullptr, seed, pair_cnt.p, st);
     pg::seq_tile_ranges(recs.p, uint32_t(pl->M), ts_d.p, tl_d.p, n_tiles, span, rlo.p, rhi.p, st);
     pg::SeqTiles tiles{n_tiles, ts_d.p, tl_d.p, te_d.p, rlo.p, rhi.p};

@@ -335,7 +335,7 @@ struct SeqInst {
   uint32_t n_tiles, tile_off;       // rows of the batch's tile arrays
   uint32_t T;                       // tile size
   uint32_t slot_off;                // chromosome tables
-  uint32_t n_blocks, blk_off;       // tile-split blocks of 64 tiles
+  uint32_t n_blocks, blk_off;       // tile-split blocks of 64 tiles (a warp each)
   uint32_t etin_off;                // edge Euler table rows (n_nodes + 2)
   uint64_t pair_off;                // pair counts [sample][tile]
   uint64_t count_off;               // alt/depth of sample s: count_off + s * count_stride + record
@@ -347,7 +347,7 @@ struct SeqBatch {
   const Key* keys;                  // sequencing key of each instance
   const uint32_t* rec_off;          // n_inst + 1: records of instance i (filled by placement)
   const uint32_t* item_off;         // n_inst + 1: first work item of each instance
-  const uint32_t* cnt_off;          // n_inst + 1: first tile-split thread of each instance
+  const uint32_t* cnt_off;          // n_inst + 1: first tile-split warp of each instance
   uint32_t n_items, n_cnt, n_tiles_all;
   const uint32_t *tile_start, *tile_len, *tile_end, *tile_inst;
   uint32_t *rec_lo, *rec_hi;        // per tile, relative to the instance's first record
@@ -403,17 +403,14 @@ void seq_build_records(const PlaceOut& sorted, uint32_t n, const uint32_t* edge_
 void seq_tile_ranges(const SeqRec* recs, uint32_t n_recs, const uint32_t* start, const uint32_t* len,
                      uint32_t n_tiles, uint32_t span, uint32_t* rlo, uint32_t* rhi, cudaStream_t st);
 // per (sample, tile) pair counts: multinomial split of each chromosome's
-// pair count over its tiles by a binary tree of binomial draws, one launch
-// per tree level (max_depth of them) with the node counts in `heap`
-// (heap_total entries per sample; chromosome slot's heap at heap_base[slot],
-// 2^(depth + 1) entries).  Tiles weigh their number of start positions, or
-// (mass_cum != NULL) their DNA mass: mass_cum[s * n_tiles + t] is the
-// sample's mass of the chromosome's tiles before t and
-// mass_tot[s * n_slots + slot] the chromosome's total.
-void seq_tile_counts(uint32_t n_samples, uint32_t n_slots, uint32_t max_depth, const uint32_t* chr_first_tile,
+// pair count over its tiles (at most max_tiles) by a binary tree of binomial
+// draws.  Tiles weigh their number of start positions, or (mass_cum != NULL)
+// their DNA mass: mass_cum[s * n_tiles + t] is the sample's mass of the
+// chromosome's tiles before t and mass_tot[s * n_slots + slot] the
+// chromosome's total.
+void seq_tile_counts(uint32_t n_samples, uint32_t n_slots, uint32_t max_tiles, const uint32_t* chr_first_tile,
                      const uint32_t* chr_ntiles, const uint32_t* chr_depth, const uint32_t* chr_nstarts,
-                     const uint32_t* chr_id, const uint64_t* chr_pairs, const uint64_t* heap_base,
-                     uint64_t heap_total, uint32_t* heap, uint32_t tile_size, uint32_t n_tiles,
+                     const uint32_t* chr_id, const uint64_t* chr_pairs, uint32_t tile_size, uint32_t n_tiles,
                      const double* mass_cum, const double* mass_tot, uint64_t seed, uint32_t* pair_cnt,
                      cudaStream_t st);
 // observed rows: flag[m] = 1 when some sample has an alt read of mutation m;

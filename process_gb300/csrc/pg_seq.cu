@@ -53,6 +53,7 @@
 
 #include "pg_common.cuh"
 #include "pg_rng.cuh"
+#include "pg_fast.cuh"
 #include "pg_kernels.h"
 #include "pg_scan.cuh"
 
@@ -128,138 +129,104 @@ struct TileSplit {
     if (n == 0 || !(wt > 0.0)) return 0.0;
     return (c(mid) - base) / wt;
   }
-  __device__ __forceinline__ uint64_t left(Key key, uint32_t h, uint32_t chr, uint32_t s, uint64_t n, uint64_t lo,
-                                           uint64_t mid, uint64_t hi) const {
+  // the pairs of node h (n of them, tiles [lo, hi)) that go left
+  __device__ __noinline__ uint64_t left(Key key, uint32_t h, uint32_t chr, uint32_t s, uint64_t n, uint64_t lo,
+                                        uint64_t mid, uint64_t hi) const {
     const double p = share(n, lo, mid, hi);
     if (!(p > 0.0)) return 0;
     Stream st{key, h, chr, s, TAG_TILE_SPLIT, 0u};
     return binomial(st, n, p);
   }
-  // left() when its draw settles in the first attempt (false: call left())
-  __device__ __forceinline__ bool left_first(Key key, uint32_t h, uint32_t chr, uint32_t s, uint64_t n, uint64_t lo,
-                                             uint64_t mid, uint64_t hi, uint64_t& nl) const {
-    const double p = share(n, lo, mid, hi);
-    if (!(p > 0.0)) { nl = 0; return true; }
-    return binomial_first(Stream{key, h, chr, s, TAG_TILE_SPLIT, 0u}, n, p, nl);
+  // left() from the FP32 sampler; false where that does not decide.  The
+  // share p = x / y and whether it exceeds one half are taken from x and y:
+  // the rounded quotient exceeds one half exactly when 2 x > y.
+  __device__ __forceinline__ bool left_fast(Key key, uint32_t h, uint32_t chr, uint32_t s, uint32_t n, uint64_t lo,
+                                            uint64_t mid, uint64_t hi, uint64_t& nl) const {
+    F2 pp;
+    bool flip;
+    nl = 0;
+    if (n == 0) return true;
+    if (cum == nullptr) {
+      const uint32_t y = uint32_t(w(lo, hi)), x = uint32_t(w(lo, mid));
+      if (x == 0) return true;
+      if (x >= y) { nl = n; return true; }
+      flip = x > y - x;
+      pp = f2_div(f2_u32(flip ? y - x : x), f2_u32(y));
+    } else {
+      const double base = c(lo), y = c(hi) - base, x = c(mid) - base;
+      if (!(y > 0.0) || !(x > 0.0)) return true;
+      if (!(x < y)) { nl = n; return true; }
+      flip = x + x > y;
+      int ex, ey;
+      const F2 fx = f2_mantissa(flip ? y - x : x, ex), fy = f2_mantissa(y, ey);
+      if (ey - ex > 60) return false;
+      pp = f2_scale(f2_div(fx, fy), pow2f(ex - ey));
+    }
+    return binomial_fast(Stream{key, h, chr, s, TAG_TILE_SPLIT, 0u}, n, pp, flip, nl);
   }
 };
 
-constexpr uint32_t SPLIT_BLOCK_LOG = 6;   // 64 tiles per thread
-
-// one thread per (sample, block of 64 tiles): walk from the root to the
-// block's node, then draw the block's 63 internal splits top-down
-__device__ __forceinline__ void tile_counts_one(uint32_t s, uint32_t bi, const uint32_t* __restrict__ blk_slot,
-                                                const uint32_t* __restrict__ blk_index,
-                                                const uint32_t* __restrict__ chr_first_tile,
-                                                const uint32_t* __restrict__ chr_ntiles,
-                                                const uint32_t* __restrict__ chr_depth,
-                                                const uint32_t* __restrict__ chr_nstarts,
-                                                const uint32_t* __restrict__ chr_id,
-                                                const uint64_t* __restrict__ chr_pairs, uint32_t T, uint32_t n_tiles,
-                                                const double* __restrict__ mass_cum,
-                                                const double* __restrict__ mass_tot, uint32_t n_slots, Key key,
-                                                uint32_t* __restrict__ pair_cnt) {
-  const uint32_t slot = blk_slot[bi], b = blk_index[bi];
-  const uint32_t D = chr_depth[slot], chr = chr_id[slot], nt = chr_ntiles[slot];
-  const uint32_t base = chr_first_tile[slot];
-  const TileSplit sp{chr_nstarts[slot], T, nt, mass_cum ? mass_cum + uint64_t(s) * n_tiles + base : nullptr,
-                     mass_cum ? mass_tot[uint64_t(s) * n_slots + slot] : 0.0};
+// One warp per (sample, block of 64 tiles).  It walks from the root of the
+// chromosome's tree to the block's node, every lane drawing the same nodes,
+// then draws the block's subtree level by level with one lane per node.  The
+// draws are a serial chain of at most D steps of about 2.5 us, most of them
+// the same in every warp of a chromosome, which costs less than a launch per
+// level: 180 us became 15 for 3 x 1 Mbp (7 levels), and at full scale
+// (16 levels, 4 samples) 1.64 ms became 0.55.
+constexpr uint32_t SPLIT_BLOCK_LOG = 6;   // 64 tiles per warp
+constexpr uint32_t SPLIT_THREADS = 128;
+__device__ __forceinline__ void tile_counts_warp(const TileSplit& sp, uint32_t s, uint32_t b, uint32_t D, uint32_t chr,
+                                                 uint64_t n_pairs, Key key, uint32_t* __restrict__ cnt) {
+  constexpr uint32_t FULL = 0xffffffffu;
+  const uint32_t lane = threadIdx.x & 31u;
   const uint32_t Db = D < SPLIT_BLOCK_LOG ? D : SPLIT_BLOCK_LOG;   // depth of the block's subtree
+  if (D == 0) {   // one tile: it takes every pair
+    if (lane == 0) cnt[0] = uint32_t(n_pairs);
+    return;
+  }
+  auto draw = [&](uint32_t h, uint32_t n, uint64_t lo, uint64_t size) {
+    uint64_t nl;
+    if (!sp.left_fast(key, h, chr, s, n, lo, lo + (size >> 1), lo + size, nl))
+      nl = sp.left(key, h, chr, s, n, lo, lo + (size >> 1), lo + size);
+    return uint32_t(nl);
+  };
   // root -> block node
-  uint64_t n = chr_pairs[slot], lo = 0, size = uint64_t(1) << D;
-  uint32_t h = 1;
-  for (uint32_t d = 0; d < D - Db; ++d) {
-    const uint64_t half = size >> 1, mid = lo + half;
-    const uint64_t nl = sp.left(key, h, chr, s, n, lo, mid, lo + size);
-    const bool right = (uint64_t(b) << Db) >= mid;   // the block lies in the right half
-    if (right) { n -= nl; lo = mid; h = 2 * h + 1; } else { n = nl; h = 2 * h; }
-    size = half;
+  uint32_t n = uint32_t(n_pairs), h = 1;
+  uint64_t lo = 0, size = uint64_t(1) << D;
+  for (uint32_t d = Db; d < D; ++d) {
+    const uint32_t nl = draw(h, n, lo, size);
+    size >>= 1;
+    const bool right = (uint64_t(b) << Db) >= lo + size;   // the block lies in the right half
+    if (right) { n -= nl; lo += size; h = 2 * h + 1; } else { n = nl; h = 2 * h; }
   }
-  // the block's subtree, breadth first (relative heap ids 1 .. 2^Db - 1)
-  uint32_t c[2 << SPLIT_BLOCK_LOG];
-  c[1] = uint32_t(n);
-  const uint32_t nint = (1u << Db) - 1;
-  for (uint32_t r = 1; r <= nint; ++r) {
-    const uint32_t level = 31 - __clz(r);
-    const uint64_t nsz = uint64_t(1) << (Db - level);
-    const uint64_t nlo = lo + uint64_t(r - (1u << level)) * nsz;
-    const uint32_t gh = (h << level) + (r - (1u << level));
-    const uint64_t nl = sp.left(key, gh, chr, s, c[r], nlo, nlo + (nsz >> 1), nlo + nsz);
-    c[2 * r] = uint32_t(nl);
-    c[2 * r + 1] = c[r] - uint32_t(nl);
-  }
-  for (uint32_t r = 0; r < (1u << Db); ++r) {
-    const uint64_t tile = lo + r;
-    if (tile < nt) pair_cnt[uint64_t(s) * n_tiles + base + tile] = c[(1u << Db) + r];
+  // the block's subtree: lane i holds node i of the level
+  for (uint32_t level = 0; level < Db; ++level, size >>= 1) {
+    const uint64_t at = lo + uint64_t(lane) * size;
+    uint32_t nl = 0;
+    if (lane < (1u << level) && at < sp.nt) nl = draw((h << level) + lane, n, at, size);
+    if (level + 1 < Db) {
+      const uint32_t a = __shfl_sync(FULL, nl, lane >> 1), t = __shfl_sync(FULL, n, lane >> 1);
+      n = (lane & 1u) ? t - a : a;
+    } else if (lane < (1u << level)) {   // the children are tiles at and at + 1
+      if (at < sp.nt) cnt[at] = nl;
+      if (at + 1 < sp.nt) cnt[at + 1] = n - nl;
+    }
   }
 }
 
-// Level-synchronous form of the same tree (the plain path): one launch per
-// level, one thread per (sample, chromosome, node of the level) whose range
-// meets the chromosome's tiles; node counts live in a per-(sample,
-// chromosome) heap in global memory.  Every node draws with its own heap id,
-// as in tile_counts_one, so the counts are the same.  A node whose draw
-// settles in BTRS's first attempt (most do) is written at once; the others
-// queue in shared memory and are drawn in full by consecutive threads, so
-// that the exact test's logarithms run on dense warps.
-constexpr uint32_t SPLIT_THREADS = 128;
-__global__ void __launch_bounds__(SPLIT_THREADS) k_tile_split_level(
-    uint32_t level, uint32_t n_slots, const uint32_t* __restrict__ chr_first_tile,
-    const uint32_t* __restrict__ chr_ntiles, const uint32_t* __restrict__ chr_depth,
-    const uint32_t* __restrict__ chr_nstarts, const uint32_t* __restrict__ chr_id,
-    const uint64_t* __restrict__ chr_pairs, const uint64_t* __restrict__ heap_base, uint64_t heap_total, uint32_t T,
-    uint32_t n_tiles, const double* __restrict__ mass_cum, const double* __restrict__ mass_tot, Key key,
-    uint32_t* __restrict__ heap, uint32_t* __restrict__ pair_cnt) {
-  __shared__ uint32_t s_q[SPLIT_THREADS];
-  __shared__ uint32_t s_nq;
-  const uint32_t s = blockIdx.z, slot = blockIdx.y;
-  const uint32_t D = chr_depth[slot], nt = chr_ntiles[slot], first = chr_first_tile[slot];
-  uint32_t* cnt = pair_cnt + uint64_t(s) * n_tiles + first;
-  if (D == 0) {   // one tile: it takes every pair
-    if (level == 0 && blockIdx.x == 0 && threadIdx.x == 0) cnt[0] = uint32_t(chr_pairs[slot]);
-    return;
-  }
-  // whole blocks past the level's nodes leave together
-  if (level >= D || uint64_t(blockIdx.x) * SPLIT_THREADS >= (uint64_t(1) << level)) return;
-  if (threadIdx.x == 0) s_nq = 0;
-  __syncthreads();
+__global__ void __launch_bounds__(SPLIT_THREADS) k_tile_split(
+    uint32_t n_slots, const uint32_t* __restrict__ chr_first_tile, const uint32_t* __restrict__ chr_ntiles,
+    const uint32_t* __restrict__ chr_depth, const uint32_t* __restrict__ chr_nstarts,
+    const uint32_t* __restrict__ chr_id, const uint64_t* __restrict__ chr_pairs, uint32_t T, uint32_t n_tiles,
+    const double* __restrict__ mass_cum, const double* __restrict__ mass_tot, Key key,
+    uint32_t* __restrict__ pair_cnt) {
+  const uint32_t s = blockIdx.z, slot = blockIdx.y, b = (blockIdx.x * SPLIT_THREADS + threadIdx.x) >> 5;
+  const uint32_t nt = chr_ntiles[slot], first = chr_first_tile[slot];
+  if (uint64_t(b) << SPLIT_BLOCK_LOG >= nt) return;   // whole warps
   const TileSplit sp{chr_nstarts[slot], T, nt, mass_cum ? mass_cum + uint64_t(s) * n_tiles + first : nullptr,
                      mass_cum ? mass_tot[uint64_t(s) * n_slots + slot] : 0.0};
-  uint32_t* hp = heap + uint64_t(s) * heap_total + heap_base[slot];
-  const uint64_t size = uint64_t(1) << (D - level);
-  const uint32_t chr = chr_id[slot];
-  // node of thread x of the block: its index in the level (valid when its
-  // range meets the tiles), heap id, pair count
-  auto node = [&](uint32_t x, uint64_t& i, uint32_t& h, uint64_t& n) {
-    i = uint64_t(blockIdx.x) * SPLIT_THREADS + x;
-    if (i >= (uint64_t(1) << level) || i * size >= nt) return false;
-    h = uint32_t((uint64_t(1) << level) + i);
-    n = level == 0 ? chr_pairs[slot] : hp[h];
-    return true;
-  };
-  auto put = [&](uint64_t i, uint32_t h, uint64_t n, uint64_t nl) {
-    const uint64_t lo = i * size;
-    if (level + 1 == D) {   // the children are tiles lo and lo + 1
-      cnt[lo] = uint32_t(nl);
-      if (lo + 1 < nt) cnt[lo + 1] = uint32_t(n - nl);
-    } else {
-      hp[2 * h] = uint32_t(nl);
-      hp[2 * h + 1] = uint32_t(n - nl);
-    }
-  };
-  uint64_t i, n;
-  uint32_t h;
-  if (node(threadIdx.x, i, h, n)) {
-    const uint64_t lo = i * size;
-    uint64_t nl;
-    if (sp.left_first(key, h, chr, s, n, lo, lo + (size >> 1), lo + size, nl)) put(i, h, n, nl);
-    else s_q[atomicAdd(&s_nq, 1u)] = threadIdx.x;
-  }
-  __syncthreads();
-  if (threadIdx.x < s_nq && node(s_q[threadIdx.x], i, h, n)) {
-    const uint64_t lo = i * size;
-    put(i, h, n, sp.left(key, h, chr, s, n, lo, lo + (size >> 1), lo + size));
-  }
+  tile_counts_warp(sp, s, b, chr_depth[slot], chr_id[slot], chr_pairs[slot], key,
+                   pair_cnt + uint64_t(s) * n_tiles + first);
 }
 
 // Error words.  A mate's word: the fragment's error word for mate 0, an
@@ -898,16 +865,16 @@ __global__ void k_tile_ranges_b(SeqBatch b, const SeqRec* __restrict__ recs) {
   b.rec_hi[t] = lower_bound_rec(recs + r0, nr, start + b.tile_len[t] - 1 + b.inst[i].prm.span);
 }
 
-__global__ void k_tile_counts_b(SeqBatch b) {
-  const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(SPLIT_THREADS) k_tile_counts_b(SeqBatch b) {
+  const uint32_t gid = (blockIdx.x * SPLIT_THREADS + threadIdx.x) >> 5;   // one warp per block of tiles
   if (gid >= b.n_cnt) return;
   const uint32_t i = batch_index(b.cnt_off, b.n_inst, gid);
   const SeqInst& in = b.inst[i];
-  const uint32_t local = gid - b.cnt_off[i];
-  tile_counts_one(local / in.n_blocks, local % in.n_blocks, b.blk_slot + in.blk_off, b.blk_index + in.blk_off,
-                  b.c_first + in.slot_off, b.c_ntiles + in.slot_off, b.c_depth + in.slot_off,
-                  b.c_nstarts + in.slot_off, b.c_id + in.slot_off, b.c_pairs + in.slot_off, in.T, in.n_tiles,
-                  nullptr, nullptr, 0, b.keys[i], b.pair_cnt + in.pair_off);
+  const uint32_t local = gid - b.cnt_off[i], s = local / in.n_blocks, bi = in.blk_off + local % in.n_blocks;
+  const uint32_t slot = in.slot_off + b.blk_slot[bi], first = b.c_first[slot];
+  const TileSplit sp{b.c_nstarts[slot], in.T, b.c_ntiles[slot], nullptr, 0.0};
+  tile_counts_warp(sp, s, b.blk_index[bi], b.c_depth[slot], b.c_id[slot], b.c_pairs[slot], b.keys[i],
+                   b.pair_cnt + in.pair_off + uint64_t(s) * in.n_tiles + first);
 }
 
 // Persistent read kernel of a batch: each CTA takes work items from a global
@@ -1169,21 +1136,18 @@ void seq_tile_ranges(const SeqRec* recs, uint32_t n_recs, const uint32_t* start,
   if (n_tiles) { k_tile_ranges<<<nblk(n_tiles), 256, 0, st>>>(recs, n_recs, start, len, n_tiles, span, rlo, rhi); note_launch(); }
 }
 
-void seq_tile_counts(uint32_t n_samples, uint32_t n_slots, uint32_t max_depth, const uint32_t* chr_first_tile,
+void seq_tile_counts(uint32_t n_samples, uint32_t n_slots, uint32_t max_tiles, const uint32_t* chr_first_tile,
                      const uint32_t* chr_ntiles, const uint32_t* chr_depth, const uint32_t* chr_nstarts,
-                     const uint32_t* chr_id, const uint64_t* chr_pairs, const uint64_t* heap_base,
-                     uint64_t heap_total, uint32_t* heap, uint32_t tile_size, uint32_t n_tiles,
+                     const uint32_t* chr_id, const uint64_t* chr_pairs, uint32_t tile_size, uint32_t n_tiles,
                      const double* mass_cum, const double* mass_tot, uint64_t seed, uint32_t* pair_cnt,
                      cudaStream_t st) {
   if (n_samples == 0 || n_slots == 0) return;
-  const Key key = make_key(seed);
-  for (uint32_t level = 0; level < std::max<uint32_t>(max_depth, 1); ++level) {
-    const dim3 grid(nblk(uint64_t(1) << level, SPLIT_THREADS), n_slots, n_samples);
-    k_tile_split_level<<<grid, SPLIT_THREADS, 0, st>>>(level, n_slots, chr_first_tile, chr_ntiles, chr_depth, chr_nstarts,
-                                             chr_id, chr_pairs, heap_base, heap_total, tile_size, n_tiles, mass_cum,
-                                             mass_tot, key, heap, pair_cnt);
-    note_launch();
-  }
+  const uint32_t warps = (max_tiles + (1u << SPLIT_BLOCK_LOG) - 1) >> SPLIT_BLOCK_LOG;
+  const dim3 grid(nblk(uint64_t(warps) * 32, SPLIT_THREADS), n_slots, n_samples);
+  k_tile_split<<<grid, SPLIT_THREADS, 0, st>>>(n_slots, chr_first_tile, chr_ntiles, chr_depth, chr_nstarts, chr_id,
+                                               chr_pairs, tile_size, n_tiles, mass_cum, mass_tot, make_key(seed),
+                                               pair_cnt);
+  note_launch();
 }
 
 // ------------------------------------------------------------ observed rows
@@ -1249,7 +1213,7 @@ int seq_reads_batch_occupancy() {
 }
 
 void seq_batch_reads(const SeqBatch& b, const SeqRec* recs, uint32_t grid, cudaStream_t st) {
-  if (b.n_cnt) { k_tile_counts_b<<<nblk(b.n_cnt, 64), 64, 0, st>>>(b); note_launch(); }
+  if (b.n_cnt) { k_tile_counts_b<<<nblk(uint64_t(b.n_cnt) * 32, SPLIT_THREADS), SPLIT_THREADS, 0, st>>>(b); note_launch(); }
   if (b.n_tiles_all) { k_tile_ranges_b<<<nblk(b.n_tiles_all), 256, 0, st>>>(b, recs); note_launch(); }
   cudaMemsetAsync(b.counter, 0, sizeof(uint32_t), st);
   if (b.n_items) { k_reads_batch<<<grid, SEQ_THREADS, 0, st>>>(b, recs); note_launch(); }

@@ -60,3 +60,34 @@ def test_read_kernel_tables(gpu_lib, orc, copies, reads):
         oalt, odep, _ = op.sequence(c, 17, flavour=0)
         np.testing.assert_array_equal(dep, odep)
         np.testing.assert_array_equal(alt, oalt)
+
+
+@pytest.mark.parametrize("tile", [64, 448, 8_192])
+@pytest.mark.parametrize("coverage", [0.05, 3, 700])
+@pytest.mark.parametrize("cna", [False, True])
+def test_tile_split(gpu_lib, orc, tile, coverage, cna):
+    """Pair counts per tile over chromosomes of one start position, one tile,
+    a tile and a bit, one block of 64 tiles more or less, and many: from
+    counts in the inversion range of the binomial to large ones, by start
+    positions and by DNA mass."""
+    from process_gb300 import CNA, synth
+    from process_gb300.engine import seq_cfg, sequence_counts
+    w = synth.plain_3mbp(seed=5, n_leaves=30)
+    w.genome.chr_names = [str(i + 1) for i in range(6)]
+    w.genome.chr_lengths = [50, 49 + 64, 49 + 65, 49 + 64 * 64, 49 + 64 * 64 + 1, 40_000]
+    (na, ra, _), (nb, rb, _) = w.mutants
+    rate = {"SNV": 1e-5, "indel": 1e-6}
+    drivers = [CNA("A", "6", 3_001, 7_000), CNA("D", "6", 20_001, 9_000, allele=0)] if cna else []
+    w.mutants = [(na, rate, drivers), (nb, rate, [])]
+    eng = synth.build_engine(w)
+    o = orc.OracleEngine.like(w)
+    f = w.forest
+    pf = eng.place_mutations(f, 30, 3, seed=2)
+    op = o.place(f, _forest_species(o, f), 30, 0, 3, 0, seed=2)
+    cfg = dict(coverage=coverage, read_size=50, insert_size_mean=0, error_rate=0.0, purity=0.5, tile_size=tile)
+    for seed in (4, 5):
+        alt, dep = sequence_counts(pf, seed, **cfg).counts()
+        c, _ = seq_cfg(chr_index=eng._chr_index, **cfg)
+        oalt, odep, _ = op.sequence(c, seed, flavour=0)
+        np.testing.assert_array_equal(dep, odep)
+        np.testing.assert_array_equal(alt, oalt)
