@@ -278,7 +278,7 @@ struct pg_placed {
   std::vector<int32_t> parent;
   std::vector<std::vector<uint32_t>> leaves;
   uint64_t M = 0;
-  DBuf<uint32_t> locus, edge, aux, attempt;
+  DBuf<uint32_t> locus, edge, aux;
   DBuf<uint8_t> cls, sig, kind, nature;
   DBuf<uint16_t> allele, seq;
   float kernel_ms = 0;
@@ -312,7 +312,7 @@ struct pg_placed {
   std::vector<uint32_t> bf_chr, bf_begin, bf_end, bf_major, bf_minor;
   std::vector<double> bf_ratio;
   pg::PlaceOut view() const {
-    return {locus.p, edge.p, aux.p, cls.p, sig.p, allele.p, seq.p, kind.p, nature.p, attempt.p};
+    return {locus.p, edge.p, aux.p, cls.p, sig.p, allele.p, seq.p, kind.p, nature.p};
   }
   pg::GenomeClasses classes_view() const {
     return {n_classes, node_class.p, seg_off.p, seg_start.p, seg_end.p, seg_ioff.p, seg_icnt.p, inst_list.p};
@@ -364,6 +364,10 @@ struct Timer {
   }
   ~Timer() { if (a) cudaEventDestroy(a); if (b) cudaEventDestroy(b); }
 };
+
+// slots up to which a placement sizes its redraw tables without reading the
+// number of redraws back
+constexpr uint32_t TAIL_NO_READ = 1u << 19;
 
 void select_device(const pg_engine* e) { ck(cudaSetDevice(e->device), "cudaSetDevice"); }
 
@@ -1285,10 +1289,9 @@ pg_status pg_place_mutations(pg_engine* e, const pg_forest* f, uint32_t n_pre_sn
     require(n_all < (1ull << 31), "too many mutations for one placement call");
     // ---- outputs
     pl->M = n_all;
-    DBuf<uint32_t> locus(P, n_all), edge(P, n_all), aux(P, n_all), attempt(P, n_all);
-    DBuf<uint8_t> cls(P, n_all), sig(P, n_all), kind(P, n_all), nature(P, n_all);
-    DBuf<uint16_t> allele(P, n_all), seqv(P, n_all);
-    pg::PlaceOut o{locus.p, edge.p, aux.p, cls.p, sig.p, allele.p, seqv.p, kind.p, nature.p, attempt.p};
+    DBuf<uint32_t> locus(P, n_all);
+    DBuf<uint4> raw(P, n_all);
+    const pg::PlaceRaw o{locus.p, raw.p};
     DBuf<uint32_t> err(P, 1);
     ck(cudaMemsetAsync(err.p, 0, sizeof(uint32_t), st), "memset");
     // infinite sites: the first draw goes into the first round's table as it
@@ -1306,12 +1309,8 @@ pg_status pg_place_mutations(pg_engine* e, const pg_forest* f, uint32_t n_pre_sn
       fmask = uint32_t(fcap - 1);
       lost1 = DBuf<uint8_t>(P, n_slots);
       ck(cudaMemsetAsync(first.p, 0xff, sizeof(unsigned long long) * fcap, st), "memset");
-      pg::place_first_round(t, o, seed, off_snv.p, off_id.p, uint32_t(n_snv), n_slots, first.p, fmask, lost1.p, err.p,
-                            st);
-    } else {
-      pg::place_mutations_launch(t, o, seed, off_snv.p, off_id.p, uint32_t(n_snv), uint32_t(n_id), nullptr, n_slots, 0,
-                                 err.p, st);
     }
+    pg::place_first_round(t, o, seed, off_snv.p, off_id.p, uint32_t(n_snv), n_slots, first.p, fmask, lost1.p, err.p, st);
     auto drv_d = upload(P, drv, st);
     pg::place_drivers(o, drv_d.p, uint32_t(drv.size()), n_slots, st);
     // the handle's host columns, while the first round runs
@@ -1324,69 +1323,47 @@ pg_status pg_place_mutations(pg_engine* e, const pg_forest* f, uint32_t n_pre_sn
       for (uint32_t v = 0; v < f->n; ++v)
         if (!has_kid[v] && f->sample[v] >= 0) pl->leaf_cls[f->sample[v]].push_back(node_class[v]);
     }
-    // ---- infinite sites, and loci drawn where the cell has no allele left.
-    // Infinite sites: the first round over all slots against one table of
-    // its candidates (drivers first), read back once to size the later
-    // rounds' tables; every later round runs in one cooperative launch.
+    // ---- redraws: infinite sites (the losers of the first round over all
+    // slots, drivers first), or loci drawn where the cell has no allele left
     DBuf<pg::TailCtl> tail_ctl;
     if ((unique || pl->has_cna) && n_slots > 0) {
-      uint32_t n_tail = 0;
-      pg::TailArgs ta{};
-      ta.unique = unique ? 1 : 0;
-      DBuf<uint32_t> pend_a, pend_b, hkeys, ckeys, cvals, hpos;
-      if (unique) {
-        pend_a = DBuf<uint32_t>(P, n_slots);
-        DBuf<uint32_t> n_next(P, 1);
-        ck(cudaMemsetAsync(n_next.p, 0, sizeof(uint32_t), st), "memset");
-        pg::sites_first_finish(locus.p + n_slots, uint32_t(drv.size()), first.p, fmask, lost1.p, n_slots, pend_a.p,
-                               n_next.p, err.p, st);
+      tail_ctl = DBuf<pg::TailCtl>(P, 1);
+      ck(cudaMemsetAsync(tail_ctl.p, 0, sizeof(pg::TailCtl), st), "memset");
+    }
+    if (unique && n_slots > 0) {
+      DBuf<uint32_t> pend(P, n_slots), n_next(P, 1);
+      ck(cudaMemsetAsync(n_next.p, 0, sizeof(uint32_t), st), "memset");
+      pg::sites_first_finish(locus.p + n_slots, uint32_t(drv.size()), first.p, fmask, lost1.p, n_slots, pend.p,
+                             n_next.p, err.p, st);
+      // the host reads how many lost, to size the tables; where tables for
+      // every slot are small (12 MB) that wait costs more than they do
+      uint32_t n_tail = n_slots;
+      if (n_slots > TAIL_NO_READ) {
         ck(cudaMemcpyAsync(&n_tail, n_next.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "round");
         ck(cudaStreamSynchronize(st), "first round");
-        uint32_t cap = 1024;
-        while (cap < 2 * uint64_t(n_tail)) cap <<= 1;
-        pend_b = DBuf<uint32_t>(P, n_tail);
-        hpos = DBuf<uint32_t>(P, n_tail);
-        hkeys = DBuf<uint32_t>(P, cap); ckeys = DBuf<uint32_t>(P, cap); cvals = DBuf<uint32_t>(P, cap);
-        ck(cudaMemsetAsync(hkeys.p, 0xff, sizeof(uint32_t) * cap, st), "memset");
-        ck(cudaMemsetAsync(ckeys.p, 0xff, sizeof(uint32_t) * cap, st), "memset");
-        ck(cudaMemsetAsync(cvals.p, 0xff, sizeof(uint32_t) * cap, st), "memset");
-        ta.redraw_first = 1;
-        ta.round0 = 1;
-        ta.hkeys = hkeys.p; ta.hmask = cap - 1;
-        ta.ckeys = ckeys.p; ta.cvals = cvals.p; ta.cmask = cap - 1;
-        ta.hpos = hpos.p;
-        ta.first = first.p; ta.fmask = fmask;
-      } else {
-        // loci without an allele: round 0 looks at every slot
-        n_tail = n_slots;
-        pend_a = DBuf<uint32_t>(P, n_slots);
-        pend_b = DBuf<uint32_t>(P, n_slots);
-        ta.identity_first = 1;
-        ta.round0 = 0;
       }
-      ta.list[0] = pend_a.p;
-      ta.list[1] = pend_b.p;
       if (n_tail) {
-        tail_ctl = DBuf<pg::TailCtl>(P, 1);
-        pg::TailCtl c0{};
-        c0.count[0] = n_tail;
-        ck(cudaMemcpyAsync(tail_ctl.p, &c0, sizeof(c0), cudaMemcpyHostToDevice, st), "rounds");
-        if (const char* msg = pg::sites_tail(t, o, seed, off_snv.p, off_id.p, uint32_t(n_snv), ta, n_tail, tail_ctl.p,
-                                             err.p, st))
-          throw std::runtime_error(msg);
+        uint64_t cap = 1024;
+        while (cap < 2 * uint64_t(n_tail)) cap <<= 1;
+        DBuf<uint32_t> keys(P, cap);
+        DBuf<unsigned long long> held(P, cap);
+        ck(cudaMemsetAsync(keys.p, 0xff, sizeof(uint32_t) * cap, st), "memset");
+        ck(cudaMemsetAsync(held.p, 0xff, sizeof(unsigned long long) * cap, st), "memset");
+        pg::sites_settle(t, o, seed, off_snv.p, off_id.p, uint32_t(n_snv), pend.p, n_next.p, n_tail, first.p, fmask,
+                         keys.p, held.p, cap, tail_ctl.p, err.p, st);
       }
+    } else if (tail_ctl.p) {
+      pg::sites_covered(t, o, seed, off_snv.p, off_id.p, uint32_t(n_snv), n_slots, tail_ctl.p, err.p, st);
     }
     // ---- sort by locus
     const uint32_t nb = pg::sort_num_buckets(e->G);
     DBuf<uint32_t> bcnt(P, nb), bfill(P, nb), bpart(P, pg::scan_part_elems(nb, 1)), order(P, n_all);
     pl->locus = DBuf<uint32_t>(P, n_all); pl->edge = DBuf<uint32_t>(P, n_all); pl->aux = DBuf<uint32_t>(P, n_all);
-    pl->attempt = DBuf<uint32_t>(P, n_all);
     pl->cls = DBuf<uint8_t>(P, n_all); pl->sig = DBuf<uint8_t>(P, n_all); pl->allele = DBuf<uint16_t>(P, n_all);
     pl->seq = DBuf<uint16_t>(P, n_all);
     pl->kind = DBuf<uint8_t>(P, n_all); pl->nature = DBuf<uint8_t>(P, n_all);
     DBuf<unsigned long long> skeys(P, n_all);
-    DBuf<uint4> recs(P, 2 * n_all);   // 32-byte records of the gather
-    pg::sort_by_locus(o, uint32_t(n_all), e->G, bcnt.p, bfill.p, bpart.p, order.p, pl->view(), skeys.p, recs.p, st);
+    pg::sort_by_locus(o, uint32_t(n_all), e->G, bcnt.p, bfill.p, bpart.p, order.p, pl->view(), skeys.p, st);
     pl->kernel_ms = timer.stop();
     ck(cudaGetLastError(), "placement kernels");
     uint32_t err_h = 0;
@@ -1394,7 +1371,6 @@ pg_status pg_place_mutations(pg_engine* e, const pg_forest* f, uint32_t n_pre_sn
     if (tail_ctl.p) {
       pg::TailCtl c{};
       ck(cudaMemcpy(&c, tail_ctl.p, sizeof(c), cudaMemcpyDeviceToHost), "rounds");
-      if (c.status & pg::TAIL_BARRIER_TIMEOUT) throw std::runtime_error("a grid barrier of the redraw rounds timed out");
       require(!(c.status & pg::TAIL_ROUNDS_EXHAUSTED), unique ? "infinite sites model: no free locus left for some mutations"
                                                               : "no allele left where some mutations were drawn");
       pl->redraw_rounds = c.rounds;

@@ -112,7 +112,6 @@ std::unique_ptr<pg_placed> placed_deserialize(pg_engine* e, const uint8_t* buf, 
   up(p->locus, r.vec<uint32_t>()); up(p->edge, r.vec<uint32_t>()); up(p->aux, r.vec<uint32_t>());
   up(p->cls, r.vec<uint8_t>()); up(p->sig, r.vec<uint8_t>()); up(p->kind, r.vec<uint8_t>());
   up(p->nature, r.vec<uint8_t>()); up(p->allele, r.vec<uint16_t>()); up(p->seq, r.vec<uint16_t>());
-  p->attempt = DBuf<uint32_t>(P, p->M);
   p->has_cna = r.get<uint8_t>() != 0; p->cn_max = r.get<uint32_t>(); p->n_classes = r.get<uint32_t>();
   p->node_class_h = r.vec<uint32_t>();
   p->leaf_cls.resize(r.get<uint64_t>());

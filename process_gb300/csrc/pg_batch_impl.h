@@ -48,9 +48,10 @@ struct pg_batch {
   DBuf<pg::Key> pkeys, skeys;
   // placement outputs (capacity slot_cap)
   uint64_t slot_cap = 0, n_all = 0;
-  DBuf<uint32_t> locus, edge, aux, attempt, s_locus, s_edge, s_aux, s_attempt;
-  DBuf<uint8_t> cls, sig, kind, nature, s_cls, s_sig, s_kind, s_nature;
-  DBuf<uint16_t> allele, seqo, inst_of, s_allele, s_seq, s_inst;
+  DBuf<uint32_t> locus, s_locus, s_edge, s_aux;
+  DBuf<uint4> raw;
+  DBuf<uint8_t> s_cls, s_sig, s_kind, s_nature;
+  DBuf<uint16_t> inst_of, s_allele, s_seq, s_inst;
   DBuf<uint32_t> rec_off_d, n_all_d;
   std::vector<uint32_t> rec_off;
   // sequencing layout (rebuilt when tile sizes change or an instance outgrows its capacity)
@@ -75,11 +76,8 @@ struct pg_batch {
   ~pg_batch() {
     if (graph) cudaGraphExecDestroy(graph);
   }
-  pg::PlaceOut out_view() {
-    return {locus.p, edge.p, aux.p, cls.p, sig.p, allele.p, seqo.p, kind.p, nature.p, attempt.p};
-  }
   pg::PlaceOut sorted_view() {
-    return {s_locus.p, s_edge.p, s_aux.p, s_cls.p, s_sig.p, s_allele.p, s_seq.p, s_kind.p, s_nature.p, s_attempt.p};
+    return {s_locus.p, s_edge.p, s_aux.p, s_cls.p, s_sig.p, s_allele.p, s_seq.p, s_kind.p, s_nature.p};
   }
 };
 
@@ -125,77 +123,58 @@ void batch_place(pg_batch* b, const uint64_t* place_seed) {
   b->n_all = n_all;
   if (n_all > b->slot_cap) {
     const uint64_t cap = n_all + n_all / 8 + 4096;
-    b->locus = DBuf<uint32_t>(P, cap); b->edge = DBuf<uint32_t>(P, cap); b->aux = DBuf<uint32_t>(P, cap);
-    b->attempt = DBuf<uint32_t>(P, cap);
+    b->locus = DBuf<uint32_t>(P, cap); b->raw = DBuf<uint4>(P, cap); b->inst_of = DBuf<uint16_t>(P, cap);
     b->s_locus = DBuf<uint32_t>(P, cap); b->s_edge = DBuf<uint32_t>(P, cap); b->s_aux = DBuf<uint32_t>(P, cap);
-    b->s_attempt = DBuf<uint32_t>(P, cap);
-    b->cls = DBuf<uint8_t>(P, cap); b->sig = DBuf<uint8_t>(P, cap); b->kind = DBuf<uint8_t>(P, cap);
-    b->nature = DBuf<uint8_t>(P, cap);
     b->s_cls = DBuf<uint8_t>(P, cap); b->s_sig = DBuf<uint8_t>(P, cap); b->s_kind = DBuf<uint8_t>(P, cap);
     b->s_nature = DBuf<uint8_t>(P, cap);
-    b->allele = DBuf<uint16_t>(P, cap); b->seqo = DBuf<uint16_t>(P, cap); b->inst_of = DBuf<uint16_t>(P, cap);
     b->s_allele = DBuf<uint16_t>(P, cap); b->s_seq = DBuf<uint16_t>(P, cap); b->s_inst = DBuf<uint16_t>(P, cap);
     b->slot_cap = cap;
     b->layout_ok = false;          // the records buffer follows the slot capacity
   }
-  const pg::PlaceOut o = b->out_view();
+  const pg::PlaceRaw o{b->locus.p, b->raw.p};
   DBuf<uint32_t> err(P, 1);
   DBuf<pg::TailCtl> tail_ctl;
   ck(cudaMemsetAsync(err.p, 0, sizeof(uint32_t), st), "memset");
-  pg::place_mutations_batch(b->tabs.p, B, b->cell_off_d.p, b->pkeys.p, o, b->inst_of.p, cnt_snv.p, cnt_id.p,
-                            uint32_t(n_snv), nullptr, uint32_t(n_all), 0, err.p, st);
-  if (e->infinite_sites && n_all > 0) {
-    DBuf<uint32_t> pend_a(P, n_all), pend_b(P, n_all), n_next(P, 1);
-    DBuf<uint8_t> lost(P, n_all);
-    const uint32_t* pending = nullptr;
-    uint32_t n_pend = uint32_t(n_all);
-    uint32_t* next = pend_a.p;
-    // the first round (no drivers in a batch, so nothing is taken yet) keeps
-    // its candidate table, which then holds exactly the taken keys; the
-    // later rounds test it beside their own accepted set, sized by what the
-    // first round leaves
-    uint64_t fcap = 1024;
+  const bool unique = e->infinite_sites && n_all > 0;
+  // the first round (no drivers in a batch, so nothing is taken yet): its
+  // table then holds exactly the taken keys
+  DBuf<uint64_t> fkeys;
+  DBuf<uint32_t> fslot, pend, n_next;
+  DBuf<uint8_t> lost;
+  uint64_t fcap = 1024;
+  if (unique) {
     while (fcap < 2 * n_all) fcap <<= 1;
-    DBuf<uint64_t> fkeys(P, fcap);
-    {
-      DBuf<uint32_t> fvals(P, fcap);
-      ck(cudaMemsetAsync(fkeys.p, 0xff, sizeof(uint64_t) * fcap, st), "memset");
-      ck(cudaMemsetAsync(fvals.p, 0xff, sizeof(uint32_t) * fcap, st), "memset");
-      ck(cudaMemsetAsync(n_next.p, 0, sizeof(uint32_t), st), "memset");
-      pg::sites_round_batch(b->locus.p, b->inst_of.p, nullptr, n_pend, nullptr, 0, fkeys.p, fvals.p, fcap - 1, lost.p,
-                            next, n_next.p, err.p, st);
-      uint32_t nn = 0;
-      ck(cudaMemcpyAsync(&nn, n_next.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "round");
+    fkeys = DBuf<uint64_t>(P, fcap);
+    fslot = DBuf<uint32_t>(P, fcap);
+    lost = DBuf<uint8_t>(P, n_all);
+    pend = DBuf<uint32_t>(P, n_all);
+    n_next = DBuf<uint32_t>(P, 1);
+    ck(cudaMemsetAsync(fkeys.p, 0xff, sizeof(uint64_t) * fcap, st), "memset");
+    ck(cudaMemsetAsync(fslot.p, 0xff, sizeof(uint32_t) * fcap, st), "memset");
+    ck(cudaMemsetAsync(n_next.p, 0, sizeof(uint32_t), st), "memset");
+  }
+  pg::place_first_round_batch(b->tabs.p, B, b->cell_off_d.p, b->pkeys.p, o, b->inst_of.p, cnt_snv.p, cnt_id.p,
+                              uint32_t(n_snv), uint32_t(n_all), fkeys.p, fslot.p, fcap - 1, lost.p, pend.p, n_next.p,
+                              err.p, st);
+  if (unique) {
+    uint32_t n_tail = uint32_t(n_all);   // read back as in pg_place_mutations
+    if (n_all > TAIL_NO_READ) {
+      ck(cudaMemcpyAsync(&n_tail, n_next.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "round");
       ck(cudaStreamSynchronize(st), "first round");
-      pending = next;
-      n_pend = nn;
     }
-    // every later round (the losers' redraws first) in one cooperative
-    // launch, its tables sized by what the first round leaves
-    uint64_t cap = 1024;
-    while (cap < 2 * uint64_t(n_pend)) cap <<= 1;
-    if (n_pend) {
-      DBuf<unsigned long long> hkeys(P, cap), ckeys(P, cap);
-      DBuf<uint32_t> cvals(P, cap);
-      DBuf<uint64_t> hpos(P, n_pend);
+    if (n_tail) {
+      uint64_t cap = 1024;
+      while (cap < 2 * uint64_t(n_tail)) cap <<= 1;
+      DBuf<uint64_t> hkeys(P, cap);
+      DBuf<unsigned long long> held(P, cap);
       ck(cudaMemsetAsync(hkeys.p, 0xff, sizeof(uint64_t) * cap, st), "memset");
-      ck(cudaMemsetAsync(ckeys.p, 0xff, sizeof(uint64_t) * cap, st), "memset");
-      ck(cudaMemsetAsync(cvals.p, 0xff, sizeof(uint32_t) * cap, st), "memset");
+      ck(cudaMemsetAsync(held.p, 0xff, sizeof(unsigned long long) * cap, st), "memset");
       tail_ctl = DBuf<pg::TailCtl>(P, 1);
-      pg::TailCtl c0{};
-      c0.count[0] = n_pend;
-      ck(cudaMemcpyAsync(tail_ctl.p, &c0, sizeof(c0), cudaMemcpyHostToDevice, st), "rounds");
-      pg::TailArgsB ta{};
-      ta.list[0] = const_cast<uint32_t*>(pending);
-      ta.list[1] = pend_b.p;
-      ta.hkeys = hkeys.p; ta.hmask = cap - 1;
-      ta.ckeys = ckeys.p; ta.cvals = cvals.p; ta.cmask = cap - 1;
-      ta.hpos = hpos.p;
-      ta.fkeys = fkeys.p; ta.fmask = fcap - 1;
-      if (const char* msg = pg::sites_tail_batch(b->tabs.p, B, b->cell_off_d.p, b->pkeys.p, o, b->inst_of.p, cnt_snv.p,
-                                                 cnt_id.p, uint32_t(n_snv), ta, n_pend, tail_ctl.p, err.p, st))
-        throw std::runtime_error(msg);
-      // the tables live until the launch ends: the engine's pool hands them
+      ck(cudaMemsetAsync(tail_ctl.p, 0, sizeof(pg::TailCtl), st), "memset");
+      pg::sites_settle_batch(b->tabs.p, B, b->cell_off_d.p, b->pkeys.p, o, b->inst_of.p, cnt_snv.p, cnt_id.p,
+                             uint32_t(n_snv), pend.p, n_next.p, n_tail, fkeys.p, fcap - 1, hkeys.p, held.p, cap,
+                             tail_ctl.p, err.p, st);
+      // the tables live until the launches end: the engine's pool hands them
       // out again only to later work on this stream
     }
   }
@@ -205,9 +184,8 @@ void batch_place(pg_batch* b, const uint64_t* place_seed) {
   const uint64_t nbt = uint64_t(nb) * B;
   DBuf<uint32_t> bcnt(P, nbt + 1), bfill(P, nbt), bpart(P, pg::scan_part_elems(nbt, 1)), order(P, n_all);
   DBuf<unsigned long long> skeys(P, n_all);
-  DBuf<uint4> recs(P, 2 * n_all);
   pg::sort_batch(o, b->inst_of.p, uint32_t(n_all), B, e->G, bcnt.p, bfill.p, bpart.p, order.p, b->sorted_view(),
-                 b->s_inst.p, skeys.p, recs.p, st);
+                 b->s_inst.p, skeys.p, st);
   if (n_all > 0) {
     ck(cudaMemcpy2DAsync(b->rec_off_d.p, sizeof(uint32_t), bcnt.p, sizeof(uint32_t) * nb, sizeof(uint32_t), B,
                          cudaMemcpyDeviceToDevice, st), "record offsets");
@@ -225,7 +203,6 @@ void batch_place(pg_batch* b, const uint64_t* place_seed) {
   pg::TailCtl tc{};
   if (tail_ctl.p) ck(cudaMemcpyAsync(&tc, tail_ctl.p, sizeof(tc), cudaMemcpyDeviceToHost, st), "rounds");
   ck(cudaStreamSynchronize(st), "batch placement");
-  if (tc.status & pg::TAIL_BARRIER_TIMEOUT) throw std::runtime_error("a grid barrier of the redraw rounds timed out");
   require(!(tc.status & pg::TAIL_ROUNDS_EXHAUSTED), "infinite sites model: no free locus left for some mutations");
   if (err_h & pg::ERR_EMPTY_CLASS) throw std::runtime_error("a drawn mutation class has no indexed positions");
   if (err_h & pg::ERR_CAPACITY) throw std::runtime_error("internal hash table capacity exceeded");

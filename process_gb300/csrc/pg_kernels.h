@@ -108,7 +108,13 @@ struct PlaceOut {
   uint16_t* seq;      // order on the edge: driver event index, 0x7fff passengers, 0 preneoplastic
   uint8_t* kind;
   uint8_t* nature;
-  uint32_t* attempt;
+};
+
+// Mutations in slot order, before the sort: the locus and a record {edge, aux,
+// allele | seq << 16, cls | sig << 8 | kind << 16 | nature << 24}
+struct PlaceRaw {
+  uint32_t* locus;
+  uint4* rec;
 };
 
 struct DriverRec {
@@ -119,66 +125,39 @@ struct DriverRec {
 void place_cna_counts(const PlaceTables& t, uint32_t* cnt_cna, uint64_t seed, double germline_size, cudaStream_t st);
 void place_edge_counts(const PlaceTables& t, uint32_t* cnt_snv, uint32_t* cnt_id, uint64_t seed,
                        uint32_t n_pre_snv, uint32_t n_pre_id, cudaStream_t st);
-// n_dev (optional): the number of pending slots in device memory (<= n_pending,
-// which sizes the grid); the redraw rounds run without reading it on the host
-void place_mutations_launch(const PlaceTables& t, const PlaceOut& o, uint64_t seed, const uint32_t* off_snv,
-                            const uint32_t* off_id, uint32_t n_snv, uint32_t n_id, const uint32_t* pending,
-                            uint32_t n_pending, int redraw, uint32_t* err, cudaStream_t st,
-                            const uint32_t* n_dev = nullptr);
-void place_drivers(const PlaceOut& o, const DriverRec* drv, uint32_t n_drv, uint32_t base_slot, cudaStream_t st);
-// the first draw of slots [0, n_slots) fused with their insertion into the
-// first round's table `first` (fmask + 1 entries, all ones on entry; lost:
-// n_slots bytes of scratch); then sites_first_finish inserts the drivers'
-// loci and lists the losing slots in next
-void place_first_round(const PlaceTables& t, const PlaceOut& o, uint64_t seed, const uint32_t* off_snv,
+void place_drivers(const PlaceRaw& o, const DriverRec* drv, uint32_t n_drv, uint32_t base_slot, cudaStream_t st);
+// the first draw of slots [0, n_slots); with first, fused with their insertion
+// into the first round's table `first` (fmask + 1 entries, all ones on entry;
+// lost: n_slots bytes of scratch).  Then sites_first_finish inserts the
+// drivers' loci and lists the losing slots in next.
+void place_first_round(const PlaceTables& t, const PlaceRaw& o, uint64_t seed, const uint32_t* off_snv,
                        const uint32_t* off_id, uint32_t n_snv, uint32_t n_slots, unsigned long long* first,
                        uint32_t fmask, uint8_t* lost, uint32_t* err, cudaStream_t st);
 void sites_first_finish(const uint32_t* drv_locus, uint32_t n_drv, unsigned long long* first, uint32_t fmask,
                         uint8_t* lost, uint32_t n_slots, uint32_t* next, uint32_t* n_next, uint32_t* err,
                         cudaStream_t st);
-// All redraw rounds after the first in one cooperative launch (k_sites_tail).
-// list[0] holds the n0 pending slots (identity_first: slots 0 .. n0 - 1, no
-// list); redraw_first: they are redrawn before the first round.  unique:
-// infinite sites (hkeys accepted set, ckeys/cvals candidate table, all
-// EMPTY on entry, capacities powers of two >= 2 n0; hpos n0 entries; first:
-// the first round's table or NULL); else only loci without an allele are
-// redrawn.  ctl (zeroed, count[0] = n0) reports the rounds and the status.
+// The redraws of the *n (<= n_max, in device memory) slots of list: keys and
+// held (both all ones) have cap entries, a power of two >= 2 n_max.  ctl
+// (zeroed) reports the rounds (one more than the last attempt needed; 0:
+// nothing was pending) and the status.
 constexpr uint32_t TAIL_MAX_ROUND = 256;
-enum : uint32_t { TAIL_ROUNDS_EXHAUSTED = 1u, TAIL_BARRIER_TIMEOUT = 2u };
+enum : uint32_t { TAIL_ROUNDS_EXHAUSTED = 1u };
 struct TailCtl {
-  uint32_t count[2];     // pending slots of the two lists
-  uint32_t bar_count, bar_gen;
   uint32_t status;
-  uint32_t rounds;       // the round counter after the last round run
+  uint32_t rounds;
 };
-struct TailArgs {
-  uint32_t* list[2];
-  int identity_first, redraw_first, unique;
-  uint32_t round0;
-  uint32_t* hkeys; uint32_t hmask;
-  uint32_t* ckeys; uint32_t* cvals; uint32_t cmask;
-  uint32_t* hpos;
-  const unsigned long long* first; uint32_t fmask;
-};
-// the batched form: keys (instance << 32 | locus); list 0 holds the first
-// round's losers, redrawn first; fkeys: the first round's table
-struct TailArgsB {
-  uint32_t* list[2];
-  unsigned long long* hkeys; uint64_t hmask;
-  unsigned long long* ckeys; uint32_t* cvals; uint64_t cmask;
-  uint64_t* hpos;
-  const uint64_t* fkeys; uint64_t fmask;
-};
-// returns nullptr, or a message when the launch could not be made
-const char* sites_tail(const PlaceTables& t, const PlaceOut& o, uint64_t seed, const uint32_t* off_snv,
-                       const uint32_t* off_id, uint32_t n_snv, const TailArgs& a, uint32_t n0, TailCtl* ctl,
-                       uint32_t* err, cudaStream_t st);
-uint32_t sort_num_buckets(uint64_t G);
-// sort by (locus, slot) into `sorted`; keys: n 64-bit keys, recs: 2n
-// 16-byte words (the 32-byte records of the gather)
-void sort_by_locus(const PlaceOut& o, uint32_t n, uint64_t G, uint32_t* bcnt, uint32_t* bfill, uint32_t* part,
-                   uint32_t* order, const PlaceOut& sorted, unsigned long long* keys, uint4* recs,
+void sites_settle(const PlaceTables& t, const PlaceRaw& o, uint64_t seed, const uint32_t* off_snv,
+                  const uint32_t* off_id, uint32_t n_snv, const uint32_t* list, const uint32_t* n, uint32_t n_max,
+                  const unsigned long long* first, uint32_t fmask, uint32_t* keys, unsigned long long* held,
+                  uint64_t cap, TailCtl* ctl, uint32_t* err, cudaStream_t st);
+// without infinite sites: redraws of the slots whose locus has no allele
+void sites_covered(const PlaceTables& t, const PlaceRaw& o, uint64_t seed, const uint32_t* off_snv,
+                   const uint32_t* off_id, uint32_t n_snv, uint32_t n_slots, TailCtl* ctl, uint32_t* err,
                    cudaStream_t st);
+uint32_t sort_num_buckets(uint64_t G);
+// sort by (locus, slot) into `sorted`; keys: n 64-bit keys
+void sort_by_locus(const PlaceRaw& o, uint32_t n, uint64_t G, uint32_t* bcnt, uint32_t* bfill, uint32_t* part,
+                   uint32_t* order, const PlaceOut& sorted, unsigned long long* keys, cudaStream_t st);
 
 // ---------------------------------------------------------------- sequencing
 struct SeqRec {            // 16 B, one per placed mutation, sorted by locus
@@ -367,30 +346,25 @@ struct SeqBatch {
 void place_edge_counts_batch(const PlaceTables* tabs, uint32_t n_inst, const uint32_t* node_off, uint32_t n_nodes_all,
                              const uint32_t* cell_off, const Key* keys, const uint32_t* pre_snv, const uint32_t* pre_id,
                              uint32_t* cnt_snv, uint32_t* cnt_id, cudaStream_t st);
-void place_mutations_batch(const PlaceTables* tabs, uint32_t n_inst, const uint32_t* cell_off, const Key* keys,
-                           const PlaceOut& o, uint16_t* inst_of, const uint32_t* off_snv, const uint32_t* off_id,
-                           uint32_t n_snv, const uint32_t* pending, uint32_t n_pending, int redraw, uint32_t* err,
-                           cudaStream_t st, const uint32_t* n_dev = nullptr);
-// hkeys NULL: no accepted set (the first round, whose candidate table then
-// holds the taken keys); fkeys (optional): that first round's table, tested
-// as taken by the later rounds
-void sites_round_batch(const uint32_t* locus, const uint16_t* inst_of, const uint32_t* pending, uint32_t n,
-                       uint64_t* hkeys, uint64_t hmask, uint64_t* ckeys, uint32_t* cvals, uint64_t cmask,
-                       uint8_t* lost, uint32_t* next, uint32_t* n_next, uint32_t* err, cudaStream_t st,
-                       const uint32_t* n_dev = nullptr, const uint64_t* fkeys = nullptr, uint64_t fmask = 0);
-// every round after the first in one cooperative launch (k_sites_tail_b);
-// list 0 of `a` holds the n0 losers of the first round; returns nullptr or
-// a message when the launch could not be made
-const char* sites_tail_batch(const PlaceTables* tabs, uint32_t n_inst, const uint32_t* cell_off, const Key* keys,
-                             const PlaceOut& o, uint16_t* inst_of, const uint32_t* off_snv, const uint32_t* off_id,
-                             uint32_t n_snv, const TailArgsB& a, uint32_t n0, TailCtl* ctl, uint32_t* err,
-                             cudaStream_t st);
+// the first draw of a batch's slots; with fkeys (fmask + 1 entries, all ones)
+// also the first infinite-sites round (fslot: as many entries, all ones;
+// lost: n_slots bytes), whose losers go to next
+void place_first_round_batch(const PlaceTables* tabs, uint32_t n_inst, const uint32_t* cell_off, const Key* keys,
+                             const PlaceRaw& o, uint16_t* inst_of, const uint32_t* off_snv, const uint32_t* off_id,
+                             uint32_t n_snv, uint32_t n_slots, uint64_t* fkeys, uint32_t* fslot, uint64_t fmask,
+                             uint8_t* lost, uint32_t* next, uint32_t* n_next, uint32_t* err, cudaStream_t st);
+// sites_settle for a batch, keyed by (instance << 32 | locus)
+void sites_settle_batch(const PlaceTables* tabs, uint32_t n_inst, const uint32_t* cell_off, const Key* keys,
+                        const PlaceRaw& o, uint16_t* inst_of, const uint32_t* off_snv, const uint32_t* off_id,
+                        uint32_t n_snv, const uint32_t* list, const uint32_t* n, uint32_t n_max, const uint64_t* fkeys,
+                        uint64_t fmask, uint64_t* hkeys, unsigned long long* held, uint64_t cap, TailCtl* ctl,
+                        uint32_t* err, cudaStream_t st);
 // sort by (instance, locus, slot); bcnt holds n_inst * sort_num_buckets(G)
 // + 1 entries and ends as the exclusive scan of the bucket counts; keys: n
-// 64-bit keys, recs: 2n 16-byte words
-void sort_batch(const PlaceOut& o, const uint16_t* inst_of, uint32_t n, uint32_t n_inst, uint64_t G, uint32_t* bcnt,
+// 64-bit keys
+void sort_batch(const PlaceRaw& o, const uint16_t* inst_of, uint32_t n, uint32_t n_inst, uint64_t G, uint32_t* bcnt,
                 uint32_t* bfill, uint32_t* part, uint32_t* order, const PlaceOut& sorted, uint16_t* inst_sorted,
-                unsigned long long* keys, uint4* recs, cudaStream_t st);
+                unsigned long long* keys, cudaStream_t st);
 // resident CTAs per SM of the persistent read kernel
 int seq_reads_batch_occupancy();
 // records of the first *n_dev sorted mutations of a batch (cap >= *n_dev)

@@ -91,3 +91,61 @@ def test_tile_split(gpu_lib, orc, tile, coverage, cna):
         oalt, odep, _ = op.sequence(c, seed, flavour=0)
         np.testing.assert_array_equal(dep, odep)
         np.testing.assert_array_equal(alt, oalt)
+
+
+@pytest.mark.parametrize("infinite", [True, False])
+@pytest.mark.parametrize("rate,leaves,sampling", [(1e-6, 8, 1), (6e-5, 40, 1), (2e-4, 60, 1), (2e-5, 60, 10)])
+def test_redraws(gpu_lib, orc, infinite, rate, leaves, sampling):
+    """Placements from almost no collisions to position lists so full that
+    slots take many attempts (and another class from the fourth on), with
+    regions that some or all cells have lost on both alleles."""
+    from process_gb300 import CNA, SNV, synth
+    w = synth.plain_3mbp(seed=8, n_leaves=leaves)
+    w.genome.chr_lengths = [40_000, 1_500, 30_011]
+    w.context_sampling = sampling
+    (na, _, _), (nb, _, _) = w.mutants
+    rates = {"SNV": rate, "indel": 0.05 * rate}
+    w.mutants = [(na, rates, [SNV("1", 500, "T"), CNA("D", "1", 10_001, 9_000, allele=0),
+                              CNA("D", "1", 10_001, 9_000, allele=0)]),
+                 (nb, rates, [CNA("D", "3", 1, 20_000, allele=1), CNA("D", "3", 1, 8_000, allele=0)])]
+    eng = synth.build_engine(w)
+    eng.infinite_sites_model = infinite
+    o = orc.OracleEngine.like(w)
+    o.set_infinite_sites(infinite)
+    f = w.forest
+    for seed in (3, 4, 5):
+        t = eng.place_mutations(f, 40, 5, seed=seed).table()
+        ot = o.place(f, _forest_species(o, f), 40, 0, 5, 0, seed=seed).table()
+        assert len(t["locus"]) == len(ot["locus"])
+        for k in ("locus", "edge", "aux", "cls", "sig", "allele", "kind", "nature"):
+            np.testing.assert_array_equal(t[k], ot[k], err_msg=k)
+
+
+@pytest.mark.parametrize("rate", [1e-9, 1e-4, 1e-3, 4e-3])
+def test_edge_counts(gpu_lib, orc, rate):
+    """Mutations per (edge, epoch): Poisson means in the inversion range, near
+    its end and far above it; edges that start or end at an epoch's start or
+    span epochs."""
+    from process_gb300 import SamplesForest, synth
+    w = synth.plain_3mbp(seed=9, n_leaves=50)
+    w.genome.chr_lengths = [3_000, 3_000, 3_000]
+    f0 = w.forest
+    nodes = f0.get_nodes()
+    birth = np.round(f0.birth_time)                       # many edges end exactly at an epoch's start
+    w.forest = SamplesForest(nodes["cell_id"], nodes["ancestor"], np.full(f0.num_of_nodes, "A", dtype=object),
+                             np.full(f0.num_of_nodes, "", dtype=object), nodes["sample"], birth,
+                             np.arange(f0.num_of_nodes) % 7 + 1)
+    w.mutants = [("A", {"SNV": [rate, 2 * rate, 0.5 * rate], "indel": [0.1 * rate, 0.0, rate]}, [])]
+    t_end = float(birth.max())
+    w.exposures = [(t, {"SBS1": 1.0, "ID1": 1.0}) for t in (0.0, np.round(t_end / 3), np.round(t_end / 2))]
+    eng = synth.build_engine(w)
+    eng.infinite_sites_model = False
+    o = orc.OracleEngine.like(w)
+    o.set_infinite_sites(False)
+    f = w.forest
+    sp = np.zeros(f.num_of_nodes, dtype=np.uint32)
+    for seed in (1, 2):
+        t = eng.place_mutations(f, 3, 2, seed=seed).table()
+        ot = o.place(f, sp, 3, 0, 2, 0, seed=seed).table()
+        np.testing.assert_array_equal(t["edge"], ot["edge"])
+        np.testing.assert_array_equal(t["locus"], ot["locus"])
