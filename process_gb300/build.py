@@ -29,6 +29,7 @@ UNITS = {
     "pg_place.cu": False,
     "pg_seq.cu": False,
     "pg_calib.cu": True,
+    "pg_calib_hi.cu": True,
     "pg_api.cpp": False,
 }
 

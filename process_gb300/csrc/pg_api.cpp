@@ -2080,35 +2080,42 @@ pg_status pg_seq_result_tile_size(const pg_seq_result* r, uint32_t* tile_size) {
 }  // extern "C"
 
 // ====================================================================== calibration
-constexpr uint32_t CALIB_CHUNK = 16384;   // sites per CTA of the site kernel
+// Sites of a segment at most: longer per-thread FP32 sums lose precision (65536
+// doubled the gradient error of a table of 2e5 sites), and at least: one
+// 16-byte load of each column per thread.
+constexpr uint32_t CALIB_SEG = 16384, CALIB_MIN_SEG = 1024;
 
 struct pg_calib {
   int device = 0;
   cudaStream_t st = nullptr, own_st = nullptr;
   Pool pool;
-  uint32_t n_rep = 0, K = 0, J = 0, C = 0, P = 0, n_chunks = 0;
+  uint32_t n_rep = 0, K = 0, J = 0, C = 0, P = 0, n_segs = 0;
   DBuf<int32_t> alt, depth, cls;
-  DBuf<uint64_t> site_off, chunk_start;
-  DBuf<uint32_t> chunk_rep, rep_first_chunk, step;
-  DBuf<float> sig, sig_rows, epoch_w, phi, partial, m, v, tab;
-  std::vector<uint32_t> rep_first_chunk_h;
-  uint32_t part_stride = 0, tab_stride = 0;
+  DBuf<uint64_t> seg_start;
+  DBuf<uint32_t> seg_rep, seg_len, rep_first_seg, rep_done, rep_step;   // rep_step: one more entry, the status
+  DBuf<float> sig_rows, epoch_w, phi, tab, m, v;
+  DBuf<float2> partial;
+  bool split = false;                // more segments than the GPU holds at a time
+  std::vector<uint32_t> rep_first_seg_h;
+  uint32_t part_stride = 0;
   cudaGraphExec_t graph = nullptr;
   struct { float* params = nullptr; uint32_t steps = 0; float lr = 0, b1 = 0, b2 = 0, eps = 0; float* nll = nullptr; cudaStream_t st = nullptr; } gkey;
   pg::CalibArgs args() const {
     pg::CalibArgs a{};
     a.K = K; a.J = J; a.C = C; a.P = P;
-    a.alt = alt.p; a.depth = depth.p; a.cls = cls.p; a.site_off = site_off.p;
-    a.sig = sig.p; a.epoch_w = epoch_w.p; a.phi = phi.p;
-    a.chunk = CALIB_CHUNK; a.part_stride = part_stride;
-    a.sig_rows = sig_rows.p; a.tab = tab.p; a.tab_stride = tab_stride;
+    a.alt = alt.p; a.depth = depth.p; a.cls = cls.p;
+    a.epoch_w = epoch_w.p; a.phi = phi.p; a.sig_rows = sig_rows.p;
+    a.seg_rep = seg_rep.p; a.seg_start = seg_start.p; a.seg_len = seg_len.p;
+    a.rep_first_seg = rep_first_seg.p; a.rep_done = rep_done.p;
+    a.partial = partial.p; a.part_stride = part_stride; a.tab = split ? tab.p : nullptr;
+    a.steps = 1;
     return a;
   }
   ~pg_calib() {
     if (graph) cudaGraphExecDestroy(graph);
-    alt.reset(); depth.reset(); cls.reset(); site_off.reset(); chunk_start.reset(); chunk_rep.reset();
-    rep_first_chunk.reset(); step.reset(); sig.reset(); epoch_w.reset(); phi.reset(); partial.reset(); m.reset();
-    v.reset(); tab.reset(); sig_rows.reset();
+    alt.reset(); depth.reset(); cls.reset(); seg_start.reset(); seg_rep.reset(); seg_len.reset();
+    rep_first_seg.reset(); rep_done.reset(); rep_step.reset(); sig_rows.reset(); epoch_w.reset();
+    phi.reset(); partial.reset(); tab.reset(); m.reset(); v.reset();
     pool.release_all();
     if (own_st) cudaStreamDestroy(own_st);
   }
@@ -2147,7 +2154,6 @@ pg_status pg_calib_create(uint32_t n_rep, const uint64_t* site_off, const int32_
     cudaStream_t st = c->st;
     std::vector<int32_t> va(alt, alt + n), vd(depth, depth + n), vc(cls, cls + n);
     c->alt = upload(P, va, st); c->depth = upload(P, vd, st); c->cls = upload(P, vc, st);
-    c->site_off = upload(P, std::vector<uint64_t>(site_off, site_off + n_rep + 1), st);
     std::vector<float> fs(uint64_t(J) * C), fw(uint64_t(n_rep) * K), fp(uint64_t(n_rep) * K);
     for (uint32_t j = 0; j < J; ++j) {   // signatures normalised to sum 1 over the classes
       double tot = 0;
@@ -2156,7 +2162,7 @@ pg_status pg_calib_create(uint32_t n_rep, const uint64_t* site_off, const int32_
       for (uint32_t k = 0; k < C; ++k) fs[uint64_t(j) * C + k] = float(signatures[uint64_t(j) * C + k] / tot);
     }
     for (uint64_t x = 0; x < fw.size(); ++x) { fw[x] = float(epoch_weight[x]); fp[x] = float(phi[x]); }
-    c->sig = upload(P, fs, st); c->epoch_w = upload(P, fw, st); c->phi = upload(P, fp, st);
+    c->epoch_w = upload(P, fw, st); c->phi = upload(P, fp, st);
     {   // signatures by class, rows of 4 or 8 floats
       const uint32_t JP = J > 4 ? 8 : 4;
       std::vector<float> rows(size_t(C) * JP, 0.f);
@@ -2164,26 +2170,50 @@ pg_status pg_calib_create(uint32_t n_rep, const uint64_t* site_off, const int32_
         for (uint32_t cl = 0; cl < C; ++cl) rows[size_t(cl) * JP + j] = fs[size_t(j) * C + cl];
       c->sig_rows = upload(P, rows, st);
     }
-    // chunks of CALIB_CHUNK sites, never across replicates
-    std::vector<uint32_t> crep;
-    std::vector<uint64_t> cstart;
-    c->rep_first_chunk_h.assign(n_rep + 1, 0);
-    for (uint32_t r = 0; r < n_rep; ++r) {
-      c->rep_first_chunk_h[r] = uint32_t(crep.size());
-      for (uint64_t i = site_off[r]; i < site_off[r + 1]; i += CALIB_CHUNK) { crep.push_back(r); cstart.push_back(i); }
+    // segments: the smallest size that needs no more rounds of resident CTAs
+    // than CALIB_SEG does (one round where possible; a last round of a few
+    // CTAs would take as long as a full one), equal within a replicate
+    int sms = 0;
+    ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device), "device attribute");
+    const uint64_t resident = uint64_t(std::max(1, sms)) * uint64_t(pg::calib_ctas_per_sm(K, J));
+    auto segs_at = [&](uint64_t size) {
+      uint64_t k = 0;
+      for (uint32_t r = 0; r < n_rep; ++r) k += std::max<uint64_t>(1, (site_off[r + 1] - site_off[r] + size - 1) / size);
+      return k;
+    };
+    const uint64_t room = (segs_at(CALIB_SEG) + resident - 1) / resident * resident;
+    uint64_t size = CALIB_MIN_SEG;
+    for (uint64_t hi = CALIB_SEG; size < hi;) {
+      const uint64_t mid = (size + hi) / 2;
+      if (segs_at(mid) <= room) hi = mid; else size = mid + 1;
     }
-    c->rep_first_chunk_h[n_rep] = uint32_t(crep.size());
-    c->n_chunks = uint32_t(crep.size());
-    c->chunk_rep = upload(P, crep, st); c->chunk_start = upload(P, cstart, st);
-    c->rep_first_chunk = upload(P, c->rep_first_chunk_h, st);
+    std::vector<uint32_t> srep, slen;
+    std::vector<uint64_t> sstart;
+    c->rep_first_seg_h.assign(n_rep + 1, 0);
+    for (uint32_t r = 0; r < n_rep; ++r) {
+      c->rep_first_seg_h[r] = uint32_t(srep.size());
+      const uint64_t nr = site_off[r + 1] - site_off[r], k = std::max<uint64_t>(1, (nr + size - 1) / size);
+      // cut at multiples of four sites (the 16-byte loads)
+      auto cut = [&](uint64_t q) { return q == k ? site_off[r + 1] : q == 0 ? site_off[r] : (site_off[r] + nr * q / k) & ~uint64_t(3); };
+      for (uint64_t q = 0; q < k; ++q) {
+        const uint64_t at = std::max(cut(q), site_off[r]);
+        srep.push_back(r); sstart.push_back(at); slen.push_back(uint32_t(std::max(cut(q + 1), at) - at));
+      }
+    }
+    c->rep_first_seg_h[n_rep] = uint32_t(srep.size());
+    c->n_segs = uint32_t(srep.size());
+    c->split = c->n_segs > resident;
+    c->seg_rep = upload(P, srep, st); c->seg_start = upload(P, sstart, st); c->seg_len = upload(P, slen, st);
+    c->rep_first_seg = upload(P, c->rep_first_seg_h, st);
+    c->rep_done = DBuf<uint32_t>(P, n_rep);
+    ck(cudaMemsetAsync(c->rep_done.p, 0, sizeof(uint32_t) * n_rep, st), "memset");
     c->part_stride = (1 + 3 * K + K * J + 3) & ~3u;
-    // per replicate: log(exp(lr_k) L_k / Z), log v_k, log(1 - v_k) (K each), w_kj (K J)
-    c->tab_stride = (3 * K + K * J + 3) & ~3u;
-    c->tab = DBuf<float>(P, uint64_t(n_rep) * c->tab_stride);
-    c->partial = DBuf<float>(P, uint64_t(std::max<uint32_t>(c->n_chunks, 1)) * c->part_stride);
+    c->partial = DBuf<float2>(P, uint64_t(srep.size()) * c->part_stride);
+    if (c->split) c->tab = DBuf<float>(P, uint64_t(n_rep) * c->part_stride);
     c->m = DBuf<float>(P, uint64_t(n_rep) * c->P);
     c->v = DBuf<float>(P, uint64_t(n_rep) * c->P);
-    c->step = DBuf<uint32_t>(P, n_rep);
+    c->rep_step = DBuf<uint32_t>(P, n_rep + 1);
+    ck(cudaMemsetAsync(c->rep_step.p, 0, sizeof(uint32_t) * (n_rep + 1), st), "memset");
     ck(cudaStreamSynchronize(st), "calibration upload");
     *out = c.release();
   });
@@ -2211,8 +2241,7 @@ pg_status pg_calib_nll_grad(pg_calib* c, const float* params, float* nll, float*
     require(c && params, "NULL argument");
     ck(cudaSetDevice(c->device), "cudaSetDevice");
     pg::AdamArgs no{};
-    pg::calib_launch(c->args(), const_cast<float*>(params), c->chunk_rep.p, c->chunk_start.p, c->n_chunks,
-                     c->rep_first_chunk.p, c->n_rep, c->partial.p, nll, grad, no, c->st);
+    pg::calib_launch(c->args(), c->n_segs, c->n_rep, const_cast<float*>(params), nll, grad, no, c->st);
     ck(cudaGetLastError(), "calibration kernels");
   });
 }
@@ -2223,12 +2252,12 @@ pg_status pg_calib_nll_grad_one(pg_calib* c, uint32_t rep, const float* params, 
     require(rep < c->n_rep, "replicate out of range");
     ck(cudaSetDevice(c->device), "cudaSetDevice");
     pg::CalibArgs a = c->args();
-    a.chunk0 = c->rep_first_chunk_h[rep];
+    a.seg0 = c->rep_first_seg_h[rep];
     a.rep0 = rep;
+    a.tab = nullptr;                   // few segments
     pg::AdamArgs no{};
-    pg::calib_launch(a, const_cast<float*>(params), c->chunk_rep.p, c->chunk_start.p,
-                     c->rep_first_chunk_h[rep + 1] - c->rep_first_chunk_h[rep], c->rep_first_chunk.p, 1,
-                     c->partial.p, nll, grad, no, c->st);
+    pg::calib_launch(a, c->rep_first_seg_h[rep + 1] - c->rep_first_seg_h[rep], 1, const_cast<float*>(params), nll, grad,
+                     no, c->st);
     ck(cudaGetLastError(), "calibration kernels");
   });
 }
@@ -2243,19 +2272,30 @@ pg_status pg_calib_adam(pg_calib* c, float* params, uint32_t steps, float lr, fl
     cudaStream_t st = c->st;
     ck(cudaMemsetAsync(c->m.p, 0, sizeof(float) * c->n_rep * c->P, st), "memset");
     ck(cudaMemsetAsync(c->v.p, 0, sizeof(float) * c->n_rep * c->P, st), "memset");
-    ck(cudaMemsetAsync(c->step.p, 0, sizeof(uint32_t) * c->n_rep, st), "memset");
+    if (!c->split && steps > 1) {
+      // every step in one launch, whose CTAs are resident together
+      pg::CalibArgs a = c->args();
+      a.steps = steps;
+      a.rep_step = c->rep_step.p;
+      a.status = c->rep_step.p + c->n_rep;
+      ck(cudaMemsetAsync(c->rep_step.p, 0, sizeof(uint32_t) * (c->n_rep + 1), st), "memset");
+      pg::calib_launch(a, c->n_segs, c->n_rep, params, nll, nullptr, pg::AdamArgs{c->m.p, c->v.p, 0, lr, beta1, beta2, eps}, st);
+      // (zero already, unless a wait ran out)
+      ck(cudaMemsetAsync(c->rep_done.p, 0, sizeof(uint32_t) * c->n_rep, st), "memset");
+      ck(cudaGetLastError(), "calibration steps");
+      return;
+    }
     const bool same = c->graph && c->gkey.params == params && c->gkey.steps == steps && c->gkey.lr == lr &&
                       c->gkey.b1 == beta1 && c->gkey.b2 == beta2 && c->gkey.eps == eps && c->gkey.nll == nll &&
                       c->gkey.st == st;
     if (!same) {
       if (c->graph) { cudaGraphExecDestroy(c->graph); c->graph = nullptr; }
-      pg::AdamArgs ad{c->m.p, c->v.p, c->step.p, lr, beta1, beta2, eps};
+      pg::AdamArgs ad{c->m.p, c->v.p, 0, lr, beta1, beta2, eps};
       cudaGraph_t g = nullptr;
       const uint64_t counted = g_launches.load();   // captured kernels are not launches yet
       ck(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "begin capture");
-      for (uint32_t s = 0; s < steps; ++s)
-        pg::calib_launch(c->args(), params, c->chunk_rep.p, c->chunk_start.p, c->n_chunks, c->rep_first_chunk.p,
-                         c->n_rep, c->partial.p, s + 1 == steps ? nll : nullptr, nullptr, ad, st);
+      for (uint32_t s = 0; s < steps; ++s, ad.t = s)
+        pg::calib_launch(c->args(), c->n_segs, c->n_rep, params, s + 1 == steps ? nll : nullptr, nullptr, ad, st);
       const cudaError_t ce = cudaStreamEndCapture(st, &g);
       ck(ce, "end capture");
       const cudaError_t ie = cudaGraphInstantiate(&c->graph, g, 0);
@@ -2265,7 +2305,7 @@ pg_status pg_calib_adam(pg_calib* c, float* params, uint32_t steps, float lr, fl
       g_launches.store(counted);
     }
     ck(cudaGraphLaunch(c->graph, st), "graph launch");
-    pg::note_launch(2 * steps);
+    pg::note_launch(c->split ? 3 * steps : steps);
     ck(cudaGetLastError(), "calibration graph");
   });
 }

@@ -1,0 +1,547 @@
+// Expected-VAF binomial-mixture likelihood of an alt/depth table and its
+// adjoint, batched over replicates (no reference counterpart: ProCESS has no
+// calibration path; this is the differentiable form of the sequencing output
+// used to fit epoch rates, exposures and purity to observed VAFs).
+//
+// Model of replicate r with K epochs, J signatures S_j over C classes:
+//   w_k      = softmax(theta_k)                   (exposures of epoch k)
+//   M_k(c)   = sum_j w_kj S_j(c)
+//   pi_k(c)  = exp(lr_k) L_k M_k(c) / Z,   Z = sum_k exp(lr_k) L_k
+//   v_k      = sigmoid(rho) phi_k / 2              (expected VAF of epoch k)
+//   NLL      = - sum_i log sum_k pi_k(c_i) v_k^a_i (1 - v_k)^(d_i - a_i)
+// (the binomial coefficient, constant in the parameters, is left out).
+// Parameters per replicate, in order: lr_0..K-1, theta_00..theta_K-1,J-1, rho.
+//
+// The kernel is k_calib, one CTA per segment: a replicate's sites are cut into
+// equal segments of at most CALIB_SEG sites, smaller ones where that fills the
+// GPU.  A CTA computes the per-site log-likelihoods and responsibilities in
+// FP32 with the replicate's constants and mixture weights in registers and
+// only the site class's signature row S(c) gathered from shared memory:
+//   u_k = log(exp(lr_k) L_k / Z) + a log v_k + (d - a) log(1 - v_k)
+//   e_k = exp(u_k - max u),  q_k = M_k(c) e_k,  s = sum_k q_k
+//   gamma_k = q_k / s,  log-likelihood = max u + log s
+// and reduces
+//   G_k = sum_i gamma_ik,  A_k = sum gamma_ik a_i,  B_k = sum gamma_ik (d_i - a_i),
+//   H_kj = sum_i gamma_ik S_j(c_i) / M_k(c_i) = sum_i e_ik S_j(c_i) / s_i,  NLL
+// (H carries the class dependence of the exposure gradient, so no per-class
+// bins are needed) with per-thread FP32 sums over the thread's sites in
+// order, a fixed warp tree and a Neumaier-compensated sum over the warps.  A
+// replicate's segments are then added in a fixed order (compensated) and the
+// chain rule applied, optionally followed by an Adam step on the parameters.
+// Every sum has a fixed order: results are deterministic.
+//
+// While all segments are resident together, one launch does it all: each CTA
+// derives its replicate's constants and the one that finishes a replicate's
+// last segment runs its epilogue.  An evaluation of 2e5 sites took 24.7 us with
+// separate kernels (and 13 CTAs of 16384 sites), now 10.8.  Adam steps repeat
+// inside that launch, each replicate going on when its epilogue is through:
+// 200 steps over 64 x 5e4 sites took 5.4 ms as a graph of three kernels a step,
+// 3.4 ms now.  With more segments than that, the constants and the
+// epilogues are launches of their own (in k_calib they keep a CTA's slot from
+// the next segment): 512 x 1e5 sites in 147 us.
+// Persistent CTAs with equal shares of all sites took 190 us there: they reach
+// their reductions together instead of overlapping them.
+#pragma once
+#include <cstdint>
+
+#include "pg_kernels.h"
+
+namespace pg {
+
+constexpr int CAL_THREADS = 256;
+constexpr int CAL_WARPS = CAL_THREADS / 32;
+constexpr uint32_t CAL_MAXK = 8, CAL_MAXJ = 8, CAL_MAXC = 128;
+constexpr uint32_t CAL_SPIN_LIMIT = 1u << 22;   // polls of a wait, 64 ns or more each
+
+struct Neu {   // Neumaier-compensated FP32 sum
+  float s = 0.f, c = 0.f;
+  __device__ __forceinline__ void add(float x) {
+    const float t = s + x;
+    c += (fabsf(s) >= fabsf(x)) ? ((s - t) + x) : ((x - t) + s);
+    s = t;
+  }
+  __device__ __forceinline__ float value() const { return s + c; }
+  __device__ __forceinline__ float2 both() const {   // the value and what its rounding leaves
+    const float v = s + c;
+    return make_float2(v, (s - v) + c);
+  }
+};
+
+// A replicate's parameters and constants in shared memory (one round of loads
+// for all of them), then by the threads k < K: log(exp(lr_k) L_k / Z) (K),
+// log v_k (K), log(1 - v_k) (K), the exposures w_kj (K x J).
+template <uint32_t K, uint32_t J>
+struct CalibRow {
+  float p[K + K * J + 1], ew[K], phi[K];
+  float row[3 * K + K * J];
+};
+template <uint32_t K, uint32_t J>
+__device__ __forceinline__ void calib_tables(CalibRow<K, J>& sh, const CalibArgs& a, const float* __restrict__ params,
+                                             uint32_t r) {
+  constexpr uint32_t P = K + K * J + 1;
+  const uint32_t t = threadIdx.x;
+  if (t < P) sh.p[t] = __ldcg(params + uint64_t(r) * P + t);   // (another SM may have written them)
+  else if (t >= 128 && t < 128 + K) sh.ew[t - 128] = a.epoch_w[r * K + t - 128];
+  else if (t >= 160 && t < 160 + K) sh.phi[t - 160] = a.phi[r * K + t - 160];
+  __syncthreads();
+  if (t < K) {
+    float Z = 0.f;
+#pragma unroll
+    for (uint32_t q = 0; q < K; ++q) Z += expf(sh.p[q]) * sh.ew[q];
+    sh.row[t] = sh.p[t] + logf(sh.ew[t]) - logf(Z);
+  } else if (t >= 32 && t < 32 + K) {
+    const uint32_t k = t - 32;
+    const float sig = 1.f / (1.f + expf(-sh.p[K + K * J]));
+    const float v = sig * sh.phi[k] * 0.5f;
+    sh.row[K + k] = logf(v);
+    sh.row[2 * K + k] = log1pf(-v);
+  } else if (t >= 64 && t < 64 + K) {
+    const uint32_t k = t - 64;
+    const float* th = sh.p + K + k * J;
+    float mx = th[0];
+#pragma unroll
+    for (uint32_t j = 1; j < J; ++j) mx = fmaxf(mx, th[j]);
+    float den = 0.f;
+#pragma unroll
+    for (uint32_t j = 0; j < J; ++j) den += expf(th[j] - mx);
+#pragma unroll
+    for (uint32_t j = 0; j < J; ++j) sh.row[3 * K + k * J + j] = expf(th[j] - mx) / den;
+  }
+  __syncthreads();
+}
+
+// Per-site work: every thread takes sites i0 + tid, i0 + tid + 256, ...
+// (coalesced, four sites' loads in flight at a time) and keeps plain FP32
+// sums over its sites, in site order.  The signature rows in shared memory
+// are JP floats (J rounded up to 4 or 8, zero beyond J).
+// packed f32x2 arithmetic (two lanes of one 64-bit register pair, each
+// rounded as the scalar operation)
+__device__ __forceinline__ float2 f2fma(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
+      "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+// four values read once: not kept in L1
+__device__ __forceinline__ int4 load4(const int4* p) {
+  int4 v;
+  asm("ld.global.nc.L1::no_allocate.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+// base-2 exponential and logarithm (the PTX approximate instructions, FTZ)
+__device__ __forceinline__ float ex2_approx(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float lg2_approx(float x) {
+  float y;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+#define PG_F2OP(NAME, OP)                                                                                        \
+  __device__ __forceinline__ float2 NAME(float2 a, float2 b) {                                                \
+    float2 d;                                                                                                  \
+    asm("{\n\t.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t" OP " rd, ra, rb;\n\t" \
+        "mov.b64 {%0, %1}, rd;\n\t}"                                                                          \
+        : "=f"(d.x), "=f"(d.y)                                                                                 \
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));                                                             \
+    return d;                                                                                                  \
+  }
+PG_F2OP(f2mul, "mul.rn.f32x2")
+PG_F2OP(f2add, "add.rn.f32x2")
+#undef PG_F2OP
+
+// CTAs per SM asked of the register allocator: the per-thread constants and
+// sums take about 1 + 6K + 2KJ registers, plus K of per-site temporaries
+// (4 CTAs, 64 registers, for the small shapes whose sums fit: 5% faster at
+// K = 4, J = 3 than 3 CTAs)
+constexpr uint32_t calib_min_blocks(uint32_t K, uint32_t J) {
+  return (K + K % 2) * (J + 4) <= 28 && J <= 7 ? 4
+         : 1 + 7 * K + 2 * K * J <= 53        ? 3
+         : 1 + 7 * K + 2 * K * J <= 96        ? 2
+                                              : 1;
+}
+
+// sum of v[x] over the warp for x < N (N <= 32): lane x ends with the sum of
+// v[x].  Each step sends the half of the values the partner keeps: 31
+// shuffles for 32 values instead of 160.
+template <uint32_t N>
+__device__ __forceinline__ float warp_transpose_sum(const float* v, uint32_t lane) {
+  float w[32];
+#pragma unroll
+  for (uint32_t x = 0; x < 32; ++x) w[x] = x < N ? v[x] : 0.f;
+#pragma unroll
+  for (uint32_t h = 16; h >= 1; h >>= 1) {
+    const bool up = (lane & h) != 0;
+#pragma unroll
+    for (uint32_t x = 0; x < h; ++x) {
+      if (x >= N) continue;                 // both halves are padding
+      const float send = up ? w[x] : w[x + h], keep = up ? w[x + h] : w[x];
+      w[x] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+    }
+  }
+  return w[0];
+}
+
+// a replicate's segment sums -> NLL and gradient (-> Adam step), by the CTA
+// that finished its last segment
+struct CalibEpilogue {
+  float grp[CAL_THREADS / 32][1 + 3 * CAL_MAXK + CAL_MAXK * CAL_MAXJ][2];
+  float2 tot[1 + 3 * CAL_MAXK + CAL_MAXK * CAL_MAXJ];
+  float grad[CAL_MAXK + CAL_MAXK * CAL_MAXJ + 1];
+};
+template <uint32_t K, uint32_t J>
+__device__ __forceinline__ void calib_epilogue(CalibEpilogue& sh, const CalibRow<K, J>& c, const CalibArgs& a,
+                                               float* __restrict__ params, uint32_t r, const float2* partial, float* __restrict__ nll_out,
+                                               float* __restrict__ grad_out, const AdamArgs& adam,
+                                               uint32_t step) {
+  constexpr uint32_t P = K + K * J + 1, NV = 1 + 3 * K + K * J;
+  const uint32_t c0 = a.rep_first_seg[r], c1 = a.rep_first_seg[r + 1];
+  // warp g takes segments c0 + g, c0 + g + 8, ..., a lane one value (or three);
+  // then the warps' sums in order
+  const uint32_t lane = threadIdx.x & 31u, g = threadIdx.x >> 5;
+  for (uint32_t x = lane; x < NV; x += 32) {
+    Neu t;
+#pragma unroll 4
+    for (uint32_t q = c0 + g; q < c1; q += CAL_WARPS) {
+      const float2 y = __ldcg(partial + uint64_t(q) * a.part_stride + x);
+      t.add(y.x);
+      t.c += y.y;
+    }
+    sh.grp[g][x][0] = t.s;
+    sh.grp[g][x][1] = t.c;
+  }
+  __syncthreads();
+  for (uint32_t x = threadIdx.x; x < NV; x += CAL_THREADS) {
+    Neu t;
+    for (uint32_t w = 0; w < CAL_WARPS; ++w) { t.add(sh.grp[w][x][0]); t.c += sh.grp[w][x][1]; }
+    sh.tot[x] = t.both();
+  }
+  __syncthreads();
+  // the gradient is a difference of sums that nearly cancel: the sums keep the
+  // remainders of their rounding, and products enter unrounded (fma)
+  const float2* G = sh.tot + 1 + 2 * K;
+  const float2* H = sh.tot + 1 + 3 * K;
+  // d/d lr_k = -G_k + N r_k L_k / Z   (N = sum_k G_k = number of sites)
+  if (threadIdx.x < K) {
+    const uint32_t k = threadIdx.x;
+    float Z = 0.f;
+    Neu N;
+#pragma unroll
+    for (uint32_t q = 0; q < K; ++q) { Z += expf(c.p[q]) * c.ew[q]; N.add(G[q].x); N.c += G[q].y; }
+    const float2 n = N.both();
+    const float pk = expf(c.p[k]) * c.ew[k] / Z;
+    sh.grad[k] = __fmaf_rn(n.x, pk, -G[k].x) + (n.y * pk - G[k].y);
+  }
+  if (threadIdx.x == 32) {
+    // d/d rho = -(1 - sigma) sum_k (A_k - B_k v_k / (1 - v_k))
+    const float sig = 1.f / (1.f + expf(-c.p[K + K * J]));
+    float acc = 0.f;
+#pragma unroll
+    for (uint32_t k = 0; k < K; ++k) {
+      const float v = sig * c.phi[k] * 0.5f, odds = v / (1.f - v);
+      acc += __fmaf_rn(-sh.tot[1 + K + k].x, odds, sh.tot[1 + k].x) + (sh.tot[1 + k].y - sh.tot[1 + K + k].y * odds);
+    }
+    sh.grad[K + K * J] = -(1.f - sig) * acc;
+  }
+  // d/d theta_kj = -w_kj (sum_i gamma_ik S_j(c_i) / M_k(c_i) - G_k) = -w_kj (H_kj - G_k)
+  if (threadIdx.x >= 64 && threadIdx.x < 64 + K * J) {
+    const uint32_t x = threadIdx.x - 64;
+    sh.grad[K + x] = -c.row[3 * K + x] * ((H[x].x - G[x / J].x) + (H[x].y - G[x / J].y));
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && nll_out) nll_out[r] = sh.tot[0].x;
+  for (uint32_t q = threadIdx.x; q < P; q += CAL_THREADS) {
+    const float gq = sh.grad[q];
+    if (grad_out) grad_out[uint64_t(r) * P + q] = gq;
+    if (adam.m) {   // Adam step `step` (from 0) on the parameters (bias-corrected)
+      const uint64_t o = uint64_t(r) * P + q;
+      const float t = float(step + 1);
+      const float m = adam.beta1 * __ldcg(adam.m + o) + (1.f - adam.beta1) * gq;
+      const float v = adam.beta2 * __ldcg(adam.v + o) + (1.f - adam.beta2) * gq * gq;
+      adam.m[o] = m; adam.v[o] = v;
+      const float mh = m / (1.f - powf(adam.beta1, t)), vh = v / (1.f - powf(adam.beta2, t));
+      params[o] = c.p[q] - adam.lr * mh / (sqrtf(vh) + adam.eps);
+    }
+  }
+}
+
+// STEPS: a.steps Adam steps in a cooperative launch (an instance of its own: in
+// the other the step's state would spill)
+template <uint32_t K, uint32_t J, bool STEPS>
+__global__ void __launch_bounds__(CAL_THREADS, calib_min_blocks(K, J)) k_calib(CalibArgs a, float* __restrict__ params,
+                                                                               float* __restrict__ nll_out,
+                                                                               float* __restrict__ grad_out,
+                                                                               AdamArgs adam) {
+  constexpr uint32_t JP = J > 4 ? 8 : 4;
+  constexpr uint32_t NV = 1 + 3 * K + K * J;   // nll, A, B, G, H
+  // signature rows, eight copies of each 16 bytes: a lane reads the copy in its
+  // own banks, so the gather is free of conflicts (one copy: 2.9 lanes a bank)
+  // The mixtures M_k(c) likewise, by class.
+  constexpr uint32_t KP = K > 4 ? 8 : 4;
+  __shared__ float4 s_sig[JP / 4][CAL_MAXC * 8], s_mix[KP / 4][CAL_MAXC * 8];
+  __shared__ CalibRow<K, J> s_c;
+  __shared__ union { float red[CAL_WARPS][NV]; CalibEpilogue epi; } s_u;
+  __shared__ uint32_t s_go, s_step;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t seg = a.seg0 + blockIdx.x, r = a.seg_rep[seg];
+  const uint64_t i0 = a.seg_start[seg], i1 = i0 + a.seg_len[seg];
+  if (STEPS && threadIdx.x == 0) s_step = 0;
+  for (;;) {   // a.steps evaluations (STEPS), or one
+  if (!STEPS && a.tab) {
+    for (uint32_t x = threadIdx.x; x < 3 * K + K * J; x += CAL_THREADS) s_c.row[x] = a.tab[uint64_t(r) * a.part_stride + x];
+    __syncthreads();
+  } else {
+    calib_tables<K, J>(s_c, a, params, r);
+  }
+  const float* s_row = s_c.row;
+  for (uint32_t x = threadIdx.x; x < a.C * 8; x += CAL_THREADS) {
+    float sg[JP], m[KP];
+#pragma unroll
+    for (uint32_t j = 0; j < JP; j += 4) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(a.sig_rows) + ((x >> 3) * JP + j) / 4);
+      s_sig[j / 4][x] = v;
+      sg[j] = v.x; sg[j + 1] = v.y; sg[j + 2] = v.z; sg[j + 3] = v.w;
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < KP; ++k) {
+      m[k] = 0.f;
+      if (k < K) {
+        m[k] = s_row[3 * K + k * J] * sg[0];
+#pragma unroll
+        for (uint32_t j = 1; j < J; ++j) m[k] = __fmaf_rn(s_row[3 * K + k * J + j], sg[j], m[k]);
+      }
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < KP; k += 4) s_mix[k / 4][x] = make_float4(m[k], m[k + 1], m[k + 2], m[k + 3]);
+  }
+  __syncthreads();
+  // epochs in pairs (packed f32x2 arithmetic); an odd K gets a padding
+  // epoch of weight exp(-inf) = 0
+  constexpr uint32_t KH = (K + 1) / 2;
+  float2 cst[KH], dlv[KH], l1v[KH];
+  auto at = [&](uint32_t k, uint32_t off, float pad) { return k < K ? s_row[off + k] : pad; };
+  // the log-domain terms in base 2 (ex2 / lg2 directly, the NLL scaled back by ln 2)
+  constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
+#pragma unroll
+  for (uint32_t h = 0; h < KH; ++h) {
+    cst[h] = make_float2(LOG2E * at(2 * h, 0, 0.f), at(2 * h + 1, 0, -INFINITY) * LOG2E);
+    // u_k = cst_k + a log v_k + (d - a) log(1 - v_k) = cst_k + a dlv_k + d l1v_k
+    l1v[h] = make_float2(LOG2E * at(2 * h, 2 * K, 0.f), LOG2E * at(2 * h + 1, 2 * K, 0.f));
+    dlv[h] = make_float2(LOG2E * at(2 * h, K, 0.f) - l1v[h].x, LOG2E * at(2 * h + 1, K, 0.f) - l1v[h].y);
+  }
+  float nll = 0.f;
+  float2 A[KH], D[KH], G[KH], H[J][KH];   // D_k = sum gamma_ik d_i (B_k = D_k - A_k)
+#pragma unroll
+  for (uint32_t h = 0; h < KH; ++h) {
+    A[h] = D[h] = G[h] = make_float2(0.f, 0.f);
+#pragma unroll
+    for (uint32_t j = 0; j < J; ++j) H[j][h] = make_float2(0.f, 0.f);
+  }
+  auto site = [&](float al, float dl, int32_t c) {
+    const uint32_t row = uint32_t(c) * 8 + (threadIdx.x & 7u);
+    float sg[JP];
+#pragma unroll
+    for (uint32_t j = 0; j < JP; j += 4) {
+      const float4 x = s_sig[j / 4][row];
+      sg[j] = x.x; sg[j + 1] = x.y; sg[j + 2] = x.z; sg[j + 3] = x.w;
+    }
+    float2 m[(KP + 1) / 2];
+#pragma unroll
+    for (uint32_t k = 0; k < KP; k += 4) {
+      const float4 x = s_mix[k / 4][row];
+      m[k / 2] = make_float2(x.x, x.y); m[k / 2 + 1] = make_float2(x.z, x.w);
+    }
+    const float2 al2 = make_float2(al, al), dl2 = make_float2(dl, dl);
+    float2 u[KH];
+    float umax = -INFINITY;
+#pragma unroll
+    for (uint32_t h = 0; h < KH; ++h) {
+      u[h] = f2fma(dl2, l1v[h], f2fma(al2, dlv[h], cst[h]));
+      umax = fmaxf(umax, fmaxf(u[h].x, u[h].y));
+    }
+    float2 e[KH], q[KH], s2;
+    const float2 nmax = make_float2(-umax, -umax);
+#pragma unroll
+    for (uint32_t h = 0; h < KH; ++h) {
+      const float2 z = f2add(u[h], nmax);
+      e[h] = make_float2(ex2_approx(z.x), ex2_approx(z.y));
+      q[h] = f2mul(m[h], e[h]);
+      s2 = h ? f2add(s2, q[h]) : q[h];
+    }
+    // a class that no epoch's mixture can emit (every M_k(c) = 0) keeps a
+    // finite, tiny sum
+    const float sum = fmaxf(s2.x + s2.y, 1e-30f);
+    const float inv = __fdividef(1.f, sum);
+    nll -= umax + lg2_approx(sum);
+    const float2 inv2 = make_float2(inv, inv);
+#pragma unroll
+    for (uint32_t h = 0; h < KH; ++h) {
+      const float2 g = f2mul(q[h], inv2), r = f2mul(e[h], inv2);
+      A[h] = f2fma(g, al2, A[h]);
+      D[h] = f2fma(g, dl2, D[h]);
+      G[h] = f2add(G[h], g);
+#pragma unroll
+      for (uint32_t j = 0; j < J; ++j) H[j][h] = f2fma(r, make_float2(sg[j], sg[j]), H[j][h]);
+    }
+  };
+  auto site_at = [&](uint64_t x) { site(float(__ldg(a.alt + x)), float(__ldg(a.depth + x)), __ldg(a.cls + x)); };
+  auto site4 = [&](const int4& x, const int4& y, const int4& z) {
+    site(float(x.x), float(y.x), z.x); site(float(x.y), float(y.y), z.y);
+    site(float(x.z), float(y.z), z.z); site(float(x.w), float(y.w), z.w);
+  };
+  {
+    // four consecutive sites per 16-byte load of each column (the columns
+    // are 16-byte aligned); the unaligned head [i0, v0) and tail [v1, i1)
+    // (under four sites each) site by site
+    const uint64_t v0 = min((i0 + 3) & ~uint64_t(3), i1), v1 = max(i1 & ~uint64_t(3), v0);
+    if (threadIdx.x < v0 - i0) site_at(i0 + threadIdx.x);
+    if (threadIdx.x < i1 - v1) site_at(v1 + threadIdx.x);
+    const int4* a4 = reinterpret_cast<const int4*>(a.alt) + v0 / 4;
+    const int4* d4 = reinterpret_cast<const int4*>(a.depth) + v0 / 4;
+    const int4* c4 = reinterpret_cast<const int4*>(a.cls) + v0 / 4;
+    const uint32_t n4 = uint32_t((v1 - v0) / 4);
+    // unrolled by three for the small shapes: 148 us for 512 x 1e5 sites (one
+    // group a turn 165, two 153, four 164: spills)
+#pragma unroll (K * J <= 16 ? 3 : 1)
+    for (uint32_t q = threadIdx.x; q < n4; q += CAL_THREADS) site4(load4(a4 + q), load4(d4 + q), load4(c4 + q));
+  }
+  // block partial: warp trees, then a compensated sum over the warps
+  float acc[NV];
+  acc[0] = nll * LN2;
+#pragma unroll
+  for (uint32_t k = 0; k < K; ++k) {
+    const bool hi = k & 1;
+    acc[1 + k] = hi ? A[k / 2].y : A[k / 2].x;
+    acc[1 + K + k] = hi ? D[k / 2].y - A[k / 2].y : D[k / 2].x - A[k / 2].x;
+    acc[1 + 2 * K + k] = hi ? G[k / 2].y : G[k / 2].x;
+#pragma unroll
+    for (uint32_t j = 0; j < J; ++j) acc[1 + 3 * K + k * J + j] = hi ? H[j][k / 2].y : H[j][k / 2].x;
+  }
+#pragma unroll
+  for (uint32_t q = 0; q < NV; q += 32) {
+    constexpr uint32_t tail = NV % 32 ? NV % 32 : 32;
+    const float v = q + 32 <= NV ? warp_transpose_sum<32>(acc + q, lane) : warp_transpose_sum<tail>(acc + q, lane);
+    if (q + lane < NV) s_u.red[warp][q + lane] = v;
+  }
+  __syncthreads();
+  // segment sums: nll, A_k, B_k, G_k, H_kj (j < J)
+  float2* out = a.partial + uint64_t(seg) * a.part_stride;
+  for (uint32_t x = threadIdx.x; x < NV; x += CAL_THREADS) {
+    Neu t;
+    for (uint32_t w = 0; w < CAL_WARPS; ++w) t.add(s_u.red[w][x]);
+    out[x] = t.both();
+  }
+  if (!STEPS && a.tab) return;
+  // the CTA that finishes the replicate's last segment runs the epilogue (the
+  // count is left at zero for the next evaluation)
+  __threadfence();
+  __syncthreads();
+  const uint32_t step = STEPS ? s_step : adam.t;
+  const bool end = !STEPS || step + 1 == a.steps;
+  if (threadIdx.x == 0) {
+    const uint32_t n = a.rep_first_seg[r + 1] - a.rep_first_seg[r];
+    s_go = atomicAdd(a.rep_done + r, 1u) + 1u == n ? 1u : 0u;
+    if (s_go) a.rep_done[r] = 0u;
+    __threadfence();
+  }
+  __syncthreads();
+  if (s_go) {
+    calib_epilogue<K, J>(s_u.epi, s_c, a, params, r, a.partial, end ? nll_out : nullptr, grad_out, adam, step);
+    __threadfence();
+  }
+  if (end) return;
+  __syncthreads();
+  // the next evaluation starts when the replicate's epilogue is through.  The
+  // CTAs are all resident (a cooperative launch); a wait that runs out all the
+  // same marks the call and every CTA leaves at its next look
+  if (threadIdx.x == 0) {
+    uint32_t go = 1;
+    if (s_go) {
+      atomicExch(a.rep_step + r, step + 1);
+    } else {
+      uint32_t polls = 0;
+      while (*reinterpret_cast<volatile uint32_t*>(a.rep_step + r) <= step) {
+        if (++polls > CAL_SPIN_LIMIT || *reinterpret_cast<volatile uint32_t*>(a.status)) { go = 0; break; }
+        __nanosleep(64);
+      }
+      __threadfence();
+      if (!go) atomicExch(a.status, 1u);
+    }
+    s_go = go;
+    s_step = step + 1;
+  }
+  __syncthreads();
+  if (!s_go) {
+    if (threadIdx.x == 0) {                    // no result: NaN
+      params[uint64_t(r) * (K + K * J + 1)] = __int_as_float(0x7fc00000);
+      if (nll_out) nll_out[r] = __int_as_float(0x7fc00000);
+    }
+    return;
+  }
+  }
+}
+
+// The constants and the epilogues in launches of their own, one CTA per
+// replicate (see calib_launch)
+template <uint32_t K, uint32_t J>
+__global__ void __launch_bounds__(CAL_THREADS) k_calib_tables(CalibArgs a, const float* __restrict__ params) {
+  __shared__ CalibRow<K, J> s_c;
+  const uint32_t r = a.rep0 + blockIdx.x;
+  calib_tables<K, J>(s_c, a, params, r);
+  for (uint32_t x = threadIdx.x; x < 3 * K + K * J; x += CAL_THREADS) a.tab[uint64_t(r) * a.part_stride + x] = s_c.row[x];
+}
+template <uint32_t K, uint32_t J>
+__global__ void __launch_bounds__(CAL_THREADS) k_calib_epilogue(CalibArgs a, float* __restrict__ params,
+                                                                float* __restrict__ nll_out,
+                                                                float* __restrict__ grad_out, AdamArgs adam) {
+  __shared__ CalibRow<K, J> s_c;
+  __shared__ CalibEpilogue s_epi;
+  const uint32_t r = a.rep0 + blockIdx.x;
+  calib_tables<K, J>(s_c, a, params, r);
+  calib_epilogue<K, J>(s_epi, s_c, a, params, r, a.partial, nll_out, grad_out, adam, adam.t);
+}
+
+template <uint32_t K, uint32_t J>
+static void calib_run(const CalibArgs& a, uint32_t n_segs, uint32_t n_rep, float* params, float* nll, float* grad,
+                      const AdamArgs& adam, cudaStream_t st) {
+  if (a.tab) k_calib_tables<K, J><<<n_rep, CAL_THREADS, 0, st>>>(a, params);
+  if (a.steps == 1) {
+    k_calib<K, J, false><<<n_segs, CAL_THREADS, 0, st>>>(a, params, nll, grad, adam);
+  } else {
+    CalibArgs aa = a;
+    AdamArgs ad = adam;
+    void* args[] = {&aa, &params, &nll, &grad, &ad};
+    cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_calib<K, J, true>), dim3(n_segs), dim3(CAL_THREADS), args, 0, st);
+  }
+  if (a.tab) k_calib_epilogue<K, J><<<n_rep, CAL_THREADS, 0, st>>>(a, params, nll, grad, adam);
+  note_launch(a.tab ? 3 : 1);
+}
+
+template <uint32_t K, uint32_t J>
+static int calib_resident() {
+  int n = 0, m = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_calib<K, J, false>, CAL_THREADS, 0) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, k_calib<K, J, true>, CAL_THREADS, 0) != cudaSuccess)
+    return 1;
+  n = n < m ? n : m;
+  return n > 0 ? n : 1;
+}
+
+#define PG_CALIB_J(KK, JJ) case KK * 8 + JJ - 9: PG_CALIB_DO(KK, JJ); break;
+#define PG_CALIB_K(KK) PG_CALIB_J(KK, 1) PG_CALIB_J(KK, 2) PG_CALIB_J(KK, 3) PG_CALIB_J(KK, 4) \
+                       PG_CALIB_J(KK, 5) PG_CALIB_J(KK, 6) PG_CALIB_J(KK, 7) PG_CALIB_J(KK, 8)
+
+// the launcher and the residency of the shapes with at most four epochs and
+// with more, in translation units of their own (they compile in parallel)
+void calib_launch_lo(const CalibArgs& a, uint32_t n_segs, uint32_t n_rep, float* params, float* nll, float* grad,
+                     const AdamArgs& adam, cudaStream_t st);
+void calib_launch_hi(const CalibArgs& a, uint32_t n_segs, uint32_t n_rep, float* params, float* nll, float* grad,
+                     const AdamArgs& adam, cudaStream_t st);
+int calib_ctas_lo(uint32_t K, uint32_t J);
+int calib_ctas_hi(uint32_t K, uint32_t J);
+
+}  // namespace pg

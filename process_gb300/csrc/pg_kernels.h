@@ -400,28 +400,36 @@ void seq_reads(const SeqRec* recs, uint32_t n_recs, const SeqTiles& tiles, const
 // ---------------------------------------------------------------- calibration
 struct CalibArgs {
   uint32_t K, J, C, P;          // epochs, signatures, classes, parameters per replicate
-  const int32_t* alt;           // sites of all replicates, concatenated
+  const int32_t* alt;           // sites of all replicates, concatenated (16-byte aligned columns)
   const int32_t* depth;
   const int32_t* cls;
-  const uint64_t* site_off;     // n_rep + 1
-  const float* sig;             // J x C
   const float* epoch_w;         // n_rep x K  (L_k: relative length of epoch k)
   const float* phi;             // n_rep x K  (mean cellular fraction of epoch-k mutations)
-  uint32_t chunk;               // sites per CTA
-  uint32_t part_stride;         // floats per chunk partial (>= 1 + 3K + K J)
-  uint32_t chunk0, rep0;        // first chunk / replicate of a launch (sub-range launches)
   const float* sig_rows;        // C x JP: S_j(c) by class, JP = 4 (J <= 4) or 8 floats, zero beyond J
-  float* tab;                   // per replicate: log(exp(lr_k) L_k / Z), log v_k, log(1 - v_k), w_kj
-  uint32_t tab_stride;          // floats per replicate in tab
+  // segments: sites [seg_start, + seg_len) of replicate seg_rep, in order (a
+  // replicate without sites has one empty segment)
+  const uint32_t* seg_rep;
+  const uint64_t* seg_start;
+  const uint32_t* seg_len;
+  const uint32_t* rep_first_seg;  // n_rep + 1
+  uint32_t* rep_done;             // n_rep counts, zero between launches
+  float2* partial;                // per segment, part_stride sums (>= 1 + 3K + K J) and their remainders
+  uint32_t part_stride;
+  uint32_t seg0, rep0;            // first segment and replicate of the launch
+  uint32_t steps;                 // evaluations of the launch (above 1: Adam steps, without tab)
+  uint32_t* rep_step;             // with steps > 1, zeroed: steps done per replicate
+  uint32_t* status;               // set when a wait between the steps ran out
+  float* tab;                     // per replicate, part_stride floats: its constants, where they and the
+                                  //   epilogues have launches of their own; else NULL
 };
 struct AdamArgs {               // m == nullptr: no optimizer step
-  float* m; float* v; uint32_t* step;
+  float* m; float* v;
+  uint32_t t;                   // the step's number, from 0 (launches of one step)
   float lr, beta1, beta2, eps;
 };
-// k_calib_sites over chunks [a.chunk0, a.chunk0 + n_chunks), then the
-// epilogue for replicates [a.rep0, a.rep0 + n_rep)
-void calib_launch(const CalibArgs& a, float* params, const uint32_t* chunk_rep, const uint64_t* chunk_start,
-                  uint32_t n_chunks, const uint32_t* rep_first_chunk, uint32_t n_rep, float* partial, float* nll,
-                  float* grad, const AdamArgs& adam, cudaStream_t st);
+// one evaluation over the segments [a.seg0, a.seg0 + n_segs): whole replicates
+void calib_launch(const CalibArgs& a, uint32_t n_segs, uint32_t n_rep, float* params, float* nll, float* grad,
+                  const AdamArgs& adam, cudaStream_t st);
+int calib_ctas_per_sm(uint32_t K, uint32_t J);   // resident CTAs of the evaluation kernel
 
 }  // namespace pg
