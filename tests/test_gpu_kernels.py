@@ -149,3 +149,25 @@ def test_edge_counts(gpu_lib, orc, rate):
         ot = o.place(f, sp, 3, 0, 2, 0, seed=seed).table()
         np.testing.assert_array_equal(t["edge"], ot["edge"])
         np.testing.assert_array_equal(t["locus"], ot["locus"])
+
+
+@pytest.mark.parametrize("sampling,max_rep", [(1, 1), (1, 40), (2, 1000), (7, 500_000), (1023, 3), (1024, 100), (5000, 17)])
+def test_index_strides(gpu_lib, orc, sampling, max_rep):
+    """Position lists at strides from 1 to beyond a round of the emit pass,
+    over repeats, chromosomes that start and end inside a round, and unknown
+    stretches."""
+    from process_gb300 import GenomeSpec, MutationEngine
+    rng = np.random.default_rng(sampling)
+    lengths = [9_001, 31, 4_097, 1, 20_000]
+    bases = rng.integers(0, 4, sum(lengths)).astype(np.uint8)
+    bases[500:900] = 2                                     # long runs and short repeats
+    bases[5_000:6_000] = np.tile([0, 3], 500)
+    bases[12_000:14_000] = np.resize([1, 0, 2, 2, 3], 2_000)
+    bases[3_000:3_100] = 4
+    bases[13_100] = 4
+    g = GenomeSpec(["a", "b", "c", "d", "e"], lengths, bases=bases)
+    eng = MutationEngine(g, context_sampling=sampling, max_repetition_storage=max_rep)
+    o = orc.OracleEngine(lengths, bases, context_sampling=sampling, max_rep=max_rep)
+    for which, n in ((0, 32), (1, 83)):
+        for k in range(n):
+            np.testing.assert_array_equal(eng.read_index(which, k), o.read_index(which, k), err_msg=f"{which} {k}")
