@@ -66,7 +66,10 @@ void require(bool c, const char* msg) { if (!c) throw DomainError(msg); }
 
 // ---------------------------------------------------------------- device memory
 // A small caching pool: freed blocks are kept per engine and reused by size,
-// so repeated place/sequence calls do not pay cudaMalloc/cudaFree.
+// so repeated place/sequence calls do not pay cudaMalloc/cudaFree.  Blocks of
+// up to 2 MB are cut from slabs of 2 to 16 MB: an engine with an index takes
+// some 60 of them, at 3 us (100 us from 1 MB on) for each cudaMalloc and as
+// much again to free them.
 class Pool {
  public:
   ~Pool() { release_all(); }
@@ -75,41 +78,78 @@ class Pool {
     bytes = (bytes + 255) & ~size_t(255);
     auto it = free_.lower_bound(bytes);
     if (it != free_.end() && it->first <= 2 * bytes) {
-      void* p = it->second;
-      sizes_[p] = it->first;
+      const Free f = it->second;
+      used_[f.p] = {it->first, f.slab};
+      if (f.slab != OWN) ++slabs_[f.slab].live;
       free_.erase(it);
+      return f.p;
+    }
+    if (bytes <= SLAB_MAX_BLOCK) {
+      if (cur_ == OWN || slabs_[cur_].size - slabs_[cur_].used < bytes) {
+        Slab s;
+        s.size = std::min<size_t>(size_t(2) << 20 << std::min<size_t>(slabs_.size(), 3), size_t(16) << 20);
+        s.p = static_cast<char*>(allocate(s.size));
+        slabs_.push_back(s);
+        cur_ = uint32_t(slabs_.size() - 1);
+      }
+      Slab& s = slabs_[cur_];
+      void* p = s.p + s.used;
+      used_[p] = {bytes, cur_};
+      s.used += bytes;
+      ++s.live;
       return p;
     }
-    void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, bytes);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      release_free();
-      ck(cudaMalloc(&p, bytes), "cudaMalloc");
-    }
-    sizes_[p] = bytes;
+    void* p = allocate(bytes);
+    used_[p] = {bytes, OWN};
     return p;
   }
   void put(void* p) {
     if (!p) return;
-    auto it = sizes_.find(p);
-    if (it == sizes_.end()) return;
-    free_.emplace(it->second, p);
-    sizes_.erase(it);
+    auto it = used_.find(p);
+    if (it == used_.end()) return;
+    const Block b = it->second;
+    free_.emplace(b.size, Free{p, b.slab});
+    if (b.slab != OWN) --slabs_[b.slab].live;
+    used_.erase(it);
   }
+  // gives back every free block, and the slabs none of whose blocks are in use
   void release_free() {
-    for (auto& kv : free_) cudaFree(kv.second);
-    free_.clear();
+    for (auto it = free_.begin(); it != free_.end();) {
+      const Free f = it->second;
+      if (f.slab != OWN && slabs_[f.slab].live) { ++it; continue; }
+      if (f.slab == OWN) cudaFree(f.p);
+      it = free_.erase(it);
+    }
+    for (Slab& s : slabs_)
+      if (!s.live && s.p) { cudaFree(s.p); s = Slab(); }
   }
   void release_all() {
-    release_free();
-    for (auto& kv : sizes_) cudaFree(kv.first);
-    sizes_.clear();
+    for (auto& kv : free_) if (kv.second.slab == OWN) cudaFree(kv.second.p);
+    for (auto& kv : used_) if (kv.second.slab == OWN) cudaFree(kv.first);
+    for (Slab& s : slabs_) if (s.p) cudaFree(s.p);
+    free_.clear(); used_.clear(); slabs_.clear();
+    cur_ = OWN;
   }
 
  private:
-  std::multimap<size_t, void*> free_;
-  std::map<void*, size_t> sizes_;
+  static constexpr uint32_t OWN = 0xffffffffu;             // a block with an allocation of its own
+  static constexpr size_t SLAB_MAX_BLOCK = size_t(2) << 20;
+  struct Slab { char* p = nullptr; size_t size = 0, used = 0; uint32_t live = 0; };
+  struct Block { size_t size; uint32_t slab; };
+  struct Free { void* p; uint32_t slab; };
+  void* allocate(size_t bytes) {
+    void* p = nullptr;
+    if (cudaMalloc(&p, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      release_free();
+      ck(cudaMalloc(&p, bytes), "cudaMalloc");
+    }
+    return p;
+  }
+  std::vector<Slab> slabs_;
+  uint32_t cur_ = OWN;                                     // the slab blocks are cut from
+  std::multimap<size_t, Free> free_;
+  std::map<void*, Block> used_;
 };
 
 template <class T>
@@ -136,6 +176,52 @@ DBuf<T> upload(Pool* pool, const std::vector<T>& v, cudaStream_t st) {
   if (!v.empty()) ck(cudaMemcpyAsync(b.p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, st), "upload");
   return b;
 }
+
+// The small tables of a call, sent to the device together.  add() hands out a
+// table's device buffer and keeps its bytes, send() copies what was added
+// since the last send(); the buffers are parts of one block that lives as
+// long as the Stage (or its owner, after take()).  A copy of a few hundred
+// bytes from pageable memory takes the host and the stream 2 to 4 us whatever
+// its size, and a placement or sequencing call has some 20 of them.  Larger
+// tables are copied on their own, straight from the vector.
+class Stage {
+ public:
+  Stage(Pool* pool, cudaStream_t st) : pool_(pool), st_(st) {}
+  template <class T>
+  DBuf<T> add(const std::vector<T>& v) {
+    const size_t bytes = (sizeof(T) * std::max<size_t>(v.size(), 1) + 255) & ~size_t(255);
+    if (bytes > MAX_TABLE) return upload(pool_, v, st_);
+    if (blocks_.empty() || host_.size() + bytes > BLOCK) {
+      send();
+      host_.clear();
+      sent_ = 0;
+      host_.reserve(BLOCK);
+      blocks_.emplace_back(pool_, BLOCK);
+    }
+    DBuf<T> b;                       // no pool: the block is the Stage's
+    b.p = reinterpret_cast<T*>(blocks_.back().p + host_.size());
+    b.n = v.size();
+    const size_t at = host_.size();
+    host_.resize(at + bytes);
+    if (!v.empty()) std::memcpy(host_.data() + at, v.data(), sizeof(T) * v.size());
+    return b;
+  }
+  void send() {
+    if (host_.size() > sent_)
+      ck(cudaMemcpyAsync(blocks_.back().p + sent_, host_.data() + sent_, host_.size() - sent_, cudaMemcpyHostToDevice,
+                         st_), "upload");
+    sent_ = host_.size();
+  }
+  std::vector<DBuf<char>> take() { send(); host_.clear(); sent_ = 0; return std::move(blocks_); }
+
+ private:
+  static constexpr size_t BLOCK = size_t(64) << 10, MAX_TABLE = size_t(16) << 10;
+  Pool* pool_;
+  cudaStream_t st_;
+  std::vector<DBuf<char>> blocks_;
+  std::vector<char> host_;           // the last block's bytes
+  size_t sent_ = 0;
+};
 
 // ---------------------------------------------------------------- CDF tables
 // thresholds floor(CDF * 2^31); the last class with positive mass gets 2^31
@@ -299,6 +385,7 @@ struct pg_placed {
   std::vector<uint16_t> chain_anc_h;
   std::vector<uint64_t> chain_key_h;
   std::vector<uint8_t> inst_root_h;
+  std::vector<DBuf<char>> tables;      // holds the tables below that came with one copy
   DBuf<uint32_t> atom_start, atom_ioff, atom_icnt;
   DBuf<uint32_t> node_class, seg_off, seg_start, seg_end, seg_ioff, seg_icnt, chain_off;
   DBuf<uint16_t> inst_list, chain_anc;
@@ -355,12 +442,16 @@ struct Timer {
     ck(cudaEventCreate(&a), "event"); ck(cudaEventCreate(&b), "event");
     ck(cudaEventRecord(a, st), "event");
   }
-  float stop() {
-    ck(cudaEventRecord(b, st), "event");
-    ck(cudaEventSynchronize(b), "event");
+  void mark() { ck(cudaEventRecord(b, st), "event"); }
+  float elapsed() {                 // once the stream has passed the mark
     float ms = 0;
     cudaEventElapsedTime(&ms, a, b);
     return ms;
+  }
+  float stop() {
+    mark();
+    ck(cudaEventSynchronize(b), "event");
+    return elapsed();
   }
   ~Timer() { if (a) cudaEventDestroy(a); if (b) cudaEventDestroy(b); }
 };
@@ -1029,13 +1120,10 @@ pg_status pg_place_mutations(pg_engine* e, const pg_forest* f, uint32_t n_pre_sn
       e->fc_div = upload(P, f->divisions, st);
       e->fc_uid = f->uid;
     }
-    auto times_d = upload(P, times, st);
-    auto snv_d = upload(P, snv_rate, st);
-    auto id_d = upload(P, id_rate, st);
-    auto sbs_sig_d = upload(P, sig_cdf[0], st);
-    auto id_sig_d = upload(P, sig_cdf[1], st);
-    auto sbs_expo_d = upload(P, expo_cdf[0], st);
-    auto id_expo_d = upload(P, expo_cdf[1], st);
+    Stage tables(P, st);
+    auto times_d = tables.add(times), snv_d = tables.add(snv_rate), id_d = tables.add(id_rate);
+    auto sbs_sig_d = tables.add(sig_cdf[0]), id_sig_d = tables.add(sig_cdf[1]);
+    auto sbs_expo_d = tables.add(expo_cdf[0]), id_expo_d = tables.add(expo_cdf[1]);
     std::vector<double> cna_rate(S, 0.0);
     bool passenger_cnas = false;
     for (uint32_t s2 = 0; s2 < S; ++s2) {
@@ -1044,7 +1132,7 @@ pg_status pg_place_mutations(pg_engine* e, const pg_forest* f, uint32_t n_pre_sn
       passenger_cnas = passenger_cnas || (used[s2] && cna_rate[s2] > 0);
     }
     passenger_cnas = passenger_cnas && !e->cna_cands.empty();
-    auto cna_d = upload(P, cna_rate, st);
+    auto cna_d = tables.add(cna_rate);
     pg::PlaceTables t{};
     t.n_nodes = f->n; t.parent = e->fc_parent.p; t.birth = e->fc_birth.p; t.species = e->fc_species.p;
     t.divisions = e->fc_div.p;
@@ -1059,6 +1147,7 @@ pg_status pg_place_mutations(pg_engine* e, const pg_forest* f, uint32_t n_pre_sn
     // ---- passenger CNA counts (germline-size rate, so they do not depend on the events)
     std::vector<uint32_t> cnt_cna(f->n, 0);
     if (passenger_cnas) {
+      tables.send();
       DBuf<uint32_t> cc(P, f->n);
       pg::place_cna_counts(t, cc.p, seed, 2.0 * double(e->G), st);
       ck(cudaMemcpyAsync(cnt_cna.data(), cc.p, sizeof(uint32_t) * f->n, cudaMemcpyDeviceToHost, st), "cna counts");
@@ -1197,7 +1286,9 @@ pg_status pg_place_mutations(pg_engine* e, const pg_forest* f, uint32_t n_pre_sn
     std::vector<double> node_size(f->n + 1);
     for (uint32_t v = 0; v < f->n; ++v) node_size[v] = class_size[node_class[v]];
     node_size[f->n] = class_size[0];
-    auto node_size_d = upload(P, node_size, st);
+    auto node_size_d = tables.add(node_size);
+    auto drv_d = tables.add(drv);
+    tables.send();
     t.node_size = node_size_d.p;
     const uint64_t ncell = uint64_t(f->n + 1) * E;
     DBuf<uint32_t> cnt_snv(P, ncell), cnt_id(P, ncell), off_snv(P, ncell), off_id(P, ncell);
@@ -1241,7 +1332,8 @@ pg_status pg_place_mutations(pg_engine* e, const pg_forest* f, uint32_t n_pre_sn
     pl->cn_max = std::max<uint32_t>(cn_max, 2);
     pl->n_classes = uint32_t(classes.size());
     pl->node_class_h = node_class;
-    pl->node_class = upload(P, node_class, st);
+    Stage kept(P, st);
+    pl->node_class = kept.add(node_class);
     {
       // atoms: cut at every segment boundary of every class, then merge
       // neighbours on which every class sits in the same segment
@@ -1269,16 +1361,17 @@ pg_status pg_place_mutations(pg_engine* e, const pg_forest* f, uint32_t n_pre_sn
           pl->atom_icnt_h.push_back(in ? seg_icnt[cur[c]] : 0u);
         }
       }
-      pl->atom_start = upload(P, pl->atom_start_h, st);
-      pl->atom_ioff = upload(P, atom_ioff, st);
-      pl->atom_icnt = upload(P, pl->atom_icnt_h, st);
+      pl->atom_start = kept.add(pl->atom_start_h);
+      pl->atom_ioff = kept.add(atom_ioff);
+      pl->atom_icnt = kept.add(pl->atom_icnt_h);
     }
-    pl->seg_off = upload(P, seg_off, st); pl->seg_start = upload(P, seg_start, st); pl->seg_end = upload(P, seg_end, st);
-    pl->seg_ioff = upload(P, seg_ioff, st); pl->seg_icnt = upload(P, seg_icnt, st);
+    pl->seg_off = kept.add(seg_off); pl->seg_start = kept.add(seg_start); pl->seg_end = kept.add(seg_end);
+    pl->seg_ioff = kept.add(seg_ioff); pl->seg_icnt = kept.add(seg_icnt);
     if (inst_list.empty()) inst_list.push_back(0);
-    pl->inst_list = upload(P, inst_list, st);
+    pl->inst_list = kept.add(inst_list);
     if (chain_anc.empty()) { chain_anc.push_back(0); chain_key.push_back(0); }
-    pl->chain_off = upload(P, chain_off, st); pl->chain_anc = upload(P, chain_anc, st); pl->chain_key = upload(P, chain_key, st);
+    pl->chain_off = kept.add(chain_off); pl->chain_anc = kept.add(chain_anc); pl->chain_key = kept.add(chain_key);
+    pl->tables = kept.take();
     t.gc = pl->classes_view();
     // ---- the edge counts' totals size the outputs
     uint32_t tot_h[2];
@@ -1292,8 +1385,12 @@ pg_status pg_place_mutations(pg_engine* e, const pg_forest* f, uint32_t n_pre_sn
     DBuf<uint32_t> locus(P, n_all);
     DBuf<uint4> raw(P, n_all);
     const pg::PlaceRaw o{locus.p, raw.p};
-    DBuf<uint32_t> err(P, 1);
-    ck(cudaMemsetAsync(err.p, 0, sizeof(uint32_t), st), "memset");
+    // the error flag, the number of redraws and their status, cleared and read
+    // back together
+    struct Ctl { uint32_t err, n_next; pg::TailCtl tail; };
+    DBuf<Ctl> ctl(P, 1);
+    ck(cudaMemsetAsync(ctl.p, 0, sizeof(Ctl), st), "memset");
+    uint32_t* const err = &ctl.p->err;
     // infinite sites: the first draw goes into the first round's table as it
     // is made (the drivers' loci follow; the losers are read back below)
     const bool unique = e->infinite_sites;
@@ -1310,8 +1407,7 @@ pg_status pg_place_mutations(pg_engine* e, const pg_forest* f, uint32_t n_pre_sn
       lost1 = DBuf<uint8_t>(P, n_slots);
       ck(cudaMemsetAsync(first.p, 0xff, sizeof(unsigned long long) * fcap, st), "memset");
     }
-    pg::place_first_round(t, o, seed, off_snv.p, off_id.p, uint32_t(n_snv), n_slots, first.p, fmask, lost1.p, err.p, st);
-    auto drv_d = upload(P, drv, st);
+    pg::place_first_round(t, o, seed, off_snv.p, off_id.p, uint32_t(n_snv), n_slots, first.p, fmask, lost1.p, err, st);
     pg::place_drivers(o, drv_d.p, uint32_t(drv.size()), n_slots, st);
     // the handle's host columns, while the first round runs
     pl->eng = e; pl->n_nodes = f->n; pl->n_samples = f->n_samples;
@@ -1325,35 +1421,30 @@ pg_status pg_place_mutations(pg_engine* e, const pg_forest* f, uint32_t n_pre_sn
     }
     // ---- redraws: infinite sites (the losers of the first round over all
     // slots, drivers first), or loci drawn where the cell has no allele left
-    DBuf<pg::TailCtl> tail_ctl;
-    if ((unique || pl->has_cna) && n_slots > 0) {
-      tail_ctl = DBuf<pg::TailCtl>(P, 1);
-      ck(cudaMemsetAsync(tail_ctl.p, 0, sizeof(pg::TailCtl), st), "memset");
-    }
     if (unique && n_slots > 0) {
-      DBuf<uint32_t> pend(P, n_slots), n_next(P, 1);
-      ck(cudaMemsetAsync(n_next.p, 0, sizeof(uint32_t), st), "memset");
+      DBuf<uint32_t> pend(P, n_slots);
+      uint32_t* const n_next = &ctl.p->n_next;
       pg::sites_first_finish(locus.p + n_slots, uint32_t(drv.size()), first.p, fmask, lost1.p, n_slots, pend.p,
-                             n_next.p, err.p, st);
+                             n_next, err, st);
       // the host reads how many lost, to size the tables; where tables for
       // every slot are small (12 MB) that wait costs more than they do
       uint32_t n_tail = n_slots;
       if (n_slots > TAIL_NO_READ) {
-        ck(cudaMemcpyAsync(&n_tail, n_next.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "round");
+        ck(cudaMemcpyAsync(&n_tail, n_next, sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "round");
         ck(cudaStreamSynchronize(st), "first round");
       }
       if (n_tail) {
         uint64_t cap = 1024;
         while (cap < 2 * uint64_t(n_tail)) cap <<= 1;
-        DBuf<uint32_t> keys(P, cap);
-        DBuf<unsigned long long> held(P, cap);
-        ck(cudaMemsetAsync(keys.p, 0xff, sizeof(uint32_t) * cap, st), "memset");
-        ck(cudaMemsetAsync(held.p, 0xff, sizeof(unsigned long long) * cap, st), "memset");
-        pg::sites_settle(t, o, seed, off_snv.p, off_id.p, uint32_t(n_snv), pend.p, n_next.p, n_tail, first.p, fmask,
-                         keys.p, held.p, cap, tail_ctl.p, err.p, st);
+        DBuf<uint32_t> table(P, 3 * cap);     // holders (8 bytes), then keys (4): one memset for both
+        unsigned long long* const held = reinterpret_cast<unsigned long long*>(table.p);
+        uint32_t* const keys = table.p + 2 * cap;
+        ck(cudaMemsetAsync(table.p, 0xff, sizeof(uint32_t) * 3 * cap, st), "memset");
+        pg::sites_settle(t, o, seed, off_snv.p, off_id.p, uint32_t(n_snv), pend.p, n_next, n_tail, first.p, fmask,
+                         keys, held, cap, &ctl.p->tail, err, st);
       }
-    } else if (tail_ctl.p) {
-      pg::sites_covered(t, o, seed, off_snv.p, off_id.p, uint32_t(n_snv), n_slots, tail_ctl.p, err.p, st);
+    } else if (pl->has_cna && n_slots > 0) {
+      pg::sites_covered(t, o, seed, off_snv.p, off_id.p, uint32_t(n_snv), n_slots, &ctl.p->tail, err, st);
     }
     // ---- sort by locus
     const uint32_t nb = pg::sort_num_buckets(e->G);
@@ -1364,19 +1455,17 @@ pg_status pg_place_mutations(pg_engine* e, const pg_forest* f, uint32_t n_pre_sn
     pl->kind = DBuf<uint8_t>(P, n_all); pl->nature = DBuf<uint8_t>(P, n_all);
     DBuf<unsigned long long> skeys(P, n_all);
     pg::sort_by_locus(o, uint32_t(n_all), e->G, bcnt.p, bfill.p, bpart.p, order.p, pl->view(), skeys.p, st);
-    pl->kernel_ms = timer.stop();
+    Ctl c{};
+    timer.mark();
+    ck(cudaMemcpyAsync(&c, ctl.p, sizeof(c), cudaMemcpyDeviceToHost, st), "error flag");
+    ck(cudaStreamSynchronize(st), "placement");
+    pl->kernel_ms = timer.elapsed();
     ck(cudaGetLastError(), "placement kernels");
-    uint32_t err_h = 0;
-    ck(cudaMemcpy(&err_h, err.p, sizeof(uint32_t), cudaMemcpyDeviceToHost), "error flag");
-    if (tail_ctl.p) {
-      pg::TailCtl c{};
-      ck(cudaMemcpy(&c, tail_ctl.p, sizeof(c), cudaMemcpyDeviceToHost), "rounds");
-      require(!(c.status & pg::TAIL_ROUNDS_EXHAUSTED), unique ? "infinite sites model: no free locus left for some mutations"
-                                                              : "no allele left where some mutations were drawn");
-      pl->redraw_rounds = c.rounds;
-    }
-    if (err_h & pg::ERR_EMPTY_CLASS) throw std::runtime_error("a drawn mutation class has no indexed positions");
-    if (err_h & pg::ERR_CAPACITY) throw std::runtime_error("internal hash table capacity exceeded");
+    require(!(c.tail.status & pg::TAIL_ROUNDS_EXHAUSTED), unique ? "infinite sites model: no free locus left for some mutations"
+                                                                 : "no allele left where some mutations were drawn");
+    pl->redraw_rounds = c.tail.rounds;
+    if (c.err & pg::ERR_EMPTY_CLASS) throw std::runtime_error("a drawn mutation class has no indexed positions");
+    if (c.err & pg::ERR_CAPACITY) throw std::runtime_error("internal hash table capacity exceeded");
     engine_retain(e);
     *out = pl.release();
   });
@@ -1907,29 +1996,38 @@ void simulate_seq_impl(const pg_placed* pl, const pg_seq_cfg* c, uint64_t seed, 
       *out = res.release();
       return;
     }
-    auto etin_d = upload(P, etin, st), etout_d = upload(P, etout, st);
-    DBuf<uint32_t> ts_d(P, n_tiles), tl_d(P, n_tiles), te_d(P, n_tiles);
-    {
-      auto cf = upload(P, c_first, st), cn = upload(P, c_ntiles, st), cs = upload(P, c_start, st);
-      auto cns = upload(P, c_nstarts, st), cen = upload(P, c_end, st);
-      pg::seq_make_tiles(uint32_t(c_first.size()), cf.p, cn.p, cs.p, cns.p, cen.p, T, n_tiles, ts_d.p, tl_d.p,
-                         te_d.p, st);
-    }
-    auto cnt_d = upload(P, c_ntiles, st), cns_d = upload(P, c_nstarts, st), cid_d = upload(P, c_id, st);
-    auto cf_d = upload(P, c_first, st), cd_d = upload(P, c_depth, st);
-    auto cp_d = upload(P, c_pairs, st);
-    auto smp_d = upload(P, samples, st);
-    auto leaf_d = upload(P, leaf_tin, st);
-    auto ins_d = upload(P, ins_thr, st);
+    Stage tables(P, st);
+    auto etin_d = tables.add(etin), etout_d = tables.add(etout);
+    auto cf_d = tables.add(c_first), cnt_d = tables.add(c_ntiles), cst_d = tables.add(c_start);
+    auto cns_d = tables.add(c_nstarts), cen_d = tables.add(c_end), cid_d = tables.add(c_id);
+    auto cd_d = tables.add(c_depth);
+    auto cp_d = tables.add(c_pairs);
+    auto smp_d = tables.add(samples);
+    auto leaf_d = tables.add(leaf_tin);
+    auto ins_d = tables.add(ins_thr);
     std::vector<uint32_t> guide(pg::SEQ_GUIDE, 0);
     if (ins_thr.size() <= pg::SEQ_GUIDE_INS)
-      for (uint32_t g = 0; g < pg::SEQ_GUIDE; ++g) guide[g] = pg::insert_guide(ins_thr.data(), uint32_t(ins_thr.size()), g);
-    auto guide_d = upload(P, guide, st);
+      for (uint32_t g = 0, at = 0; g < pg::SEQ_GUIDE; ++g)
+        guide[g] = pg::insert_guide(ins_thr.data(), uint32_t(ins_thr.size()), g, at);
+    auto guide_d = tables.add(guide);
+    DBuf<double> wn_d, wt_d;
+    DBuf<uint64_t> nl_d, i0_d, cs_d;
+    DBuf<uint32_t> ocls_d, oloff_d, onl_d, cltin_d, ocdf_d;
+    if (pl->has_cna) {
+      wn_d = tables.add(s_wn); wt_d = tables.add(s_wt);
+      nl_d = tables.add(s_nl); i0_d = tables.add(s_icnt0); cs_d = tables.add(s_copy);
+      ocls_d = tables.add(opt_class); oloff_d = tables.add(opt_leaf_off); onl_d = tables.add(opt_nleaf);
+      cltin_d = tables.add(cls_leaf_tin); ocdf_d = tables.add(opt_cdf);
+    }
+    tables.send();
+    DBuf<uint32_t> ts_d(P, n_tiles), tl_d(P, n_tiles), te_d(P, n_tiles);
+    pg::seq_make_tiles(uint32_t(c_first.size()), cf_d.p, cnt_d.p, cst_d.p, cns_d.p, cen_d.p, T, n_tiles, ts_d.p, tl_d.p,
+                       te_d.p, st);
     DBuf<pg::SeqRec> recs(P, pl->M);
     DBuf<uint32_t> pair_cnt(P, uint64_t(n_tiles) * samples.size()), rlo(P, n_tiles), rhi(P, n_tiles);
     pg::seq_build_records(pl->view(), uint32_t(pl->M), etin_d.p, etout_d.p, recs.p, st);
     DBuf<double> mcum_d, mtot_d;
-    DBuf<uint32_t> poff_d, pstart_d, plen_d, patom_d, pcdf_d, ocls_d, oloff_d, onl_d, cltin_d, ocdf_d;
+    DBuf<uint32_t> poff_d, pstart_d, plen_d, patom_d, pcdf_d;
     uint32_t n_parts_cap = 0;
     if (pl->has_cna) {
       const uint32_t NS = uint32_t(samples.size()), NA = uint32_t(pl->atom_start_h.size());
@@ -1940,17 +2038,12 @@ void simulate_seq_impl(const pg_placed* pl, const pg_seq_cfg* c, uint64_t seed, 
       DBuf<uint32_t> scan_part(P, pg::scan_part_elems(n_tiles, 1));
       pg::seq_tile_parts(n_tiles, ts_d.p, tl_d.p, pl->atom_start.p, NA, uint32_t(e->G), poff_d.p, scan_part.p,
                          pstart_d.p, plen_d.p, patom_d.p, st);
-      auto wn_d = upload(P, s_wn, st), wt_d = upload(P, s_wt, st);
-      auto nl_d = upload(P, s_nl, st), i0_d = upload(P, s_icnt0, st), cs_d = upload(P, s_copy, st);
-      auto cf_d2 = upload(P, c_first, st), cn_d2 = upload(P, c_ntiles, st);
       mcum_d = DBuf<double>(P, uint64_t(NS) * n_tiles);
       mtot_d = DBuf<double>(P, uint64_t(NS) * c_id.size());
       DBuf<uint64_t> tsums(P, 2 * uint64_t(NS) * n_tiles);
-      pg::seq_tile_mass(NS, uint32_t(c_id.size()), cf_d2.p, cn_d2.p, poff_d.p, plen_d.p, patom_d.p, NA, wn_d.p,
+      pg::seq_tile_mass(NS, uint32_t(c_id.size()), cf_d.p, cnt_d.p, poff_d.p, plen_d.p, patom_d.p, NA, wn_d.p,
                         wt_d.p, nl_d.p, i0_d.p, cs_d.p, n_tiles, n_parts_cap, tsums.p, mcum_d.p, mtot_d.p, pcdf_d.p,
                         st);
-      ocls_d = upload(P, opt_class, st); oloff_d = upload(P, opt_leaf_off, st); onl_d = upload(P, opt_nleaf, st);
-      cltin_d = upload(P, cls_leaf_tin, st); ocdf_d = upload(P, opt_cdf, st);
     }
     pg::seq_tile_counts(uint32_t(samples.size()), uint32_t(c_id.size()), max_tiles, cf_d.p, cnt_d.p, cd_d.p, cns_d.p,
                         cid_d.p, cp_d.p, T, n_tiles, pl->has_cna ? mcum_d.p : nullptr,

@@ -316,8 +316,8 @@ void batch_layout(pg_batch* b) {
     prm.ins_cdf = reinterpret_cast<const uint32_t*>(uintptr_t(ins_cdf.size()));
     prm.ins_guide = reinterpret_cast<const uint32_t*>(uintptr_t(guide_all.size()));
     ins_cdf.insert(ins_cdf.end(), thr.begin(), thr.end());
-    for (uint32_t g = 0; g < pg::SEQ_GUIDE; ++g)
-      guide_all.push_back(thr.size() <= pg::SEQ_GUIDE_INS ? pg::insert_guide(thr.data(), uint32_t(thr.size()), g) : 0u);
+    for (uint32_t g = 0, at = 0; g < pg::SEQ_GUIDE; ++g)
+      guide_all.push_back(thr.size() <= pg::SEQ_GUIDE_INS ? pg::insert_guide(thr.data(), uint32_t(thr.size()), g, at) : 0u);
     // counts and work items
     S.pair_off = pair_total;
     pair_total += uint64_t(S.n_samples) * n_tiles;

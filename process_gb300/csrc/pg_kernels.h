@@ -179,10 +179,12 @@ constexpr uint32_t SEQ_FRAGS_PER_BATCH = 1280;
 // one word in a hundred of a normal-shaped table to the walk (256 left one in
 // thirty, so that most warps had a lane in it).
 constexpr uint32_t SEQ_GUIDE = 1024, SEQ_GUIDE_INS = 1024;
-inline uint32_t insert_guide(const uint32_t* thr, uint32_t n, uint32_t g) {
+// Cells are asked for in ascending order: at is the previous cell's entry (0
+// at the first).
+inline uint32_t insert_guide(const uint32_t* thr, uint32_t n, uint32_t g, uint32_t& at) {
   const uint32_t first = g << 21, next = first + (1u << 21);   // cells end at 2^31 at the latest
-  uint32_t lo = 0, hi = n;
-  while (lo < hi) { const uint32_t mid = (lo + hi) / 2; if (thr[mid] <= first) lo = mid + 1; else hi = mid; }
+  while (at < n && thr[at] <= first) ++at;
+  const uint32_t lo = at;
   if (lo >= n || thr[lo] >= next) return (lo < n ? lo : n - 1) | 0x7ffffc00u;
   const bool walk = lo + 1 >= n || thr[lo + 1] < next;
   return lo | (thr[lo] - first - 1u) << 10 | (walk ? 0x80000000u : 0u);

@@ -18,6 +18,7 @@ library through the C-ABI; this module only validates and arranges inputs.
 """
 from __future__ import annotations
 
+import copy
 import ctypes as C
 import os
 import itertools
@@ -698,14 +699,14 @@ class MutationEngine:
 
     def _config(self) -> dict:
         """JSON-ready copy of the engine's configuration."""
-        import copy
         return {"context_sampling": self.context_sampling, "max_motif_size": self.max_motif_size,
                 "max_repetition_storage": self.max_repetition_storage,
                 "avoid_homozygous_losses": self.avoid_homozygous_losses,
                 "infinite_sites_model": self.infinite_sites_model,
-                "SBS_signatures": _plain(self._sigs[0]), "indel_signatures": _plain(self._sigs[1]),
-                "exposures": copy.deepcopy(_plain(self._exposures)),
-                "mutants": copy.deepcopy(_plain(self._mutant_specs)),
+                # lists of floats (set_signatures)
+                "SBS_signatures": {str(k): v.copy() for k, v in self._sigs[0].items()},
+                "indel_signatures": {str(k): v.copy() for k, v in self._sigs[1].items()},
+                "exposures": _plain(self._exposures), "mutants": _plain(self._mutant_specs),
                 "passenger_CNAs": _plain(self.passenger_CNAs),
                 "regions_to_avoid": _plain(getattr(self, "regions_to_avoid", []))}
 
@@ -1068,6 +1069,8 @@ FOREST_VERSION = 2
 
 def _plain(x):
     """JSON-ready copy of rates, exposures and driver specifications."""
+    if type(x) in _ATOMS:
+        return x
     if isinstance(x, dict):
         return {str(k): _plain(v) for k, v in x.items()}
     if isinstance(x, (list, tuple)):
@@ -1084,7 +1087,10 @@ def _plain(x):
                 "allele": x.allele, "src_allele": x.src_allele}
     if x is WGD:
         return {"kind": "WGD"}
-    return x
+    return copy.deepcopy(x)
+
+
+_ATOMS = frozenset((str, int, float, bool, type(None)))
 
 
 def _driver(d):
@@ -1439,7 +1445,15 @@ def _sid_strings(buf: np.ndarray, n: int) -> np.ndarray:
     """Strings of a buffer of n NUL-padded SID_CHARS-byte fields."""
     if n == 0:
         return np.zeros(0, dtype=object)
-    return buf.reshape(n, _lib.SID_CHARS).view(f"S{_lib.SID_CHARS}").ravel().astype(str).astype(object)
+    rows = buf.reshape(n, _lib.SID_CHARS)
+    out = _CHARS[rows[:, 0] & 127]      # an SNV's base by one lookup, the few longer fields by conversion
+    rest = np.nonzero((rows[:, 0] > 127) | (rows[:, 1] != 0))[0]
+    if len(rest):
+        out[rest] = rows[rest].view(f"S{_lib.SID_CHARS}").ravel().astype(str).astype(object)
+    return out
+
+
+_CHARS = np.array([""] + [chr(i) for i in range(1, 128)], dtype=object)
 
 
 def _cbuf(arr: np.ndarray):
@@ -1483,17 +1497,11 @@ def _result_frame(res: "SeqResult", pf: PhylogeneticForest, include_non_sequence
     check(lib().pg_seq_result_frame_copy(res._h, ptr(chr_, C.c_uint32), ptr(pos, C.c_uint32), _cbuf(ref), _cbuf(alt),
                                          ptr(coff, C.c_uint64), _cbuf(cb), ptr(classes, C.c_uint8),
                                          ptr(occ, C.c_int32), ptr(cov, C.c_int32), ptr(vaf, C.c_double)))
-    # causes: the joined strings into fixed-width fields, empty ones NA (None)
-    lens = np.diff(coff).astype(np.int64)
-    width = int(lens.max()) if R else 0
-    causes = np.full(R, None, dtype=object)
-    if width:
-        grid = np.zeros((R, width), np.uint8)
-        rows = np.repeat(np.arange(R), lens)
-        cols = np.arange(int(lens.sum())) - np.repeat(coff[:-1].astype(np.int64), lens)
-        grid[rows, cols] = cb[:int(lens.sum())]
-        txt = grid.view(f"S{width}").ravel().astype(str).astype(object)
-        causes[lens > 0] = txt[lens > 0]
+    # causes: cut out of the joined bytes, empty ones NA (None)
+    txt = cb[:int(coff[-1])].tobytes().decode("ascii")
+    ends = coff.tolist()
+    causes = np.empty(R, dtype=object)
+    causes[:] = [txt[i:j] or None for i, j in zip(ends, ends[1:])]
     names = np.array(pf.engine.chr_names, dtype=object)
     df = {"chr": names[chr_], "chr_pos": pos.astype(np.int64), "ref": _sid_strings(ref, R),
           "alt": _sid_strings(alt, R), "causes": causes, "classes": _class_names()[classes & 15]}
