@@ -2027,7 +2027,8 @@ void simulate_seq_impl(const pg_placed* pl, const pg_seq_cfg* c, uint64_t seed, 
     DBuf<uint32_t> pair_cnt(P, uint64_t(n_tiles) * samples.size()), rlo(P, n_tiles), rhi(P, n_tiles);
     pg::seq_build_records(pl->view(), uint32_t(pl->M), etin_d.p, etout_d.p, recs.p, st);
     DBuf<double> mcum_d, mtot_d;
-    DBuf<uint32_t> poff_d, pstart_d, plen_d, patom_d, pcdf_d;
+    DBuf<uint32_t> poff_d, pstart_d, plen_d, patom_d, pcdf_d, tatom_d;
+    DBuf<pg::CnRow> cnrow_d;
     uint32_t n_parts_cap = 0;
     if (pl->has_cna) {
       const uint32_t NS = uint32_t(samples.size()), NA = uint32_t(pl->atom_start_h.size());
@@ -2035,9 +2036,11 @@ void simulate_seq_impl(const pg_placed* pl, const pg_seq_cfg* c, uint64_t seed, 
       poff_d = DBuf<uint32_t>(P, uint64_t(n_tiles) + 1);
       pstart_d = DBuf<uint32_t>(P, n_parts_cap); plen_d = DBuf<uint32_t>(P, n_parts_cap);
       patom_d = DBuf<uint32_t>(P, n_parts_cap); pcdf_d = DBuf<uint32_t>(P, uint64_t(NS) * n_parts_cap);
+      tatom_d = DBuf<uint32_t>(P, n_tiles);
+      cnrow_d = DBuf<pg::CnRow>(P, uint64_t(NS) * NA);
       DBuf<uint32_t> scan_part(P, pg::scan_part_elems(n_tiles, 1));
       pg::seq_tile_parts(n_tiles, ts_d.p, tl_d.p, pl->atom_start.p, NA, uint32_t(e->G), poff_d.p, scan_part.p,
-                         pstart_d.p, plen_d.p, patom_d.p, st);
+                         pstart_d.p, plen_d.p, patom_d.p, tatom_d.p, st);
       mcum_d = DBuf<double>(P, uint64_t(NS) * n_tiles);
       mtot_d = DBuf<double>(P, uint64_t(NS) * c_id.size());
       DBuf<uint64_t> tsums(P, 2 * uint64_t(NS) * n_tiles);
@@ -2070,6 +2073,8 @@ void simulate_seq_impl(const pg_placed* pl, const pg_seq_cfg* c, uint64_t seed, 
       prm.part_cdf = pcdf_d.p; prm.n_parts = n_parts_cap;
       prm.opt_class = ocls_d.p; prm.opt_leaf_off = oloff_d.p; prm.opt_nleaf = onl_d.p;
       prm.cls_leaf_tin = cltin_d.p; prm.opt_cdf = ocdf_d.p;
+      prm.tile_atom = tatom_d.p; prm.cn_rows = cnrow_d.p; prm.n_atoms = uint32_t(pl->atom_start_h.size());
+      pg::seq_cn_rows(prm, smp_d.p, uint32_t(samples.size()), cnrow_d.p, st);
     }
     Timer timer(st);
     pg::seq_reads(recs.p, uint32_t(pl->M), tiles, pair_cnt.p, smp_d.p, uint32_t(samples.size()), leaf_d.p, prm, seed,

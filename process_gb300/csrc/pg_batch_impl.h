@@ -9,14 +9,14 @@
 // species 0 has those rates and that exposure at time 0, called with the
 // same seeds and tile size:
 //   * placement runs as single launches over every instance (edge counts,
-//     mutation placement, infinite-sites rounds keyed by (instance, locus),
+//     mutation placement, infinite-sites redraws keyed by (instance, locus),
 //     one sort by (instance, locus)); slots of one instance keep their order;
-//   * sequencing runs as one persistent read kernel over every (instance,
+//   * sequencing runs as one read kernel over every (instance,
 //     sample, tile), after batched tile splits and record ranges; the stage is
 //     captured into a CUDA graph on its first run and replayed afterwards
 //     (sizes it depends on live in device memory; capacities grow, and the
 //     graph is captured again, only when an instance outgrows them);
-//   * the autotuner times the persistent kernel over candidate tile sizes
+//   * the autotuner times the read kernel over candidate tile sizes
 //     for every instance and keeps the fastest.
 
 struct BatchInst {
@@ -60,17 +60,16 @@ struct pg_batch {
   std::vector<pg::SeqInst> sinst;
   pg::SeqBatch sb{};
   DBuf<pg::SeqInst> sinst_d;
-  DBuf<uint32_t> item_off_d, cnt_off_d, t_start, t_len, t_end, t_inst, rec_lo, rec_hi;
+  DBuf<uint32_t> cnt_off_d, t_start, t_len, t_end, t_inst, rec_lo, rec_hi;
   DBuf<uint32_t> c_first, c_ntiles, c_depth, c_nstarts, c_id, blk_slot, blk_index, pair_cnt;
   DBuf<uint64_t> c_pairs;
   DBuf<pg::SeqSample> samples;
-  DBuf<uint32_t> leaf_tin, etin, etout, ins_cdf, counter, alt, depth;
+  DBuf<uint32_t> leaf_tin, etin, etout, ins_cdf, alt, depth;
   DBuf<uint32_t> ins_guide;
   DBuf<pg::SeqRec> recs;
   uint64_t rec_cap = 0;
   cudaGraphExec_t graph = nullptr;
   uint32_t graph_kernels = 0;     // kernels one replay launches
-  uint32_t grid = 0;
   float place_ms = 0, seq_ms = 0;
 
   ~pg_batch() {
@@ -221,7 +220,7 @@ void batch_layout(pg_batch* b) {
   Pool* P = &e->pool;
   const uint32_t B = uint32_t(b->in.size());
   std::vector<uint32_t> t_start, t_len, t_end, t_inst, c_first, c_ntiles, c_depth, c_nstarts, c_id, blk_slot,
-      blk_index, leaf_tin, etin, etout, ins_cdf, item_off{0}, cnt_off{0};
+      blk_index, leaf_tin, etin, etout, ins_cdf, cnt_off{0};
   std::vector<uint64_t> c_pairs;
   std::vector<uint32_t> guide_all;
   std::vector<pg::SeqSample> samples;
@@ -326,7 +325,6 @@ void batch_layout(pg_batch* b) {
     S.count_stride = b->stride[i];
     S.count_off = count_total;
     count_total += uint64_t(S.n_samples) * S.count_stride;
-    item_off.push_back(item_off.back() + S.n_samples * n_tiles);
     cnt_off.push_back(cnt_off.back() + S.n_samples * S.n_blocks);
   }
   if (leaf_tin.empty()) leaf_tin.push_back(0);
@@ -346,26 +344,22 @@ void batch_layout(pg_batch* b) {
     S.prm.ins_guide = b->ins_guide.p + uintptr_t(S.prm.ins_guide);
   }
   b->sinst_d = upload(P, b->sinst, st);
-  b->item_off_d = upload(P, item_off, st); b->cnt_off_d = upload(P, cnt_off, st);
-  b->counter = DBuf<uint32_t>(P, 1);
+  b->cnt_off_d = upload(P, cnt_off, st);
   b->alt = DBuf<uint32_t>(P, count_total); b->depth = DBuf<uint32_t>(P, count_total);
   b->recs = DBuf<pg::SeqRec>(P, b->slot_cap);
   b->rec_cap = b->slot_cap;
   pg::SeqBatch& sb = b->sb;
   sb = pg::SeqBatch{};
   sb.n_inst = B; sb.inst = b->sinst_d.p; sb.keys = b->skeys.p; sb.rec_off = b->rec_off_d.p;
-  sb.item_off = b->item_off_d.p; sb.cnt_off = b->cnt_off_d.p;
-  sb.n_items = item_off.back(); sb.n_cnt = cnt_off.back(); sb.n_tiles_all = uint32_t(t_start.size());
+  sb.cnt_off = b->cnt_off_d.p;
+  for (const auto& S : b->sinst) sb.max_samples = std::max(sb.max_samples, S.n_samples);
+  sb.n_cnt = cnt_off.back(); sb.n_tiles_all = uint32_t(t_start.size());
   sb.tile_start = b->t_start.p; sb.tile_len = b->t_len.p; sb.tile_end = b->t_end.p; sb.tile_inst = b->t_inst.p;
   sb.rec_lo = b->rec_lo.p; sb.rec_hi = b->rec_hi.p;
   sb.c_first = b->c_first.p; sb.c_ntiles = b->c_ntiles.p; sb.c_depth = b->c_depth.p; sb.c_nstarts = b->c_nstarts.p;
   sb.c_id = b->c_id.p; sb.c_pairs = b->c_pairs.p; sb.blk_slot = b->blk_slot.p; sb.blk_index = b->blk_index.p;
   sb.pair_cnt = b->pair_cnt.p; sb.samples = b->samples.p; sb.leaf_tin = b->leaf_tin.p;
-  sb.etin = b->etin.p; sb.etout = b->etout.p; sb.counter = b->counter.p; sb.alt = b->alt.p; sb.depth = b->depth.p;
-  int sms = 0, per_sm = 0;
-  ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device), "device attribute");
-  per_sm = pg::seq_reads_batch_occupancy();
-  b->grid = uint32_t(std::max(1, sms * std::max(1, per_sm)));
+  sb.etin = b->etin.p; sb.etout = b->etout.p; sb.alt = b->alt.p; sb.depth = b->depth.p;
   if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
   ck(cudaStreamSynchronize(st), "batch layout");
   b->layout_ok = true;
@@ -383,7 +377,7 @@ void batch_sequence(pg_batch* b) {
     cudaMemsetAsync(b->alt.p, 0, sizeof(uint32_t) * nc, st);
     cudaMemsetAsync(b->depth.p, 0, sizeof(uint32_t) * nc, st);
     pg::seq_batch_records(b->sorted_view(), b->s_inst.p, b->n_all_d.p, uint32_t(b->rec_cap), b->sb, b->recs.p, st);
-    pg::seq_batch_reads(b->sb, b->recs.p, b->grid, st);
+    pg::seq_batch_reads(b->sb, b->recs.p, st);
     ck(cudaStreamEndCapture(st, &g), "stream capture");
     b->graph_kernels = uint32_t(g_launches.load() - counted);
     g_launches.store(counted);
@@ -623,7 +617,7 @@ pg_status pg_batch_autotune(pg_batch* b, const uint64_t* place_seed, const uint6
     ck(cudaMemcpyAsync(b->skeys.p, keys.data(), sizeof(pg::Key) * B, cudaMemcpyHostToDevice, st), "keys");
     // candidates: multiples of each instance's analytic size (the fragment
     // count of a tile 4 sigma below one shared-memory batch; 1.5 and 2 give
-    // tiles of two batches), timed as one whole persistent launch; the best
+    // tiles of two batches), timed as one whole launch; the best
     // of two repetitions counts
     const double mult[] = {0.5, 0.75, 1.0, 1.25, 1.5, 2.0};
     double best = 1e300;

@@ -172,9 +172,10 @@ constexpr uint32_t SEQ_FRAGS_PER_BATCH = 1280;
 
 // The insert-size lookup of a 31-bit word v: entry g = v >> 21 of the guide
 // covers the words of one cell and holds k, the first index whose threshold
-// exceeds the cell's first word (bits 0-9), the last word of the cell that
-// still gets k, relative to the cell's first (bits 10-30), and whether later
-// words need a walk over the thresholds (bit 31; else they get k + 1).  Tables
+// exceeds the cell's first word (bits 0-9), whether words past that threshold
+// need a walk over the following ones (bit 10; else they get k + 1), and the
+// last word of the cell that still gets k, relative to the cell's first (bits
+// 11-31: one comparison with the word's own low bits at the top).  Tables
 // of at most SEQ_GUIDE_INS thresholds have a guide: 1024 cells leave about
 // one word in a hundred of a normal-shaped table to the walk (256 left one in
 // thirty, so that most warps had a lane in it).
@@ -185,9 +186,9 @@ inline uint32_t insert_guide(const uint32_t* thr, uint32_t n, uint32_t g, uint32
   const uint32_t first = g << 21, next = first + (1u << 21);   // cells end at 2^31 at the latest
   while (at < n && thr[at] <= first) ++at;
   const uint32_t lo = at;
-  if (lo >= n || thr[lo] >= next) return (lo < n ? lo : n - 1) | 0x7ffffc00u;
+  if (lo >= n || thr[lo] >= next) return (lo < n ? lo : n - 1) | 0xfffff800u;
   const bool walk = lo + 1 >= n || thr[lo + 1] < next;
-  return lo | (thr[lo] - first - 1u) << 10 | (walk ? 0x80000000u : 0u);
+  return lo | (thr[lo] - first - 1u) << 11 | (walk ? 0x400u : 0u);
 }
 
 struct SeqTiles {
@@ -252,6 +253,11 @@ struct SeqParams {
   const uint32_t* opt_nleaf;      // 0: the normal cells
   const uint32_t* cls_leaf_tin;   // every sample's leaves grouped by class (Euler indices)
   const uint32_t* opt_cdf;        // option thresholds (see SeqSample)
+  // for a tile inside one atom: the atom (else 0xffffffff), and the draw
+  // tables of (sample, atom), row sample * n_atoms + atom (see CnRow)
+  const uint32_t* tile_atom;
+  const struct CnRow* cn_rows;
+  uint32_t n_atoms;
   const uint32_t* nmask;          // unknown reference bases (N), one bit each, or NULL (SAM output)
 };
 
@@ -266,6 +272,7 @@ void seq_make_tiles(uint32_t n_slots, const uint32_t* c_first, const uint32_t* c
 void seq_tile_parts(uint32_t n_tiles, const uint32_t* tile_start, const uint32_t* tile_len,
                     const uint32_t* atom_start, uint32_t n_atoms, uint32_t genome_len, uint32_t* part_off,
                     uint32_t* scan_part, uint32_t* part_start, uint32_t* part_len, uint32_t* part_atom,
+                    uint32_t* tile_atom,
                     cudaStream_t st);
 // Per (sample, tile) its integer copy sums (I0, S) (scratch tile_sums,
 // 2 * n_samples * n_tiles) and, for tiles of several parts, the thresholds
@@ -310,6 +317,20 @@ void seq_sam_reads(const SeqRec* recs, uint32_t n_recs, const uint32_t* aux, con
 // (sample, tile) pairs, sample-major; every table row below is relative to
 // the instance's offsets, so each instance computes exactly what the plain
 // path computes for it alone with the same tile size and seed.
+// The copy-number draw tables of one (atom, sample), laid out for a read CTA:
+// per cell option its threshold (the last one takes what is left; unused ones
+// past any 31-bit word), its covering instances, leaves, first leaf and the
+// mate tag of its first instance.  The instances of all options are numbered
+// through as local ids (the instance of id l: linst[l]); n_ids exceeds
+// SEQ_CN_IDS when they, or the options, do not fit (the row is then not used).
+constexpr uint32_t SEQ_CN_OPTS = 8, SEQ_CN_IDS = 16;
+struct alignas(16) CnRow {
+  uint32_t thr[SEQ_CN_OPTS];
+  uint4 opt[SEQ_CN_OPTS];
+  uint32_t linst[SEQ_CN_IDS];
+  uint32_t n_ids, pad[3];
+};
+
 struct SeqInst {
   SeqParams prm;
   uint32_t n_samples, sample_off;   // rows of the batch's SeqSample array
@@ -327,9 +348,8 @@ struct SeqBatch {
   const SeqInst* inst;
   const Key* keys;                  // sequencing key of each instance
   const uint32_t* rec_off;          // n_inst + 1: records of instance i (filled by placement)
-  const uint32_t* item_off;         // n_inst + 1: first work item of each instance
   const uint32_t* cnt_off;          // n_inst + 1: first tile-split warp of each instance
-  uint32_t n_items, n_cnt, n_tiles_all;
+  uint32_t max_samples, n_cnt, n_tiles_all;
   const uint32_t *tile_start, *tile_len, *tile_end, *tile_inst;
   uint32_t *rec_lo, *rec_hi;        // per tile, relative to the instance's first record
   const uint32_t *c_first, *c_ntiles, *c_depth, *c_nstarts, *c_id;
@@ -339,7 +359,6 @@ struct SeqBatch {
   const SeqSample* samples;
   const uint32_t* leaf_tin;
   const uint32_t *etin, *etout;
-  uint32_t* counter;                // work-item counter of the persistent read kernel
   uint32_t *alt, *depth;
 };
 // batched placement (launchers in pg_place.cu): cells of instance i are
@@ -367,13 +386,11 @@ void sites_settle_batch(const PlaceTables* tabs, uint32_t n_inst, const uint32_t
 void sort_batch(const PlaceRaw& o, const uint16_t* inst_of, uint32_t n, uint32_t n_inst, uint64_t G, uint32_t* bcnt,
                 uint32_t* bfill, uint32_t* part, uint32_t* order, const PlaceOut& sorted, uint16_t* inst_sorted,
                 unsigned long long* keys, cudaStream_t st);
-// resident CTAs per SM of the persistent read kernel
-int seq_reads_batch_occupancy();
 // records of the first *n_dev sorted mutations of a batch (cap >= *n_dev)
 void seq_batch_records(const PlaceOut& sorted, const uint16_t* inst_sorted, const uint32_t* n_dev, uint32_t cap,
                        const SeqBatch& b, SeqRec* recs, cudaStream_t st);
-// tile split, record ranges and the persistent read kernel over every work item
-void seq_batch_reads(const SeqBatch& b, const SeqRec* recs, uint32_t grid, cudaStream_t st);
+// tile split, record ranges and the read kernel over every (tile, sample)
+void seq_batch_reads(const SeqBatch& b, const SeqRec* recs, cudaStream_t st);
 void seq_build_records(const PlaceOut& sorted, uint32_t n, const uint32_t* edge_tin, const uint32_t* edge_tout,
                        SeqRec* recs, cudaStream_t st);
 void seq_tile_ranges(const SeqRec* recs, uint32_t n_recs, const uint32_t* start, const uint32_t* len,
@@ -395,6 +412,8 @@ void seq_tile_counts(uint32_t n_samples, uint32_t n_slots, uint32_t max_tiles, c
 void seq_active_flags(const uint32_t* alt, uint32_t n_samples, uint64_t M, uint32_t* flag, cudaStream_t st);
 void seq_active_gather(const uint32_t* alt, const uint32_t* depth, uint32_t n_samples, uint64_t M, const uint32_t* pos,
                        uint32_t n_active, uint32_t* index, uint32_t* a_out, uint32_t* d_out, cudaStream_t st);
+// the rows prm.cn_rows of n_samples samples (prm's other copy-number fields set)
+void seq_cn_rows(const SeqParams& prm, const SeqSample* samples, uint32_t n_samples, CnRow* rows, cudaStream_t st);
 void seq_reads(const SeqRec* recs, uint32_t n_recs, const SeqTiles& tiles, const uint32_t* pair_cnt,
                const SeqSample* samples, uint32_t n_samples, const uint32_t* leaf_tin, const SeqParams& prm,
                uint64_t seed, uint32_t* alt, uint32_t* depth, cudaStream_t st);

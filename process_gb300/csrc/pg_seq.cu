@@ -33,22 +33,22 @@
 //   phase A  every thread generates fragments (one Philox block each); their
 //            two mates go to shared memory in the order of their start
 //            buckets (16 bp, counting sort);
-//   phase B  four lanes share a mutation record and visit the mates of the
+//   phase B  a few lanes share a mutation record and visit the mates of the
 //            buckets that may cover it, counting depth and alt in registers.
 // Windows with more records than shared memory holds run a per-read loop on
 // the global arrays instead.
 //
-// Bound by instruction issue (62% of the slots, 11 warp instructions per
-// fragment) and by shared-memory wavefronts (72%), not by HBM.  At 155 Mbp,
-// 100x paired, four samples with copy-number events (2.07e8 fragments) the
-// launch takes 2.88 ms.  The form with evenly split candidate runs (a thread
-// walks 17 or so candidates across record borders), a lineage walk and two
-// table lookups per draw took 4.53 ms at 18.6 warp instructions per fragment.
-// Lanes per record in phase B, same launch: 32 3.50 ms, 16 3.37, 8 3.01,
-// 4 2.92 (2.89 with two candidates per step), 2 2.87: fewer lanes amortise a
-// record's set-up over more records per warp; four keeps more warps busy
-// where windows hold few records.  One batch per tile in CTAs of 512 threads
-// took 3.25 ms.
+// Bound by shared-memory wavefronts (73% of the pipe; about 90 per 32
+// fragments: 35 for the counting sort, 35 for the visits, the draws' lookups)
+// and instruction issue (60%, 10 warp instructions per fragment) around four
+// barriers a batch, not by HBM.  At 155 Mbp, 100x paired, four samples with
+// copy-number events (2.07e8 fragments) the launch takes 2.64 ms.  The form
+// with evenly split candidate runs (a thread walks 17 or so candidates across
+// record borders), a lineage walk and two table lookups per draw took 4.53 ms
+// at 18.6 warp instructions per fragment; with the draws in absolute
+// positions, an eight-way option comparison and the tile's copy-number tables
+// gathered in the kernel, 2.88 ms.  Two fragments' draws interleaved per
+// thread (2.72), one batch per tile in CTAs of 512 threads (3.25) were slower.
 #include <type_traits>
 
 #include "pg_common.cuh"
@@ -62,7 +62,6 @@ namespace pg {
 constexpr int SEQ_THREADS = 256;
 constexpr uint32_t SEQ_CAP = 512;        // mutation records staged per CTA
 constexpr uint32_t SEQ_MCAP = 2 * SEQ_FRAGS_PER_BATCH;   // mates per batch
-constexpr uint32_t SEQ_REC_LANES = 4;    // lanes that share a record in phase B
 constexpr uint32_t SEQ_BW = 16;          // start bucket width (bp)
 constexpr uint32_t SEQ_NBK = 1024;       // start buckets per window (window <= 16 kbp)
 static_assert(SEQ_NBK == 4 * SEQ_THREADS, "the bucket scan takes four buckets per thread");
@@ -299,50 +298,85 @@ struct Fragment {
 };
 
 // The copy-number draw tables of one (tile, sample) staged in shared memory:
-// the tile's parts with their thresholds and, per part, the option
-// thresholds of its atom (unused ones past any 31-bit word) and each option's
-// covering instances there.  The instances of all (part, option) pairs are
-// numbered through as local ids (the instance of id l: linst[l]), so that a
+// the tile's parts with their thresholds and, per part, a CnRow's tables for
+// its atom, the local ids numbered through over the parts.  With them a
 // fragment's instance draw needs no lookup and a record can hold the set of
-// instances that carry it as a bit mask over the ids.
-constexpr uint32_t SEQ_CN_PARTS = 4, SEQ_CN_OPTS = 8, SEQ_CN_IDS = 16;
+// instances that carry it as a bit mask over the ids.  Almost every tile lies
+// in one atom: its tables come as a row made once per call, one load after
+// the tile's header, where reading them here through part, atom and class
+// held the CTA back for five dependent loads.
+constexpr uint32_t SEQ_CN_PARTS = 4;
 struct CnCache {
-  uint4 othr[SEQ_CN_PARTS][SEQ_CN_OPTS / 4];   // option thresholds
-  uint4 opt[SEQ_CN_PARTS][SEQ_CN_OPTS];        // covering instances, leaves, first leaf, first local id
+  uint4 othr[SEQ_CN_PARTS][SEQ_CN_OPTS];       // option thresholds (.x; the stride of opt, so that one offset serves both)
+  uint4 opt[SEQ_CN_PARTS][SEQ_CN_OPTS];        // covering instances, leaves, first leaf, tag of the first instance
+  uint4 linst[SEQ_CN_IDS / 4];
   uint32_t pstart[SEQ_CN_PARTS], plen[SEQ_CN_PARTS], pthr[SEQ_CN_PARTS];
-  uint32_t linst[SEQ_CN_IDS];
-  uint32_t n_parts, n_opt, n_ids;
+  uint32_t n_parts, n_ids;
 };
 
-// one warp fills the cache; n_ids exceeds SEQ_CN_IDS when the local ids do
-// not fit (linst is then incomplete and the cache is not used)
+// one option's draw table entries in an atom: its threshold, {covering
+// instances, leaves, first leaf, 0} and the offset of its instance list
+__device__ __forceinline__ uint32_t cn_option(const SeqParams& prm, const SeqSample& sm, uint32_t atom, uint32_t o,
+                                              uint4& op, uint32_t& ioff) {
+  const uint32_t ai = atom * prm.n_classes + prm.opt_class[sm.opt_off + o];
+  ioff = prm.atom_ioff[ai];
+  op = make_uint4(prm.atom_icnt[ai], prm.opt_nleaf[sm.opt_off + o], prm.opt_leaf_off[sm.opt_off + o], 0u);
+  return o + 1 < sm.n_opt ? prm.opt_cdf[sm.opt_cdf_off + atom * sm.n_opt + o] : 0xffffffffu;
+}
+// the mate tag of local id l (see ReadSmem), or that of a dropped fragment
+__device__ __forceinline__ uint32_t cn_tag(uint32_t icnt, uint32_t l) { return icnt ? 0x10000u << (l & 15u) : 0x8000u; }
+
+// one warp fills the cache of a tile of up to SEQ_CN_PARTS parts (and the
+// sample of up to SEQ_CN_OPTS options); linst is incomplete when n_ids
+// exceeds SEQ_CN_IDS
 __device__ __forceinline__ void fill_cn_cache(CnCache& c, const SeqParams& prm, const SeqSample& sm, uint32_t t,
                                               uint32_t s, uint32_t lane) {
-  const uint32_t pb = prm.part_off[t], pn = prm.part_off[t + 1] - pb, no = sm.n_opt;
+  const uint32_t pb = prm.part_off[t], pn = prm.part_off[t + 1] - pb;
   if (lane < pn) {
     c.pstart[lane] = prm.part_start[pb + lane];
     c.plen[lane] = prm.part_len[pb + lane];
     c.pthr[lane] = prm.part_cdf[uint64_t(s) * prm.n_parts + pb + lane];
   }
   const uint32_t p = lane / SEQ_CN_OPTS, o = lane % SEQ_CN_OPTS;   // SEQ_CN_PARTS x SEQ_CN_OPTS = 32 lanes
-  const bool mine = p < pn && o < no;
-  uint32_t thr = 0xffffffffu, icnt = 0, ioff = 0, nl = 0, lo = 0;
-  if (mine) {
-    const uint32_t atom = prm.part_atom[pb + p];
-    thr = prm.opt_cdf[sm.opt_cdf_off + atom * no + o];
-    const uint32_t ai = atom * prm.n_classes + prm.opt_class[sm.opt_off + o];
-    ioff = prm.atom_ioff[ai];
-    icnt = prm.atom_icnt[ai];
-    nl = prm.opt_nleaf[sm.opt_off + o];
-    lo = prm.opt_leaf_off[sm.opt_off + o];
-  }
-  const uint32_t incl = warp_incl_scan(icnt), id0 = incl - icnt;
-  reinterpret_cast<uint32_t*>(c.othr[p])[o] = thr;
-  c.opt[p][o] = make_uint4(icnt, nl, lo, id0);
-  for (uint32_t i = 0; i < icnt && id0 + i < SEQ_CN_IDS; ++i) c.linst[id0 + i] = prm.gc.inst_list[ioff + i];
-  if (lane == 31) { c.n_parts = pn; c.n_opt = no; c.n_ids = incl; }
+  uint32_t thr = 0xffffffffu, ioff = 0;
+  uint4 op = make_uint4(0u, 0u, 0u, 0u);
+  if (p < pn && o < sm.n_opt) thr = cn_option(prm, sm, prm.part_atom[pb + p], o, op, ioff);
+  const uint32_t incl = warp_incl_scan(op.x), id0 = incl - op.x;
+  op.w = cn_tag(op.x, id0);
+  c.othr[p][o].x = thr;
+  c.opt[p][o] = op;
+  uint32_t* linst = reinterpret_cast<uint32_t*>(c.linst);
+  for (uint32_t i = 0; i < op.x && id0 + i < SEQ_CN_IDS; ++i) linst[id0 + i] = prm.gc.inst_list[ioff + i];
+  if (lane == 31) { c.n_parts = pn; c.n_ids = incl; }
 }
 static_assert(SEQ_CN_PARTS * SEQ_CN_OPTS == 32 && SEQ_CN_OPTS == 8, "one lane per (part, option)");
+
+// the same tables of whole atoms: eight lanes per (sample, atom)
+__global__ void k_cn_rows(SeqParams prm, const SeqSample* __restrict__ samples, uint32_t n_samples,
+                          CnRow* __restrict__ rows) {
+  const uint64_t row = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / SEQ_CN_OPTS;
+  const uint32_t o = threadIdx.x % SEQ_CN_OPTS;
+  const bool mine = row < uint64_t(n_samples) * prm.n_atoms;
+  const SeqSample sm = samples[mine ? row / prm.n_atoms : 0];
+  const bool fits = sm.n_opt <= SEQ_CN_OPTS;
+  uint32_t thr = 0xffffffffu, ioff = 0;
+  uint4 op = make_uint4(0u, 0u, 0u, 0u);
+  if (mine && fits && o < sm.n_opt) thr = cn_option(prm, sm, uint32_t(row % prm.n_atoms), o, op, ioff);
+  uint32_t incl = op.x;
+#pragma unroll
+  for (uint32_t d = 1; d < SEQ_CN_OPTS; d <<= 1) {
+    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d, SEQ_CN_OPTS);
+    if (o >= d) incl += v;
+  }
+  if (!mine) return;
+  const uint32_t id0 = incl - op.x;
+  op.w = cn_tag(op.x, id0);
+  CnRow& r = rows[row];
+  r.thr[o] = thr;
+  r.opt[o] = op;
+  for (uint32_t i = 0; i < op.x && id0 + i < SEQ_CN_IDS; ++i) r.linst[id0 + i] = prm.gc.inst_list[ioff + i];
+  if (o == SEQ_CN_OPTS - 1) r.n_ids = fits ? incl : 0xffffffffu;
+}
 
 // cdf_lookup for tables of at most NMAX (a power of two) thresholds: the
 // count of thresholds <= u >> 1 by binary lifting, without a data-dependent
@@ -363,10 +397,6 @@ __device__ __forceinline__ uint32_t part_offset(uint32_t u, uint32_t lo, uint32_
   return uint32_t((uint64_t((u >> 1) - lo) * plen) / uint64_t(hi - lo));
 }
 
-// CN selects the copy-number path at compile time (0: no copy-number
-// events, 1: the tile's tables in shared memory, and inst is the mate tag of
-// the drawn local id (see ReadSmem), 2: the tables in global memory) or, -1, at run time from prm.has_cna
-// (0 or 2).
 // (KeyT: Key, or the precomputed RoundKeys of the same key)
 __device__ __forceinline__ U4 pair_block(const Key& key, uint32_t j, uint32_t t, uint32_t s) {
   return philox(key.k0, key.k1, j, t, s, TAG_PAIR);
@@ -375,40 +405,34 @@ __device__ __forceinline__ U4 pair_block(const RoundKeys& rk, uint32_t j, uint32
   return philox(rk, j, t, s, TAG_PAIR);
 }
 
-template <bool INS_SMEM, int CN = -1, class KeyT>
+// index of the insert size: by the guide (one lookup, but where several
+// thresholds share the word's cell) or by binary search
+template <bool GUIDE>
+__device__ __forceinline__ uint32_t insert_index(const SeqParams& prm, const uint32_t* guide, uint32_t u) {
+  if (!GUIDE) return cdf_lookup(prm.ins_cdf, prm.n_ins, u);
+  const uint32_t g = guide[u >> 22];
+  const bool past = (u << 10) > (g | 0x7ffu);
+  uint32_t k = (g & 1023u) + (past ? 1u : 0u);
+  if (past && (g & 1024u))
+    while (__ldg(prm.ins_cdf + k) <= (u >> 1)) ++k;   // the last threshold is 2^31, past every word
+  return k;
+}
+
+// CN: with copy-number events (0, 1), or as prm.has_cna says (-1)
+template <bool GUIDE, int CN = -1, class KeyT>
 __device__ __forceinline__ Fragment make_fragment(const KeyT& key, uint32_t j, uint32_t t, uint32_t s, uint32_t start,
                                                   uint32_t len, uint32_t ce, const SeqSample& sm,
                                                   const uint32_t* __restrict__ leaf_tin, const SeqParams& prm,
-                                                  const uint32_t* guide, const CnCache* cc = nullptr) {
+                                                  const uint32_t* guide) {
   const U4 r = pair_block(key, j, t, s);
   Fragment f;
   const uint32_t R = prm.read_len;
-  const int path = CN >= 0 ? CN : (!prm.has_cna ? 0 : 2);
-  if (path == 0) {
+  if (CN == 0 || (CN < 0 && !prm.has_cna)) {
     f.p0 = start + __umulhi(r.x, len);
     const bool normal = sm.all_normal || r.y < sm.normal_thr;
     f.inst = __umulhi(r.w, prm.n_alleles);
     f.cell = normal ? prm.normal_tin
                     : __ldg(leaf_tin + sm.leaf_off + __umulhi(r.w * prm.n_alleles, sm.n_leaves));
-  } else if (path == 1) {
-    uint32_t part = 0;
-    if (cc->n_parts > 1) {
-      part = cdf_lookup_small<SEQ_CN_PARTS>(cc->pthr, cc->n_parts, r.x);
-      f.p0 = cc->pstart[part] + part_offset(r.x, part ? cc->pthr[part - 1] : 0u, cc->pthr[part], cc->plen[part]);
-    } else {
-      f.p0 = cc->pstart[0] + __umulhi(r.x, cc->plen[0]);
-    }
-    // the option: the number of thresholds at or below the 31-bit word
-    const uint32_t v = r.y >> 1, no = cc->n_opt;
-    const uint4 h = cc->othr[part][0];
-    uint32_t o = uint32_t(h.x <= v) + uint32_t(h.y <= v) + uint32_t(h.z <= v) + uint32_t(h.w <= v);
-    if (no > 4) {
-      const uint4 g = cc->othr[part][1];
-      o += uint32_t(g.x <= v) + uint32_t(g.y <= v) + uint32_t(g.z <= v) + uint32_t(g.w <= v);
-    }
-    const uint4 op = cc->opt[part][min(o, no - 1)];   // {covering instances, leaves, first leaf, first id}
-    f.inst = op.x ? 0x10000u << ((op.w + __umulhi(r.w, op.x)) & 15u) : 0x8000u;
-    f.cell = op.y ? __ldg(prm.cls_leaf_tin + op.z + __umulhi(r.w * op.x, op.y)) : prm.normal_tin;
   } else {
     const uint32_t pb = __ldg(prm.part_off + t), pn = __ldg(prm.part_off + t + 1) - pb;
     uint32_t part = pb;
@@ -432,18 +456,7 @@ __device__ __forceinline__ Fragment make_fragment(const KeyT& key, uint32_t j, u
   f.w = r.x ^ r.y ^ r.z ^ r.w;
   f.p1 = f.p0;
   if (prm.paired) {
-    uint32_t k;
-    if (INS_SMEM) {
-      // one lookup, but where several thresholds share the word's cell
-      const uint32_t g = guide[r.z >> 22];
-      const bool past = (g & 0x7ffffc00u) < ((r.z << 9) & 0x7ffffc00u);
-      k = (g & 1023u) + (past ? 1u : 0u);
-      if (past && int32_t(g) < 0)
-        while (__ldg(prm.ins_cdf + k) <= (r.z >> 1)) ++k;   // the last threshold is 2^31, past every word
-    } else {
-      k = cdf_lookup(prm.ins_cdf, prm.n_ins, r.z);
-    }
-    uint32_t p1 = f.p0 + prm.ins_min + k - R;
+    uint32_t p1 = f.p0 + prm.ins_min + insert_index<GUIDE>(prm, guide, r.z) - R;
     if (p1 > ce - R) p1 = ce - R;
     f.p1 = p1;
   }
@@ -477,15 +490,15 @@ struct ReadSmem {
 //
 // The fragments go through in batches.  Phase A draws them, a histogram's
 // atomics giving each mate its rank in its 16 bp start bucket, and places the
-// mates in bucket order.  Phase B takes one record per warp: its candidate
+// mates in bucket order.  Phase B takes a record per group of lanes: its candidate
 // mates (those starting in the buckets of [L - R + 1, L]) are one contiguous
-// run, visited 32 at a time with the record's terms the same in every lane.
+// run, dealt out to the record's lanes.
 // Instruction issue bounds the kernel, so what a visit needs is prepared per
 // record: "the mate's instance carries the mutation" is one bit of the
 // record's mask, and the error thresholds of an indel are 0.
 template <class KeyT>
 __device__ __forceinline__ void read_tile(ReadSmem& sh, const SeqRec* __restrict__ g_recs, uint32_t t, uint32_t s,
-                                          uint32_t n_pairs, uint32_t lo, uint32_t nw, uint32_t start, uint32_t len,
+                                          uint32_t atom, uint32_t n_pairs, uint32_t lo, uint32_t nw, uint32_t start, uint32_t len,
                                           uint32_t ce, const SeqSample& sm, const uint32_t* __restrict__ leaf_tin,
                                           const SeqParams& prm, const KeyT& key, uint32_t* __restrict__ g_alt_row,
                                           uint32_t* __restrict__ g_dep_row) {
@@ -520,17 +533,27 @@ __device__ __forceinline__ void read_tile(ReadSmem& sh, const SeqRec* __restrict
   }
 
   // copy-number draws from shared memory when the tile's tables fit
-  const bool cn_fits = prm.has_cna && prm.part_off[t + 1] - prm.part_off[t] <= SEQ_CN_PARTS &&
-                       sm.n_opt <= SEQ_CN_OPTS;
+  const bool row = prm.has_cna && atom != 0xffffffffu;
+  const bool parts = prm.has_cna && !row && sm.n_opt <= SEQ_CN_OPTS &&
+                     prm.part_off[t + 1] - prm.part_off[t] <= SEQ_CN_PARTS;
   // (the first records are on their way meanwhile)
   SeqRec r{};
   if (tid / 4 < nw) r = grec[tid / 4];
-  if (cn_fits && warp == 0) fill_cn_cache(sh.s_cn, prm, sm, t, s, lane);
+  if (row) {
+    const CnRow& cr = prm.cn_rows[uint64_t(s) * prm.n_atoms + atom];
+    if (tid < SEQ_CN_OPTS) sh.s_cn.othr[0][tid].x = __ldg(cr.thr + tid);
+    else if (tid < 2 * SEQ_CN_OPTS) sh.s_cn.opt[0][tid - SEQ_CN_OPTS] = __ldg(cr.opt + tid - SEQ_CN_OPTS);
+    else if (tid < 2 * SEQ_CN_OPTS + SEQ_CN_IDS / 4)
+      sh.s_cn.linst[tid - 2 * SEQ_CN_OPTS] = __ldg(reinterpret_cast<const uint4*>(cr.linst) + tid - 2 * SEQ_CN_OPTS);
+    else if (tid == 31) sh.s_cn.n_ids = __ldg(&cr.n_ids);
+  } else if (parts && warp == 0) {
+    fill_cn_cache(sh.s_cn, prm, sm, t, s, lane);
+  }
   if (ins_smem) sh.s_guide[tid] = __ldg(reinterpret_cast<const uint4*>(prm.ins_guide) + tid);
   __syncthreads();
-  const int cn = !prm.has_cna ? 0 : (cn_fits && sh.s_cn.n_ids <= SEQ_CN_IDS ? 1 : 2);
+  const int cn = !prm.has_cna ? 0 : !((row || parts) && sh.s_cn.n_ids <= SEQ_CN_IDS) ? 2 : row ? 1 : 3;
   // the records, four threads each (they share the walk over the local ids)
-  const uint32_t n_ids = cn == 1 ? sh.s_cn.n_ids : 0u;
+  const uint32_t n_ids = cn & 1 ? sh.s_cn.n_ids : 0u;
   for (uint32_t i0 = 0; i0 < nw; i0 += SEQ_THREADS / 4) {
     const uint32_t i = i0 + tid / 4, sub = tid % 4;
     if (i0 > 0 && i < nw) r = grec[i];
@@ -541,7 +564,7 @@ __device__ __forceinline__ void read_tile(ReadSmem& sh, const SeqRec* __restrict
       for (uint32_t l = sub; l < n_ids; l += 4) {
         // a copy has a larger instance number than its source, and instances
         // 0 and 1 have no source
-        const uint32_t y = sh.s_cn.linst[l];
+        const uint32_t y = reinterpret_cast<const uint32_t*>(sh.s_cn.linst)[l];
         if (y == x || (y > max(x, 1u) && inst_carries(prm, y, x, km))) m |= 1u << l;
       }
     m |= __shfl_xor_sync(0xffffffffu, m, 1);
@@ -554,6 +577,13 @@ __device__ __forceinline__ void read_tile(ReadSmem& sh, const SeqRec* __restrict
     }
   }
 
+  // phase B's lanes per record: as many as take all records in one pass (a
+  // second, nearly empty pass holds the CTA's other warps at the barrier), but
+  // 2 to 16, and 4 from three passes on.  Against 4 throughout: a batch of
+  // 24 genomes (5 to 60 records a window) 9.86 -> 9.38 ms, 81 records a
+  // window the same within 0.3%.
+  const uint32_t lsh = nw <= 16 ? 4u : nw <= 32 ? 3u : nw <= 64 ? 2u : nw <= 128 ? 1u : 2u;
+  const uint32_t lanes = 1u << lsh, sub = tid & (lanes - 1u);
   constexpr uint32_t per_batch = SEQ_MCAP / 2;
   constexpr uint32_t FPT = per_batch / SEQ_THREADS;   // fragments per thread and batch
   uint32_t* hist = reinterpret_cast<uint32_t*>(sh.s_hist);
@@ -567,28 +597,63 @@ __device__ __forceinline__ void read_tile(ReadSmem& sh, const SeqRec* __restrict
     // cleared by the last scan.)
     uint32_t o01[FPT], ca[FPT], fi[FPT], fw[FPT], rk01[FPT];
     // one instance of the draw code per (copy-number path, insert table)
-    // pair, chosen once per tile: the unrolled loop holds only that path
-    auto gen = [&](auto cn_tag, auto ins_tag) {
+    // pair, chosen once per tile: the unrolled loop holds only that path.
+    // The draws are make_fragment's, as window offsets and mate tags, and run
+    // in the lanes past the batch's end too (only their ranks are not taken).
+    auto gen = [&](auto path, auto insert) {
+      constexpr int CN = decltype(path)::value;           // 0 none, 1 one atom, 3 several, 2 tables in global memory
+      constexpr bool GUIDE = decltype(insert)::value;     // (paired)
+      const CnCache& cc = sh.s_cn;
+      const uint32_t* guide = reinterpret_cast<const uint32_t*>(sh.s_guide);
+      const uint32_t last = ce - R - start, ins0 = prm.ins_min - R;
+      const uint32_t t3 = CN == 1 ? cc.othr[0][3].x : 0u;
 #pragma unroll
       for (uint32_t q = 0; q < FPT; ++q) {
         const uint32_t k = tid + q * SEQ_THREADS;
-        if (k < nb_pairs) {
-          const Fragment f = make_fragment<decltype(ins_tag)::value, decltype(cn_tag)::value>(
-              key, b0 + k, t, s, start, len, ce, sm, leaf_tin, prm, reinterpret_cast<const uint32_t*>(sh.s_guide),
-              &sh.s_cn);
+        if (!__any_sync(0xffffffffu, k < nb_pairs)) break;
+        uint32_t o0, o1 = 0;
+        if constexpr (CN == 2) {
+          const Fragment f = make_fragment<GUIDE, 1>(key, b0 + k, t, s, start, len, ce, sm, leaf_tin, prm, guide);
+          o0 = f.p0 - start; o1 = f.p1 - start;
           ca[q] = f.cell;
-          if constexpr (decltype(cn_tag)::value == 0) fi[q] = 0x10000u << (f.inst & 15u);
-          else if constexpr (decltype(cn_tag)::value == 1) fi[q] = f.inst;
-          else fi[q] = f.inst == 0xffffu ? 0x8000u : f.inst << 16;
+          fi[q] = f.inst == 0xffffu ? 0x8000u : f.inst << 16;
           fw[q] = f.w;
-          const uint32_t o0 = f.p0 - start;
-          uint32_t rk = atomicAdd(hist + o0 / SEQ_BW, 1u);
-          uint32_t o1 = 0;
-          if (paired) {
-            o1 = f.p1 - start;
-            rk |= atomicAdd(hist + o1 / SEQ_BW, 1u) << 16;
+        } else {
+          const U4 r = pair_block(key, b0 + k, t, s);
+          uint32_t cell = prm.normal_tin;
+          if constexpr (CN == 0) {
+            o0 = __umulhi(r.x, len);
+            fi[q] = 0x10000u << (__umulhi(r.w, prm.n_alleles) & 15u);
+            if (!sm.all_normal && r.y >= sm.normal_thr)
+              cell = __ldg(leaf_tin + sm.leaf_off + __umulhi(r.w * prm.n_alleles, sm.n_leaves));
+          } else {
+            uint32_t part = 0;
+            if constexpr (CN == 1) {
+              o0 = __umulhi(r.x, len);
+            } else {
+              part = cdf_lookup_small<SEQ_CN_PARTS>(cc.pthr, cc.n_parts, r.x);
+              o0 = cc.pstart[part] - start +
+                   part_offset(r.x, part ? cc.pthr[part - 1] : 0u, cc.pthr[part], cc.plen[part]);
+            }
+            // the option: the number of thresholds at or below the 31-bit
+            // word, in units of the tables' stride
+            const char* thr = reinterpret_cast<const char*>(cc.othr[part]);
+            const uint32_t v = r.y >> 1;
+            uint32_t o = (CN == 1 ? t3 : cc.othr[part][3].x) <= v ? 64u : 0u;
+            if (*reinterpret_cast<const uint32_t*>(thr + o + 16) <= v) o += 32u;
+            if (*reinterpret_cast<const uint32_t*>(thr + o) <= v) o += 16u;
+            const uint4 op = *reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(cc.opt[part]) + o);
+            fi[q] = op.w << __umulhi(r.w, op.x);
+            if (op.y) cell = __ldg(prm.cls_leaf_tin + op.z + __umulhi(r.w * op.x, op.y));
           }
-          o01[q] = o0 | (o1 << 16);
+          ca[q] = cell;
+          fw[q] = r.x ^ r.y ^ r.z ^ r.w;
+          if (GUIDE || paired) o1 = min(o0 + ins0 + insert_index<GUIDE>(prm, guide, r.z), last);
+        }
+        o01[q] = o0 | (o1 << 16);
+        if (k < nb_pairs) {
+          uint32_t rk = atomicAdd(hist + o0 / SEQ_BW, 1u);
+          if (GUIDE || paired) rk |= atomicAdd(hist + o1 / SEQ_BW, 1u) << 16;
           rk01[q] = rk;
         }
       }
@@ -596,11 +661,13 @@ __device__ __forceinline__ void read_tile(ReadSmem& sh, const SeqRec* __restrict
     using T0 = std::integral_constant<int, 0>;
     using T1 = std::integral_constant<int, 1>;
     using T2 = std::integral_constant<int, 2>;
+    using T3 = std::integral_constant<int, 3>;
     using YES = std::true_type;
     using NO = std::false_type;
     if (cn == 0) { if (ins_smem) gen(T0{}, YES{}); else gen(T0{}, NO{}); }
     else if (cn == 1) { if (ins_smem) gen(T1{}, YES{}); else gen(T1{}, NO{}); }
-    else { if (ins_smem) gen(T2{}, YES{}); else gen(T2{}, NO{}); }
+    else if (cn == 2) { if (ins_smem) gen(T2{}, YES{}); else gen(T2{}, NO{}); }
+    else { if (ins_smem) gen(T3{}, YES{}); else gen(T3{}, NO{}); }
     __syncthreads();
     // bucket offsets: exclusive scan of the 1024 counts, four per thread,
     // the counts cleared for the next batch
@@ -634,12 +701,12 @@ __device__ __forceinline__ void read_tile(ReadSmem& sh, const SeqRec* __restrict
       }
     }
     __syncthreads();
-    // phase B: SEQ_REC_LANES lanes per record
+    // phase B: 1 << lsh lanes per record
     const uint32_t err_thr = prm.err_thr, err_t1 = prm.err_t1, R16 = R << 16, lc0 = start * ERR_LOCUS;
     auto visits = [&](auto ids_tag) {
       constexpr bool IDS = decltype(ids_tag)::value;
-      for (uint32_t i0 = 0; i0 < nw; i0 += SEQ_THREADS / SEQ_REC_LANES) {
-        const uint32_t i = i0 + tid / SEQ_REC_LANES;
+      for (uint32_t i0 = 0; i0 < nw; i0 += SEQ_THREADS >> lsh) {
+        const uint32_t i = i0 + (tid >> lsh);
         uint32_t acc = 0;                    // depth | alt << 16 (a batch holds 2560 mates)
         if (i < nw) {
           const uint4 r = sh.s_rec[i];
@@ -647,7 +714,7 @@ __device__ __forceinline__ void read_tile(ReadSmem& sh, const SeqRec* __restrict
           const uint32_t off16 = r.x & 0xffff0000u, lc = (r.x >> 16) * ERR_LOCUS + lc0;
           const uint32_t thr = (r.x & 1u) ? 0u : err_thr, t1 = (r.x & 1u) ? 0u : err_t1;
 #pragma unroll 2
-          for (uint32_t k = sh.s_boff[bnd & 0xffffu] + tid % SEQ_REC_LANES; k < e; k += SEQ_REC_LANES) {
+          for (uint32_t k = sh.s_boff[bnd & 0xffffu] + sub; k < e; k += lanes) {
             const uint32_t pi = sh.s_mpi[k];
             const uint2 cw = sh.s_mcw[k];
             // the mate covers L when its start o is in (L - R, L] (unsigned: o > off wraps)
@@ -670,9 +737,8 @@ __device__ __forceinline__ void read_tile(ReadSmem& sh, const SeqRec* __restrict
             if (cov) acc += one;
           }
         }
-#pragma unroll
-        for (uint32_t o = SEQ_REC_LANES / 2; o >= 1; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (acc && tid % SEQ_REC_LANES == 0) {
+        for (uint32_t o = lanes >> 1; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (acc && sub == 0) {
           uint2 c = sh.s_cnt[i];
           c.x += acc & 0xffffu;
           c.y += acc >> 16;
@@ -704,7 +770,8 @@ __global__ void __launch_bounds__(SEQ_THREADS, 4) k_reads(const SeqRec* __restri
   sh.s_hist[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
   const uint32_t lo = tiles.rec_lo[t];
   const SeqSample sm = samples[s];
-  read_tile(sh, g_recs, t, s, pair_cnt[uint64_t(s) * tiles.n_tiles + t], lo, tiles.rec_hi[t] - lo, tiles.start[t],
+  const uint32_t atom = prm.has_cna ? prm.tile_atom[t] : 0u;
+  read_tile(sh, g_recs, t, s, atom, pair_cnt[uint64_t(s) * tiles.n_tiles + t], lo, tiles.rec_hi[t] - lo, tiles.start[t],
             tiles.len[t], tiles.chr_end[t], sm, leaf_tin, prm, key, g_alt + uint64_t(s) * n_recs,
             g_dep + uint64_t(s) * n_recs);
 }
@@ -877,56 +944,29 @@ __global__ void __launch_bounds__(SPLIT_THREADS) k_tile_counts_b(SeqBatch b) {
                    b.pair_cnt + in.pair_off + uint64_t(s) * in.n_tiles + first);
 }
 
-// Persistent read kernel of a batch: each CTA takes work items from a global
-// counter until none is left; an item is one (instance, sample, tile).
+// Read kernel of a batch: CTA (x, y) takes tile x of all the instances' tiles
+// for the instance's sample y, if it has that many.  (Resident CTAs that took
+// items from a counter were no faster: 9.80 ms against 9.82 over 24 genomes.)
 static_assert(sizeof(SeqParams) % 4 == 0 && sizeof(SeqParams) / 4 <= SEQ_THREADS, "SeqParams staging");
 
 __global__ void __launch_bounds__(SEQ_THREADS, 4) k_reads_batch(SeqBatch b, const SeqRec* __restrict__ g_recs) {
   __shared__ __align__(16) ReadSmem sh;
-  __shared__ SeqParams s_prm;        // the item's instance parameters, staged once per instance change
-  __shared__ SeqSample s_sm;
-  __shared__ Key s_key;
-  __shared__ uint32_t s_item, s_inst, s_t, s_s, s_pairs, s_lo, s_nw, s_start, s_len, s_ce;
-  __shared__ const SeqRec* s_recs;
-  __shared__ uint64_t s_row;
-  uint32_t cur = 0xffffffffu;        // instance whose parameters s_prm holds
+  __shared__ SeqParams s_prm;
+  const uint32_t gt = blockIdx.x, s = blockIdx.y, i = b.tile_inst[gt];
+  const SeqInst& in = b.inst[i];
+  if (s >= in.n_samples) return;
   sh.s_hist[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
-  for (;;) {
-    if (threadIdx.x == 0) {
-      // decode the next work item once for the CTA
-      const uint32_t item = atomicAdd(b.counter, 1u);
-      s_item = item;
-      if (item < b.n_items) {
-        const uint32_t i = batch_index(b.item_off, b.n_inst, item);
-        const SeqInst& in = b.inst[i];
-        const uint32_t local = item - b.item_off[i];
-        const uint32_t s = local / in.n_tiles, t = local % in.n_tiles, gt = in.tile_off + t;
-        s_inst = i; s_t = t; s_s = s;
-        s_lo = b.rec_lo[gt]; s_nw = b.rec_hi[gt] - s_lo;
-        s_pairs = b.pair_cnt[in.pair_off + uint64_t(s) * in.n_tiles + t];
-        s_start = b.tile_start[gt]; s_len = b.tile_len[gt]; s_ce = b.tile_end[gt];
-        s_sm = b.samples[in.sample_off + s];
-        s_key = b.keys[i];
-        s_recs = g_recs + b.rec_off[i];
-        s_row = in.count_off + uint64_t(s) * in.count_stride;
-      }
-    }
-    __syncthreads();
-    if (s_item >= b.n_items) return;
-    const uint32_t i = s_inst;
-    if (i != cur) {                  // block-uniform
-      if (threadIdx.x < sizeof(SeqParams) / 4)
-        reinterpret_cast<uint32_t*>(&s_prm)[threadIdx.x] =
-            reinterpret_cast<const uint32_t*>(&b.inst[i].prm)[threadIdx.x];
-      cur = i;
-      __syncthreads();
-    }
-    read_tile(sh, s_recs, s_t, s_s, s_pairs, s_lo, s_nw, s_start, s_len, s_ce, s_sm, b.leaf_tin, s_prm, s_key,
-              b.alt + s_row, b.depth + s_row);
-    __syncthreads();
-  }
+  if (threadIdx.x < sizeof(SeqParams) / 4)
+    reinterpret_cast<uint32_t*>(&s_prm)[threadIdx.x] = reinterpret_cast<const uint32_t*>(&in.prm)[threadIdx.x];
+  const uint32_t t = gt - in.tile_off, lo = b.rec_lo[gt];
+  const uint64_t rows = in.count_off + uint64_t(s) * in.count_stride;
+  const SeqSample sm = b.samples[in.sample_off + s];
+  const uint32_t n_pairs = b.pair_cnt[in.pair_off + uint64_t(s) * in.n_tiles + t];
+  const SeqRec* recs = g_recs + b.rec_off[i];
+  __syncthreads();
+  read_tile(sh, recs, t, s, 0u, n_pairs, lo, b.rec_hi[gt] - lo, b.tile_start[gt], b.tile_len[gt], b.tile_end[gt], sm,
+            b.leaf_tin, s_prm, b.keys[i], b.alt + rows, b.depth + rows);
 }
-
 
 
 __global__ void k_make_tiles(uint32_t n_slots, const uint32_t* __restrict__ c_first,
@@ -967,7 +1007,7 @@ __global__ void k_part_emit(uint32_t n_tiles, const uint32_t* __restrict__ tile_
                             const uint32_t* __restrict__ tile_len, const uint32_t* __restrict__ atom_start,
                             uint32_t n_atoms, uint32_t genome_len, const uint32_t* __restrict__ part_off,
                             uint32_t* __restrict__ part_start, uint32_t* __restrict__ part_len,
-                            uint32_t* __restrict__ part_atom) {
+                            uint32_t* __restrict__ part_atom, uint32_t* __restrict__ tile_atom) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n_tiles) return;
   const uint32_t a = tile_start[t], b = a + tile_len[t];
@@ -977,6 +1017,7 @@ __global__ void k_part_emit(uint32_t n_tiles, const uint32_t* __restrict__ tile_
     const uint32_t hi = min(b, x + 1 < n_atoms ? atom_start[x + 1] : genome_len);
     part_start[q] = lo; part_len[q] = hi - lo; part_atom[q] = x;
   }
+  tile_atom[t] = q - part_off[t] == 1 ? part_atom[q - 1] : 0xffffffffu;
 }
 
 // mass of one stretch of starts with integer copy sums (i0, sum)
@@ -1095,13 +1136,13 @@ __global__ void __launch_bounds__(256) k_mass_prefix(uint32_t n_slots, const uin
 void seq_tile_parts(uint32_t n_tiles, const uint32_t* tile_start, const uint32_t* tile_len,
                     const uint32_t* atom_start, uint32_t n_atoms, uint32_t genome_len, uint32_t* part_off,
                     uint32_t* scan_part, uint32_t* part_start, uint32_t* part_len, uint32_t* part_atom,
-                    cudaStream_t st) {
+                    uint32_t* tile_atom, cudaStream_t st) {
   if (!n_tiles) return;
   k_part_counts<<<nblk(n_tiles), 256, 0, st>>>(n_tiles, tile_start, tile_len, atom_start, n_atoms, part_off);
   note_launch();
   scan_rows<uint32_t>(part_off, part_off, n_tiles, 1, scan_part, part_off + n_tiles, st);
   k_part_emit<<<nblk(n_tiles), 256, 0, st>>>(n_tiles, tile_start, tile_len, atom_start, n_atoms, genome_len,
-                                             part_off, part_start, part_len, part_atom);
+                                             part_off, part_start, part_len, part_atom, tile_atom);
   note_launch();
 }
 
@@ -1201,21 +1242,22 @@ void seq_reads(const SeqRec* recs, uint32_t n_recs, const SeqTiles& tiles, const
                                          alt, depth); note_launch();
 }
 
+void seq_cn_rows(const SeqParams& prm, const SeqSample* samples, uint32_t n_samples, CnRow* rows, cudaStream_t st) {
+  const uint64_t n = uint64_t(n_samples) * prm.n_atoms * SEQ_CN_OPTS;
+  if (n) { k_cn_rows<<<nblk(n), 256, 0, st>>>(prm, samples, n_samples, rows); note_launch(); }
+}
+
 void seq_batch_records(const PlaceOut& sorted, const uint16_t* inst_sorted, const uint32_t* n_dev, uint32_t cap,
                        const SeqBatch& b, SeqRec* recs, cudaStream_t st) {
   if (cap) { k_seq_records_b<<<nblk(cap), 256, 0, st>>>(sorted, inst_sorted, n_dev, cap, b, recs); note_launch(); }
 }
 
-int seq_reads_batch_occupancy() {
-  int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_reads_batch, SEQ_THREADS, 0) != cudaSuccess) return 1;
-  return n;
-}
-
-void seq_batch_reads(const SeqBatch& b, const SeqRec* recs, uint32_t grid, cudaStream_t st) {
+void seq_batch_reads(const SeqBatch& b, const SeqRec* recs, cudaStream_t st) {
   if (b.n_cnt) { k_tile_counts_b<<<nblk(uint64_t(b.n_cnt) * 32, SPLIT_THREADS), SPLIT_THREADS, 0, st>>>(b); note_launch(); }
-  if (b.n_tiles_all) { k_tile_ranges_b<<<nblk(b.n_tiles_all), 256, 0, st>>>(b, recs); note_launch(); }
-  cudaMemsetAsync(b.counter, 0, sizeof(uint32_t), st);
-  if (b.n_items) { k_reads_batch<<<grid, SEQ_THREADS, 0, st>>>(b, recs); note_launch(); }
+  if (!b.n_tiles_all) return;
+  k_tile_ranges_b<<<nblk(b.n_tiles_all), 256, 0, st>>>(b, recs); note_launch();
+  if (b.max_samples) {
+    k_reads_batch<<<dim3(b.n_tiles_all, b.max_samples), SEQ_THREADS, 0, st>>>(b, recs); note_launch();
+  }
 }
 }  // namespace pg

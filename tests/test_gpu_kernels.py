@@ -171,3 +171,29 @@ def test_index_strides(gpu_lib, orc, sampling, max_rep):
     for which, n in ((0, 32), (1, 83)):
         for k in range(n):
             np.testing.assert_array_equal(eng.read_index(which, k), o.read_index(which, k), err_msg=f"{which} {k}")
+
+
+@pytest.mark.parametrize("reads", [0, 3])
+@pytest.mark.parametrize("tile", [64, 192, 448, 1_088, 2_304, 2_560, 10_048])
+def test_read_windows_by_records(gpu_lib, orc, tile, reads):
+    """Windows of a few records to more than shared memory holds (0.05 per
+    position): every number of lanes that share a record, tiles in one atom
+    and across atoms, one and several batches of fragments."""
+    from process_gb300 import CNA, synth
+    from process_gb300.engine import seq_cfg, sequence_counts
+    w = synth.plain_3mbp(seed=12, n_leaves=50)
+    w.genome.chr_lengths = [30_000, 900, 20_011]
+    (na, _, _), (nb, _, _) = w.mutants
+    rate = {"SNV": 5e-5, "indel": 2e-6}
+    w.mutants = [(na, rate, [CNA("A", "1", 8_001, 12_000)]), (nb, rate, [CNA("D", "3", 1, 9_000, allele=1)])]
+    eng = synth.build_engine(w)
+    o = orc.OracleEngine.like(w)
+    f = w.forest
+    pf = eng.place_mutations(f, 2_000, 50, seed=6)
+    op = o.place(f, _forest_species(o, f), 2_000, 0, 50, 0, seed=6)
+    cfg = dict(error_rate=5e-3, purity=0.7, with_normal_sample=True, tile_size=tile, **READS[reads])
+    alt, dep = sequence_counts(pf, 23, **cfg).counts()
+    c, _ = seq_cfg(chr_index=eng._chr_index, **cfg)
+    oalt, odep, _ = op.sequence(c, 23, flavour=0)
+    np.testing.assert_array_equal(dep, odep)
+    np.testing.assert_array_equal(alt, oalt)
