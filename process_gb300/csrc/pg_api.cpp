@@ -1291,11 +1291,10 @@ pg_status pg_place_mutations(pg_engine* e, const pg_forest* f, uint32_t n_pre_sn
     tables.send();
     t.node_size = node_size_d.p;
     const uint64_t ncell = uint64_t(f->n + 1) * E;
-    DBuf<uint32_t> cnt_snv(P, ncell), cnt_id(P, ncell), off_snv(P, ncell), off_id(P, ncell);
-    DBuf<uint32_t> part(P, pg::scan_part_elems(ncell, 1)), tot(P, 2);
-    pg::place_edge_counts(t, cnt_snv.p, cnt_id.p, seed, n_pre_snv, n_pre_id, st);
-    pg::scan_rows<uint32_t>(cnt_snv.p, off_snv.p, ncell, 1, part.p, tot.p, st);
-    pg::scan_rows<uint32_t>(cnt_id.p, off_id.p, ncell, 1, part.p, tot.p + 1, st);
+    DBuf<uint32_t> cnt(P, 2 * ncell), part(P, pg::scan_part_elems(ncell, 2)), tot(P, 2);   // SNVs, then indels
+    const uint32_t *const off_snv = cnt.p, *const off_id = cnt.p + ncell;
+    pg::place_edge_counts(t, cnt.p, cnt.p + ncell, seed, n_pre_snv, n_pre_id, st);
+    pg::scan_rows<uint32_t>(cnt.p, cnt.p, ncell, 2, part.p, tot.p, st);
     // ---- class tables (segments) and instance lineage chains
     std::vector<uint32_t> seg_off{0}, seg_start, seg_end, seg_ioff, seg_icnt;
     std::vector<uint16_t> inst_list;
@@ -1407,7 +1406,7 @@ pg_status pg_place_mutations(pg_engine* e, const pg_forest* f, uint32_t n_pre_sn
       lost1 = DBuf<uint8_t>(P, n_slots);
       ck(cudaMemsetAsync(first.p, 0xff, sizeof(unsigned long long) * fcap, st), "memset");
     }
-    pg::place_first_round(t, o, seed, off_snv.p, off_id.p, uint32_t(n_snv), n_slots, first.p, fmask, lost1.p, err, st);
+    pg::place_first_round(t, o, seed, off_snv, off_id, uint32_t(n_snv), n_slots, first.p, fmask, lost1.p, err, st);
     pg::place_drivers(o, drv_d.p, uint32_t(drv.size()), n_slots, st);
     // the handle's host columns, while the first round runs
     pl->eng = e; pl->n_nodes = f->n; pl->n_samples = f->n_samples;
@@ -1440,21 +1439,21 @@ pg_status pg_place_mutations(pg_engine* e, const pg_forest* f, uint32_t n_pre_sn
         unsigned long long* const held = reinterpret_cast<unsigned long long*>(table.p);
         uint32_t* const keys = table.p + 2 * cap;
         ck(cudaMemsetAsync(table.p, 0xff, sizeof(uint32_t) * 3 * cap, st), "memset");
-        pg::sites_settle(t, o, seed, off_snv.p, off_id.p, uint32_t(n_snv), pend.p, n_next, n_tail, first.p, fmask,
+        pg::sites_settle(t, o, seed, off_snv, off_id, uint32_t(n_snv), pend.p, n_next, n_tail, first.p, fmask,
                          keys, held, cap, &ctl.p->tail, err, st);
       }
     } else if (pl->has_cna && n_slots > 0) {
-      pg::sites_covered(t, o, seed, off_snv.p, off_id.p, uint32_t(n_snv), n_slots, &ctl.p->tail, err, st);
+      pg::sites_covered(t, o, seed, off_snv, off_id, uint32_t(n_snv), n_slots, &ctl.p->tail, err, st);
     }
     // ---- sort by locus
     const uint32_t nb = pg::sort_num_buckets(e->G);
-    DBuf<uint32_t> bcnt(P, nb), bfill(P, nb), bpart(P, pg::scan_part_elems(nb, 1)), order(P, n_all);
+    DBuf<uint32_t> bcnt(P, 2 * uint64_t(nb)), bpart(P, pg::scan_part_elems(nb, 1)), order(P, n_all);
     pl->locus = DBuf<uint32_t>(P, n_all); pl->edge = DBuf<uint32_t>(P, n_all); pl->aux = DBuf<uint32_t>(P, n_all);
     pl->cls = DBuf<uint8_t>(P, n_all); pl->sig = DBuf<uint8_t>(P, n_all); pl->allele = DBuf<uint16_t>(P, n_all);
     pl->seq = DBuf<uint16_t>(P, n_all);
     pl->kind = DBuf<uint8_t>(P, n_all); pl->nature = DBuf<uint8_t>(P, n_all);
     DBuf<unsigned long long> skeys(P, n_all);
-    pg::sort_by_locus(o, uint32_t(n_all), e->G, bcnt.p, bfill.p, bpart.p, order.p, pl->view(), skeys.p, st);
+    pg::sort_by_locus(o, uint32_t(n_all), e->G, bcnt.p, bpart.p, order.p, pl->view(), skeys.p, st);
     Ctl c{};
     timer.mark();
     ck(cudaMemcpyAsync(&c, ctl.p, sizeof(c), cudaMemcpyDeviceToHost, st), "error flag");
@@ -2021,17 +2020,20 @@ void simulate_seq_impl(const pg_placed* pl, const pg_seq_cfg* c, uint64_t seed, 
     }
     tables.send();
     DBuf<uint32_t> ts_d(P, n_tiles), tl_d(P, n_tiles), te_d(P, n_tiles);
-    pg::seq_make_tiles(uint32_t(c_first.size()), cf_d.p, cnt_d.p, cst_d.p, cns_d.p, cen_d.p, T, n_tiles, ts_d.p, tl_d.p,
-                       te_d.p, st);
     DBuf<pg::SeqRec> recs(P, pl->M);
     DBuf<uint32_t> pair_cnt(P, uint64_t(n_tiles) * samples.size()), rlo(P, n_tiles), rhi(P, n_tiles);
-    pg::seq_build_records(pl->view(), uint32_t(pl->M), etin_d.p, etout_d.p, recs.p, st);
+    const uint32_t n_slots = uint32_t(c_id.size()), NS = uint32_t(samples.size());
+    const pg::SeqChroms chroms{n_slots, cf_d.p, cnt_d.p, cst_d.p, cns_d.p, cen_d.p, cd_d.p, cid_d.p, cp_d.p, T, n_tiles,
+                               max_tiles};
+    pg::SeqTiles tiles{n_tiles, ts_d.p, tl_d.p, te_d.p, rlo.p, rhi.p};
+    pg::seq_prepare(chroms, tiles, pl->view(), uint32_t(pl->M), etin_d.p, etout_d.p, span, recs.p,
+                    pl->has_cna ? 0u : NS, seed, pair_cnt.p, st);
     DBuf<double> mcum_d, mtot_d;
     DBuf<uint32_t> poff_d, pstart_d, plen_d, patom_d, pcdf_d, tatom_d;
     DBuf<pg::CnRow> cnrow_d;
     uint32_t n_parts_cap = 0;
     if (pl->has_cna) {
-      const uint32_t NS = uint32_t(samples.size()), NA = uint32_t(pl->atom_start_h.size());
+      const uint32_t NA = uint32_t(pl->atom_start_h.size());
       n_parts_cap = n_tiles + NA;   // each atom boundary splits at most one tile
       poff_d = DBuf<uint32_t>(P, uint64_t(n_tiles) + 1);
       pstart_d = DBuf<uint32_t>(P, n_parts_cap); plen_d = DBuf<uint32_t>(P, n_parts_cap);
@@ -2047,12 +2049,8 @@ void simulate_seq_impl(const pg_placed* pl, const pg_seq_cfg* c, uint64_t seed, 
       pg::seq_tile_mass(NS, uint32_t(c_id.size()), cf_d.p, cnt_d.p, poff_d.p, plen_d.p, patom_d.p, NA, wn_d.p,
                         wt_d.p, nl_d.p, i0_d.p, cs_d.p, n_tiles, n_parts_cap, tsums.p, mcum_d.p, mtot_d.p, pcdf_d.p,
                         st);
+      pg::seq_tile_counts(chroms, NS, mcum_d.p, mtot_d.p, seed, pair_cnt.p, st);
     }
-    pg::seq_tile_counts(uint32_t(samples.size()), uint32_t(c_id.size()), max_tiles, cf_d.p, cnt_d.p, cd_d.p, cns_d.p,
-                        cid_d.p, cp_d.p, T, n_tiles, pl->has_cna ? mcum_d.p : nullptr,
-                        pl->has_cna ? mtot_d.p : nullptr, seed, pair_cnt.p, st);
-    pg::seq_tile_ranges(recs.p, uint32_t(pl->M), ts_d.p, tl_d.p, n_tiles, span, rlo.p, rhi.p, st);
-    pg::SeqTiles tiles{n_tiles, ts_d.p, tl_d.p, te_d.p, rlo.p, rhi.p};
     pg::SeqParams prm{};
     prm.read_len = R; prm.paired = paired ? 1u : 0u; prm.span = span;
     prm.ins_min = ins_min; prm.n_ins = uint32_t(ins_thr.size()); prm.ins_cdf = ins_d.p;

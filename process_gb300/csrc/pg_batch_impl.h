@@ -109,11 +109,11 @@ void batch_place(pg_batch* b, const uint64_t* place_seed) {
   for (uint32_t i = 0; i < B; ++i) keys[i] = pg::make_key(place_seed[i]);
   ck(cudaMemcpyAsync(b->pkeys.p, keys.data(), sizeof(pg::Key) * B, cudaMemcpyHostToDevice, st), "keys");
   const uint32_t n_cells = b->cell_off[B];
-  DBuf<uint32_t> cnt_snv(P, n_cells), cnt_id(P, n_cells), part(P, pg::scan_part_elems(n_cells, 1)), tot(P, 2);
+  DBuf<uint32_t> cnt(P, 2 * uint64_t(n_cells)), part(P, pg::scan_part_elems(n_cells, 2)), tot(P, 2);   // SNVs, then indels
+  uint32_t *const cnt_snv = cnt.p, *const cnt_id = cnt.p + n_cells;
   pg::place_edge_counts_batch(b->tabs.p, B, b->node_off_d.p, b->node_off[B], b->cell_off_d.p, b->pkeys.p,
-                              b->pre_snv_d.p, b->pre_id_d.p, cnt_snv.p, cnt_id.p, st);
-  pg::scan_rows<uint32_t>(cnt_snv.p, cnt_snv.p, n_cells, 1, part.p, tot.p, st);
-  pg::scan_rows<uint32_t>(cnt_id.p, cnt_id.p, n_cells, 1, part.p, tot.p + 1, st);
+                              b->pre_snv_d.p, b->pre_id_d.p, cnt_snv, cnt_id, st);
+  pg::scan_rows<uint32_t>(cnt.p, cnt.p, n_cells, 2, part.p, tot.p, st);
   uint32_t tot_h[2];
   ck(cudaMemcpyAsync(tot_h, tot.p, sizeof(tot_h), cudaMemcpyDeviceToHost, st), "counts");
   ck(cudaStreamSynchronize(st), "batch counts");
@@ -152,7 +152,7 @@ void batch_place(pg_batch* b, const uint64_t* place_seed) {
     ck(cudaMemsetAsync(fslot.p, 0xff, sizeof(uint32_t) * fcap, st), "memset");
     ck(cudaMemsetAsync(n_next.p, 0, sizeof(uint32_t), st), "memset");
   }
-  pg::place_first_round_batch(b->tabs.p, B, b->cell_off_d.p, b->pkeys.p, o, b->inst_of.p, cnt_snv.p, cnt_id.p,
+  pg::place_first_round_batch(b->tabs.p, B, b->cell_off_d.p, b->pkeys.p, o, b->inst_of.p, cnt_snv, cnt_id,
                               uint32_t(n_snv), uint32_t(n_all), fkeys.p, fslot.p, fcap - 1, lost.p, pend.p, n_next.p,
                               err.p, st);
   if (unique) {
@@ -170,7 +170,7 @@ void batch_place(pg_batch* b, const uint64_t* place_seed) {
       ck(cudaMemsetAsync(held.p, 0xff, sizeof(unsigned long long) * cap, st), "memset");
       tail_ctl = DBuf<pg::TailCtl>(P, 1);
       ck(cudaMemsetAsync(tail_ctl.p, 0, sizeof(pg::TailCtl), st), "memset");
-      pg::sites_settle_batch(b->tabs.p, B, b->cell_off_d.p, b->pkeys.p, o, b->inst_of.p, cnt_snv.p, cnt_id.p,
+      pg::sites_settle_batch(b->tabs.p, B, b->cell_off_d.p, b->pkeys.p, o, b->inst_of.p, cnt_snv, cnt_id,
                              uint32_t(n_snv), pend.p, n_next.p, n_tail, fkeys.p, fcap - 1, hkeys.p, held.p, cap,
                              tail_ctl.p, err.p, st);
       // the tables live until the launches end: the engine's pool hands them

@@ -155,9 +155,10 @@ void sites_covered(const PlaceTables& t, const PlaceRaw& o, uint64_t seed, const
                    const uint32_t* off_id, uint32_t n_snv, uint32_t n_slots, TailCtl* ctl, uint32_t* err,
                    cudaStream_t st);
 uint32_t sort_num_buckets(uint64_t G);
-// sort by (locus, slot) into `sorted`; keys: n 64-bit keys
-void sort_by_locus(const PlaceRaw& o, uint32_t n, uint64_t G, uint32_t* bcnt, uint32_t* bfill, uint32_t* part,
-                   uint32_t* order, const PlaceOut& sorted, unsigned long long* keys, cudaStream_t st);
+// sort by (locus, slot) into `sorted`; bcnt: 2 sort_num_buckets(G) entries,
+// keys: n 64-bit keys
+void sort_by_locus(const PlaceRaw& o, uint32_t n, uint64_t G, uint32_t* bcnt, uint32_t* part, uint32_t* order,
+                   const PlaceOut& sorted, unsigned long long* keys, cudaStream_t st);
 
 // ---------------------------------------------------------------- sequencing
 struct SeqRec {            // 16 B, one per placed mutation, sorted by locus
@@ -193,11 +194,11 @@ inline uint32_t insert_guide(const uint32_t* thr, uint32_t n, uint32_t g, uint32
 
 struct SeqTiles {
   uint32_t n_tiles;        // over all selected chromosomes
-  const uint32_t* start;   // first start position of the tile (absolute)
-  const uint32_t* len;     // number of start positions in the tile
-  const uint32_t* chr_end; // absolute end of the tile's chromosome
-  const uint32_t* rec_lo;  // records of the tile's window [start, start + len - 1 + span)
-  const uint32_t* rec_hi;
+  uint32_t* start;   // first start position of the tile (absolute)
+  uint32_t* len;     // number of start positions in the tile
+  uint32_t* chr_end; // absolute end of the tile's chromosome
+  uint32_t* rec_lo;  // records of the tile's window [start, start + len - 1 + span)
+  uint32_t* rec_hi;
 };
 
 struct SeqSample {
@@ -261,11 +262,24 @@ struct SeqParams {
   const uint32_t* nmask;          // unknown reference bases (N), one bit each, or NULL (SAM output)
 };
 
-// tile t of chromosome slot c (c_first[c] <= t < c_first[c] + c_ntiles[c],
-// k = t - c_first[c]) covers the starts [c_start + k T, + min(T, S - k T))
-void seq_make_tiles(uint32_t n_slots, const uint32_t* c_first, const uint32_t* c_ntiles, const uint32_t* c_start,
-                    const uint32_t* c_nstarts, const uint32_t* c_end, uint32_t T, uint32_t n_tiles, uint32_t* start,
-                    uint32_t* len, uint32_t* end, cudaStream_t st);
+// The chromosomes of a sequencing call: tile t of slot c (first[c] <= t <
+// first[c] + ntiles[c], k = t - first[c]) covers the starts
+// [start[c] + k T, + min(T, nstarts[c] - k T)).
+struct SeqChroms {
+  uint32_t n_slots;
+  const uint32_t *first, *ntiles, *start, *nstarts, *end;
+  const uint32_t* depth;    // levels of the tile-split tree
+  const uint32_t* id;       // chromosome numbers (keys of the tree's draws)
+  const uint64_t* pairs;    // fragments
+  uint32_t T, n_tiles, max_tiles;
+};
+// What the read kernel needs that depends on no copy-number table, in one
+// launch: the tiles and the ranges of their windows' records, the records
+// and, for the first n_split samples (all, or none), the fragments per tile
+// by start positions (see seq_tile_counts).
+void seq_prepare(const SeqChroms& c, const SeqTiles& tiles, const PlaceOut& sorted, uint32_t n_recs,
+                 const uint32_t* edge_tin, const uint32_t* edge_tout, uint32_t span, SeqRec* recs, uint32_t n_split,
+                 uint64_t seed, uint32_t* pair_cnt, cudaStream_t st);
 // Copy-number tables of a sequencing call.  Parts: tile t's start range cut
 // at atom boundaries, at part_off[t] .. part_off[t + 1] (part_off holds
 // n_tiles + 1 entries; `part` is scan scratch of scan_part_elems(n_tiles, 1)).
@@ -391,21 +405,13 @@ void seq_batch_records(const PlaceOut& sorted, const uint16_t* inst_sorted, cons
                        const SeqBatch& b, SeqRec* recs, cudaStream_t st);
 // tile split, record ranges and the read kernel over every (tile, sample)
 void seq_batch_reads(const SeqBatch& b, const SeqRec* recs, cudaStream_t st);
-void seq_build_records(const PlaceOut& sorted, uint32_t n, const uint32_t* edge_tin, const uint32_t* edge_tout,
-                       SeqRec* recs, cudaStream_t st);
-void seq_tile_ranges(const SeqRec* recs, uint32_t n_recs, const uint32_t* start, const uint32_t* len,
-                     uint32_t n_tiles, uint32_t span, uint32_t* rlo, uint32_t* rhi, cudaStream_t st);
 // per (sample, tile) pair counts: multinomial split of each chromosome's
-// pair count over its tiles (at most max_tiles) by a binary tree of binomial
-// draws.  Tiles weigh their number of start positions, or (mass_cum != NULL)
-// their DNA mass: mass_cum[s * n_tiles + t] is the sample's mass of the
-// chromosome's tiles before t and mass_tot[s * n_slots + slot] the
-// chromosome's total.
-void seq_tile_counts(uint32_t n_samples, uint32_t n_slots, uint32_t max_tiles, const uint32_t* chr_first_tile,
-                     const uint32_t* chr_ntiles, const uint32_t* chr_depth, const uint32_t* chr_nstarts,
-                     const uint32_t* chr_id, const uint64_t* chr_pairs, uint32_t tile_size, uint32_t n_tiles,
-                     const double* mass_cum, const double* mass_tot, uint64_t seed, uint32_t* pair_cnt,
-                     cudaStream_t st);
+// pair count over its tiles by a binary tree of binomial draws.  Tiles weigh
+// their number of start positions (seq_prepare), or their DNA mass:
+// mass_cum[s * n_tiles + t] is the sample's mass of the chromosome's tiles
+// before t and mass_tot[s * n_slots + slot] the chromosome's total.
+void seq_tile_counts(const SeqChroms& c, uint32_t n_samples, const double* mass_cum, const double* mass_tot,
+                     uint64_t seed, uint32_t* pair_cnt, cudaStream_t st);
 // observed rows: flag[m] = 1 when some sample has an alt read of mutation m;
 // with pos the exclusive scan of the flags (n_active rows), the compact
 // [sample][row] alt / depth tables and each row's mutation index

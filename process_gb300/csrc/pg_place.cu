@@ -758,11 +758,11 @@ void sites_covered(const PlaceTables& t, const PlaceRaw& o, uint64_t seed, const
   note_launch();
 }
 
-void sort_by_locus(const PlaceRaw& o, uint32_t n, uint64_t G, uint32_t* bcnt, uint32_t* bfill, uint32_t* part,
-                   uint32_t* order, const PlaceOut& sorted, unsigned long long* keys, cudaStream_t st) {
+void sort_by_locus(const PlaceRaw& o, uint32_t n, uint64_t G, uint32_t* bcnt, uint32_t* part, uint32_t* order,
+                   const PlaceOut& sorted, unsigned long long* keys, cudaStream_t st) {
   const uint32_t nb = uint32_t((G >> BUCKET_SHIFT) + 1);
-  cudaMemsetAsync(bcnt, 0, sizeof(uint32_t) * nb, st);
-  cudaMemsetAsync(bfill, 0, sizeof(uint32_t) * nb, st);
+  uint32_t* const bfill = bcnt + nb;
+  cudaMemsetAsync(bcnt, 0, sizeof(uint32_t) * 2 * nb, st);
   if (n == 0) return;
   k_bucket_count<<<nblk(n), 256, 0, st>>>(o.locus, n, bcnt); note_launch();
   scan_rows<uint32_t>(bcnt, bcnt, nb, 1, part, nullptr, st);

@@ -68,33 +68,10 @@ static_assert(SEQ_NBK == 4 * SEQ_THREADS, "the bucket scan takes four buckets pe
 static_assert(SEQ_GUIDE == 4 * SEQ_THREADS, "the insert table is staged by one 16-byte load per thread");
 static_assert(SEQ_MCAP < 65536, "bucket offsets and a batch's counts are 16-bit");
 
-__global__ void k_seq_records(PlaceOut s, uint32_t n, const uint32_t* __restrict__ edge_tin,
-                              const uint32_t* __restrict__ edge_tout, SeqRec* __restrict__ recs) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t e = s.edge[i];
-  SeqRec r;
-  r.locus = s.locus[i];
-  r.tin = edge_tin[e];
-  r.tout = edge_tout[e];
-  r.info = uint32_t(s.allele[i]) | ((uint32_t(s.seq[i]) & 0x7fffu) << 16) | (uint32_t(s.kind[i]) << 31);
-  recs[i] = r;
-}
-
 __device__ __forceinline__ uint32_t lower_bound_rec(const SeqRec* __restrict__ recs, uint32_t n, uint32_t key) {
   uint32_t lo = 0, hi = n;
   while (lo < hi) { const uint32_t mid = (lo + hi) >> 1; if (recs[mid].locus < key) lo = mid + 1; else hi = mid; }
   return lo;
-}
-
-// record range [lo, hi) of every tile's window [start, start + len - 1 + span)
-__global__ void k_tile_ranges(const SeqRec* __restrict__ recs, uint32_t n_recs, const uint32_t* __restrict__ start,
-                              const uint32_t* __restrict__ len, uint32_t n_tiles, uint32_t span,
-                              uint32_t* __restrict__ rlo, uint32_t* __restrict__ rhi) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n_tiles) return;
-  rlo[t] = lower_bound_rec(recs, n_recs, start[t]);
-  rhi[t] = lower_bound_rec(recs, n_recs, start[t] + len[t] - 1 + span);
 }
 
 // Multinomial split of a chromosome's fragments over its n tiles: a binary
@@ -174,6 +151,11 @@ struct TileSplit {
 // (16 levels, 4 samples) 1.64 ms became 0.55.
 constexpr uint32_t SPLIT_BLOCK_LOG = 6;   // 64 tiles per warp
 constexpr uint32_t SPLIT_THREADS = 128;
+// blocks per (sample, chromosome slot)
+__host__ __device__ inline uint32_t split_blocks(const SeqChroms& c) {
+  const uint32_t tiles = SPLIT_THREADS / 32 << SPLIT_BLOCK_LOG;
+  return (c.max_tiles + tiles - 1) / tiles;
+}
 __device__ __forceinline__ void tile_counts_warp(const TileSplit& sp, uint32_t s, uint32_t b, uint32_t D, uint32_t chr,
                                                  uint64_t n_pairs, Key key, uint32_t* __restrict__ cnt) {
   constexpr uint32_t FULL = 0xffffffffu;
@@ -213,19 +195,71 @@ __device__ __forceinline__ void tile_counts_warp(const TileSplit& sp, uint32_t s
   }
 }
 
-__global__ void __launch_bounds__(SPLIT_THREADS) k_tile_split(
-    uint32_t n_slots, const uint32_t* __restrict__ chr_first_tile, const uint32_t* __restrict__ chr_ntiles,
-    const uint32_t* __restrict__ chr_depth, const uint32_t* __restrict__ chr_nstarts,
-    const uint32_t* __restrict__ chr_id, const uint64_t* __restrict__ chr_pairs, uint32_t T, uint32_t n_tiles,
-    const double* __restrict__ mass_cum, const double* __restrict__ mass_tot, Key key,
-    uint32_t* __restrict__ pair_cnt) {
-  const uint32_t s = blockIdx.z, slot = blockIdx.y, b = (blockIdx.x * SPLIT_THREADS + threadIdx.x) >> 5;
-  const uint32_t nt = chr_ntiles[slot], first = chr_first_tile[slot];
+// block x of the tile split: 64 tiles per warp of a (sample, chromosome slot)
+__device__ __forceinline__ void split_block(const SeqChroms& c, uint32_t x, const double* __restrict__ mass_cum,
+                                            const double* __restrict__ mass_tot, Key key,
+                                            uint32_t* __restrict__ pair_cnt) {
+  const uint32_t per = split_blocks(c), row = x / per, s = row / c.n_slots, slot = row % c.n_slots;
+  const uint32_t b = (x % per * SPLIT_THREADS + threadIdx.x) >> 5;
+  const uint32_t nt = c.ntiles[slot], first = c.first[slot];
   if (uint64_t(b) << SPLIT_BLOCK_LOG >= nt) return;   // whole warps
-  const TileSplit sp{chr_nstarts[slot], T, nt, mass_cum ? mass_cum + uint64_t(s) * n_tiles + first : nullptr,
-                     mass_cum ? mass_tot[uint64_t(s) * n_slots + slot] : 0.0};
-  tile_counts_warp(sp, s, b, chr_depth[slot], chr_id[slot], chr_pairs[slot], key,
-                   pair_cnt + uint64_t(s) * n_tiles + first);
+  const TileSplit sp{c.nstarts[slot], c.T, nt, mass_cum ? mass_cum + uint64_t(s) * c.n_tiles + first : nullptr,
+                     mass_cum ? mass_tot[uint64_t(s) * c.n_slots + slot] : 0.0};
+  tile_counts_warp(sp, s, b, c.depth[slot], c.id[slot], c.pairs[slot], key,
+                   pair_cnt + uint64_t(s) * c.n_tiles + first);
+}
+
+__global__ void __launch_bounds__(SPLIT_THREADS) k_tile_split(SeqChroms c, const double* __restrict__ mass_cum,
+                                                              const double* __restrict__ mass_tot, Key key,
+                                                              uint32_t* __restrict__ pair_cnt) {
+  split_block(c, blockIdx.x, mass_cum, mass_tot, key, pair_cnt);
+}
+
+// The steps before the read kernel that wait for nothing, each a range of
+// blocks: the tile split (a chain of dependent draws, so first), the tiles
+// with their windows' records (two binary searches over the loci, in step),
+// the records (a gather, bound by memory).  Of 3 Mbp: 16 us, against 29 as
+// four launches one after the other.
+template <bool SPLIT>
+__global__ void __launch_bounds__(SPLIT_THREADS) k_seq_prepare(SeqChroms c, SeqTiles tiles, PlaceOut s, uint32_t n_recs,
+                                                               const uint32_t* __restrict__ edge_tin,
+                                                               const uint32_t* __restrict__ edge_tout, uint32_t span,
+                                                               SeqRec* __restrict__ recs, uint32_t split_end,
+                                                               uint32_t tiles_end, Key key,
+                                                               uint32_t* __restrict__ pair_cnt) {
+  if (SPLIT && blockIdx.x < split_end) {
+    split_block(c, blockIdx.x, nullptr, nullptr, key, pair_cnt);
+  } else if (blockIdx.x < tiles_end) {
+    const uint32_t t = (blockIdx.x - split_end) * SPLIT_THREADS + threadIdx.x;
+    if (t >= c.n_tiles) return;
+    uint32_t lo = 0, hi = c.n_slots;          // last slot whose first tile is <= t
+    while (hi - lo > 1) { const uint32_t mid = (lo + hi) >> 1; if (c.first[mid] <= t) lo = mid; else hi = mid; }
+    const uint32_t k = t - c.first[lo], start = c.start[lo] + k * c.T, len = min(c.T, c.nstarts[lo] - k * c.T);
+    tiles.start[t] = start;
+    tiles.len[t] = len;
+    tiles.chr_end[t] = c.end[lo];
+    // records [r0, r1) of the window [start, start + len - 1 + span)
+    const uint32_t end = start + len - 1 + span;
+    uint32_t r0 = 0, n0 = n_recs, r1 = 0, n1 = n_recs;
+    while (r0 < n0 || r1 < n1) {
+      const uint32_t m0 = (r0 + n0) >> 1, m1 = (r1 + n1) >> 1;
+      const uint32_t l0 = r0 < n0 ? s.locus[m0] : 0u, l1 = r1 < n1 ? s.locus[m1] : 0u;
+      if (r0 < n0) { if (l0 < start) r0 = m0 + 1; else n0 = m0; }
+      if (r1 < n1) { if (l1 < end) r1 = m1 + 1; else n1 = m1; }
+    }
+    tiles.rec_lo[t] = r0;
+    tiles.rec_hi[t] = r1;
+  } else {
+    const uint32_t i = (blockIdx.x - tiles_end) * SPLIT_THREADS + threadIdx.x;
+    if (i >= n_recs) return;
+    const uint32_t e = s.edge[i];
+    SeqRec r;
+    r.locus = s.locus[i];
+    r.tin = edge_tin[e];
+    r.tout = edge_tout[e];
+    r.info = uint32_t(s.allele[i]) | ((uint32_t(s.seq[i]) & 0x7fffu) << 16) | (uint32_t(s.kind[i]) << 31);
+    recs[i] = r;
+  }
 }
 
 // Error words.  A mate's word: the fragment's error word for mate 0, an
@@ -969,22 +1003,6 @@ __global__ void __launch_bounds__(SEQ_THREADS, 4) k_reads_batch(SeqBatch b, cons
 }
 
 
-__global__ void k_make_tiles(uint32_t n_slots, const uint32_t* __restrict__ c_first,
-                             const uint32_t* __restrict__ c_ntiles, const uint32_t* __restrict__ c_start,
-                             const uint32_t* __restrict__ c_nstarts, const uint32_t* __restrict__ c_end, uint32_t T,
-                             uint32_t n_tiles, uint32_t* __restrict__ start, uint32_t* __restrict__ len,
-                             uint32_t* __restrict__ end) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n_tiles) return;
-  uint32_t lo = 0, hi = n_slots;          // last slot whose first tile is <= t
-  while (hi - lo > 1) { const uint32_t mid = (lo + hi) >> 1; if (c_first[mid] <= t) lo = mid; else hi = mid; }
-  const uint32_t k = t - c_first[lo];
-  start[t] = c_start[lo] + k * T;
-  len[t] = min(T, c_nstarts[lo] - k * T);
-  end[t] = c_end[lo];
-  (void)c_ntiles;
-}
-
 // last atom starting at or before position a
 __device__ __forceinline__ uint32_t atom_of(const uint32_t* __restrict__ atom_start, uint32_t n_atoms, uint32_t a) {
   uint32_t lo = 0, hi = n_atoms;
@@ -1160,34 +1178,27 @@ void seq_tile_mass(uint32_t n_samples, uint32_t n_slots, const uint32_t* c_first
   note_launch(2);
 }
 
-void seq_make_tiles(uint32_t n_slots, const uint32_t* c_first, const uint32_t* c_ntiles, const uint32_t* c_start,
-                    const uint32_t* c_nstarts, const uint32_t* c_end, uint32_t T, uint32_t n_tiles, uint32_t* start,
-                    uint32_t* len, uint32_t* end, cudaStream_t st) {
-  if (n_tiles) { k_make_tiles<<<nblk(n_tiles), 256, 0, st>>>(n_slots, c_first, c_ntiles, c_start, c_nstarts, c_end, T,
-                                                             n_tiles, start, len, end); note_launch(); }
+void seq_prepare(const SeqChroms& c, const SeqTiles& tiles, const PlaceOut& sorted, uint32_t n_recs,
+                 const uint32_t* edge_tin, const uint32_t* edge_tout, uint32_t span, SeqRec* recs, uint32_t n_split,
+                 uint64_t seed, uint32_t* pair_cnt, cudaStream_t st) {
+  const uint32_t split_end = n_split * c.n_slots * split_blocks(c), tiles_end = split_end + nblk(c.n_tiles, SPLIT_THREADS);
+  const uint32_t grid = tiles_end + nblk(n_recs, SPLIT_THREADS);
+  if (!grid) return;
+  const Key key = make_key(seed);
+  if (split_end)
+    k_seq_prepare<true><<<grid, SPLIT_THREADS, 0, st>>>(c, tiles, sorted, n_recs, edge_tin, edge_tout, span, recs,
+                                                        split_end, tiles_end, key, pair_cnt);
+  else
+    k_seq_prepare<false><<<grid, SPLIT_THREADS, 0, st>>>(c, tiles, sorted, n_recs, edge_tin, edge_tout, span, recs,
+                                                         split_end, tiles_end, key, pair_cnt);
+  note_launch();
 }
 
-void seq_build_records(const PlaceOut& sorted, uint32_t n, const uint32_t* edge_tin, const uint32_t* edge_tout,
-                       SeqRec* recs, cudaStream_t st) {
-  if (n) { k_seq_records<<<nblk(n), 256, 0, st>>>(sorted, n, edge_tin, edge_tout, recs); note_launch(); }
-}
-
-void seq_tile_ranges(const SeqRec* recs, uint32_t n_recs, const uint32_t* start, const uint32_t* len,
-                     uint32_t n_tiles, uint32_t span, uint32_t* rlo, uint32_t* rhi, cudaStream_t st) {
-  if (n_tiles) { k_tile_ranges<<<nblk(n_tiles), 256, 0, st>>>(recs, n_recs, start, len, n_tiles, span, rlo, rhi); note_launch(); }
-}
-
-void seq_tile_counts(uint32_t n_samples, uint32_t n_slots, uint32_t max_tiles, const uint32_t* chr_first_tile,
-                     const uint32_t* chr_ntiles, const uint32_t* chr_depth, const uint32_t* chr_nstarts,
-                     const uint32_t* chr_id, const uint64_t* chr_pairs, uint32_t tile_size, uint32_t n_tiles,
-                     const double* mass_cum, const double* mass_tot, uint64_t seed, uint32_t* pair_cnt,
-                     cudaStream_t st) {
-  if (n_samples == 0 || n_slots == 0) return;
-  const uint32_t warps = (max_tiles + (1u << SPLIT_BLOCK_LOG) - 1) >> SPLIT_BLOCK_LOG;
-  const dim3 grid(nblk(uint64_t(warps) * 32, SPLIT_THREADS), n_slots, n_samples);
-  k_tile_split<<<grid, SPLIT_THREADS, 0, st>>>(n_slots, chr_first_tile, chr_ntiles, chr_depth, chr_nstarts, chr_id,
-                                               chr_pairs, tile_size, n_tiles, mass_cum, mass_tot, make_key(seed),
-                                               pair_cnt);
+void seq_tile_counts(const SeqChroms& c, uint32_t n_samples, const double* mass_cum, const double* mass_tot,
+                     uint64_t seed, uint32_t* pair_cnt, cudaStream_t st) {
+  const uint32_t grid = n_samples * c.n_slots * split_blocks(c);
+  if (!grid) return;
+  k_tile_split<<<grid, SPLIT_THREADS, 0, st>>>(c, mass_cum, mass_tot, make_key(seed), pair_cnt);
   note_launch();
 }
 

@@ -197,3 +197,26 @@ def test_read_windows_by_records(gpu_lib, orc, tile, reads):
     oalt, odep, _ = op.sequence(c, 23, flavour=0)
     np.testing.assert_array_equal(dep, odep)
     np.testing.assert_array_equal(alt, oalt)
+
+
+@pytest.mark.parametrize("leaves,epochs", [(3, 1), (682, 3), (683, 3), (2_730, 3), (2_731, 3)])
+def test_edge_offsets_by_size(gpu_lib, orc, leaves, epochs):
+    """Placements whose (edge, epoch) cells fill less than a chunk of the
+    one-launch prefix sum, one chunk, a chunk and a bit, and more than it
+    takes."""
+    from process_gb300 import synth
+    w = synth.plain_3mbp(seed=4, n_leaves=leaves)
+    w.genome.chr_lengths = [70_000, 30_001]
+    w.genome.chr_names = ["1", "2"]
+    first = w.exposures[0][1] if w.exposures else {}
+    w.exposures = [(float(t * 10), first) for t in range(epochs)]
+    (na, _, _), (nb, _, _) = w.mutants
+    rate = {"SNV": 2e-9 * 1000 / leaves, "indel": 1e-9}
+    w.mutants = [(na, rate, []), (nb, rate, [])]
+    eng = synth.build_engine(w)
+    o = orc.OracleEngine.like(w)
+    f = w.forest
+    pf = eng.place_mutations(f, 500, 20, seed=9)
+    op = o.place(f, _forest_species(o, f), 500, 0, 20, 0, seed=9)
+    for col in ("locus", "edge", "aux"):
+        np.testing.assert_array_equal(pf.table()[col], op.table()[col])
