@@ -28,20 +28,18 @@ namespace pg {
 
 
 // ------------------------------------------------------------ genome fill
-__global__ void k_genome_synth(uint32_t* __restrict__ words, uint64_t G, uint64_t nwords,
-                               Key key, uint32_t gc_thr) {
-  const uint64_t w = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (w >= nwords) return;
+// one word (16 bases) per thread; FULL: all of them inside the genome
+template <bool FULL>
+__device__ __forceinline__ uint32_t synth_word(uint64_t w, uint64_t G, const RoundKeys& key, uint32_t gc_thr) {
   uint32_t out = 0;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const uint64_t blk = w * 4 + q;               // Philox block = 4 bases
-    const U4 r = philox(key.k0, key.k1, uint32_t(blk), uint32_t(blk >> 32), 0u, TAG_GENOME);
+    const U4 r = philox(key, uint32_t(blk), uint32_t(blk >> 32), 0u, TAG_GENOME);
     const uint32_t rw[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const uint64_t i = blk * 4 + j;
-      if (i < G) {
+      if (FULL || blk * 4 + j < G) {
         const uint32_t u = rw[j];
         // GC with probability gc_thr/2^32, then C/G or A/T by the low bit
         const uint32_t b = (u < gc_thr) ? (1u + (u & 1u)) : ((u & 1u) ? 3u : 0u);
@@ -49,7 +47,14 @@ __global__ void k_genome_synth(uint32_t* __restrict__ words, uint64_t G, uint64_
       }
     }
   }
-  words[w] = out;
+  return out;
+}
+
+__global__ void k_genome_synth(uint32_t* __restrict__ words, uint64_t G, uint64_t nwords, RoundKeys key,
+                               uint32_t gc_thr) {
+  const uint64_t w = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (w >= nwords) return;
+  words[w] = (w + 1) * 16 <= G ? synth_word<true>(w, G, key, gc_thr) : synth_word<false>(w, G, key, gc_thr);
 }
 
 __global__ void k_genome_pack(uint32_t* __restrict__ words, const uint8_t* __restrict__ codes,
@@ -75,20 +80,37 @@ __device__ __forceinline__ bool base_unknown(const uint32_t* __restrict__ nmask,
 // (bit i for position base + i): the bases as two bit planes (the low and
 // the high bit of the 2-bit code), a validity plane (known bases of the
 // position's chromosome), and from these one mask per class.  Features are
-// computed on 64-bit windows (bit j = position q0 + j, q0 = base - 16 or
-// base) whose bits 16..31 are the window's 16 positions; classes are
-// bitwise functions of the features, so the two windows' features are
-// packed side by side into 32-bit position masks first.
+// 32-bit masks, read off the planes or off longer bit strings derived from
+// them by one funnel shift each; classes are bitwise functions of the
+// features.
+struct Window {      // bits of positions base - 16 .. base + 63
+  uint32_t x[3];
+  // positions base + o .. base + o + 31 (a constant o, -16 <= o <= 32)
+  __device__ __forceinline__ uint32_t at(int o) const {
+    return o < 16 ? __funnelshift_r(x[0], x[1], 16 + o) : __funnelshift_r(x[1], x[2], o - 16);
+  }
+};
 struct Planes {
-  uint64_t p0, p1;   // low and high bit of each base
-  uint64_t v;        // known base inside the position's chromosome
+  Window p0, p1;     // low and high bit of each base
+  Window v;          // known base inside the position's chromosome
 };
 
-__device__ __forceinline__ uint64_t eq_shift(const Planes& w, int s) {   // base(j) == base(j + s), both valid
-  return w.v & (w.v >> s) & ~((w.p0 ^ (w.p0 >> s)) | (w.p1 ^ (w.p1 >> s)));
+struct Run64 {       // bits of positions base - 5 .. base + 58
+  uint32_t lo, hi;
+  // positions base + o .. base + o + 31 (-5 <= o <= 26)
+  __device__ __forceinline__ uint32_t at(int o) const { return __funnelshift_r(lo, hi, o + 5); }
+  // *this at the positions where it holds s further on as well
+  __device__ __forceinline__ Run64 both(const Run64& y, int s) const {
+    return {lo & __funnelshift_r(y.lo, y.hi, s), hi & (y.hi >> s)};
+  }
+};
+// base(j) == base(j + s), both known (up to base + 58; s <= 5)
+__device__ __forceinline__ Run64 eq_shift(const Planes& w, int s) {
+  Run64 r;
+  r.lo = w.v.at(-5) & w.v.at(s - 5) & ~((w.p0.at(-5) ^ w.p0.at(s - 5)) | (w.p1.at(-5) ^ w.p1.at(s - 5)));
+  r.hi = w.v.at(27) & w.v.at(s + 27) & ~((w.p0.at(27) ^ w.p0.at(s + 27)) | (w.p1.at(27) ^ w.p1.at(s + 27)));
+  return r;
 }
-
-__device__ __forceinline__ uint32_t pos16(uint64_t x) { return uint32_t(x >> 16) & 0xFFFFu; }
 
 // SBS: one family, the pyrimidine-centred trinucleotide context of p (p - 1,
 // p and p + 1 known and in p's chromosome; p not in a region to avoid).
@@ -100,14 +122,11 @@ struct SbsFamilies {
   static constexpr int NF = 7;
   static constexpr bool AVOIDABLE = true;    // positions of the regions to avoid are not indexed
   // features: 0 indexable; 1, 2 planes of p - 1; 3, 4 of p; 5, 6 of p + 1
-  __device__ static void features(const Planes& w, uint64_t avoid, uint32_t* f, uint32_t keep, int sh) {
-    f[0] |= (pos16(w.v & (w.v << 1) & (w.v >> 1) & ~avoid) << sh) & keep;
-    f[1] |= (pos16(w.p0 << 1) << sh) & keep;
-    f[2] |= (pos16(w.p1 << 1) << sh) & keep;
-    f[3] |= (pos16(w.p0) << sh) & keep;
-    f[4] |= (pos16(w.p1) << sh) & keep;
-    f[5] |= (pos16(w.p0 >> 1) << sh) & keep;
-    f[6] |= (pos16(w.p1 >> 1) << sh) & keep;
+  __device__ static void features(const Planes& w, uint32_t avoid, uint32_t* f, uint32_t keep) {
+    f[0] |= w.v.at(-1) & w.v.at(0) & w.v.at(1) & ~avoid & keep;
+    f[1] = w.p0.at(-1); f[2] = w.p1.at(-1);      // (bases, whatever the chromosome)
+    f[3] = w.p0.at(0); f[4] = w.p1.at(0);
+    f[5] = w.p0.at(1); f[6] = w.p1.at(1);
   }
   template <class Sink>
   __device__ static void classes(const uint32_t* f, Sink sink) {
@@ -125,6 +144,15 @@ struct SbsFamilies {
 #pragma unroll
         for (int c = 0; c < 4; ++c)
           sink(s * 16 + a * 4 + c, ok & ((cen(s) & ex(a) & ez(c)) | (rev(s) & ez(3 - a) & ex(3 - c))));
+  }
+  // the bits of the context number, one plane each (meaningful at indexable positions)
+  __device__ static void number(const uint32_t* f, uint32_t (&k)[5]) {
+    const uint32_t fwd = f[3];                 // C and T have an odd code
+    k[0] = (fwd & f[5]) | ~(fwd | f[1]);
+    k[1] = (fwd & f[6]) | ~(fwd | f[2]);
+    k[2] = (fwd & f[1]) | ~(fwd | f[5]);
+    k[3] = (fwd & f[2]) | ~(fwd | f[6]);
+    k[4] = ~(f[3] ^ f[4]);
   }
 };
 
@@ -153,33 +181,36 @@ struct IdFamilies {
   static constexpr bool AVOIDABLE = false;
   // features: 0 p and p-1 known; 1 run start; 2, 3 base of p / p-1 is A or T;
   // 4..8 h >= 2..6; then per l = 2..5: the family applies, r >= 2..6, m >= 1..l-1
-  __device__ static void features(const Planes& w, uint64_t, uint32_t* f, uint32_t keep, int sh) {
-    auto put = [&](int x, uint64_t m) { f[x] |= (pos16(m) << sh) & keep; };
-    const uint64_t v = w.v, e1 = eq_shift(w, 1), bv = v & (v << 1), pt = ~(w.p0 ^ w.p1);
+  __device__ static void features(const Planes& w, uint32_t, uint32_t* f, uint32_t keep) {
+    auto put = [&](int x, uint32_t m) { f[x] |= m & keep; };
+    const uint32_t bv = w.v.at(0) & w.v.at(-1);
+    const Run64 e1 = eq_shift(w, 1);
     put(0, bv);
-    put(1, bv & ~(e1 << 1));
-    put(2, pt);
-    put(3, pt << 1);
-    uint64_t h = e1;
+    put(1, bv & ~e1.at(-1));
+    put(2, ~(w.p0.at(0) ^ w.p1.at(0)));
+    put(3, ~(w.p0.at(-1) ^ w.p1.at(-1)));
+    uint32_t h = e1.at(0);
     put(4, h);
 #pragma unroll
-    for (int k = 1; k <= 4; ++k) { h &= e1 >> k; put(4 + k, h); }
+    for (int k = 1; k <= 4; ++k) { h &= e1.at(k); put(4 + k, h); }
     int o = 9;
 #pragma unroll
     for (int l = 2; l <= 5; ++l) {
-      const uint64_t el = eq_shift(w, l);
-      uint64_t vl = v, u = el, sb = el << 1;
+      const Run64 el = eq_shift(w, l);
+      uint32_t vl = bv, sb = el.at(-1);
 #pragma unroll
-      for (int i = 1; i < l; ++i) { vl &= v >> i; u &= el >> i; sb &= el << (i + 1); }
-      put(o, bv & vl & ~sb);
-      uint64_t r = u;
+      for (int i = 1; i < l; ++i) { vl &= w.v.at(i); sb &= el.at(-1 - i); }
+      put(o, vl & ~sb);
+      const Run64 e2 = el.both(el, 1);           // u: el at the l positions from here
+      const Run64 u = l == 2 ? e2 : l == 3 ? e2.both(el, 2) : l == 4 ? e2.both(e2, 2) : e2.both(e2, 2).both(el, 4);
+      uint32_t r = u.at(0);
       put(o + 1, r);
 #pragma unroll
-      for (int q = 2; q <= 5; ++q) { r &= u >> ((q - 1) * l); put(o + q, r); }
-      uint64_t m = el;
+      for (int q = 2; q <= 5; ++q) { r &= u.at((q - 1) * l); put(o + q, r); }
+      uint32_t m = el.at(0);
       put(o + 6, m);
 #pragma unroll
-      for (int j = 2; j < l; ++j) { m &= el >> (j - 1); put(o + 5 + j, m); }
+      for (int j = 2; j < l; ++j) { m &= el.at(j - 1); put(o + 5 + j, m); }
       o += 5 + l;
     }
   }
@@ -251,13 +282,12 @@ __device__ __forceinline__ uint32_t unshuffle32(uint32_t x) {
   return x;
 }
 
-// bits [lo, hi) of a 64-bit window, clamped to the window
-__device__ __forceinline__ uint64_t range_bits(int64_t lo, int64_t hi) {
+// bits [lo, hi) of a 32-bit window, clamped to the window
+__device__ __forceinline__ uint32_t range_bits(int64_t lo, int64_t hi) {
   lo = lo < 0 ? 0 : lo;
-  hi = hi > 64 ? 64 : hi;
+  hi = hi > 32 ? 32 : hi;
   if (hi <= lo) return 0;
-  const uint64_t top = hi >= 64 ? ~0ull : ((1ull << hi) - 1ull);
-  return top & ~((1ull << lo) - 1ull);
+  return 0xffffffffu >> (32 - int(hi - lo)) << int(lo);
 }
 
 // unknown base (N) masks and the like: 1 bit per position, bit q % 32 of word q / 32
@@ -265,19 +295,32 @@ __device__ __forceinline__ uint32_t mask_word(const uint32_t* __restrict__ m, in
   return (m && wi >= 0 && uint64_t(wi) < nw) ? __ldg(m + wi) : 0u;
 }
 
-// MODE 0: the count pass.  MODE 1: the emit pass at any strides.  A round's
+// MODE 0: the count pass.  Each lane adds up its counts over the unit's
+// rounds, four classes to a word, and the warp adds the lanes' once per unit.
+// Of 310 Mbp: contexts 0.23 ms, ID classes 0.43 (at 64 registers with some
+// spilled; 0.44 at 80, 0.51 at 117 without spills, half as many warps); one
+// reduction per class and round took 0.29 and 0.54.
+// MODE 1: the emit pass at any strides.  A round's
 // class masks go to shared memory; then a lane per class counts its hits,
 // which tells how many of them are written, and the written positions of all
 // classes are dealt out evenly to the lanes, each found by a search over its
 // class's partial counts.  (Ranking one class at a time over the lanes took 13
 // warp instructions per position for the 83 ID classes, 21.4 ms for 3.1 Gbp;
-// 10.7 ms this way.)  MODE 2: every position written (SBS).
+// 10.7 ms this way.)
+// MODE 2: every position written (SBS).  The round's positions are grouped by
+// class in shared memory, then written run by run, consecutive lanes to
+// consecutive entries.  A position's slot is its lane's first slot in the
+// class's run (a packed prefix sum over the lanes, two classes to a word) and
+// the lane's hits below it; its class number comes from five bit planes,
+// spread to bytes four positions at a time.  (A prefix sum per class and a
+// shared-memory counter per class and lane took 1.04 ms for 310 Mbp, this form
+// 0.86.)
 // warps per block: the emit passes keep a round's masks per warp in shared
 // memory, so their blocks are smaller
 __host__ __device__ constexpr int ix_warps(int mode) { return mode == 0 ? IX_WARPS : IX_WARPS / 2; }
 
 template <class F, int MODE>
-__global__ void __launch_bounds__(32 * ix_warps(MODE)) k_index_scan(const uint32_t* __restrict__ g,
+__global__ void __launch_bounds__(32 * ix_warps(MODE), MODE == 0 ? 4 : 0) k_index_scan(const uint32_t* __restrict__ g,
                                                                    const uint32_t* __restrict__ nmask,
                                                                    const uint32_t* __restrict__ amask, uint64_t G,
                                                                    const uint32_t* __restrict__ chr_off, int n_chr,
@@ -293,6 +336,7 @@ __global__ void __launch_bounds__(32 * ix_warps(MODE)) k_index_scan(const uint32
   constexpr int SN = MODE >= 1 ? F::NC : 1;
   constexpr int QW = MODE == 1 ? W : 1, QN = MODE == 1 ? F::NC : 1;
   constexpr int PW = MODE == 2 ? W : 1, PN = MODE == 2 ? 32 : 1, PB = MODE == 2 ? 32 * IX_LANE_POS : 1;
+  constexpr int CN = MODE == 0 ? (F::NC + 3) / 4 : 1, PK = MODE == 2 ? 16 : 1;
   __shared__ uint32_t s_stride[SN], s_len[SN];
   __shared__ uint64_t s_off[SN];
   // MODE 1, per warp and class: the lanes' masks of the round (rows of 33
@@ -302,13 +346,14 @@ __global__ void __launch_bounds__(32 * ix_warps(MODE)) k_index_scan(const uint32
   __shared__ uint32_t s_mask[QW][QN][33];
   __shared__ uint16_t s_pre[QW][QN][8];
   __shared__ uint32_t s_dist[QW][QN], s_kidx[QW][QN], s_item[QW][QN];
-  // MODE 2 (every position written), per warp: the round's positions grouped
-  // by class (class runs in class order, in position order within a run), per
-  // class and lane the lane's next slot in the run, per class the run's start,
-  // its first list index and the next round's
-  __shared__ uint32_t s_ppos[PW][PN][32], s_pbuf[PW][PB];
-  __shared__ uint8_t s_pcls[PW][PB];
-  __shared__ uint32_t s_prun[PW][PN], s_plist[PW][PN], s_pnext[PW][PN];
+  // MODE 2, per warp: each lane's masks and first slots by class (a lane's
+  // words all in its bank), the round's positions in class order (position
+  // in the round | class << 10), the runs' lengths by packed pairs, their
+  // starts, and the distance from slot to list index
+  __shared__ uint32_t s_pmask[PW][PN][32], s_pslot[PW][PN][32];
+  __shared__ uint16_t s_pbuf[PW][PB];
+  __shared__ uint32_t s_ptot[PW][PK], s_plist[PW][PN];
+  __shared__ uint4 s_prun[PW][PN / 4 + 1];
   if (MODE >= 1) {
     for (int k = threadIdx.x; k < F::NC; k += blockDim.x) {
       s_stride[k] = stride[k];
@@ -320,10 +365,12 @@ __global__ void __launch_bounds__(32 * ix_warps(MODE)) k_index_scan(const uint32
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const uint32_t unit = blockIdx.x * W + w;
   if (unit >= n_units) return;
-  // MODE 0: per class k the count, held by lane k % 32 in slot k / 32
-  uint32_t run[NS];
+  // MODE 0: the lane's counts, class k in byte k % 4 of word k / 4 (at most
+  // 128: a unit's positions of one lane)
+  static_assert(IX_LANE_POS * IX_ROUNDS < 256, "a lane's counts fit a byte");
+  uint32_t run[CN];
 #pragma unroll
-  for (int s = 0; s < NS; ++s) run[s] = 0;
+  for (int s = 0; s < CN; ++s) run[s] = 0;
   // MODE 1: lane k % 32 keeps class k's state
   uint32_t dist[NS], kidx[NS];
 #pragma unroll
@@ -338,10 +385,7 @@ __global__ void __launch_bounds__(32 * ix_warps(MODE)) k_index_scan(const uint32
     }
   }
   const uint32_t qw = MODE == 1 ? w : 0, pw = MODE == 2 ? w : 0;
-  if (MODE == 2) {
-    s_pnext[pw][lane] = cnt[uint64_t(lane) * n_units + unit];
-    __syncwarp();
-  }
+  uint32_t next = MODE == 2 ? cnt[uint64_t(lane) * n_units + unit] : 0u;   // lane k: class k's next list index
   const uint64_t n_gw = (G + 15) / 16, n_mw = (G + 31) / 32;
   for (uint32_t round = 0; round < IX_ROUNDS; ++round) {
     const uint64_t wbase = uint64_t(unit) * IX_UNIT + uint64_t(round) * (32 * IX_LANE_POS);
@@ -351,22 +395,26 @@ __global__ void __launch_bounds__(32 * ix_warps(MODE)) k_index_scan(const uint32
 #pragma unroll
     for (int x = 0; x < F::NF; ++x) f[x] = 0;
     if (base < G) {
-      // bases [base - 16, base + 64) as bit planes, 16 positions per half word
-      uint32_t lo[5], hi[5];
+      // bases [base - 16, base + 64) as bit planes: 16 positions per word, low
+      // bits in its low half, then 32 positions per plane word
+      uint32_t u[6];
 #pragma unroll
       for (int i = 0; i < 5; ++i) {
         const int64_t wi = int64_t(base >> 4) - 1 + i;
-        const uint32_t u = unshuffle32((wi >= 0 && uint64_t(wi) < n_gw) ? __ldg(g + wi) : 0u);
-        lo[i] = u & 0xFFFFu;
-        hi[i] = u >> 16;
+        u[i] = unshuffle32((wi >= 0 && uint64_t(wi) < n_gw) ? __ldg(g + wi) : 0u);
       }
-      uint32_t nw[3], aw[3];
+      u[5] = 0;
+      Planes wd;
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
-        const int64_t wi = int64_t(base >> 5) - 1 + i;
-        nw[i] = mask_word(nmask, wi, n_mw);
-        aw[i] = F::AVOIDABLE ? mask_word(amask, wi, n_mw) : 0u;
+        wd.p0.x[i] = __byte_perm(u[2 * i], u[2 * i + 1], 0x5410);
+        wd.p1.x[i] = __byte_perm(u[2 * i], u[2 * i + 1], 0x7632);
       }
+      uint32_t nw[3];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) nw[i] = mask_word(nmask, int64_t(base >> 5) - 1 + i, n_mw);
+      const uint32_t known[3] = {~__funnelshift_r(nw[0], nw[1], 16), ~__funnelshift_r(nw[1], nw[2], 16), ~(nw[2] >> 16)};
+      const uint32_t avoid = F::AVOIDABLE ? mask_word(amask, int64_t(base >> 5), n_mw) : 0u;
       // chromosome of base: the largest c with chr_off[c] <= base
       int c = 0;
       {
@@ -382,81 +430,80 @@ __global__ void __launch_bounds__(32 * ix_warps(MODE)) k_index_scan(const uint32
         const uint64_t cs = __ldg(chr_off + c), ce = __ldg(chr_off + c + 1);
         if (cs >= base + IX_LANE_POS) break;
         if (ce <= base) continue;
-        const uint32_t keep = uint32_t(range_bits(int64_t(cs) - int64_t(base), int64_t(ce) - int64_t(base)));
+        const uint32_t keep = range_bits(int64_t(cs) - int64_t(base), int64_t(ce) - int64_t(base));
+        const int64_t q0 = int64_t(base) - 16;
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          const int64_t q0 = int64_t(base) - 16 + 16 * half;
-          Planes wd;
-          wd.p0 = uint64_t(lo[half]) | (uint64_t(lo[half + 1]) << 16) | (uint64_t(lo[half + 2]) << 32) |
-                  (uint64_t(lo[half + 3]) << 48);
-          wd.p1 = uint64_t(hi[half]) | (uint64_t(hi[half + 1]) << 16) | (uint64_t(hi[half + 2]) << 32) |
-                  (uint64_t(hi[half + 3]) << 48);
-          const uint64_t nm = half == 0 ? (uint64_t(nw[0] >> 16) | (uint64_t(nw[1]) << 16) | (uint64_t(nw[2]) << 48))
-                                        : (uint64_t(nw[1]) | (uint64_t(nw[2]) << 32));
-          const uint64_t am = half == 0 ? (uint64_t(aw[0] >> 16) | (uint64_t(aw[1]) << 16) | (uint64_t(aw[2]) << 48))
-                                        : (uint64_t(aw[1]) | (uint64_t(aw[2]) << 32));
-          wd.v = ~nm & range_bits(int64_t(cs) - q0, int64_t(ce) - q0);
-          F::features(wd, am, f, keep, 16 * half);
-        }
+        for (int i = 0; i < 3; ++i)
+          wd.v.x[i] = known[i] & range_bits(int64_t(cs) - q0 - 32 * i, min(int64_t(ce) - q0, int64_t(80)) - 32 * i);
+        F::features(wd, avoid, f, keep);
       }
     }
-    uint32_t tk = 0;
-    F::classes(f, [&](int k, uint32_t m) {
-      if constexpr (MODE == 2) {
-        // the lane's first slot in the class's run, and the run's length (held by lane k)
-        const uint32_t c = __popc(m);
-        uint32_t incl = c;
+    uint32_t pk[PK];                 // MODE 2: the lane's counts, classes 2j and 2j + 1 in word j
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const uint32_t y = __shfl_up_sync(FULL, incl, o);
-          if (lane >= uint32_t(o)) incl += y;
-        }
-        s_ppos[pw][k][lane] = incl - c;
-        const uint32_t t = __shfl_sync(FULL, incl, 31);
-        if (lane == uint32_t(k)) tk = t;
-        return;
-      }
+    for (int j = 0; j < PK; ++j) pk[j] = 0;
+    F::classes(f, [&](int k, uint32_t m) {
       if constexpr (MODE == 0) {
-        const uint32_t t = __reduce_add_sync(FULL, uint32_t(__popc(m)));
-        if (lane == (uint32_t(k) & 31u)) run[k >> 5] += t;
-      } else {
+        run[k >> 2] += uint32_t(__popc(m)) << (8 * (k & 3));
+      } else if constexpr (MODE == 1) {
         s_mask[qw][k][lane] = m;
+      } else {
+        s_pmask[pw][k][lane] = m;
+        pk[k >> 1] += uint32_t(__popc(m)) << (16 * (k & 1));
       }
     });
     if constexpr (MODE == 2) {
-      // class runs in class order: lane k holds class k's run length tk
-      uint32_t incl = tk;
+      uint32_t in[PK];               // inclusive over the lanes (a class has at most 1024)
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(FULL, incl, o);
-        if (lane >= uint32_t(o)) incl += y;
-      }
-      const uint32_t tot = __shfl_sync(FULL, incl, 31);
-      s_prun[pw][lane] = incl - tk;
-      s_plist[pw][lane] = s_pnext[pw][lane];
-      s_pnext[pw][lane] += tk;
+      for (int j = 0; j < PK; ++j) in[j] = pk[j];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+        for (int j = 0; j < PK; ++j) {
+          const uint32_t y = __shfl_up_sync(FULL, in[j], o);
+          if (lane >= uint32_t(o)) in[j] += y;
+        }
+      if (lane == 31)
+#pragma unroll
+        for (int j = 0; j < PK; ++j) s_ptot[pw][j] = in[j];
       __syncwarp();
-      // each lane's positions into their class runs, in position order
+      // lane k: class k's run
+      const uint32_t tk = reinterpret_cast<const uint16_t*>(s_ptot[pw])[lane], incl = warp_incl_scan(tk);
+      const uint32_t tot = __shfl_sync(FULL, incl, 31);
+      reinterpret_cast<uint32_t*>(s_prun[pw])[lane] = incl - tk;
+      s_plist[pw][lane] = next - (incl - tk);
+      next += tk;
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < PK; j += 2) {
+        const uint4 r = s_prun[pw][j / 2];
+        const uint32_t e0 = in[j] - pk[j], e1 = in[j + 1] - pk[j + 1];
+        s_pslot[pw][2 * j][lane] = r.x + (e0 & 0xffffu);
+        s_pslot[pw][2 * j + 1][lane] = r.y + (e0 >> 16);
+        s_pslot[pw][2 * j + 2][lane] = r.z + (e1 & 0xffffu);
+        s_pslot[pw][2 * j + 3][lane] = r.w + (e1 >> 16);
+      }
+      // each lane's positions into their class runs, in position order (a
+      // lane reads only what it wrote itself)
       const uint32_t ok = f[0];
-#pragma unroll 4
-      for (uint32_t i = 0; i < IX_LANE_POS; ++i) {
-        if ((ok >> i) & 1u) {
-          const uint32_t x = ((f[1] >> i) & 1u) | (((f[2] >> i) & 1u) << 1);
-          const uint32_t y0 = (f[3] >> i) & 1u, y1 = (f[4] >> i) & 1u;
-          const uint32_t z = ((f[5] >> i) & 1u) | (((f[6] >> i) & 1u) << 1);
-          // the context as SbsFamilies::classes numbers it
-          const uint32_t k = y0 ? ((y1 << 4) | (x << 2) | z) : (((y1 ^ 1u) << 4) | ((3u - z) << 2) | (3u - x));
-          const uint32_t slot = s_prun[pw][k] + s_ppos[pw][k][lane]++;
-          s_pbuf[pw][slot] = uint32_t(base) + i;
-          s_pcls[pw][slot] = uint8_t(k);
+      uint32_t kp[5];
+      F::number(f, kp);
+#pragma unroll
+      for (uint32_t n = 0; n < IX_LANE_POS; n += 4) {
+        uint32_t k4 = 0;             // the class numbers of four positions, a byte each
+#pragma unroll
+        for (int p = 4; p >= 0; --p) k4 = 2u * k4 + (((kp[p] >> n) & 15u) * 0x00204081u & 0x01010101u);
+#pragma unroll
+        for (uint32_t i = n; i < n + 4; ++i) {
+          const uint32_t k = (k4 >> (8 * (i - n))) & 0xffu;
+          const uint32_t slot = s_pslot[pw][k][lane] + __popc(s_pmask[pw][k][lane] & ((1u << i) - 1u));
+          if ((ok >> i) & 1u) s_pbuf[pw][slot] = uint16_t(k << 10 | (lane * IX_LANE_POS + i));
         }
       }
       __syncwarp();
       // the runs to the class lists, consecutive lanes to consecutive entries
       for (uint32_t e = lane; e < tot; e += 32) {
-        const uint32_t k = s_pcls[pw][e];
-        const uint32_t idx = s_plist[pw][k] + (e - s_prun[pw][k]);
-        if (idx < s_len[k]) lists[s_off[k] + idx] = s_pbuf[pw][e];
+        const uint32_t v = s_pbuf[pw][e], k = v >> 10, idx = s_plist[pw][k] + e;
+        if (idx < s_len[k]) lists[s_off[k] + idx] = uint32_t(wbase) + (v & 1023u);
       }
       __syncwarp();
     }
@@ -516,11 +563,24 @@ __global__ void __launch_bounds__(32 * ix_warps(MODE)) k_index_scan(const uint32
       __syncwarp();
     }
   }
-  if (MODE == 0) {
+  if constexpr (MODE == 0) {
+    uint32_t t[NS];                  // lane k % 32: class k's count, in slot k / 32
+#pragma unroll
+    for (int s = 0; s < NS; ++s) t[s] = 0;
+#pragma unroll
+    for (int j = 0; j < CN; ++j) {
+      // two classes to a reduction: at most 4096 each
+      const uint32_t a = __reduce_add_sync(FULL, run[j] & 0x00ff00ffu);
+      const uint32_t b = __reduce_add_sync(FULL, (run[j] >> 8) & 0x00ff00ffu);
+      const uint32_t c[4] = {a & 0xffffu, b & 0xffffu, a >> 16, b >> 16};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (4 * j + i < F::NC && lane == uint32_t((4 * j + i) & 31)) t[(4 * j + i) >> 5] = c[i];
+    }
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
       const uint32_t k = s * 32 + lane;
-      if (k < uint32_t(F::NC)) cnt[uint64_t(k) * n_units + unit] = run[s];
+      if (k < uint32_t(F::NC)) cnt[uint64_t(k) * n_units + unit] = t[s];
     }
   }
 }
@@ -530,7 +590,9 @@ void genome_synth(uint32_t* words, uint64_t G, uint64_t seed, double gc, cudaStr
   const uint64_t nwords = (G + 15) / 16;
   double t = gc * 4294967296.0;
   uint32_t thr = t >= 4294967295.0 ? 0xffffffffu : uint32_t(t);
-  k_genome_synth<<<unsigned((nwords + 255) / 256), 256, 0, st>>>(words, G, nwords, make_key(seed), thr); note_launch();
+  const Key k = make_key(seed);
+  k_genome_synth<<<unsigned((nwords + 255) / 256), 256, 0, st>>>(words, G, nwords, round_keys(k.k0, k.k1), thr);
+  note_launch();
 }
 
 void genome_pack(uint32_t* words, const uint8_t* codes, uint64_t G, cudaStream_t st) {
