@@ -405,6 +405,12 @@ __device__ __forceinline__ bool taken_first(const PlainSlots&, const unsigned lo
   return first_find(tab, uint32_t(mask), k) != FIRST_EMPTY;
 }
 
+// A slot that is given up (the call fails) gets a locus the sort can take.
+__device__ __forceinline__ void give_up(const PlaceRaw& o, uint32_t slot, uint32_t* flags, uint32_t bit) {
+  atomicOr(flags, bit);
+  o.locus[slot] = 0;
+}
+
 // pending slots list[0 .. *n) (n <= cap, which sizes the grid)
 template <class S, class First>
 __global__ void __launch_bounds__(128) k_sites_settle(S s, PlaceRaw o, const uint32_t* __restrict__ list,
@@ -422,14 +428,17 @@ __global__ void __launch_bounds__(128) k_sites_settle(S s, PlaceRaw o, const uin
     const PlaceTables& t = s.tables(ref);
     const Key key = s.key(ref);
     for (;; ++attempt) {                        // the slot's next attempt at a locus that is not taken
-      if (attempt >= TAIL_MAX_ROUND) { atomicOr(&ctl->status, TAIL_ROUNDS_EXHAUSTED); return; }
+      if (attempt >= TAIL_MAX_ROUND) { give_up(o, slot, &ctl->status, TAIL_ROUNDS_EXHAUSTED); return; }
       Site x;
-      if (!draw_site(t, key, u, attempt, r.w & 0xffu, (r.w >> 8) & 0xffu, x)) { atomicOr(err, ERR_EMPTY_CLASS); return; }
+      if (!draw_site(t, key, u, attempt, r.w & 0xffu, (r.w >> 8) & 0xffu, x)) {
+        give_up(o, slot, err, ERR_EMPTY_CLASS);
+        return;
+      }
       if (x.locus == LOCUS_INVALID) continue;
       const typename S::TabKey k = s.tab_key(x.locus, ref);
       if (taken_first(s, first, fmask, k)) continue;
       uint64_t h;
-      if (!key_entry(keys, mask, k, h)) { atomicOr(err, ERR_CAPACITY); return; }
+      if (!key_entry(keys, mask, k, h)) { give_up(o, slot, err, ERR_CAPACITY); return; }
       const unsigned long long mine = (static_cast<unsigned long long>(attempt) << 32) | slot;
       const unsigned long long old = atomicMin(held + h, mine);
       if (old == SITE_FREE) return;
@@ -458,7 +467,7 @@ __global__ void __launch_bounds__(256) k_sites_final(S s, PlaceRaw o, const unsi
     const Mut u = s.again(slot, r.x, ref);
     const uint32_t sig = (r.w >> 8) & 0xffu;
     Site x;
-    if (!draw_site(s.tables(ref), s.key(ref), u, attempt, r.w & 0xffu, sig, x)) atomicOr(err, ERR_EMPTY_CLASS);
+    if (!draw_site(s.tables(ref), s.key(ref), u, attempt, r.w & 0xffu, sig, x)) give_up(o, slot, err, ERR_EMPTY_CLASS);
     else put_site(s.tables(ref), o, slot, u, sig, x);
   }
   attempt = __reduce_max_sync(0xffffffffu, attempt);
@@ -479,8 +488,8 @@ __global__ void __launch_bounds__(128) k_sites_covered(PlainSlots s, PlaceRaw o,
     const uint32_t sig = (r.w >> 8) & 0xffu;
     Site x;
     do {
-      if (++attempt >= TAIL_MAX_ROUND) { atomicOr(&ctl->status, TAIL_ROUNDS_EXHAUSTED); return; }
-      if (!draw_site(s.t, s.k, u, attempt, r.w & 0xffu, sig, x)) { atomicOr(err, ERR_EMPTY_CLASS); return; }
+      if (++attempt >= TAIL_MAX_ROUND) { give_up(o, slot, &ctl->status, TAIL_ROUNDS_EXHAUSTED); return; }
+      if (!draw_site(s.t, s.k, u, attempt, r.w & 0xffu, sig, x)) { give_up(o, slot, err, ERR_EMPTY_CLASS); return; }
     } while (x.locus == LOCUS_INVALID);
     put_site(s.t, o, slot, u, sig, x);
   }

@@ -220,3 +220,27 @@ def test_edge_offsets_by_size(gpu_lib, orc, leaves, epochs):
     op = o.place(f, _forest_species(o, f), 500, 0, 20, 0, seed=9)
     for col in ("locus", "edge", "aux"):
         np.testing.assert_array_equal(pf.table()[col], op.table()[col])
+
+
+@pytest.mark.parametrize("infinite", [True, False])
+def test_no_allele_left(gpu_lib, infinite):
+    """A class whose every position the cells have lost on both alleles: the
+    call fails, whatever the draws left in the columns, and the engine goes
+    on."""
+    from process_gb300 import CNA, SBS_CLASSES, DomainError, GenomeSpec, synth
+    w = synth.plain_3mbp(seed=3, n_leaves=20)
+    bases = np.zeros(60_000, np.uint8)                       # poly-A, and A C A repeats on the second
+    bases[40_000:] = np.resize([0, 1], 20_000)
+    w.genome = GenomeSpec(["1", "2"], [40_000, 20_000], bases=bases)
+    sig = np.zeros(96)
+    sig[SBS_CLASSES.index("A[C>T]A")] = 1.0
+    w.sbs = {"SBS1": sig}
+    (na, _, _), (nb, _, _) = w.mutants
+    lost = [CNA("D", "2", 1, 20_000, allele=0), CNA("D", "2", 1, 20_000, allele=0)]
+    w.mutants = [(na, {"SNV": 1e-5, "indel": 0.0}, lost), (nb, {"SNV": 1e-5, "indel": 0.0}, [])]
+    eng = synth.build_engine(w)
+    eng.infinite_sites_model = infinite
+    with pytest.raises(DomainError, match="left"):
+        eng.place_mutations(w.forest, 0, 0, seed=2)
+    ok = synth.plain_3mbp(seed=3, n_leaves=20)
+    assert synth.build_engine(ok).place_mutations(ok.forest, 10, 1, seed=2).num_of_mutations > 0
