@@ -123,6 +123,29 @@ __device__ __forceinline__ uint32_t find_cell(const uint32_t* __restrict__ off, 
   return lo;
 }
 
+// The same for a whole warp of consecutive slots (i - lane the first; lanes
+// past the end may repeat the last): a 32-way search for the first slot's
+// cell, then the lanes rank themselves among the next 32 offsets: 4 or 5
+// dependent loads where a search per lane takes 16 (60 000 cells).
+__device__ __forceinline__ uint32_t find_cell_warp(const uint32_t* __restrict__ off, uint32_t ncell, uint32_t i) {
+  constexpr uint32_t FULL = 0xffffffffu;
+  const uint32_t lane = threadIdx.x & 31u, i0 = __shfl_sync(FULL, i, 0);
+  uint32_t lo = 0, hi = ncell;                 // off[lo] <= i0 < off[hi]
+  while (hi - lo > 1) {
+    const uint32_t step = (hi - lo + 31) / 32, at = lo + (lane + 1) * step;
+    const uint32_t below = __popc(__ballot_sync(FULL, at < hi && off[at] <= i0));   // (ascending: a run of lanes)
+    lo += below * step;
+    hi = min(hi, lo + step);
+  }
+  const uint32_t b = lo + 1 + lane < ncell ? off[lo + 1 + lane] : 0xffffffffu;
+  if (__shfl_sync(FULL, b, 31) <= i0 + 31u) return lo + find_cell(off + lo, ncell - lo, i);
+  uint32_t c = 0;                              // offsets at or below i
+#pragma unroll
+  for (uint32_t step = 16; step >= 1; step >>= 1)
+    if (__shfl_sync(FULL, b, c + step - 1) <= i) c += step;
+  return lo + c;
+}
+
 // A slot's mutation in unsorted order: its locus and a 16-byte record of the
 // other columns (PlaceRaw), written once and gathered once by the sort.
 __device__ __forceinline__ uint4 raw_record(uint32_t edge, uint32_t aux, uint32_t allele, uint32_t seq, uint32_t cls,
@@ -160,8 +183,9 @@ __device__ __forceinline__ void draw_class(const PlaceTables& t, Key key, const 
 struct Site {
   uint32_t p, locus, allele, cls, w;
 };
-__device__ __forceinline__ bool draw_site(const PlaceTables& t, Key key, const Mut& u, uint32_t attempt, uint32_t cls,
-                                          uint32_t sig, Site& out) {
+// its position (locus: before the alleles are known; allele: the word that draws it)
+__device__ __forceinline__ bool draw_position(const PlaceTables& t, Key key, const Mut& u, uint32_t attempt,
+                                              uint32_t cls, uint32_t sig, Site& out) {
   Stream st{key, u.m, u.v, u.e, u.is_id ? TAG_INDEL : TAG_SNV, 1u + attempt};
   const U4 r = st.next();
   if (attempt >= RECLASS_ATTEMPTS)
@@ -174,23 +198,38 @@ __device__ __forceinline__ bool draw_site(const PlaceTables& t, Key key, const M
   out.cls = cls;
   out.w = r.w;
   out.locus = u.is_id ? out.p - 1 : out.p;          // an indel's locus is its anchor base
+  out.allele = r.z;
+  return true;
+}
+// its allele among those of genotype class node_cls
+__device__ __forceinline__ void draw_allele(const PlaceTables& t, uint32_t node_cls, Site& x) {
   if (t.gc.n_classes == 1) {                        // no copy-number events: instances 0 and 1 everywhere
-    out.allele = uniform_index32(r.z, 2u);
-    return true;
+    x.allele = uniform_index32(x.allele, 2u);
+    return;
   }
   uint32_t ioff = 0;
-  const uint32_t n = covering(t.gc, t.gc.node_class[u.v], out.locus, &ioff);
-  if (n == 0) out.locus = LOCUS_INVALID;            // deleted here: redrawn
-  else out.allele = t.gc.inst_list[ioff + uniform_index32(r.z, n)];
+  const uint32_t n = covering(t.gc, node_cls, x.locus, &ioff);
+  if (n == 0) x.locus = LOCUS_INVALID;              // deleted here: redrawn
+  else x.allele = t.gc.inst_list[ioff + uniform_index32(x.allele, n)];
+}
+__device__ __forceinline__ uint32_t node_class_of(const PlaceTables& t, uint32_t v) {
+  return t.gc.n_classes == 1 ? 0u : t.gc.node_class[v];
+}
+__device__ __forceinline__ bool draw_site(const PlaceTables& t, Key key, const Mut& u, uint32_t attempt, uint32_t cls,
+                                          uint32_t sig, Site& out) {
+  if (!draw_position(t, key, u, attempt, cls, sig, out)) return false;
+  draw_allele(t, node_class_of(t, u.v), out);
   return true;
 }
 
-// SNV: the alt base on the forward strand; indel: its descriptor (bit 0
-// insertion, bits 1-3 length, bits 8.. inserted bases, 2 bits each)
-__device__ __forceinline__ uint32_t site_aux(const PlaceTables& t, bool is_id, const Site& x) {
-  const uint32_t p = x.p, cls = x.cls;
+// What a mutation of class cls at p (its locus, or the base after an indel's)
+// does, from the bases there and its word w.  SNV: the alt base on the forward
+// strand; indel: its descriptor (bit 0 insertion, bits 1-3 length, bits 8..
+// inserted bases, 2 bits each).
+__device__ __forceinline__ uint32_t site_aux(const uint32_t* __restrict__ genome, bool is_id, uint32_t p, uint32_t cls,
+                                             uint32_t w) {
+  const uint32_t ref = base_at(genome, p);
   if (!is_id) {
-    const uint32_t ref = base_at(t.genome, p);
     const uint32_t alt_pyr = sbs_class_alt(int(cls));
     const bool fwd = (ref == 1u || ref == 3u);
     return fwd ? alt_pyr : 3u - alt_pyr;
@@ -200,25 +239,27 @@ __device__ __forceinline__ uint32_t site_aux(const PlaceTables& t, bool is_id, c
   else if (cls < 24) {
     ins = 1; l = 1;
     const uint32_t idx = (cls - 12) % 6;
-    if (idx >= 1) bases = base_at(t.genome, p);
-    else bases = (cls < 18) ? ((x.w & 1u) ? 2u : 1u) : ((x.w & 1u) ? 0u : 3u);
+    if (idx >= 1) bases = ref;
+    else bases = (cls < 18) ? ((w & 1u) ? 2u : 1u) : ((w & 1u) ? 0u : 3u);
   } else if (cls < 48) { ins = 0; l = (cls - 24) / 6 + 2; }
   else if (cls < 72) {
     ins = 1; l = (cls - 48) / 6 + 2;
-    if ((cls - 48) % 6 >= 1) { for (uint32_t k = 0; k < l; ++k) bases |= base_at(t.genome, p + k) << (2 * k); }
-    else bases = x.w & ((1u << (2 * l)) - 1u);
+    if ((cls - 48) % 6 >= 1) { for (uint32_t k = 0; k < l; ++k) bases |= base_at(genome, p + k) << (2 * k); }
+    else bases = w & ((1u << (2 * l)) - 1u);
   } else {
     ins = 0; l = cls == 72 ? 2 : (cls < 75 ? 3 : (cls < 78 ? 4 : 5));
   }
   return ins | (l << 1) | (bases << 8);
 }
 
-// the slot's columns for site x
+// The slot's columns for site x.  The aux column holds the site's word for now:
+// the gather after the sort looks up the bases, in locus order (here each would
+// be a DRAM access of its own).
 __device__ __forceinline__ void put_site(const PlaceTables& t, const PlaceRaw& o, uint32_t slot, const Mut& u,
                                          uint32_t sig, const Site& x) {
   const bool pre = u.v == t.n_nodes, ok = x.locus != LOCUS_INVALID;
   o.locus[slot] = x.locus;
-  o.rec[slot] = raw_record(u.v, ok ? site_aux(t, u.is_id, x) : 0u, ok ? x.allele : 0u,
+  o.rec[slot] = raw_record(u.v, x.w, ok ? x.allele : 0u,
                            pre ? SEQ_PRENEOPLASTIC : SEQ_PASSENGER, x.cls, sig, u.is_id ? KIND_INDEL : KIND_SNV,
                            pre ? NATURE_PRENEOPLASTIC : NATURE_PASSENGER);
 }
@@ -234,11 +275,13 @@ struct PlainSlots {
   using Ref = uint32_t;      // (nothing to know beyond the slot)
   __device__ __forceinline__ const PlaceTables& tables(Ref) const { return t; }
   __device__ __forceinline__ Key key(Ref) const { return k; }
+  // (a warp of consecutive slots; see find_cell_warp)
   __device__ __forceinline__ Mut first(uint32_t slot, Ref&) const {
     const bool is_id = slot >= n_snv;
-    const uint32_t i = is_id ? slot - n_snv : slot;
+    const uint32_t i = is_id ? slot - n_snv : slot, ncell = (t.n_nodes + 1) * t.n_epochs;
     const uint32_t* off = is_id ? off_id : off_snv;
-    const uint32_t q = find_cell(off, (t.n_nodes + 1) * t.n_epochs, i);
+    const bool one = __all_sync(0xffffffffu, is_id) || !__any_sync(0xffffffffu, is_id);   // the warp has one kind
+    const uint32_t q = one ? find_cell_warp(off, ncell, i) : find_cell(off, ncell, i);
     return {q / t.n_epochs, q % t.n_epochs, i - off[q], is_id};
   }
   __device__ __forceinline__ Mut again(uint32_t slot, uint32_t edge, Ref&) const {
@@ -255,6 +298,7 @@ struct PlainSlots {
 };
 
 // ------------------------------------------------------------ hash sets
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ uint32_t hash32(uint32_t k) {
   k ^= k >> 16; k *= 0x7feb352du; k ^= k >> 15; k *= 0x846ca68bu; k ^= k >> 16;
   return k;
@@ -346,19 +390,28 @@ __global__ void __launch_bounds__(256) k_first_collect(const uint8_t* __restrict
 // gathers.  The drivers go in afterwards (k_first_insert with no passenger
 // slots); the table's final state and the marks do not depend on the order of
 // the insertions.  tab (all ones) and lost (zeros) are set by the caller.
+// Bound by the latency of dependent loads, at full scale by random DRAM
+// accesses (list entry, table entry): the cell by a search of the warp, the
+// table's entry requested before the allele is looked up, the bases left to
+// the gather after the sort.  35e6 slots on 3.1 Gbp: 2.82 -> 2.18 ms (the
+// gather 0.72 -> 0.85); 1.75e6 on 155 Mbp: 120 -> 85 us.
 __global__ void k_place_first(PlainSlots s, PlaceRaw o, uint32_t n_slots, unsigned long long* __restrict__ tab,
                               uint32_t mask, uint8_t* __restrict__ lost, uint32_t* __restrict__ err) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_slots) return;
   uint32_t ref = 0, cls, sig;
-  const Mut u = s.first(i, ref);
+  const Mut u = s.first(min(i, n_slots - 1), ref);
+  if (i >= n_slots) return;
+  const uint32_t nc = node_class_of(s.t, u.v);
   draw_class(s.t, s.k, u, cls, sig);
   Site x;
-  if (!draw_site(s.t, s.k, u, 0u, cls, sig, x)) { atomicOr(err, ERR_EMPTY_CLASS); o.locus[i] = 0; return; }
+  if (!draw_position(s.t, s.k, u, 0u, cls, sig, x)) { atomicOr(err, ERR_EMPTY_CLASS); o.locus[i] = 0; return; }
+  if (tab) prefetch_l2(tab + (hash32(x.locus) & mask));
+  draw_allele(s.t, nc, x);
+  if (tab) {
+    if (x.locus == LOCUS_INVALID) lost[i] = 1;           // no allele at the drawn position
+    else first_insert(tab, mask, x.locus, i + 1, lost, err);
+  }
   put_site(s.t, o, i, u, sig, x);
-  if (tab == nullptr) return;
-  if (x.locus == LOCUS_INVALID) lost[i] = 1;             // no allele at the drawn position
-  else first_insert(tab, mask, x.locus, i + 1, lost, err);
 }
 
 // ------------------------------------------------------------ redraws
@@ -573,15 +626,19 @@ __global__ void __launch_bounds__(SORT_THREADS) k_bucket_sort_keys(const uint32_
   }
 }
 
-// the sorted columns: one 16-byte record per mutation
+// The sorted columns: one 16-byte record per mutation, a passenger's aux from
+// the bases at its locus (drivers bring theirs).
 // (n_inst: a batch, whose instance i starts at boff[i * nb]; else 0)
 __global__ void k_gather_records(const uint4* __restrict__ rec, const uint32_t* __restrict__ order, uint32_t n,
-                                 PlaceOut s, uint16_t* __restrict__ inst_sorted, uint32_t n_inst, uint32_t nb,
-                                 const uint32_t* __restrict__ boff) {
+                                 const uint32_t* __restrict__ genome, PlaceOut s, uint16_t* __restrict__ inst_sorted,
+                                 uint32_t n_inst, uint32_t nb, const uint32_t* __restrict__ boff) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const uint4 a = rec[order[i]];
-  s.edge[i] = a.x; s.aux[i] = a.y;
+  const bool is_id = ((a.w >> 16) & 0xffu) == KIND_INDEL;
+  s.edge[i] = a.x;
+  s.aux[i] = a.w >> 24 == NATURE_DRIVER ? a.y
+                                        : site_aux(genome, is_id, s.locus[i] + (is_id ? 1u : 0u), a.w & 0xffu, a.y);
   s.allele[i] = uint16_t(a.z); s.seq[i] = uint16_t(a.z >> 16);
   s.cls[i] = uint8_t(a.w); s.sig[i] = uint8_t(a.w >> 8); s.kind[i] = uint8_t(a.w >> 16); s.nature[i] = uint8_t(a.w >> 24);
   if (n_inst) {
@@ -632,9 +689,10 @@ struct BatchSlots {
   __device__ __forceinline__ Key key(Ref i) const { return keys[i]; }
   __device__ __forceinline__ Mut first(uint32_t slot, Ref& inst) const {
     const bool is_id = slot >= n_snv;
-    const uint32_t j = is_id ? slot - n_snv : slot;
+    const uint32_t j = is_id ? slot - n_snv : slot, ncell = cell_off[n_inst];
     const uint32_t* off = is_id ? off_id : off_snv;
-    const uint32_t q = find_cell(off, cell_off[n_inst], j);        // global cell
+    const bool one = __all_sync(0xffffffffu, is_id) || !__any_sync(0xffffffffu, is_id);   // the warp has one kind
+    const uint32_t q = one ? find_cell_warp(off, ncell, j) : find_cell(off, ncell, j);    // global cell
     inst = upper_index(cell_off, n_inst, q);
     const uint32_t lq = q - cell_off[inst], E = tabs[inst].n_epochs;
     return {lq / E, lq % E, j - off[q], is_id};
@@ -674,23 +732,34 @@ __global__ void k_place_first_b(BatchSlots s, PlaceRaw o, uint32_t n_slots, uint
                                 uint32_t* __restrict__ fslot, uint64_t fmask, uint8_t* __restrict__ lost,
                                 uint32_t* __restrict__ err) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_slots) return;
   uint32_t inst, cls, sig;
-  const Mut u = s.first(i, inst);
+  const Mut u = s.first(min(i, n_slots - 1), inst);
+  if (i >= n_slots) return;
   const PlaceTables& t = s.tabs[inst];
   const Key key = s.keys[inst];
   s.inst_of[i] = uint16_t(inst);
   draw_class(t, key, u, cls, sig);
   Site x;
-  if (!draw_site(t, key, u, 0u, cls, sig, x)) { atomicOr(err, ERR_EMPTY_CLASS); o.locus[i] = 0; return; }
+  if (!draw_position(t, key, u, 0u, cls, sig, x)) { atomicOr(err, ERR_EMPTY_CLASS); o.locus[i] = 0; return; }
+  uint64_t h = 0;
+  if (fkeys) {
+    h = key_hash(s.tab_key(x.locus, inst)) & fmask;
+    prefetch_l2(fkeys + h);
+    prefetch_l2(fslot + h);
+  }
+  draw_allele(t, node_class_of(t, u.v), x);
+  if (fkeys) {
+    if (x.locus == LOCUS_INVALID) {
+      lost[i] = 1;
+    } else if (!key_entry(fkeys, fmask, s.tab_key(x.locus, inst), h)) {
+      atomicOr(err, ERR_CAPACITY);
+    } else {
+      const uint32_t old = atomicMin(fslot + h, i);
+      if (old < i) lost[i] = 1;
+      else if (old != 0xffffffffu) lost[old] = 1;
+    }
+  }
   put_site(t, o, i, u, sig, x);
-  if (fkeys == nullptr) return;
-  if (x.locus == LOCUS_INVALID) { lost[i] = 1; return; }
-  uint64_t h;
-  if (!key_entry(fkeys, fmask, s.tab_key(x.locus, inst), h)) { atomicOr(err, ERR_CAPACITY); return; }
-  const uint32_t old = atomicMin(fslot + h, i);
-  if (old < i) lost[i] = 1;
-  else if (old != 0xffffffffu) lost[old] = 1;
 }
 
 // sort of a batch by (instance, locus): bucket = instance * nb + locus >> 10
@@ -767,8 +836,8 @@ void sites_covered(const PlaceTables& t, const PlaceRaw& o, uint64_t seed, const
   note_launch();
 }
 
-void sort_by_locus(const PlaceRaw& o, uint32_t n, uint64_t G, uint32_t* bcnt, uint32_t* part, uint32_t* order,
-                   const PlaceOut& sorted, unsigned long long* keys, cudaStream_t st) {
+void sort_by_locus(const PlaceRaw& o, uint32_t n, const uint32_t* genome, uint64_t G, uint32_t* bcnt, uint32_t* part,
+                   uint32_t* order, const PlaceOut& sorted, unsigned long long* keys, cudaStream_t st) {
   const uint32_t nb = uint32_t((G >> BUCKET_SHIFT) + 1);
   uint32_t* const bfill = bcnt + nb;
   cudaMemsetAsync(bcnt, 0, sizeof(uint32_t) * 2 * nb, st);
@@ -777,7 +846,7 @@ void sort_by_locus(const PlaceRaw& o, uint32_t n, uint64_t G, uint32_t* bcnt, ui
   scan_rows<uint32_t>(bcnt, bcnt, nb, 1, part, nullptr, st);
   k_bucket_scatter_keys<<<nblk(n), 256, 0, st>>>(o.locus, n, bcnt, bfill, keys); note_launch();
   k_bucket_sort_keys<<<nblk(nb, SORT_BUCKETS), SORT_THREADS, 0, st>>>(bcnt, nb, n, keys, sorted.locus, order);
-  k_gather_records<<<nblk(n), 256, 0, st>>>(o.rec, order, n, sorted, nullptr, 0u, 0u, nullptr);
+  k_gather_records<<<nblk(n), 256, 0, st>>>(o.rec, order, n, genome, sorted, nullptr, 0u, 0u, nullptr);
   note_launch(2);
 }
 
@@ -817,8 +886,8 @@ void sites_settle_batch(const PlaceTables* tabs, uint32_t n_inst, const uint32_t
   note_launch(2);
 }
 
-void sort_batch(const PlaceRaw& o, const uint16_t* inst_of, uint32_t n, uint32_t n_inst, uint64_t G, uint32_t* bcnt,
-                uint32_t* bfill, uint32_t* part, uint32_t* order, const PlaceOut& sorted, uint16_t* inst_sorted,
+void sort_batch(const PlaceRaw& o, const uint16_t* inst_of, uint32_t n, uint32_t n_inst, const uint32_t* genome,
+                uint64_t G, uint32_t* bcnt, uint32_t* bfill, uint32_t* part, uint32_t* order, const PlaceOut& sorted, uint16_t* inst_sorted,
                 unsigned long long* keys, cudaStream_t st) {
   const uint32_t nb = uint32_t((G >> BUCKET_SHIFT) + 1);
   const uint64_t nbt = uint64_t(nb) * n_inst;
@@ -829,7 +898,7 @@ void sort_batch(const PlaceRaw& o, const uint16_t* inst_of, uint32_t n, uint32_t
   scan_rows<uint32_t>(bcnt, bcnt, nbt, 1, part, bcnt + nbt, st);
   k_bucket_scatter_b<<<nblk(n), 256, 0, st>>>(o.locus, inst_of, n, nb, bcnt, bfill, keys); note_launch();
   k_bucket_sort_keys<<<nblk(nbt, SORT_BUCKETS), SORT_THREADS, 0, st>>>(bcnt, uint32_t(nbt), n, keys, sorted.locus, order);
-  k_gather_records<<<nblk(n), 256, 0, st>>>(o.rec, order, n, sorted, inst_sorted, n_inst, nb, bcnt);
+  k_gather_records<<<nblk(n), 256, 0, st>>>(o.rec, order, n, genome, sorted, inst_sorted, n_inst, nb, bcnt);
   note_launch(2);
 }
 
