@@ -2188,7 +2188,7 @@ struct pg_calib {
   uint32_t n_rep = 0, K = 0, J = 0, C = 0, P = 0, n_segs = 0;
   DBuf<int32_t> alt, depth, cls;
   DBuf<uint64_t> seg_start;
-  DBuf<uint32_t> seg_rep, seg_len, rep_first_seg, rep_done, rep_step;   // rep_step: one more entry, the status
+  DBuf<uint32_t> seg_rep, seg_len, rep_first_seg, rep_done, status;
   DBuf<float> sig_rows, epoch_w, phi, tab, m, v;
   DBuf<float2> partial;
   bool split = false;                // more segments than the GPU holds at a time
@@ -2210,7 +2210,7 @@ struct pg_calib {
   ~pg_calib() {
     if (graph) cudaGraphExecDestroy(graph);
     alt.reset(); depth.reset(); cls.reset(); seg_start.reset(); seg_rep.reset(); seg_len.reset();
-    rep_first_seg.reset(); rep_done.reset(); rep_step.reset(); sig_rows.reset(); epoch_w.reset();
+    rep_first_seg.reset(); rep_done.reset(); status.reset(); sig_rows.reset(); epoch_w.reset();
     phi.reset(); partial.reset(); tab.reset(); m.reset(); v.reset();
     pool.release_all();
     if (own_st) cudaStreamDestroy(own_st);
@@ -2304,12 +2304,11 @@ pg_status pg_calib_create(uint32_t n_rep, const uint64_t* site_off, const int32_
     c->rep_done = DBuf<uint32_t>(P, n_rep);
     ck(cudaMemsetAsync(c->rep_done.p, 0, sizeof(uint32_t) * n_rep, st), "memset");
     c->part_stride = (1 + 3 * K + K * J + 3) & ~3u;
-    c->partial = DBuf<float2>(P, uint64_t(srep.size()) * c->part_stride);
+    c->partial = DBuf<float2>(P, (c->split ? 1 : 2) * uint64_t(srep.size()) * c->part_stride);
     if (c->split) c->tab = DBuf<float>(P, uint64_t(n_rep) * c->part_stride);
     c->m = DBuf<float>(P, uint64_t(n_rep) * c->P);
     c->v = DBuf<float>(P, uint64_t(n_rep) * c->P);
-    c->rep_step = DBuf<uint32_t>(P, n_rep + 1);
-    ck(cudaMemsetAsync(c->rep_step.p, 0, sizeof(uint32_t) * (n_rep + 1), st), "memset");
+    c->status = DBuf<uint32_t>(P, 1);
     ck(cudaStreamSynchronize(st), "calibration upload");
     *out = c.release();
   });
@@ -2366,21 +2365,19 @@ pg_status pg_calib_adam(pg_calib* c, float* params, uint32_t steps, float lr, fl
     require(lr > 0 && beta1 >= 0 && beta1 < 1 && beta2 >= 0 && beta2 < 1 && eps > 0, "invalid Adam hyperparameters");
     ck(cudaSetDevice(c->device), "cudaSetDevice");
     cudaStream_t st = c->st;
-    ck(cudaMemsetAsync(c->m.p, 0, sizeof(float) * c->n_rep * c->P, st), "memset");
-    ck(cudaMemsetAsync(c->v.p, 0, sizeof(float) * c->n_rep * c->P, st), "memset");
     if (!c->split && steps > 1) {
       // every step in one launch, whose CTAs are resident together
       pg::CalibArgs a = c->args();
       a.steps = steps;
-      a.rep_step = c->rep_step.p;
-      a.status = c->rep_step.p + c->n_rep;
-      ck(cudaMemsetAsync(c->rep_step.p, 0, sizeof(uint32_t) * (c->n_rep + 1), st), "memset");
+      a.status = c->status.p;
+      ck(cudaMemsetAsync(c->status.p, 0, sizeof(uint32_t), st), "memset");
       pg::calib_launch(a, c->n_segs, c->n_rep, params, nll, nullptr, pg::AdamArgs{c->m.p, c->v.p, 0, lr, beta1, beta2, eps}, st);
-      // (zero already, unless a wait ran out)
       ck(cudaMemsetAsync(c->rep_done.p, 0, sizeof(uint32_t) * c->n_rep, st), "memset");
       ck(cudaGetLastError(), "calibration steps");
       return;
     }
+    ck(cudaMemsetAsync(c->m.p, 0, sizeof(float) * c->n_rep * c->P, st), "memset");
+    ck(cudaMemsetAsync(c->v.p, 0, sizeof(float) * c->n_rep * c->P, st), "memset");
     const bool same = c->graph && c->gkey.params == params && c->gkey.steps == steps && c->gkey.lr == lr &&
                       c->gkey.b1 == beta1 && c->gkey.b2 == beta2 && c->gkey.eps == eps && c->gkey.nll == nll &&
                       c->gkey.st == st;

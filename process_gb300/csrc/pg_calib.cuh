@@ -34,9 +34,9 @@
 // derives its replicate's constants and the one that finishes a replicate's
 // last segment runs its epilogue.  An evaluation of 2e5 sites took 24.7 us with
 // separate kernels (and 13 CTAs of 16384 sites), now 10.8.  Adam steps repeat
-// inside that launch, each replicate going on when its epilogue is through:
+// inside that launch, each replicate going on when its sums are complete:
 // 200 steps over 64 x 5e4 sites took 5.4 ms as a graph of three kernels a step,
-// 3.4 ms now.  With more segments than that, the constants and the
+// 3.1 ms now.  With more segments than that, the constants and the
 // epilogues are launches of their own (in k_calib they keep a CTA's slot from
 // the next segment): 512 x 1e5 sites in 147 us.
 // Persistent CTAs with equal shares of all sites took 190 us there: they reach
@@ -76,14 +76,18 @@ struct CalibRow {
   float row[3 * K + K * J];
 };
 template <uint32_t K, uint32_t J>
-__device__ __forceinline__ void calib_tables(CalibRow<K, J>& sh, const CalibArgs& a, const float* __restrict__ params,
-                                             uint32_t r) {
+__device__ __forceinline__ void calib_load(CalibRow<K, J>& sh, const CalibArgs& a, const float* __restrict__ params,
+                                           uint32_t r) {
   constexpr uint32_t P = K + K * J + 1;
   const uint32_t t = threadIdx.x;
-  if (t < P) sh.p[t] = __ldcg(params + uint64_t(r) * P + t);   // (another SM may have written them)
+  if (t < P) sh.p[t] = __ldcg(params + uint64_t(r) * P + t);
   else if (t >= 128 && t < 128 + K) sh.ew[t - 128] = a.epoch_w[r * K + t - 128];
   else if (t >= 160 && t < 160 + K) sh.phi[t - 160] = a.phi[r * K + t - 160];
   __syncthreads();
+}
+template <uint32_t K, uint32_t J>
+__device__ __forceinline__ void calib_rows(CalibRow<K, J>& sh) {
+  const uint32_t t = threadIdx.x;
   if (t < K) {
     float Z = 0.f;
 #pragma unroll
@@ -108,6 +112,12 @@ __device__ __forceinline__ void calib_tables(CalibRow<K, J>& sh, const CalibArgs
     for (uint32_t j = 0; j < J; ++j) sh.row[3 * K + k * J + j] = expf(th[j] - mx) / den;
   }
   __syncthreads();
+}
+template <uint32_t K, uint32_t J>
+__device__ __forceinline__ void calib_tables(CalibRow<K, J>& sh, const CalibArgs& a, const float* __restrict__ params,
+                                             uint32_t r) {
+  calib_load<K, J>(sh, a, params, r);
+  calib_rows<K, J>(sh);
 }
 
 // Per-site work: every thread takes sites i0 + tid, i0 + tid + 256, ...
@@ -186,19 +196,16 @@ __device__ __forceinline__ float warp_transpose_sum(const float* v, uint32_t lan
   return w[0];
 }
 
-// a replicate's segment sums -> NLL and gradient (-> Adam step), by the CTA
-// that finished its last segment
+// a replicate's segment sums -> NLL (tot[0]) and gradient
 struct CalibEpilogue {
   float grp[CAL_THREADS / 32][1 + 3 * CAL_MAXK + CAL_MAXK * CAL_MAXJ][2];
   float2 tot[1 + 3 * CAL_MAXK + CAL_MAXK * CAL_MAXJ];
   float grad[CAL_MAXK + CAL_MAXK * CAL_MAXJ + 1];
 };
 template <uint32_t K, uint32_t J>
-__device__ __forceinline__ void calib_epilogue(CalibEpilogue& sh, const CalibRow<K, J>& c, const CalibArgs& a,
-                                               float* __restrict__ params, uint32_t r, const float2* partial, float* __restrict__ nll_out,
-                                               float* __restrict__ grad_out, const AdamArgs& adam,
-                                               uint32_t step) {
-  constexpr uint32_t P = K + K * J + 1, NV = 1 + 3 * K + K * J;
+__device__ __forceinline__ void calib_gradient(CalibEpilogue& sh, const CalibRow<K, J>& c, const CalibArgs& a,
+                                               uint32_t r, const float2* partial) {
+  constexpr uint32_t NV = 1 + 3 * K + K * J;
   const uint32_t c0 = a.rep_first_seg[r], c1 = a.rep_first_seg[r + 1];
   // warp g takes segments c0 + g, c0 + g + 8, ..., a lane one value (or three);
   // then the warps' sums in order
@@ -253,24 +260,48 @@ __device__ __forceinline__ void calib_epilogue(CalibEpilogue& sh, const CalibRow
     sh.grad[K + x] = -c.row[3 * K + x] * ((H[x].x - G[x / J].x) + (H[x].y - G[x / J].y));
   }
   __syncthreads();
+}
+
+// The Adam step's bias corrections of step `step` (from 0) and its update
+struct AdamBias { float m, v; };
+__device__ __forceinline__ AdamBias adam_bias(const AdamArgs& adam, uint32_t step) {
+  const float t = float(step + 1);
+  return {1.f - powf(adam.beta1, t), 1.f - powf(adam.beta2, t)};
+}
+__device__ __forceinline__ float adam_update(const AdamArgs& adam, AdamBias b, float p, float g, float& m, float& v) {
+  m = adam.beta1 * m + (1.f - adam.beta1) * g;
+  v = adam.beta2 * v + (1.f - adam.beta2) * g * g;
+  const float mh = m / b.m, vh = v / b.v;
+  return p - adam.lr * mh / (sqrtf(vh) + adam.eps);
+}
+
+// one evaluation's results (and Adam step), by one CTA per replicate
+template <uint32_t K, uint32_t J>
+__device__ __forceinline__ void calib_epilogue(CalibEpilogue& sh, const CalibRow<K, J>& c, const CalibArgs& a,
+                                               float* __restrict__ params, uint32_t r, float* __restrict__ nll_out,
+                                               float* __restrict__ grad_out, const AdamArgs& adam) {
+  constexpr uint32_t P = K + K * J + 1;
+  calib_gradient<K, J>(sh, c, a, r, a.partial);
   if (threadIdx.x == 0 && nll_out) nll_out[r] = sh.tot[0].x;
   for (uint32_t q = threadIdx.x; q < P; q += CAL_THREADS) {
+    const uint64_t o = uint64_t(r) * P + q;
     const float gq = sh.grad[q];
-    if (grad_out) grad_out[uint64_t(r) * P + q] = gq;
-    if (adam.m) {   // Adam step `step` (from 0) on the parameters (bias-corrected)
-      const uint64_t o = uint64_t(r) * P + q;
-      const float t = float(step + 1);
-      const float m = adam.beta1 * __ldcg(adam.m + o) + (1.f - adam.beta1) * gq;
-      const float v = adam.beta2 * __ldcg(adam.v + o) + (1.f - adam.beta2) * gq * gq;
+    if (grad_out) grad_out[o] = gq;
+    if (adam.m) {
+      float m = __ldcg(adam.m + o), v = __ldcg(adam.v + o);
+      params[o] = adam_update(adam, adam_bias(adam, adam.t), c.p[q], gq, m, v);
       adam.m[o] = m; adam.v[o] = v;
-      const float mh = m / (1.f - powf(adam.beta1, t)), vh = v / (1.f - powf(adam.beta2, t));
-      params[o] = c.p[q] - adam.lr * mh / (sqrtf(vh) + adam.eps);
     }
   }
 }
 
 // STEPS: a.steps Adam steps in a cooperative launch (an instance of its own: in
-// the other the step's state would spill)
+// the other the step's state would spill).  Every CTA of a replicate keeps the
+// parameters and moments and makes each step itself, from all the segments'
+// sums in the same order, so a step has one wait (the sums) where parameters
+// published by one CTA need a second: 200 steps over 64 x 5e4 sites 3.53 ->
+// 3.12 ms.  The sums alternate between two halves of a.partial: a CTA is at
+// most one step ahead of the others.
 template <uint32_t K, uint32_t J, bool STEPS>
 __global__ void __launch_bounds__(CAL_THREADS, calib_min_blocks(K, J)) k_calib(CalibArgs a, float* __restrict__ params,
                                                                                float* __restrict__ nll_out,
@@ -285,13 +316,22 @@ __global__ void __launch_bounds__(CAL_THREADS, calib_min_blocks(K, J)) k_calib(C
   __shared__ float4 s_sig[JP / 4][CAL_MAXC * 8], s_mix[KP / 4][CAL_MAXC * 8];
   __shared__ CalibRow<K, J> s_c;
   __shared__ union { float red[CAL_WARPS][NV]; CalibEpilogue epi; } s_u;
-  __shared__ uint32_t s_go, s_step;
+  __shared__ uint32_t s_go;
+  // STEPS: the moments of the parameters, the step's bias corrections
+  __shared__ float s_adam[2][STEPS ? K + K * J + 1 : 1];
+  __shared__ AdamBias s_bias;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t seg = a.seg0 + blockIdx.x, r = a.seg_rep[seg];
   const uint64_t i0 = a.seg_start[seg], i1 = i0 + a.seg_len[seg];
-  if (STEPS && threadIdx.x == 0) s_step = 0;
-  for (;;) {   // a.steps evaluations (STEPS), or one
-  if (!STEPS && a.tab) {
+  if (STEPS) {
+    if (threadIdx.x < K + K * J + 1) s_adam[0][threadIdx.x] = s_adam[1][threadIdx.x] = 0.f;
+    calib_load<K, J>(s_c, a, params, r);
+  }
+  for (uint32_t step = 0;; ++step) {   // a.steps evaluations (STEPS), or one
+  if (STEPS) {
+    if (threadIdx.x == 128) s_bias = adam_bias(adam, step);
+    calib_rows<K, J>(s_c);
+  } else if (a.tab) {
     for (uint32_t x = threadIdx.x; x < 3 * K + K * J; x += CAL_THREADS) s_c.row[x] = a.tab[uint64_t(r) * a.part_stride + x];
     __syncthreads();
   } else {
@@ -302,8 +342,13 @@ __global__ void __launch_bounds__(CAL_THREADS, calib_min_blocks(K, J)) k_calib(C
     float sg[JP], m[KP];
 #pragma unroll
     for (uint32_t j = 0; j < JP; j += 4) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(a.sig_rows) + ((x >> 3) * JP + j) / 4);
-      s_sig[j / 4][x] = v;
+      float4 v;
+      if (STEPS && step) {
+        v = s_sig[j / 4][x];
+      } else {
+        v = __ldg(reinterpret_cast<const float4*>(a.sig_rows) + ((x >> 3) * JP + j) / 4);
+        s_sig[j / 4][x] = v;
+      }
       sg[j] = v.x; sg[j + 1] = v.y; sg[j + 2] = v.z; sg[j + 3] = v.w;
     }
 #pragma unroll
@@ -429,58 +474,66 @@ __global__ void __launch_bounds__(CAL_THREADS, calib_min_blocks(K, J)) k_calib(C
   }
   __syncthreads();
   // segment sums: nll, A_k, B_k, G_k, H_kj (j < J)
-  float2* out = a.partial + uint64_t(seg) * a.part_stride;
+  float2* const sums = STEPS && (step & 1u) ? a.partial + uint64_t(gridDim.x) * a.part_stride : a.partial;
+  float2* out = sums + uint64_t(seg) * a.part_stride;
   for (uint32_t x = threadIdx.x; x < NV; x += CAL_THREADS) {
     Neu t;
     for (uint32_t w = 0; w < CAL_WARPS; ++w) t.add(s_u.red[w][x]);
     out[x] = t.both();
   }
   if (!STEPS && a.tab) return;
-  // the CTA that finishes the replicate's last segment runs the epilogue (the
-  // count is left at zero for the next evaluation)
   __threadfence();
   __syncthreads();
-  const uint32_t step = STEPS ? s_step : adam.t;
-  const bool end = !STEPS || step + 1 == a.steps;
-  if (threadIdx.x == 0) {
-    const uint32_t n = a.rep_first_seg[r + 1] - a.rep_first_seg[r];
-    s_go = atomicAdd(a.rep_done + r, 1u) + 1u == n ? 1u : 0u;
-    if (s_go) a.rep_done[r] = 0u;
-    __threadfence();
-  }
-  __syncthreads();
-  if (s_go) {
-    calib_epilogue<K, J>(s_u.epi, s_c, a, params, r, a.partial, end ? nll_out : nullptr, grad_out, adam, step);
-    __threadfence();
-  }
-  if (end) return;
-  __syncthreads();
-  // the next evaluation starts when the replicate's epilogue is through.  The
-  // CTAs are all resident (a cooperative launch); a wait that runs out all the
-  // same marks the call and every CTA leaves at its next look
-  if (threadIdx.x == 0) {
-    uint32_t go = 1;
-    if (s_go) {
-      atomicExch(a.rep_step + r, step + 1);
-    } else {
-      uint32_t polls = 0;
-      while (*reinterpret_cast<volatile uint32_t*>(a.rep_step + r) <= step) {
+  const uint32_t n = a.rep_first_seg[r + 1] - a.rep_first_seg[r];
+  if constexpr (!STEPS) {
+    // the CTA that finishes the replicate's last segment runs the epilogue (the
+    // count is left at zero for the next evaluation)
+    if (threadIdx.x == 0) {
+      s_go = atomicAdd(a.rep_done + r, 1u) + 1u == n ? 1u : 0u;
+      if (s_go) a.rep_done[r] = 0u;
+      __threadfence();
+    }
+    __syncthreads();
+    if (s_go) calib_epilogue<K, J>(s_u.epi, s_c, a, params, r, nll_out, grad_out, adam);
+    return;
+  } else {
+    constexpr uint32_t P = K + K * J + 1;
+    // All the replicate's sums of this step.  The CTAs are all resident (a
+    // cooperative launch); a wait that runs out all the same marks the call and
+    // every CTA leaves at its next look.
+    if (threadIdx.x == 0) {
+      uint32_t go = 1, polls = 0;
+      atomicAdd(a.rep_done + r, 1u);
+      while (*reinterpret_cast<volatile uint32_t*>(a.rep_done + r) < (step + 1) * n) {
         if (++polls > CAL_SPIN_LIMIT || *reinterpret_cast<volatile uint32_t*>(a.status)) { go = 0; break; }
-        __nanosleep(64);
+        __nanosleep(20);
       }
       __threadfence();
       if (!go) atomicExch(a.status, 1u);
+      s_go = go;
     }
-    s_go = go;
-    s_step = step + 1;
-  }
-  __syncthreads();
-  if (!s_go) {
-    if (threadIdx.x == 0) {                    // no result: NaN
-      params[uint64_t(r) * (K + K * J + 1)] = __int_as_float(0x7fc00000);
-      if (nll_out) nll_out[r] = __int_as_float(0x7fc00000);
+    __syncthreads();
+    const bool first = seg == a.rep_first_seg[r];
+    if (!s_go) {
+      if (threadIdx.x == 0) {                    // no result: NaN
+        params[uint64_t(r) * P] = __int_as_float(0x7fc00000);
+        if (nll_out) nll_out[r] = __int_as_float(0x7fc00000);
+      }
+      return;
     }
-    return;
+    calib_gradient<K, J>(s_u.epi, s_c, a, r, sums);
+    const bool end = step + 1 == a.steps;
+    if (threadIdx.x < P) {
+      const float p = adam_update(adam, s_bias, s_c.p[threadIdx.x], s_u.epi.grad[threadIdx.x], s_adam[0][threadIdx.x],
+                                  s_adam[1][threadIdx.x]);
+      s_c.p[threadIdx.x] = p;
+      if (end && first) params[uint64_t(r) * P + threadIdx.x] = p;
+    }
+    if (end) {
+      if (first && threadIdx.x == 0 && nll_out) nll_out[r] = s_u.epi.tot[0].x;
+      return;
+    }
+    __syncthreads();
   }
   }
 }
@@ -502,7 +555,7 @@ __global__ void __launch_bounds__(CAL_THREADS) k_calib_epilogue(CalibArgs a, flo
   __shared__ CalibEpilogue s_epi;
   const uint32_t r = a.rep0 + blockIdx.x;
   calib_tables<K, J>(s_c, a, params, r);
-  calib_epilogue<K, J>(s_epi, s_c, a, params, r, a.partial, nll_out, grad_out, adam, adam.t);
+  calib_epilogue<K, J>(s_epi, s_c, a, params, r, nll_out, grad_out, adam);
 }
 
 template <uint32_t K, uint32_t J>

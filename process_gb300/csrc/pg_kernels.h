@@ -439,12 +439,12 @@ struct CalibArgs {
   const uint64_t* seg_start;
   const uint32_t* seg_len;
   const uint32_t* rep_first_seg;  // n_rep + 1
-  uint32_t* rep_done;             // n_rep counts, zero between launches
-  float2* partial;                // per segment, part_stride sums (>= 1 + 3K + K J) and their remainders
+  uint32_t* rep_done;             // n_rep counts, zero before a launch (and after one of one evaluation)
+  float2* partial;                // per segment, part_stride sums (>= 1 + 3K + K J) and their remainders; with
+                                  //   steps > 1 twice that
   uint32_t part_stride;
   uint32_t seg0, rep0;            // first segment and replicate of the launch
   uint32_t steps;                 // evaluations of the launch (above 1: Adam steps, without tab)
-  uint32_t* rep_step;             // with steps > 1, zeroed: steps done per replicate
   uint32_t* status;               // set when a wait between the steps ran out
   float* tab;                     // per replicate, part_stride floats: its constants, where they and the
                                   //   epilogues have launches of their own; else NULL
