@@ -200,7 +200,7 @@ def reference_arm(args):
 
 def batch_bench(stream, n_inst: int, steps: int, warmup: int):
     """Batched replicates (256 forests on 100 Mbp): every instance placed and sequenced in
-    one batch run (fused placement launches, one persistent read kernel under
+    one batch run (fused placement launches, one read kernel under
     a CUDA graph, tile sizes from the autotuner).  Reads/s and placed
     mutations/s of whole runs, timed with CUDA events on the engine stream;
     beside them the plain path run instance by instance on the first 16."""
@@ -264,7 +264,7 @@ def batch_bench(stream, n_inst: int, steps: int, warmup: int):
 def calibration_bench(world: int, n_rep: int = 512, n_sites: int = 100_000, steps: int = 200):
     """Batched calibration (512 replicates x 1e5 sites, Poisson depth means
     U(30, 200), K=4, 3 exposures): gradient evaluations per second of the
-    batched kernels, of the graph-captured Adam loop, and of the per-instance
+    batched kernels, of the Adam loop, and of the per-instance
     path (one launch pair per replicate), plus the FP64 CPU oracle."""
     import torch
 
@@ -288,7 +288,7 @@ def calibration_bench(world: int, n_rep: int = 512, n_sites: int = 100_000, step
     ev[1].record(s)
     ev[1].synchronize()
     t_batched = ev[0].elapsed_time(ev[1]) / 1000.0 / reps
-    # 200 Adam steps under one CUDA graph
+    # 200 Adam steps in one call
     p = p0.clone()
     b.adam(p, steps)
     p = p0.clone()

@@ -462,7 +462,8 @@ pg_status pg_calib_nll_grad(pg_calib* cal, const float* params, float* nll, floa
 /* One replicate only (the per-instance path): same layout, replicate `rep`. */
 pg_status pg_calib_nll_grad_one(pg_calib* cal, uint32_t rep, const float* params, float* nll, float* grad);
 /* `steps` Adam steps on every replicate's parameters (device, updated in
- * place), run entirely on the device as one CUDA graph; nll (device, n_rep,
+ * place), run entirely on the device (in one launch where the
+ * segments fit the GPU at a time, else as a CUDA graph); nll (device, n_rep,
  * may be NULL) receives the NLL of the last step's parameters before the
  * update.  The optimizer state restarts at zero on each call. */
 pg_status pg_calib_adam(pg_calib* cal, float* params, uint32_t steps, float lr, float beta1, float beta2, float eps,
@@ -481,7 +482,7 @@ pg_status pg_calib_adam(pg_calib* cal, float* params, uint32_t steps, float lr, 
  * path computes for it alone (pg_place_mutations then pg_simulate_seq on an
  * engine whose species 0 has those rates and that exposure at time 0, with
  * the same seeds and the instance's tile size).  Placement runs as single
- * launches over all instances; sequencing as one persistent kernel over every
+ * launches over all instances; sequencing as one kernel over every
  * (instance, sample, tile), captured into a CUDA graph on the first run and
  * replayed afterwards. */
 typedef struct pg_batch pg_batch;
@@ -493,7 +494,7 @@ pg_status pg_batch_destroy(pg_batch* batch);
 /* place and sequence every instance with its placement and sequencing seed */
 pg_status pg_batch_run(pg_batch* batch, const uint64_t* place_seed, const uint64_t* seq_seed);
 /* The autotuner: places once with these seeds, then times the whole
- * persistent read launch for candidate tile sizes (multiples 0.5, 0.75, 1,
+ * read launch for candidate tile sizes (multiples 0.5, 0.75, 1,
  * 1.25 of every instance's analytic size) and keeps the fastest; tile_sizes
  * (may be NULL) receives the choice. */
 pg_status pg_batch_autotune(pg_batch* batch, const uint64_t* place_seed, const uint64_t* seq_seed,

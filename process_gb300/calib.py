@@ -108,7 +108,7 @@ class CalibBatch:
 
     def adam(self, params, steps: int, lr: float = 0.05, beta1: float = 0.9, beta2: float = 0.999,
              eps: float = 1e-8):
-        """``steps`` Adam steps on every replicate, in place, as one CUDA graph."""
+        """``steps`` Adam steps on every replicate, in place, without host work between them."""
         import torch
         assert params.dtype == torch.float32 and params.is_contiguous() and params.is_cuda
         nll = torch.empty(self.n_rep, dtype=torch.float32, device=params.device)

@@ -2190,7 +2190,8 @@ struct pg_calib {
   DBuf<uint64_t> seg_start;
   DBuf<uint32_t> seg_rep, seg_len, rep_first_seg, rep_done, status;
   DBuf<float> sig_rows, epoch_w, phi, tab, m, v;
-  DBuf<float2> partial;
+  DBuf<float2> partial, epoch_log;
+  DBuf<float4> rep_stat;
   bool split = false;                // more segments than the GPU holds at a time
   std::vector<uint32_t> rep_first_seg_h;
   uint32_t part_stride = 0;
@@ -2200,7 +2201,7 @@ struct pg_calib {
     pg::CalibArgs a{};
     a.K = K; a.J = J; a.C = C; a.P = P;
     a.alt = alt.p; a.depth = depth.p; a.cls = cls.p;
-    a.epoch_w = epoch_w.p; a.phi = phi.p; a.sig_rows = sig_rows.p;
+    a.epoch_w = epoch_w.p; a.phi = phi.p; a.sig_rows = sig_rows.p; a.rep_stat = rep_stat.p; a.epoch_log = epoch_log.p;
     a.seg_rep = seg_rep.p; a.seg_start = seg_start.p; a.seg_len = seg_len.p;
     a.rep_first_seg = rep_first_seg.p; a.rep_done = rep_done.p;
     a.partial = partial.p; a.part_stride = part_stride; a.tab = split ? tab.p : nullptr;
@@ -2211,7 +2212,7 @@ struct pg_calib {
     if (graph) cudaGraphExecDestroy(graph);
     alt.reset(); depth.reset(); cls.reset(); seg_start.reset(); seg_rep.reset(); seg_len.reset();
     rep_first_seg.reset(); rep_done.reset(); status.reset(); sig_rows.reset(); epoch_w.reset();
-    phi.reset(); partial.reset(); tab.reset(); m.reset(); v.reset();
+    phi.reset(); partial.reset(); rep_stat.reset(); epoch_log.reset(); tab.reset(); m.reset(); v.reset();
     pool.release_all();
     if (own_st) cudaStreamDestroy(own_st);
   }
@@ -2232,9 +2233,22 @@ pg_status pg_calib_create(uint32_t n_rep, const uint64_t* site_off, const int32_
     require(site_off[0] == 0, "site offsets start at 0");
     for (uint32_t r = 0; r < n_rep; ++r) require(site_off[r + 1] >= site_off[r], "site offsets must not decrease");
     require(n == 0 || (alt && depth && cls), "NULL site arrays");
-    for (uint64_t i = 0; i < n; ++i) {
-      require(depth[i] >= 0 && alt[i] >= 0 && alt[i] <= depth[i], "sites need 0 <= alt <= depth");
-      require(cls[i] >= 0 && uint32_t(cls[i]) < C, "site class out of range");
+    // the replicates' sites and sums, exact in two floats up to 2^48
+    std::vector<float4> stat(2 * size_t(n_rep));
+    for (uint32_t r = 0; r < n_rep; ++r) {
+      uint64_t sa = 0, sd = 0;
+      const uint64_t nr = site_off[r + 1] - site_off[r];
+      for (uint64_t i = site_off[r]; i < site_off[r + 1]; ++i) {
+        require(depth[i] >= 0 && alt[i] >= 0 && alt[i] <= depth[i], "sites need 0 <= alt <= depth");
+        require(cls[i] >= 0 && uint32_t(cls[i]) < C, "site class out of range");
+        sa += uint32_t(alt[i]);
+        sd += uint32_t(depth[i]);
+      }
+      auto two = [](uint64_t x, float& h, float& l) { h = float(double(x)); l = float(double(x) - double(h)); };
+      float4 &s0 = stat[2 * size_t(r)], &s1 = stat[2 * size_t(r) + 1];
+      two(nr, s0.x, s0.y); two(sa, s0.z, s0.w); two(sd - sa, s1.x, s1.y);
+      s1.z = nr ? float(double(sd) / double(nr)) : 0.f;
+      s1.w = 0.f;
     }
     for (uint64_t x = 0; x < uint64_t(J) * C; ++x) require(signatures[x] >= 0, "signature probabilities >= 0");
     for (uint64_t x = 0; x < uint64_t(n_rep) * K; ++x) {
@@ -2259,6 +2273,13 @@ pg_status pg_calib_create(uint32_t n_rep, const uint64_t* site_off, const int32_
     }
     for (uint64_t x = 0; x < fw.size(); ++x) { fw[x] = float(epoch_weight[x]); fp[x] = float(phi[x]); }
     c->epoch_w = upload(P, fw, st); c->phi = upload(P, fp, st);
+    std::vector<float2> logl(fw.size());
+    for (size_t x = 0; x < fw.size(); ++x) {
+      const double y = std::log2(double(fw[x]));
+      logl[x].x = float(y);
+      logl[x].y = float(y - double(logl[x].x));
+    }
+    c->epoch_log = upload(P, logl, st);
     {   // signatures by class, rows of 4 or 8 floats
       const uint32_t JP = J > 4 ? 8 : 4;
       std::vector<float> rows(size_t(C) * JP, 0.f);
@@ -2266,6 +2287,7 @@ pg_status pg_calib_create(uint32_t n_rep, const uint64_t* site_off, const int32_
         for (uint32_t cl = 0; cl < C; ++cl) rows[size_t(cl) * JP + j] = fs[size_t(j) * C + cl];
       c->sig_rows = upload(P, rows, st);
     }
+    c->rep_stat = upload(P, stat, st);
     // segments: the smallest size that needs no more rounds of resident CTAs
     // than CALIB_SEG does (one round where possible; a last round of a few
     // CTAs would take as long as a full one), equal within a replicate
@@ -2305,7 +2327,7 @@ pg_status pg_calib_create(uint32_t n_rep, const uint64_t* site_off, const int32_
     ck(cudaMemsetAsync(c->rep_done.p, 0, sizeof(uint32_t) * n_rep, st), "memset");
     c->part_stride = (1 + 3 * K + K * J + 3) & ~3u;
     c->partial = DBuf<float2>(P, (c->split ? 1 : 2) * uint64_t(srep.size()) * c->part_stride);
-    if (c->split) c->tab = DBuf<float>(P, uint64_t(n_rep) * c->part_stride);
+    if (c->split) c->tab = DBuf<float>(P, uint64_t(n_rep) * (3 * K + 2 * K * J));
     c->m = DBuf<float>(P, uint64_t(n_rep) * c->P);
     c->v = DBuf<float>(P, uint64_t(n_rep) * c->P);
     c->status = DBuf<uint32_t>(P, 1);

@@ -17,9 +17,10 @@
 // GPU.  A CTA computes the per-site log-likelihoods and responsibilities in
 // FP32 with the replicate's constants and mixture weights in registers and
 // only the site class's signature row S(c) gathered from shared memory:
-//   u_k = log(exp(lr_k) L_k / Z) + a log v_k + (d - a) log(1 - v_k)
+//   u_k = log pi'_k / pi'_r + a log v_k / v_r + (d - a) log (1 - v_k) / (1 - v_r)
+//         (pi'_k = exp(lr_k) L_k / Z, r a reference epoch)
 //   e_k = exp(u_k - max u),  q_k = M_k(c) e_k,  s = sum_k q_k
-//   gamma_k = q_k / s,  log-likelihood = max u + log s
+//   gamma_k = q_k / s,  log-likelihood = the reference's + max u + log s
 // and reduces
 //   G_k = sum_i gamma_ik,  A_k = sum gamma_ik a_i,  B_k = sum gamma_ik (d_i - a_i),
 //   H_kj = sum_i gamma_ik S_j(c_i) / M_k(c_i) = sum_i e_ik S_j(c_i) / s_i,  NLL
@@ -33,17 +34,18 @@
 // While all segments are resident together, one launch does it all: each CTA
 // derives its replicate's constants and the one that finishes a replicate's
 // last segment runs its epilogue.  An evaluation of 2e5 sites took 24.7 us with
-// separate kernels (and 13 CTAs of 16384 sites), now 10.8.  Adam steps repeat
+// separate kernels (and 13 CTAs of 16384 sites), now 12.4.  Adam steps repeat
 // inside that launch, each replicate going on when its sums are complete:
 // 200 steps over 64 x 5e4 sites took 5.4 ms as a graph of three kernels a step,
-// 3.1 ms now.  With more segments than that, the constants and the
+// 3.3 ms now.  With more segments than that, the constants and the
 // epilogues are launches of their own (in k_calib they keep a CTA's slot from
-// the next segment): 512 x 1e5 sites in 147 us.
+// the next segment): 512 x 1e5 sites in 150 us.
 // Persistent CTAs with equal shares of all sites took 190 us there: they reach
 // their reductions together instead of overlapping them.
 #pragma once
 #include <cstdint>
 
+#include "pg_f2.cuh"
 #include "pg_kernels.h"
 
 namespace pg {
@@ -67,49 +69,132 @@ struct Neu {   // Neumaier-compensated FP32 sum
   }
 };
 
-// A replicate's parameters and constants in shared memory (one round of loads
-// for all of them), then by the threads k < K: log(exp(lr_k) L_k / Z) (K),
-// log v_k (K), log(1 - v_k) (K), the exposures w_kj (K x J).
+// A replicate's parameters and constants in shared memory.  The site loop works
+// on differences of log-likelihoods from those of a reference epoch (whose own
+// sum over the sites is linear in the counts and added by the epilogue): for
+// epoch k their constant, their slope in a and their slope in d, in base 2.
+// The constants come from two-float arithmetic and are rounded together: what
+// the slopes lose is put into the constant at the replicate's mean depth and
+// the alt count expected of epoch k there, where its sites lie.  So the
+// rounding of a constant, which every site shares, no longer adds up over the
+// sites: the gradient of 512 tables of 1e5 sites is 2.0e-7 off (1.2e-6 with
+// plain FP32 constants), 200 Adam steps over 64 tables of 5e4 sites, whose
+// parameters keep their remainders too, typically 1.8e-6 (5e-6; up to 4e-5
+// where Adam's oscillation amplifies rounding, now 2e-5).  It costs 1 to 2 us
+// an evaluation.
 template <uint32_t K, uint32_t J>
 struct CalibRow {
-  float p[K + K * J + 1], ew[K], phi[K];
-  float row[3 * K + K * J];
+  float p[K + K * J + 1], pl[K + K * J + 1], ew[K], phi[K];   // pl: the parameters' remainders (Adam steps)
+  F2 logl[K];                            // log2 L_k
+  F2 e[K + K * J + 1];                   // exponentials of the parameters (see calib_rows)
+  float row[3 * K + 2 * K * J];          // constant, a, d (K each), the exposures w_kj (K x J) and their remainders
+  float4 stat[2];                        // the replicate's sites and sums of a and of d - a (two floats each), its mean depth
+  F2 c[K], lv[K], l1[K], odds[K];        // log2 exp(lr) L, log2 v, log2(1 - v), v / (1 - v)
+  F2 prob[K];                            // pi_k = exp(lr_k) L_k / Z
+  F2 logz;
+  F2 lin[3];                             // the reference's log2 pi, log2 v, log2(1 - v)
+  float v[K], sig;
 };
 template <uint32_t K, uint32_t J>
 __device__ __forceinline__ void calib_load(CalibRow<K, J>& sh, const CalibArgs& a, const float* __restrict__ params,
                                            uint32_t r) {
   constexpr uint32_t P = K + K * J + 1;
   const uint32_t t = threadIdx.x;
-  if (t < P) sh.p[t] = __ldcg(params + uint64_t(r) * P + t);
+  if (t < P) { sh.p[t] = __ldcg(params + uint64_t(r) * P + t); sh.pl[t] = 0.f; }
   else if (t >= 128 && t < 128 + K) sh.ew[t - 128] = a.epoch_w[r * K + t - 128];
   else if (t >= 160 && t < 160 + K) sh.phi[t - 160] = a.phi[r * K + t - 160];
+  else if (t >= 176 && t < 176 + K) sh.logl[t - 176] = {a.epoch_log[r * K + t - 176].x, a.epoch_log[r * K + t - 176].y};
+  else if (t >= 192 && t < 194) sh.stat[t - 192] = a.rep_stat[2 * r + t - 192];
   __syncthreads();
 }
+// One thread per function value and one copy of each function's code, loops
+// rolled: the code runs once per evaluation, from far caches (unrolled per
+// epoch and exposure it took 4.5 us longer).
 template <uint32_t K, uint32_t J>
 __device__ __forceinline__ void calib_rows(CalibRow<K, J>& sh) {
+  constexpr uint32_t P = K + K * J + 1;
+  constexpr F2 LOG2E = {1.44269502162933350f, 1.92596299e-08f}, one = {1.f, 0.f};
   const uint32_t t = threadIdx.x;
+  auto par = [&](uint32_t q) { return F2{sh.p[q], sh.pl[q]}; };
+  // x - m (infinite, or of equal infinities, as in FP32)
+  auto less = [](F2 x, F2 m) {
+    const float d = x.h == m.h ? 0.f : __fsub_rn(x.h, m.h);
+    return fabsf(d) < 1e30f && fabsf(x.h) < 1e30f ? f2_add(x, f2_neg(m)) : F2{d, 0.f};
+  };
+  auto top = [&](uint32_t first, uint32_t n) {
+    uint32_t m = first;
+#pragma unroll 1
+    for (uint32_t q = 1; q < n; ++q) m = sh.p[first + q] > sh.p[m] ? first + q : m;
+    return par(m);
+  };
+  // exp(lr_k - max lr), exp(theta_kj - max theta_k) (probabilities do not depend
+  // on a common term), exp(-|rho|)
+  if (t < P) {
+    F2 x = sh.p[t] >= 0.f ? f2_neg(par(t)) : par(t);
+    if (t < P - 1) {
+      const uint32_t first = t < K ? 0u : K + (t - K) / J * J;
+      x = less(par(t), top(first, t < K ? K : J));
+    }
+    sh.e[t] = f2_exp(x);
+  }
+  __syncthreads();
+  auto part = [&](uint32_t k) { return f2_mul(sh.e[k], {sh.ew[k], 0.f}); };
+  auto total = [&]() {
+    F2 z = {0.f, 0.f};
+#pragma unroll 1
+    for (uint32_t q = 0; q < K; ++q) z = f2_add(z, part(q));
+    return z;
+  };
+  if (t < 2 * K + 1) {                   // log2 v_k, log2(1 - v_k), log2 Z
+    const uint32_t k = t / 2;
+    F2 x;
+    if (t == 2 * K) {
+      x = total();
+    } else {
+      const F2 e = sh.e[P - 1], sig = f2_div(sh.p[P - 1] >= 0.f ? one : e, f2_add(one, e));
+      const F2 v = f2_mul(sig, {sh.phi[k] * 0.5f, 0.f}), w = f2_add(one, f2_neg(v));
+      x = t & 1u ? w : v;
+      if (t & 1u) sh.odds[k] = f2_div(v, w);
+      else sh.v[k] = v.h;
+      if (t == 0) sh.sig = sig.h;
+    }
+    const F2 y = f2_log2(x);
+    (t == 2 * K ? sh.logz : t & 1u ? sh.l1[k] : sh.lv[k]) = y;
+  } else if (t >= 32 && t < 32 + K * J) {
+    const uint32_t x = t - 32;
+    F2 den = {0.f, 0.f};
+#pragma unroll 1
+    for (uint32_t j = 0; j < J; ++j) den = f2_add(den, sh.e[K + x / J * J + j]);
+    const F2 w = f2_div(sh.e[K + x], den);
+    sh.row[3 * K + x] = w.h;
+    sh.row[3 * K + K * J + x] = w.l;
+  } else if (t >= 96 && t < 96 + K) {
+    const uint32_t k = t - 96;
+    sh.prob[k] = f2_div(part(k), total());
+    const F2 x = less(par(k), top(0, K));
+    sh.c[k] = x.h > -1e30f ? f2_add(f2_mul(x, LOG2E), sh.logl[k]) : F2{x.h, 0.f};
+  }
+  __syncthreads();
   if (t < K) {
-    float Z = 0.f;
-#pragma unroll
-    for (uint32_t q = 0; q < K; ++q) Z += expf(sh.p[q]) * sh.ew[q];
-    sh.row[t] = sh.p[t] + logf(sh.ew[t]) - logf(Z);
-  } else if (t >= 32 && t < 32 + K) {
-    const uint32_t k = t - 32;
-    const float sig = 1.f / (1.f + expf(-sh.p[K + K * J]));
-    const float v = sig * sh.phi[k] * 0.5f;
-    sh.row[K + k] = logf(v);
-    sh.row[2 * K + k] = log1pf(-v);
-  } else if (t >= 64 && t < 64 + K) {
-    const uint32_t k = t - 64;
-    const float* th = sh.p + K + k * J;
-    float mx = th[0];
-#pragma unroll
-    for (uint32_t j = 1; j < J; ++j) mx = fmaxf(mx, th[j]);
-    float den = 0.f;
-#pragma unroll
-    for (uint32_t j = 0; j < J; ++j) den += expf(th[j] - mx);
-#pragma unroll
-    for (uint32_t j = 0; j < J; ++j) sh.row[3 * K + k * J + j] = expf(th[j] - mx) / den;
+    uint32_t best = 0;
+#pragma unroll 1
+    for (uint32_t q = 1; q < K; ++q)
+      if (sh.c[q].h > sh.c[best].h) best = q;
+    // the reference: a middle epoch, unless its share is negligible
+    const uint32_t ref = sh.c[(K - 1) / 2].h >= sh.c[best].h - 30.f ? (K - 1) / 2 : best;
+    const F2 l1r = sh.l1[ref], cr = sh.c[ref];
+    const F2 d = f2_add(sh.l1[t], f2_neg(l1r));
+    const F2 a = f2_add(f2_add(sh.lv[t], f2_neg(sh.lv[ref])), f2_neg(d));
+    const F2 c = sh.c[t].h > -1e30f ? f2_add(sh.c[t], f2_neg(cr)) : sh.c[t];
+    const float md = sh.stat[1].z, ma = md * sh.v[t];
+    sh.row[t] = t == ref ? 0.f : c.h + (c.l + __fmaf_rn(ma, a.l, md * d.l));
+    sh.row[K + t] = t == ref ? 0.f : a.h;
+    sh.row[2 * K + t] = t == ref ? 0.f : d.h;
+    if (t == 0) {
+      sh.lin[0] = f2_add(cr, f2_neg(sh.logz));
+      sh.lin[1] = sh.lv[ref];
+      sh.lin[2] = l1r;
+    }
   }
   __syncthreads();
 }
@@ -200,7 +285,7 @@ __device__ __forceinline__ float warp_transpose_sum(const float* v, uint32_t lan
 struct CalibEpilogue {
   float grp[CAL_THREADS / 32][1 + 3 * CAL_MAXK + CAL_MAXK * CAL_MAXJ][2];
   float2 tot[1 + 3 * CAL_MAXK + CAL_MAXK * CAL_MAXJ];
-  float grad[CAL_MAXK + CAL_MAXK * CAL_MAXJ + 1];
+  float grad[CAL_MAXK + CAL_MAXK * CAL_MAXJ + 1], nll;
 };
 template <uint32_t K, uint32_t J>
 __device__ __forceinline__ void calib_gradient(CalibEpilogue& sh, const CalibRow<K, J>& c, const CalibArgs& a,
@@ -232,27 +317,32 @@ __device__ __forceinline__ void calib_gradient(CalibEpilogue& sh, const CalibRow
   // remainders of their rounding, and products enter unrounded (fma)
   const float2* G = sh.tot + 1 + 2 * K;
   const float2* H = sh.tot + 1 + 3 * K;
-  // d/d lr_k = -G_k + N r_k L_k / Z   (N = sum_k G_k = number of sites)
+  const F2 n = {c.stat[0].x, c.stat[0].y};
+  // d/d lr_k = N pi_k - G_k
   if (threadIdx.x < K) {
     const uint32_t k = threadIdx.x;
-    float Z = 0.f;
-    Neu N;
-#pragma unroll
-    for (uint32_t q = 0; q < K; ++q) { Z += expf(c.p[q]) * c.ew[q]; N.add(G[q].x); N.c += G[q].y; }
-    const float2 n = N.both();
-    const float pk = expf(c.p[k]) * c.ew[k] / Z;
-    sh.grad[k] = __fmaf_rn(n.x, pk, -G[k].x) + (n.y * pk - G[k].y);
+    const F2 g = f2_add(f2_mul(n, c.prob[k]), {-G[k].x, -G[k].y});
+    sh.grad[k] = g.h + g.l;
   }
   if (threadIdx.x == 32) {
     // d/d rho = -(1 - sigma) sum_k (A_k - B_k v_k / (1 - v_k))
-    const float sig = 1.f / (1.f + expf(-c.p[K + K * J]));
-    float acc = 0.f;
-#pragma unroll
+    F2 acc = {0.f, 0.f};
+#pragma unroll 1
     for (uint32_t k = 0; k < K; ++k) {
-      const float v = sig * c.phi[k] * 0.5f, odds = v / (1.f - v);
-      acc += __fmaf_rn(-sh.tot[1 + K + k].x, odds, sh.tot[1 + k].x) + (sh.tot[1 + k].y - sh.tot[1 + K + k].y * odds);
+      const float2 A = sh.tot[1 + k], B = sh.tot[1 + K + k];
+      acc = f2_add(acc, f2_add({A.x, A.y}, f2_neg(f2_mul({B.x, B.y}, c.odds[k]))));
     }
-    sh.grad[K + K * J] = -(1.f - sig) * acc;
+    sh.grad[K + K * J] = -(1.f - c.sig) * (acc.h + acc.l);
+  }
+  if (threadIdx.x == 33) {
+    // the reference epoch's log-likelihood of all sites: N log pi + sum a log v + sum (d - a) log(1 - v)
+    F2 l = {0.f, 0.f};
+    const float2* sums = reinterpret_cast<const float2*>(c.stat);
+#pragma unroll 1
+    for (uint32_t i = 0; i < 3 && n.h > 0.f; ++i) l = f2_add(l, f2_mul({sums[i].x, sums[i].y}, c.lin[i]));
+    l = f2_mul(l, {0.693147182464599609f, -1.90465432e-09f});
+    const F2 x = f2_add({sh.tot[0].x, sh.tot[0].y}, f2_neg(l));
+    sh.nll = x.h + x.l;
   }
   // d/d theta_kj = -w_kj (sum_i gamma_ik S_j(c_i) / M_k(c_i) - G_k) = -w_kj (H_kj - G_k)
   if (threadIdx.x >= 64 && threadIdx.x < 64 + K * J) {
@@ -268,11 +358,12 @@ __device__ __forceinline__ AdamBias adam_bias(const AdamArgs& adam, uint32_t ste
   const float t = float(step + 1);
   return {1.f - powf(adam.beta1, t), 1.f - powf(adam.beta2, t)};
 }
-__device__ __forceinline__ float adam_update(const AdamArgs& adam, AdamBias b, float p, float g, float& m, float& v) {
+// (the change of the parameter, to be subtracted)
+__device__ __forceinline__ float adam_update(const AdamArgs& adam, AdamBias b, float g, float& m, float& v) {
   m = adam.beta1 * m + (1.f - adam.beta1) * g;
   v = adam.beta2 * v + (1.f - adam.beta2) * g * g;
   const float mh = m / b.m, vh = v / b.v;
-  return p - adam.lr * mh / (sqrtf(vh) + adam.eps);
+  return adam.lr * mh / (sqrtf(vh) + adam.eps);
 }
 
 // one evaluation's results (and Adam step), by one CTA per replicate
@@ -282,33 +373,35 @@ __device__ __forceinline__ void calib_epilogue(CalibEpilogue& sh, const CalibRow
                                                float* __restrict__ grad_out, const AdamArgs& adam) {
   constexpr uint32_t P = K + K * J + 1;
   calib_gradient<K, J>(sh, c, a, r, a.partial);
-  if (threadIdx.x == 0 && nll_out) nll_out[r] = sh.tot[0].x;
+  if (threadIdx.x == 0 && nll_out) nll_out[r] = sh.nll;
   for (uint32_t q = threadIdx.x; q < P; q += CAL_THREADS) {
     const uint64_t o = uint64_t(r) * P + q;
     const float gq = sh.grad[q];
     if (grad_out) grad_out[o] = gq;
     if (adam.m) {
       float m = __ldcg(adam.m + o), v = __ldcg(adam.v + o);
-      params[o] = adam_update(adam, adam_bias(adam, adam.t), c.p[q], gq, m, v);
+      params[o] = c.p[q] - adam_update(adam, adam_bias(adam, adam.t), gq, m, v);
       adam.m[o] = m; adam.v[o] = v;
     }
   }
 }
 
 // STEPS: a.steps Adam steps in a cooperative launch (an instance of its own: in
-// the other the step's state would spill).  Every CTA of a replicate keeps the
+// the other the step's state would spill; with 64 registers it spills even so,
+// 4.6 ms against 3.3 with one CTA per SM less).  Every CTA of a replicate keeps the
 // parameters and moments and makes each step itself, from all the segments'
 // sums in the same order, so a step has one wait (the sums) where parameters
-// published by one CTA need a second: 200 steps over 64 x 5e4 sites 3.53 ->
-// 3.12 ms.  The sums alternate between two halves of a.partial: a CTA is at
+// published by one CTA need a second: 0.4 ms of 200 steps over 64 x 5e4 sites.
+// The sums alternate between two halves of a.partial: a CTA is at
 // most one step ahead of the others.
 template <uint32_t K, uint32_t J, bool STEPS>
-__global__ void __launch_bounds__(CAL_THREADS, calib_min_blocks(K, J)) k_calib(CalibArgs a, float* __restrict__ params,
+__global__ void __launch_bounds__(CAL_THREADS, calib_min_blocks(K, J) - (STEPS && calib_min_blocks(K, J) > 3 ? 1 : 0)) k_calib(CalibArgs a, float* __restrict__ params,
                                                                                float* __restrict__ nll_out,
                                                                                float* __restrict__ grad_out,
                                                                                AdamArgs adam) {
   constexpr uint32_t JP = J > 4 ? 8 : 4;
   constexpr uint32_t NV = 1 + 3 * K + K * J;   // nll, A, B, G, H
+  constexpr uint32_t TAB = 3 * K + 2 * K * J;
   // signature rows, eight copies of each 16 bytes: a lane reads the copy in its
   // own banks, so the gather is free of conflicts (one copy: 2.9 lanes a bank)
   // The mixtures M_k(c) likewise, by class.
@@ -332,7 +425,7 @@ __global__ void __launch_bounds__(CAL_THREADS, calib_min_blocks(K, J)) k_calib(C
     if (threadIdx.x == 128) s_bias = adam_bias(adam, step);
     calib_rows<K, J>(s_c);
   } else if (a.tab) {
-    for (uint32_t x = threadIdx.x; x < 3 * K + K * J; x += CAL_THREADS) s_c.row[x] = a.tab[uint64_t(r) * a.part_stride + x];
+    for (uint32_t x = threadIdx.x; x < TAB; x += CAL_THREADS) s_c.row[x] = a.tab[uint64_t(r) * TAB + x];
     __syncthreads();
   } else {
     calib_tables<K, J>(s_c, a, params, r);
@@ -355,9 +448,10 @@ __global__ void __launch_bounds__(CAL_THREADS, calib_min_blocks(K, J)) k_calib(C
     for (uint32_t k = 0; k < KP; ++k) {
       m[k] = 0.f;
       if (k < K) {
-        m[k] = s_row[3 * K + k * J] * sg[0];
 #pragma unroll
-        for (uint32_t j = 1; j < J; ++j) m[k] = __fmaf_rn(s_row[3 * K + k * J + j], sg[j], m[k]);
+        for (uint32_t j = 0; j < J; ++j) m[k] = __fmaf_rn(s_row[3 * K + K * J + k * J + j], sg[j], m[k]);
+#pragma unroll
+        for (uint32_t j = 0; j < J; ++j) m[k] = __fmaf_rn(s_row[3 * K + k * J + j], sg[j], m[k]);
       }
     }
 #pragma unroll
@@ -369,14 +463,14 @@ __global__ void __launch_bounds__(CAL_THREADS, calib_min_blocks(K, J)) k_calib(C
   constexpr uint32_t KH = (K + 1) / 2;
   float2 cst[KH], dlv[KH], l1v[KH];
   auto at = [&](uint32_t k, uint32_t off, float pad) { return k < K ? s_row[off + k] : pad; };
-  // the log-domain terms in base 2 (ex2 / lg2 directly, the NLL scaled back by ln 2)
-  constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
+  // the log-domain terms are in base 2 (ex2 / lg2 directly, the NLL scaled back by ln 2)
+  constexpr float LN2 = 0.6931471805599453f;
 #pragma unroll
   for (uint32_t h = 0; h < KH; ++h) {
-    cst[h] = make_float2(LOG2E * at(2 * h, 0, 0.f), at(2 * h + 1, 0, -INFINITY) * LOG2E);
-    // u_k = cst_k + a log v_k + (d - a) log(1 - v_k) = cst_k + a dlv_k + d l1v_k
-    l1v[h] = make_float2(LOG2E * at(2 * h, 2 * K, 0.f), LOG2E * at(2 * h + 1, 2 * K, 0.f));
-    dlv[h] = make_float2(LOG2E * at(2 * h, K, 0.f) - l1v[h].x, LOG2E * at(2 * h + 1, K, 0.f) - l1v[h].y);
+    cst[h] = make_float2(at(2 * h, 0, 0.f), at(2 * h + 1, 0, -INFINITY));
+    // u_k = cst_k + a dlv_k + d l1v_k
+    l1v[h] = make_float2(at(2 * h, 2 * K, 0.f), at(2 * h + 1, 2 * K, 0.f));
+    dlv[h] = make_float2(at(2 * h, K, 0.f), at(2 * h + 1, K, 0.f));
   }
   float nll = 0.f;
   float2 A[KH], D[KH], G[KH], H[J][KH];   // D_k = sum gamma_ik d_i (B_k = D_k - A_k)
@@ -524,13 +618,14 @@ __global__ void __launch_bounds__(CAL_THREADS, calib_min_blocks(K, J)) k_calib(C
     calib_gradient<K, J>(s_u.epi, s_c, a, r, sums);
     const bool end = step + 1 == a.steps;
     if (threadIdx.x < P) {
-      const float p = adam_update(adam, s_bias, s_c.p[threadIdx.x], s_u.epi.grad[threadIdx.x], s_adam[0][threadIdx.x],
-                                  s_adam[1][threadIdx.x]);
-      s_c.p[threadIdx.x] = p;
-      if (end && first) params[uint64_t(r) * P + threadIdx.x] = p;
+      const float u = adam_update(adam, s_bias, s_u.epi.grad[threadIdx.x], s_adam[0][threadIdx.x], s_adam[1][threadIdx.x]);
+      const F2 p = f2_add({s_c.p[threadIdx.x], s_c.pl[threadIdx.x]}, {-u, 0.f});
+      s_c.p[threadIdx.x] = p.h;
+      s_c.pl[threadIdx.x] = p.l;
+      if (end && first) params[uint64_t(r) * P + threadIdx.x] = p.h;
     }
     if (end) {
-      if (first && threadIdx.x == 0 && nll_out) nll_out[r] = s_u.epi.tot[0].x;
+      if (first && threadIdx.x == 0 && nll_out) nll_out[r] = s_u.epi.nll;
       return;
     }
     __syncthreads();
@@ -545,7 +640,8 @@ __global__ void __launch_bounds__(CAL_THREADS) k_calib_tables(CalibArgs a, const
   __shared__ CalibRow<K, J> s_c;
   const uint32_t r = a.rep0 + blockIdx.x;
   calib_tables<K, J>(s_c, a, params, r);
-  for (uint32_t x = threadIdx.x; x < 3 * K + K * J; x += CAL_THREADS) a.tab[uint64_t(r) * a.part_stride + x] = s_c.row[x];
+  constexpr uint32_t TAB = 3 * K + 2 * K * J;
+  for (uint32_t x = threadIdx.x; x < TAB; x += CAL_THREADS) a.tab[uint64_t(r) * TAB + x] = s_c.row[x];
 }
 template <uint32_t K, uint32_t J>
 __global__ void __launch_bounds__(CAL_THREADS) k_calib_epilogue(CalibArgs a, float* __restrict__ params,

@@ -11,47 +11,12 @@
 // sampler takes the same decisions from the same Philox words, so the result
 // is its result.  Inside a margin (under one draw in ten thousand) the
 // functions return false and the caller draws with the FP64 sampler.
-//
-// Double-float arithmetic: T. J. Dekker, "A floating-point technique for
-// extending the available precision", Numer. Math. 18, 1971; D. E. Knuth,
-// TAOCP vol. 2, 4.2.2 (the error of a sum).
 #pragma once
+#include "pg_f2.cuh"
 #include "pg_rng.cuh"
 
 namespace pg {
 
-struct F2 { float h, l; };   // h + l, |l| at most half an ulp of h
-
-__device__ __forceinline__ F2 f2_quick(float a, float b) {   // |a| >= |b|
-  const float s = __fadd_rn(a, b);
-  return {s, __fsub_rn(b, __fsub_rn(s, a))};
-}
-__device__ __forceinline__ F2 f2_sum(float a, float b) {
-  const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
-  return {s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb))};
-}
-__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
-  const F2 s = f2_sum(a.h, b.h), t = f2_sum(a.l, b.l);
-  const F2 u = f2_quick(s.h, __fadd_rn(s.l, t.h));
-  return f2_quick(u.h, __fadd_rn(u.l, t.l));
-}
-__device__ __forceinline__ F2 f2_neg(F2 a) { return {-a.h, -a.l}; }
-__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
-  const float p = __fmul_rn(a.h, b.h);
-  float e = __fmaf_rn(a.h, b.h, -p);
-  e = __fmaf_rn(a.h, b.l, e);
-  e = __fmaf_rn(a.l, b.h, e);
-  return f2_quick(p, e);
-}
-__device__ __forceinline__ F2 f2_scale(F2 a, float p2) { return {__fmul_rn(a.h, p2), __fmul_rn(a.l, p2)}; }  // p2 a power of two
-__device__ __forceinline__ F2 f2_div(F2 a, F2 b) {
-  const float q = __fdividef(a.h, b.h);
-  // a - q b, then one more quotient digit
-  const float p = __fmul_rn(q, b.h), pe = __fmaf_rn(q, b.h, -p);
-  const F2 r = f2_add(a, {-p, -__fmaf_rn(q, b.l, pe)});
-  const float q2 = __fdividef(r.h, b.h);
-  return f2_quick(q, q2);
-}
 __device__ __forceinline__ F2 f2_sqrt(F2 a) {   // a.h > 0
   const float s = __fsqrt_rn(a.h);
   const float e = __fadd_rn(__fmaf_rn(-s, s, a.h), a.l);
@@ -72,7 +37,6 @@ __device__ __forceinline__ F2 f2_mantissa(double x, int& e) {
   const uint64_t m = (bits & 0x000fffffffffffffull) | 0x0010000000000000ull;
   return f2_quick(float(uint32_t(m >> 29)) * 0x1p-23f, float(uint32_t(m) & 0x1fffffffu) * 0x1p-52f);
 }
-__device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }   // -126 <= e <= 127
 
 // floor of x (|x| < 2^33) and the distance of x to the nearest integer
 __device__ __forceinline__ int64_t f2_floor(F2 x, float& dist) {

@@ -431,7 +431,10 @@ struct CalibArgs {
   const int32_t* depth;
   const int32_t* cls;
   const float* epoch_w;         // n_rep x K  (L_k: relative length of epoch k)
+  const float2* epoch_log;      // n_rep x K: log2 L_k in two floats
   const float* phi;             // n_rep x K  (mean cellular fraction of epoch-k mutations)
+  const float4* rep_stat;       // per replicate two: {sites, sum of alt}, {sum of depth - alt, mean depth, 0}, sums as
+                                //   two floats each
   const float* sig_rows;        // C x JP: S_j(c) by class, JP = 4 (J <= 4) or 8 floats, zero beyond J
   // segments: sites [seg_start, + seg_len) of replicate seg_rep, in order (a
   // replicate without sites has one empty segment)
@@ -446,7 +449,7 @@ struct CalibArgs {
   uint32_t seg0, rep0;            // first segment and replicate of the launch
   uint32_t steps;                 // evaluations of the launch (above 1: Adam steps, without tab)
   uint32_t* status;               // set when a wait between the steps ran out
-  float* tab;                     // per replicate, part_stride floats: its constants, where they and the
+  float* tab;                     // per replicate, 3K + 2K J floats: its constants, where they and the
                                   //   epilogues have launches of their own; else NULL
 };
 struct AdamArgs {               // m == nullptr: no optimizer step
