@@ -332,7 +332,7 @@ def calibration_bench(world: int, n_rep: int = 512, n_sites: int = 100_000, step
             "per_instance": "pg_calib_nll_grad_one per replicate, stream-ordered, one synchronisation at the end",
             "adam_200_steps_ms": t_adam * 1000.0,
             "cpu_fp64_grad_evals_per_s_1core": 1.0 / t_cpu,
-            "roofline": {"kernel": "k_calib_sites+k_calib_epilogue", "bound": "hbm",
+            "roofline": {"kernel": "k_calib", "bound": "hbm",
                          "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "per_unit": "12 B/site (alt, depth, class)"}}
 
