@@ -2176,23 +2176,18 @@ pg_status pg_seq_result_tile_size(const pg_seq_result* r, uint32_t* tile_size) {
 }  // extern "C"
 
 // ====================================================================== calibration
-// Sites of a segment at most: longer per-thread FP32 sums lose precision (65536
-// doubled the gradient error of a table of 2e5 sites), and at least: one
-// 16-byte load of each column per thread.
-constexpr uint32_t CALIB_SEG = 16384, CALIB_MIN_SEG = 1024;
-
 struct pg_calib {
   int device = 0;
   cudaStream_t st = nullptr, own_st = nullptr;
   Pool pool;
   uint32_t n_rep = 0, K = 0, J = 0, C = 0, P = 0, n_segs = 0;
   DBuf<int32_t> alt, depth, cls;
-  DBuf<uint64_t> seg_start;
-  DBuf<uint32_t> seg_rep, seg_len, rep_first_seg, rep_done, status;
-  DBuf<float> sig_rows, epoch_w, phi, tab, m, v;
-  DBuf<float2> partial, epoch_log;
-  DBuf<float4> rep_stat;
+  DBuf<uint64_t> site_off;
+  DBuf<uint32_t> seg_rep, rep_first_seg, rep_first_chunk, rep_done, status;
+  DBuf<float> sig_rows, epoch_w, phi, tab, m, v, partial;
   bool split = false;                // more segments than the GPU holds at a time
+  bool by_warps = false;             // chunks dealt out by warps
+  uint32_t n_rows = 0;
   std::vector<uint32_t> rep_first_seg_h;
   uint32_t part_stride = 0;
   cudaGraphExec_t graph = nullptr;
@@ -2200,19 +2195,19 @@ struct pg_calib {
   pg::CalibArgs args() const {
     pg::CalibArgs a{};
     a.K = K; a.J = J; a.C = C; a.P = P;
-    a.alt = alt.p; a.depth = depth.p; a.cls = cls.p;
-    a.epoch_w = epoch_w.p; a.phi = phi.p; a.sig_rows = sig_rows.p; a.rep_stat = rep_stat.p; a.epoch_log = epoch_log.p;
-    a.seg_rep = seg_rep.p; a.seg_start = seg_start.p; a.seg_len = seg_len.p;
-    a.rep_first_seg = rep_first_seg.p; a.rep_done = rep_done.p;
-    a.partial = partial.p; a.part_stride = part_stride; a.tab = split ? tab.p : nullptr;
+    a.alt = alt.p; a.depth = depth.p; a.cls = cls.p; a.site_off = site_off.p;
+    a.epoch_w = epoch_w.p; a.phi = phi.p; a.sig_rows = sig_rows.p;
+    a.rep_first_chunk = rep_first_chunk.p; a.rep_first_seg = rep_first_seg.p; a.seg_rep = seg_rep.p;
+    a.by_warps = by_warps ? 1u : 0u; a.rep_done = rep_done.p;
+    a.partial = partial.p; a.part_stride = part_stride; a.n_rows = n_rows; a.tab = split ? tab.p : nullptr;
     a.steps = 1;
     return a;
   }
   ~pg_calib() {
     if (graph) cudaGraphExecDestroy(graph);
-    alt.reset(); depth.reset(); cls.reset(); seg_start.reset(); seg_rep.reset(); seg_len.reset();
-    rep_first_seg.reset(); rep_done.reset(); status.reset(); sig_rows.reset(); epoch_w.reset();
-    phi.reset(); partial.reset(); rep_stat.reset(); epoch_log.reset(); tab.reset(); m.reset(); v.reset();
+    alt.reset(); depth.reset(); cls.reset(); site_off.reset(); seg_rep.reset(); rep_first_seg.reset();
+    rep_first_chunk.reset(); rep_done.reset(); status.reset(); sig_rows.reset(); epoch_w.reset();
+    phi.reset(); partial.reset(); tab.reset(); m.reset(); v.reset();
     pool.release_all();
     if (own_st) cudaStreamDestroy(own_st);
   }
@@ -2233,22 +2228,9 @@ pg_status pg_calib_create(uint32_t n_rep, const uint64_t* site_off, const int32_
     require(site_off[0] == 0, "site offsets start at 0");
     for (uint32_t r = 0; r < n_rep; ++r) require(site_off[r + 1] >= site_off[r], "site offsets must not decrease");
     require(n == 0 || (alt && depth && cls), "NULL site arrays");
-    // the replicates' sites and sums, exact in two floats up to 2^48
-    std::vector<float4> stat(2 * size_t(n_rep));
-    for (uint32_t r = 0; r < n_rep; ++r) {
-      uint64_t sa = 0, sd = 0;
-      const uint64_t nr = site_off[r + 1] - site_off[r];
-      for (uint64_t i = site_off[r]; i < site_off[r + 1]; ++i) {
-        require(depth[i] >= 0 && alt[i] >= 0 && alt[i] <= depth[i], "sites need 0 <= alt <= depth");
-        require(cls[i] >= 0 && uint32_t(cls[i]) < C, "site class out of range");
-        sa += uint32_t(alt[i]);
-        sd += uint32_t(depth[i]);
-      }
-      auto two = [](uint64_t x, float& h, float& l) { h = float(double(x)); l = float(double(x) - double(h)); };
-      float4 &s0 = stat[2 * size_t(r)], &s1 = stat[2 * size_t(r) + 1];
-      two(nr, s0.x, s0.y); two(sa, s0.z, s0.w); two(sd - sa, s1.x, s1.y);
-      s1.z = nr ? float(double(sd) / double(nr)) : 0.f;
-      s1.w = 0.f;
+    for (uint64_t i = 0; i < n; ++i) {
+      require(depth[i] >= 0 && alt[i] >= 0 && alt[i] <= depth[i], "sites need 0 <= alt <= depth");
+      require(cls[i] >= 0 && uint32_t(cls[i]) < C, "site class out of range");
     }
     for (uint64_t x = 0; x < uint64_t(J) * C; ++x) require(signatures[x] >= 0, "signature probabilities >= 0");
     for (uint64_t x = 0; x < uint64_t(n_rep) * K; ++x) {
@@ -2264,6 +2246,7 @@ pg_status pg_calib_create(uint32_t n_rep, const uint64_t* site_off, const int32_
     cudaStream_t st = c->st;
     std::vector<int32_t> va(alt, alt + n), vd(depth, depth + n), vc(cls, cls + n);
     c->alt = upload(P, va, st); c->depth = upload(P, vd, st); c->cls = upload(P, vc, st);
+    c->site_off = upload(P, std::vector<uint64_t>(site_off, site_off + n_rep + 1), st);
     std::vector<float> fs(uint64_t(J) * C), fw(uint64_t(n_rep) * K), fp(uint64_t(n_rep) * K);
     for (uint32_t j = 0; j < J; ++j) {   // signatures normalised to sum 1 over the classes
       double tot = 0;
@@ -2273,13 +2256,6 @@ pg_status pg_calib_create(uint32_t n_rep, const uint64_t* site_off, const int32_
     }
     for (uint64_t x = 0; x < fw.size(); ++x) { fw[x] = float(epoch_weight[x]); fp[x] = float(phi[x]); }
     c->epoch_w = upload(P, fw, st); c->phi = upload(P, fp, st);
-    std::vector<float2> logl(fw.size());
-    for (size_t x = 0; x < fw.size(); ++x) {
-      const double y = std::log2(double(fw[x]));
-      logl[x].x = float(y);
-      logl[x].y = float(y - double(logl[x].x));
-    }
-    c->epoch_log = upload(P, logl, st);
     {   // signatures by class, rows of 4 or 8 floats
       const uint32_t JP = J > 4 ? 8 : 4;
       std::vector<float> rows(size_t(C) * JP, 0.f);
@@ -2287,47 +2263,50 @@ pg_status pg_calib_create(uint32_t n_rep, const uint64_t* site_off, const int32_
         for (uint32_t cl = 0; cl < C; ++cl) rows[size_t(cl) * JP + j] = fs[size_t(j) * C + cl];
       c->sig_rows = upload(P, rows, st);
     }
-    c->rep_stat = upload(P, stat, st);
-    // segments: the smallest size that needs no more rounds of resident CTAs
-    // than CALIB_SEG does (one round where possible; a last round of a few
-    // CTAs would take as long as a full one), equal within a replicate
+    // A CTA takes up to `take` of the warps of its replicate's chunks, the
+    // fewest with which all CTAs are resident together; from 129 chunks on, a
+    // chunk (all the CTAs of a replicate read its sums at each Adam step).
+    const uint64_t chunk = pg::calib_chunk(), warps = 8;
+    std::vector<uint32_t> first_chunk(n_rep + 1, 0);
+    uint32_t most = 0;
+    for (uint32_t r = 0; r < n_rep; ++r) {
+      const uint64_t k = (site_off[r + 1] - site_off[r] + chunk - 1) / chunk;
+      require(first_chunk[r] + k < (uint64_t(1) << 28), "too many sites");
+      first_chunk[r + 1] = first_chunk[r] + uint32_t(k);
+      most = std::max(most, uint32_t(k));
+    }
     int sms = 0;
     ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device), "device attribute");
     const uint64_t resident = uint64_t(std::max(1, sms)) * uint64_t(pg::calib_ctas_per_sm(K, J));
-    auto segs_at = [&](uint64_t size) {
+    auto segs = [&](uint32_t r, uint64_t take) {
+      return std::max<uint64_t>(1, (uint64_t(first_chunk[r + 1] - first_chunk[r]) * warps + take - 1) / take);
+    };
+    auto total = [&](uint64_t take) {
       uint64_t k = 0;
-      for (uint32_t r = 0; r < n_rep; ++r) k += std::max<uint64_t>(1, (site_off[r + 1] - site_off[r] + size - 1) / size);
+      for (uint32_t r = 0; r < n_rep; ++r) k += segs(r, take);
       return k;
     };
-    const uint64_t room = (segs_at(CALIB_SEG) + resident - 1) / resident * resident;
-    uint64_t size = CALIB_MIN_SEG;
-    for (uint64_t hi = CALIB_SEG; size < hi;) {
-      const uint64_t mid = (size + hi) / 2;
-      if (segs_at(mid) <= room) hi = mid; else size = mid + 1;
-    }
-    std::vector<uint32_t> srep, slen;
-    std::vector<uint64_t> sstart;
+    uint64_t take = warps;
+    c->by_warps = most <= 128 && total(warps) <= resident;
+    while (c->by_warps && take > 1 && total(take - 1) <= resident) --take;
+    std::vector<uint32_t> srep;
     c->rep_first_seg_h.assign(n_rep + 1, 0);
     for (uint32_t r = 0; r < n_rep; ++r) {
       c->rep_first_seg_h[r] = uint32_t(srep.size());
-      const uint64_t nr = site_off[r + 1] - site_off[r], k = std::max<uint64_t>(1, (nr + size - 1) / size);
-      // cut at multiples of four sites (the 16-byte loads)
-      auto cut = [&](uint64_t q) { return q == k ? site_off[r + 1] : q == 0 ? site_off[r] : (site_off[r] + nr * q / k) & ~uint64_t(3); };
-      for (uint64_t q = 0; q < k; ++q) {
-        const uint64_t at = std::max(cut(q), site_off[r]);
-        srep.push_back(r); sstart.push_back(at); slen.push_back(uint32_t(std::max(cut(q + 1), at) - at));
-      }
+      srep.insert(srep.end(), segs(r, take), r);
     }
     c->rep_first_seg_h[n_rep] = uint32_t(srep.size());
     c->n_segs = uint32_t(srep.size());
     c->split = c->n_segs > resident;
-    c->seg_rep = upload(P, srep, st); c->seg_start = upload(P, sstart, st); c->seg_len = upload(P, slen, st);
+    c->n_rows = std::max<uint32_t>(first_chunk[n_rep], 1) * (c->by_warps ? uint32_t(warps) : 1u);
+    c->seg_rep = upload(P, srep, st);
     c->rep_first_seg = upload(P, c->rep_first_seg_h, st);
+    c->rep_first_chunk = upload(P, first_chunk, st);
     c->rep_done = DBuf<uint32_t>(P, n_rep);
     ck(cudaMemsetAsync(c->rep_done.p, 0, sizeof(uint32_t) * n_rep, st), "memset");
     c->part_stride = (1 + 3 * K + K * J + 3) & ~3u;
-    c->partial = DBuf<float2>(P, (c->split ? 1 : 2) * uint64_t(srep.size()) * c->part_stride);
-    if (c->split) c->tab = DBuf<float>(P, uint64_t(n_rep) * (3 * K + 2 * K * J));
+    c->partial = DBuf<float>(P, (c->split ? 1 : 2) * uint64_t(c->n_rows) * c->part_stride);
+    if (c->split) c->tab = DBuf<float>(P, uint64_t(n_rep) * pg::calib_tab(K, J));
     c->m = DBuf<float>(P, uint64_t(n_rep) * c->P);
     c->v = DBuf<float>(P, uint64_t(n_rep) * c->P);
     c->status = DBuf<uint32_t>(P, 1);

@@ -20,6 +20,9 @@ int calib_ctas_lo(uint32_t K, uint32_t J) {
 
 int calib_ctas_per_sm(uint32_t K, uint32_t J) { return K <= 4 ? calib_ctas_lo(K, J) : calib_ctas_hi(K, J); }
 
+uint32_t calib_chunk() { return CAL_CHUNK; }
+uint32_t calib_tab(uint32_t K, uint32_t J) { return calib_row_floats(K, J); }
+
 void calib_launch(const CalibArgs& a, uint32_t n_segs, uint32_t n_rep, float* params, float* nll, float* grad,
                   const AdamArgs& adam, cudaStream_t st) {
   if (n_segs == 0) return;

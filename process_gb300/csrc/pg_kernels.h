@@ -430,26 +430,25 @@ struct CalibArgs {
   const int32_t* alt;           // sites of all replicates, concatenated (16-byte aligned columns)
   const int32_t* depth;
   const int32_t* cls;
+  const uint64_t* site_off;     // n_rep + 1
   const float* epoch_w;         // n_rep x K  (L_k: relative length of epoch k)
-  const float2* epoch_log;      // n_rep x K: log2 L_k in two floats
   const float* phi;             // n_rep x K  (mean cellular fraction of epoch-k mutations)
-  const float4* rep_stat;       // per replicate two: {sites, sum of alt}, {sum of depth - alt, mean depth, 0}, sums as
-                                //   two floats each
   const float* sig_rows;        // C x JP: S_j(c) by class, JP = 4 (J <= 4) or 8 floats, zero beyond J
-  // segments: sites [seg_start, + seg_len) of replicate seg_rep, in order (a
-  // replicate without sites has one empty segment)
+  // A replicate's chunks of CAL_CHUNK sites (chunk c: those from
+  // site_off + c CAL_CHUNK on) and segments, the CTAs it is dealt out to: a
+  // chunk each, or with by_warps the chunks' warps in turn (a replicate without
+  // sites has one segment)
+  const uint32_t* rep_first_chunk;  // n_rep + 1
+  const uint32_t* rep_first_seg;    // n_rep + 1
   const uint32_t* seg_rep;
-  const uint64_t* seg_start;
-  const uint32_t* seg_len;
-  const uint32_t* rep_first_seg;  // n_rep + 1
+  uint32_t by_warps;
   uint32_t* rep_done;             // n_rep counts, zero before a launch (and after one of one evaluation)
-  float2* partial;                // per segment, part_stride sums (>= 1 + 3K + K J) and their remainders; with
-                                  //   steps > 1 twice that
-  uint32_t part_stride;
+  float* partial;                 // per chunk, or per warp of a chunk, part_stride sums (>= 1 + 3K + K J): n_rows rows,
+  uint32_t part_stride, n_rows;   //   with steps > 1 twice that
   uint32_t seg0, rep0;            // first segment and replicate of the launch
   uint32_t steps;                 // evaluations of the launch (above 1: Adam steps, without tab)
   uint32_t* status;               // set when a wait between the steps ran out
-  float* tab;                     // per replicate, 3K + 2K J floats: its constants, where they and the
+  float* tab;                     // per replicate, calib_tab floats: its constants, where they and the
                                   //   epilogues have launches of their own; else NULL
 };
 struct AdamArgs {               // m == nullptr: no optimizer step
@@ -461,5 +460,7 @@ struct AdamArgs {               // m == nullptr: no optimizer step
 void calib_launch(const CalibArgs& a, uint32_t n_segs, uint32_t n_rep, float* params, float* nll, float* grad,
                   const AdamArgs& adam, cudaStream_t st);
 int calib_ctas_per_sm(uint32_t K, uint32_t J);   // resident CTAs of the evaluation kernel
+uint32_t calib_chunk();                          // sites of a chunk
+uint32_t calib_tab(uint32_t K, uint32_t J);      // floats of a replicate in CalibArgs::tab
 
 }  // namespace pg
