@@ -2372,6 +2372,7 @@ pg_status pg_calib_adam(pg_calib* c, float* params, uint32_t steps, float lr, fl
       a.steps = steps;
       a.status = c->status.p;
       ck(cudaMemsetAsync(c->status.p, 0, sizeof(uint32_t), st), "memset");
+      ck(cudaMemsetAsync(c->rep_done.p, 0xff, sizeof(uint32_t) * c->n_rep, st), "memset");
       pg::calib_launch(a, c->n_segs, c->n_rep, params, nll, nullptr, pg::AdamArgs{c->m.p, c->v.p, 0, lr, beta1, beta2, eps}, st);
       ck(cudaMemsetAsync(c->rep_done.p, 0, sizeof(uint32_t) * c->n_rep, st), "memset");
       ck(cudaGetLastError(), "calibration steps");

@@ -49,6 +49,7 @@
 #include <cstdint>
 
 #include "pg_kernels.h"
+#include "pg_wait.h"
 
 namespace pg {
 
@@ -56,6 +57,9 @@ constexpr int CAL_THREADS = 256;
 constexpr int CAL_WARPS = CAL_THREADS / 32;
 constexpr uint32_t CAL_MAXK = 8, CAL_MAXJ = 8, CAL_MAXC = 128;
 constexpr uint32_t CAL_CHUNK = 16384;   // sites (per-thread FP32 sums of 256 in site order)
+// the arrivals' count before the first step: it wraps at once, not only after
+// 2^32 arrivals
+constexpr uint32_t CAL_COUNT0 = 0xffffffffu;
 constexpr uint32_t CAL_SPIN_LIMIT = 1u << 22;   // polls of a wait, 64 ns or more each
 
 struct Neu {   // Neumaier-compensated FP32 sum
@@ -549,7 +553,7 @@ __global__ void __launch_bounds__(CAL_THREADS, calib_ctas(K, J, STEPS)) k_calib(
     if (threadIdx.x == 0) {
       uint32_t go = 1, polls = 0;
       atomicAdd(a.rep_done + r, 1u);
-      while (*reinterpret_cast<volatile uint32_t*>(a.rep_done + r) < (step + 1) * n_parts) {
+      while (!arrived(*reinterpret_cast<volatile uint32_t*>(a.rep_done + r), CAL_COUNT0 + (step + 1) * n_parts)) {
         if (++polls > CAL_SPIN_LIMIT || *reinterpret_cast<volatile uint32_t*>(a.status)) { go = 0; break; }
         __nanosleep(20);
       }

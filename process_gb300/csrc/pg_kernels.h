@@ -442,7 +442,8 @@ struct CalibArgs {
   const uint32_t* rep_first_seg;    // n_rep + 1
   const uint32_t* seg_rep;
   uint32_t by_warps;
-  uint32_t* rep_done;             // n_rep counts, zero before a launch (and after one of one evaluation)
+  uint32_t* rep_done;             // n_rep counts, zero before a launch of one evaluation (and after it), all ones
+                                  //   before one of several
   float* partial;                 // per chunk, or per warp of a chunk, part_stride sums (>= 1 + 3K + K J): n_rows rows,
   uint32_t part_stride, n_rows;   //   with steps > 1 twice that
   uint32_t seg0, rep0;            // first segment and replicate of the launch
