@@ -465,9 +465,19 @@ pg_status pg_calib_nll_grad_one(pg_calib* cal, uint32_t rep, const float* params
  * place), run entirely on the device (in one launch where the
  * segments fit the GPU at a time, else as a CUDA graph); nll (device, n_rep,
  * may be NULL) receives the NLL of the last step's parameters before the
- * update.  The optimizer state restarts at zero on each call. */
+ * update.  The optimizer state restarts at zero on each call.  Asynchronous
+ * on the handle's stream.  In the one-launch form the thread blocks of a
+ * replicate wait for one another at each step, for about two seconds at most;
+ * should a wait run out, the replicate's parameters and NLL become NaN and
+ * pg_calib_status reports it. */
 pg_status pg_calib_adam(pg_calib* cal, float* params, uint32_t steps, float lr, float beta1, float beta2, float eps,
                         float* nll);
+/* Synchronises the handle's stream; PG_ERR_RUNTIME when a wait of
+ * pg_calib_adam has run out since the last query. */
+pg_status pg_calib_status(pg_calib* cal);
+/* Looks after which later calls give up a wait (UINT32_MAX: the default; 0: at
+ * once, to test the failure). */
+pg_status pg_calib_set_wait_polls(pg_calib* cal, uint32_t polls);
 
 /* ------------------------------------------------------------------ batches
  * Many independent instances on one engine's genome and signatures (no

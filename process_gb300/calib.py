@@ -34,6 +34,8 @@ def _bind():
         "pg_calib_nll_grad": (C.c_int, [P, P, P, P]),
         "pg_calib_nll_grad_one": (C.c_int, [P, C.c_uint32, P, P, P]),
         "pg_calib_adam": (C.c_int, [P, P, C.c_uint32, C.c_float, C.c_float, C.c_float, C.c_float, P]),
+        "pg_calib_status": (C.c_int, [P]),
+        "pg_calib_set_wait_polls": (C.c_int, [P, C.c_uint32]),
     }
     for name, (res, args) in protos.items():
         fn = getattr(L, name)
@@ -108,7 +110,10 @@ class CalibBatch:
 
     def adam(self, params, steps: int, lr: float = 0.05, beta1: float = 0.9, beta2: float = 0.999,
              eps: float = 1e-8):
-        """``steps`` Adam steps on every replicate, in place, without host work between them."""
+        """``steps`` Adam steps on every replicate, in place, without host work between them.
+
+        A replicate whose thread blocks could not meet between two steps ends
+        as NaN; ``check`` then raises."""
         import torch
         assert params.dtype == torch.float32 and params.is_contiguous() and params.is_cuda
         nll = torch.empty(self.n_rep, dtype=torch.float32, device=params.device)
@@ -116,6 +121,10 @@ class CalibBatch:
             check(self.L.pg_calib_adam(self._h, C.c_void_p(params.data_ptr()), steps, lr, beta1, beta2, eps,
                                        C.c_void_p(nll.data_ptr())))
         return nll
+
+    def check(self):
+        """Waits for the handle's calls; raises if a wait between Adam steps ran out."""
+        check(self.L.pg_calib_status(self._h))
 
     @property
     def stream(self):

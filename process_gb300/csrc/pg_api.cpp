@@ -2176,6 +2176,10 @@ pg_status pg_seq_result_tile_size(const pg_seq_result* r, uint32_t* tile_size) {
 }  // extern "C"
 
 // ====================================================================== calibration
+// Looks at a count before a wait between Adam steps is given up: a look takes
+// an L2 round trip, some 0.5 us, so about two seconds.
+constexpr uint32_t CALIB_WAIT_POLLS = 1u << 22;
+
 struct pg_calib {
   int device = 0;
   cudaStream_t st = nullptr, own_st = nullptr;
@@ -2187,6 +2191,7 @@ struct pg_calib {
   DBuf<float> sig_rows, epoch_w, phi, tab, m, v, partial;
   bool split = false;                // more segments than the GPU holds at a time
   bool by_warps = false;             // chunks dealt out by warps
+  uint32_t wait_polls = CALIB_WAIT_POLLS;
   uint32_t n_rows = 0;
   std::vector<uint32_t> rep_first_seg_h;
   uint32_t part_stride = 0;
@@ -2302,7 +2307,7 @@ pg_status pg_calib_create(uint32_t n_rep, const uint64_t* site_off, const int32_
     c->seg_rep = upload(P, srep, st);
     c->rep_first_seg = upload(P, c->rep_first_seg_h, st);
     c->rep_first_chunk = upload(P, first_chunk, st);
-    c->rep_done = DBuf<uint32_t>(P, n_rep);
+    c->rep_done = DBuf<uint32_t>(P, 2 * uint64_t(n_rep));   // and rep_left
     ck(cudaMemsetAsync(c->rep_done.p, 0, sizeof(uint32_t) * n_rep, st), "memset");
     c->part_stride = (1 + 3 * K + K * J + 3) & ~3u;
     c->partial = DBuf<float>(P, (c->split ? 1 : 2) * uint64_t(c->n_rows) * c->part_stride);
@@ -2310,6 +2315,7 @@ pg_status pg_calib_create(uint32_t n_rep, const uint64_t* site_off, const int32_
     c->m = DBuf<float>(P, uint64_t(n_rep) * c->P);
     c->v = DBuf<float>(P, uint64_t(n_rep) * c->P);
     c->status = DBuf<uint32_t>(P, 1);
+    ck(cudaMemsetAsync(c->status.p, 0, sizeof(uint32_t), st), "memset");
     ck(cudaStreamSynchronize(st), "calibration upload");
     *out = c.release();
   });
@@ -2358,6 +2364,25 @@ pg_status pg_calib_nll_grad_one(pg_calib* c, uint32_t rep, const float* params, 
   });
 }
 
+pg_status pg_calib_set_wait_polls(pg_calib* c, uint32_t polls) {
+  return guarded([&] {
+    require(c != nullptr, "NULL handle");
+    c->wait_polls = polls == UINT32_MAX ? CALIB_WAIT_POLLS : polls;
+  });
+}
+
+pg_status pg_calib_status(pg_calib* c) {
+  return guarded([&] {
+    require(c != nullptr, "NULL handle");
+    ck(cudaSetDevice(c->device), "cudaSetDevice");
+    uint32_t s = 0;
+    ck(cudaMemcpyAsync(&s, c->status.p, sizeof(s), cudaMemcpyDeviceToHost, c->st), "status");
+    ck(cudaMemsetAsync(c->status.p, 0, sizeof(uint32_t), c->st), "status");
+    ck(cudaStreamSynchronize(c->st), "status");
+    if (s) throw std::runtime_error("a wait between Adam steps ran out: the parameters and NLL of its replicates are NaN");
+  });
+}
+
 pg_status pg_calib_adam(pg_calib* c, float* params, uint32_t steps, float lr, float beta1, float beta2, float eps,
                         float* nll) {
   return guarded([&] {
@@ -2371,8 +2396,9 @@ pg_status pg_calib_adam(pg_calib* c, float* params, uint32_t steps, float lr, fl
       pg::CalibArgs a = c->args();
       a.steps = steps;
       a.status = c->status.p;
-      ck(cudaMemsetAsync(c->status.p, 0, sizeof(uint32_t), st), "memset");
-      ck(cudaMemsetAsync(c->rep_done.p, 0xff, sizeof(uint32_t) * c->n_rep, st), "memset");
+      a.rep_left = c->rep_done.p + c->n_rep;
+      a.wait_polls = c->wait_polls;
+      ck(cudaMemsetAsync(c->rep_done.p, 0xff, 2 * sizeof(uint32_t) * c->n_rep, st), "memset");
       pg::calib_launch(a, c->n_segs, c->n_rep, params, nll, nullptr, pg::AdamArgs{c->m.p, c->v.p, 0, lr, beta1, beta2, eps}, st);
       ck(cudaMemsetAsync(c->rep_done.p, 0, sizeof(uint32_t) * c->n_rep, st), "memset");
       ck(cudaGetLastError(), "calibration steps");

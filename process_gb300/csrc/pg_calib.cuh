@@ -60,7 +60,6 @@ constexpr uint32_t CAL_CHUNK = 16384;   // sites (per-thread FP32 sums of 256 in
 // the arrivals' count before the first step: it wraps at once, not only after
 // 2^32 arrivals
 constexpr uint32_t CAL_COUNT0 = 0xffffffffu;
-constexpr uint32_t CAL_SPIN_LIMIT = 1u << 22;   // polls of a wait, 64 ns or more each
 
 struct Neu {   // Neumaier-compensated FP32 sum
   float s = 0.f, c = 0.f;
@@ -548,25 +547,29 @@ __global__ void __launch_bounds__(CAL_THREADS, calib_ctas(K, J, STEPS)) k_calib(
   } else {
     constexpr uint32_t P = K + K * J + 1;
     // All the replicate's sums of this step.  The CTAs are all resident (a
-    // cooperative launch); a wait that runs out all the same marks the call and
-    // every CTA leaves at its next look.
+    // cooperative launch); should a wait run out all the same, the CTA leaves and
+    // the replicate's others with it.  The first CTA alone writes results, so
+    // they are those of all steps or, where it had to leave, NaN.
     if (threadIdx.x == 0) {
-      uint32_t go = 1, polls = 0;
+      uint32_t go = 0;
       atomicAdd(a.rep_done + r, 1u);
-      while (!arrived(*reinterpret_cast<volatile uint32_t*>(a.rep_done + r), CAL_COUNT0 + (step + 1) * n_parts)) {
-        if (++polls > CAL_SPIN_LIMIT || *reinterpret_cast<volatile uint32_t*>(a.status)) { go = 0; break; }
+      for (uint32_t polls = 0; polls < a.wait_polls; ++polls) {
+        go = arrived(*reinterpret_cast<volatile uint32_t*>(a.rep_done + r), CAL_COUNT0 + (step + 1) * n_parts);
+        if (go || *reinterpret_cast<volatile uint32_t*>(a.rep_left + r) == 0u) break;
         __nanosleep(20);
       }
       __threadfence();
-      if (!go) atomicExch(a.status, 1u);
+      if (!go) atomicExch(a.rep_left + r, 0u);
       s_go = go;
     }
     __syncthreads();
     const bool first = s_at.first != 0;
     if (!s_go) {
-      if (threadIdx.x == 0) {                    // no result: NaN
-        params[uint64_t(r) * P] = __int_as_float(0x7fc00000);
-        if (nll_out) nll_out[r] = __int_as_float(0x7fc00000);
+      const float nan = __int_as_float(0x7fc00000);
+      if (first && threadIdx.x < P) params[uint64_t(r) * P + threadIdx.x] = nan;
+      if (first && threadIdx.x == 0) {
+        if (nll_out) nll_out[r] = nan;
+        *a.status = 1u;
       }
       return;
     }

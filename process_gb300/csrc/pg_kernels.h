@@ -448,7 +448,9 @@ struct CalibArgs {
   uint32_t part_stride, n_rows;   //   with steps > 1 twice that
   uint32_t seg0, rep0;            // first segment and replicate of the launch
   uint32_t steps;                 // evaluations of the launch (above 1: Adam steps, without tab)
-  uint32_t* status;               // set when a wait between the steps ran out
+  uint32_t* rep_left;             // several evaluations: n_rep words, all ones before the launch, 0 where a CTA left
+  uint32_t wait_polls;            //   a wait after this many looks, which
+  uint32_t* status;               //   sets this
   float* tab;                     // per replicate, calib_tab floats: its constants, where they and the
                                   //   epilogues have launches of their own; else NULL
 };
