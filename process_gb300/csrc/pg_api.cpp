@@ -1453,7 +1453,8 @@ pg_status pg_place_mutations(pg_engine* e, const pg_forest* f, uint32_t n_pre_sn
     pl->seq = DBuf<uint16_t>(P, n_all);
     pl->kind = DBuf<uint8_t>(P, n_all); pl->nature = DBuf<uint8_t>(P, n_all);
     DBuf<unsigned long long> skeys(P, n_all);
-    pg::sort_by_locus(o, uint32_t(n_all), e->genome.p, e->G, bcnt.p, bpart.p, order.p, pl->view(), skeys.p, st);
+    pg::sort_by_locus(o, uint32_t(n_all), e->genome.p, e->G, bcnt.p, bpart.p, order.p, pl->view(), skeys.p,
+                      {err, &ctl.p->tail}, st);
     Ctl c{};
     timer.mark();
     ck(cudaMemcpyAsync(&c, ctl.p, sizeof(c), cudaMemcpyDeviceToHost, st), "error flag");

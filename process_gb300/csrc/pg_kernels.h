@@ -154,11 +154,17 @@ void sites_settle(const PlaceTables& t, const PlaceRaw& o, uint64_t seed, const 
 void sites_covered(const PlaceTables& t, const PlaceRaw& o, uint64_t seed, const uint32_t* off_snv,
                    const uint32_t* off_id, uint32_t n_snv, uint32_t n_slots, TailCtl* ctl, uint32_t* err,
                    cudaStream_t st);
+// What says that a placement failed (tail may be NULL): a sort then writes nothing.
+struct PlaceFlags {
+  const uint32_t* err;
+  const TailCtl* tail;
+};
 uint32_t sort_num_buckets(uint64_t G);
 // sort by (locus, slot) into `sorted`; bcnt: 2 sort_num_buckets(G) entries,
 // keys: n 64-bit keys
 void sort_by_locus(const PlaceRaw& o, uint32_t n, const uint32_t* genome, uint64_t G, uint32_t* bcnt, uint32_t* part,
-                   uint32_t* order, const PlaceOut& sorted, unsigned long long* keys, cudaStream_t st);
+                   uint32_t* order, const PlaceOut& sorted, unsigned long long* keys, const PlaceFlags& flags,
+                   cudaStream_t st);
 
 // ---------------------------------------------------------------- sequencing
 struct SeqRec {            // 16 B, one per placed mutation, sorted by locus
@@ -399,7 +405,7 @@ void sites_settle_batch(const PlaceTables* tabs, uint32_t n_inst, const uint32_t
 // 64-bit keys
 void sort_batch(const PlaceRaw& o, const uint16_t* inst_of, uint32_t n, uint32_t n_inst, const uint32_t* genome,
                 uint64_t G, uint32_t* bcnt, uint32_t* bfill, uint32_t* part, uint32_t* order, const PlaceOut& sorted, uint16_t* inst_sorted,
-                unsigned long long* keys, cudaStream_t st);
+                unsigned long long* keys, const PlaceFlags& flags, cudaStream_t st);
 // records of the first *n_dev sorted mutations of a batch (cap >= *n_dev)
 void seq_batch_records(const PlaceOut& sorted, const uint16_t* inst_sorted, const uint32_t* n_dev, uint32_t cap,
                        const SeqBatch& b, SeqRec* recs, cudaStream_t st);

@@ -565,17 +565,25 @@ __global__ void k_drivers(PlaceRaw o, const DriverRec* __restrict__ drv, uint32_
 // ------------------------------------------------------------ locus sort
 constexpr int BUCKET_SHIFT = 10;
 
-__global__ void k_bucket_count(const uint32_t* __restrict__ locus, uint32_t n, uint32_t* __restrict__ bcnt) {
+// Whether slots were given up: the call fails, and nothing is sorted (they all
+// hold locus 0, and one thread would sort their bucket by insertion).
+__device__ __forceinline__ bool failed(const PlaceFlags& f) {
+  return *f.err != 0u || (f.tail && f.tail->status != 0u);
+}
+
+__global__ void k_bucket_count(const uint32_t* __restrict__ locus, uint32_t n, uint32_t* __restrict__ bcnt,
+                               PlaceFlags flags) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) atomicAdd(bcnt + (locus[i] >> BUCKET_SHIFT), 1u);
+  if (i < n && !failed(flags)) atomicAdd(bcnt + (locus[i] >> BUCKET_SHIFT), 1u);
 }
 // Bucket sort on 64-bit keys (locus << 32 | slot) written by the scatter:
 // the in-bucket insertion sort reads its bucket's keys contiguously, and
 // ties of a locus fall in slot order.
 __global__ void k_bucket_scatter_keys(const uint32_t* __restrict__ locus, uint32_t n, const uint32_t* __restrict__ boff,
-                                      uint32_t* __restrict__ bfill, unsigned long long* __restrict__ keys) {
+                                      uint32_t* __restrict__ bfill, unsigned long long* __restrict__ keys,
+                                      PlaceFlags flags) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  if (i >= n || failed(flags)) return;
   const uint32_t k = locus[i], b = k >> BUCKET_SHIFT;
   keys[boff[b] + atomicAdd(bfill + b, 1u)] = (static_cast<unsigned long long>(k) << 32) | i;
 }
@@ -590,9 +598,10 @@ constexpr uint32_t SORT_BUCKETS = 64, SORT_STAGE = 2560, SORT_THREADS = 256;   /
 __global__ void __launch_bounds__(SORT_THREADS) k_bucket_sort_keys(const uint32_t* __restrict__ boff, uint32_t nb,
                                                                    uint32_t n, unsigned long long* __restrict__ keys,
                                                                    uint32_t* __restrict__ locus,
-                                                                   uint32_t* __restrict__ order) {
+                                                                   uint32_t* __restrict__ order, PlaceFlags flags) {
   __shared__ unsigned long long s_keys[SORT_STAGE];
   __shared__ uint32_t s_off[SORT_BUCKETS + 1];
+  if (failed(flags)) return;
   const uint32_t b0 = blockIdx.x * SORT_BUCKETS, b1 = min(b0 + SORT_BUCKETS, nb), m = b1 - b0;
   if (threadIdx.x <= m) s_off[threadIdx.x] = b0 + threadIdx.x < nb ? boff[b0 + threadIdx.x] : n;
   __syncthreads();
@@ -631,9 +640,9 @@ __global__ void __launch_bounds__(SORT_THREADS) k_bucket_sort_keys(const uint32_
 // (n_inst: a batch, whose instance i starts at boff[i * nb]; else 0)
 __global__ void k_gather_records(const uint4* __restrict__ rec, const uint32_t* __restrict__ order, uint32_t n,
                                  const uint32_t* __restrict__ genome, PlaceOut s, uint16_t* __restrict__ inst_sorted,
-                                 uint32_t n_inst, uint32_t nb, const uint32_t* __restrict__ boff) {
+                                 uint32_t n_inst, uint32_t nb, const uint32_t* __restrict__ boff, PlaceFlags flags) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  if (i >= n || failed(flags)) return;
   const uint4 a = rec[order[i]];
   const bool is_id = ((a.w >> 16) & 0xffu) == KIND_INDEL;
   s.edge[i] = a.x;
@@ -764,15 +773,16 @@ __global__ void k_place_first_b(BatchSlots s, PlaceRaw o, uint32_t n_slots, uint
 
 // sort of a batch by (instance, locus): bucket = instance * nb + locus >> 10
 __global__ void k_bucket_count_b(const uint32_t* __restrict__ locus, const uint16_t* __restrict__ inst_of, uint32_t n,
-                                 uint32_t nb, uint32_t* __restrict__ bcnt) {
+                                 uint32_t nb, uint32_t* __restrict__ bcnt, PlaceFlags flags) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) atomicAdd(bcnt + uint64_t(inst_of[i]) * nb + (locus[i] >> BUCKET_SHIFT), 1u);
+  if (i < n && !failed(flags)) atomicAdd(bcnt + uint64_t(inst_of[i]) * nb + (locus[i] >> BUCKET_SHIFT), 1u);
 }
 __global__ void k_bucket_scatter_b(const uint32_t* __restrict__ locus, const uint16_t* __restrict__ inst_of,
                                    uint32_t n, uint32_t nb, const uint32_t* __restrict__ boff,
-                                   uint32_t* __restrict__ bfill, unsigned long long* __restrict__ keys) {
+                                   uint32_t* __restrict__ bfill, unsigned long long* __restrict__ keys,
+                                   PlaceFlags flags) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  if (i >= n || failed(flags)) return;
   const uint32_t k = locus[i];
   const uint64_t b = uint64_t(inst_of[i]) * nb + (k >> BUCKET_SHIFT);
   keys[boff[b] + atomicAdd(bfill + b, 1u)] = (static_cast<unsigned long long>(k) << 32) | i;
@@ -837,16 +847,16 @@ void sites_covered(const PlaceTables& t, const PlaceRaw& o, uint64_t seed, const
 }
 
 void sort_by_locus(const PlaceRaw& o, uint32_t n, const uint32_t* genome, uint64_t G, uint32_t* bcnt, uint32_t* part,
-                   uint32_t* order, const PlaceOut& sorted, unsigned long long* keys, cudaStream_t st) {
+                   uint32_t* order, const PlaceOut& sorted, unsigned long long* keys, const PlaceFlags& flags, cudaStream_t st) {
   const uint32_t nb = uint32_t((G >> BUCKET_SHIFT) + 1);
   uint32_t* const bfill = bcnt + nb;
   cudaMemsetAsync(bcnt, 0, sizeof(uint32_t) * 2 * nb, st);
   if (n == 0) return;
-  k_bucket_count<<<nblk(n), 256, 0, st>>>(o.locus, n, bcnt); note_launch();
+  k_bucket_count<<<nblk(n), 256, 0, st>>>(o.locus, n, bcnt, flags); note_launch();
   scan_rows<uint32_t>(bcnt, bcnt, nb, 1, part, nullptr, st);
-  k_bucket_scatter_keys<<<nblk(n), 256, 0, st>>>(o.locus, n, bcnt, bfill, keys); note_launch();
-  k_bucket_sort_keys<<<nblk(nb, SORT_BUCKETS), SORT_THREADS, 0, st>>>(bcnt, nb, n, keys, sorted.locus, order);
-  k_gather_records<<<nblk(n), 256, 0, st>>>(o.rec, order, n, genome, sorted, nullptr, 0u, 0u, nullptr);
+  k_bucket_scatter_keys<<<nblk(n), 256, 0, st>>>(o.locus, n, bcnt, bfill, keys, flags); note_launch();
+  k_bucket_sort_keys<<<nblk(nb, SORT_BUCKETS), SORT_THREADS, 0, st>>>(bcnt, nb, n, keys, sorted.locus, order, flags);
+  k_gather_records<<<nblk(n), 256, 0, st>>>(o.rec, order, n, genome, sorted, nullptr, 0u, 0u, nullptr, flags);
   note_launch(2);
 }
 
@@ -888,17 +898,17 @@ void sites_settle_batch(const PlaceTables* tabs, uint32_t n_inst, const uint32_t
 
 void sort_batch(const PlaceRaw& o, const uint16_t* inst_of, uint32_t n, uint32_t n_inst, const uint32_t* genome,
                 uint64_t G, uint32_t* bcnt, uint32_t* bfill, uint32_t* part, uint32_t* order, const PlaceOut& sorted, uint16_t* inst_sorted,
-                unsigned long long* keys, cudaStream_t st) {
+                unsigned long long* keys, const PlaceFlags& flags, cudaStream_t st) {
   const uint32_t nb = uint32_t((G >> BUCKET_SHIFT) + 1);
   const uint64_t nbt = uint64_t(nb) * n_inst;
   cudaMemsetAsync(bcnt, 0, sizeof(uint32_t) * (nbt + 1), st);
   cudaMemsetAsync(bfill, 0, sizeof(uint32_t) * nbt, st);
   if (n == 0) return;
-  k_bucket_count_b<<<nblk(n), 256, 0, st>>>(o.locus, inst_of, n, nb, bcnt); note_launch();
+  k_bucket_count_b<<<nblk(n), 256, 0, st>>>(o.locus, inst_of, n, nb, bcnt, flags); note_launch();
   scan_rows<uint32_t>(bcnt, bcnt, nbt, 1, part, bcnt + nbt, st);
-  k_bucket_scatter_b<<<nblk(n), 256, 0, st>>>(o.locus, inst_of, n, nb, bcnt, bfill, keys); note_launch();
-  k_bucket_sort_keys<<<nblk(nbt, SORT_BUCKETS), SORT_THREADS, 0, st>>>(bcnt, uint32_t(nbt), n, keys, sorted.locus, order);
-  k_gather_records<<<nblk(n), 256, 0, st>>>(o.rec, order, n, genome, sorted, inst_sorted, n_inst, nb, bcnt);
+  k_bucket_scatter_b<<<nblk(n), 256, 0, st>>>(o.locus, inst_of, n, nb, bcnt, bfill, keys, flags); note_launch();
+  k_bucket_sort_keys<<<nblk(nbt, SORT_BUCKETS), SORT_THREADS, 0, st>>>(bcnt, uint32_t(nbt), n, keys, sorted.locus, order, flags);
+  k_gather_records<<<nblk(n), 256, 0, st>>>(o.rec, order, n, genome, sorted, inst_sorted, n_inst, nb, bcnt, flags);
   note_launch(2);
 }
 
