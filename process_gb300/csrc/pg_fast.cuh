@@ -9,8 +9,12 @@
 // floats where two numbers are compared.  Each decision has a margin that
 // exceeds the error of both evaluations; outside the margins the FP64
 // sampler takes the same decisions from the same Philox words, so the result
-// is its result.  Inside a margin (under one draw in ten thousand) the
-// functions return false and the caller draws with the FP64 sampler.
+// is its result.  Inside a margin the functions return false and the caller
+// draws with the FP64 sampler.  Measured over 3.1e7 draws in each of fourteen
+// ranges (none decided otherwise): Poisson means 1e-6 to 0.1 6e-5 of the draws,
+// inversion up to means of ten 4e-4 (Poisson) and 9e-4 (binomial), rejection 3e-4
+// to 8e-4, 1.8e-3 for binomials of 2^24 to 2^32 trials (the floor's margin grows
+// with them); 1e-2 within 0.01 of a mean of ten, and every half of 20.
 #pragma once
 #include "pg_f2.cuh"
 #include "pg_rng.cuh"
@@ -75,9 +79,11 @@ __device__ __forceinline__ float stirling_tail_f(float k) {
 }
 
 // One attempt's uniforms of the transformed-rejection samplers, as FP64 sees
-// them: U = u01_open(x, y) - 1/2 and us = 1/2 - |U|, both exact in FP64 and
-// here (multiples of 2^-54; the sum inside u01_open rounds half to even), and
-// V = u01_open(z, w).  False when us is so small that two floats lose it.
+// them: U = u01_open(x, y) - 1/2 and us = 1/2 - |U|, both exact in FP64
+// (multiples of 2^-54; the sum inside u01_open rounds half to even) and taken
+// here from the same integers into two floats (2^-43 relative, which the margins
+// hold), and V = u01_open(z, w).  False when us is so small that two floats lose
+// it.
 __device__ __forceinline__ bool attempt_uniforms(const U4& r, F2& U, F2& us, float& V) {
   const uint64_t u = ((uint64_t(r.x) << 32) | r.y) >> 11;
   const uint64_t t = u >= (1ull << 52) ? 2 * (u + (u & 1)) : 2 * u + 1;   // u01 * 2^54
