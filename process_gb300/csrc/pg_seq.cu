@@ -151,7 +151,7 @@ struct TileSplit {
 // (16 levels, 4 samples) 1.64 ms became 0.55.
 constexpr uint32_t SPLIT_BLOCK_LOG = 6;   // 64 tiles per warp
 constexpr uint32_t SPLIT_THREADS = 128;
-// blocks per (sample, chromosome slot)
+// blocks per (sample, chromosome slot): as many as the longest needs
 __host__ __device__ inline uint32_t split_blocks(const SeqChroms& c) {
   const uint32_t tiles = SPLIT_THREADS / 32 << SPLIT_BLOCK_LOG;
   return (c.max_tiles + tiles - 1) / tiles;
@@ -195,12 +195,13 @@ __device__ __forceinline__ void tile_counts_warp(const TileSplit& sp, uint32_t s
   }
 }
 
-// block x of the tile split: 64 tiles per warp of a (sample, chromosome slot)
-__device__ __forceinline__ void split_block(const SeqChroms& c, uint32_t x, const double* __restrict__ mass_cum,
-                                            const double* __restrict__ mass_tot, Key key,
-                                            uint32_t* __restrict__ pair_cnt) {
-  const uint32_t per = split_blocks(c), row = x / per, s = row / c.n_slots, slot = row % c.n_slots;
-  const uint32_t b = (x % per * SPLIT_THREADS + threadIdx.x) >> 5;
+// block x of row `row` of the tile split (a row: a sample's chromosome slot):
+// 64 tiles per warp
+__device__ __forceinline__ void split_block(const SeqChroms& c, uint64_t row, uint32_t x,
+                                            const double* __restrict__ mass_cum, const double* __restrict__ mass_tot,
+                                            Key key, uint32_t* __restrict__ pair_cnt) {
+  const uint32_t s = uint32_t(row / c.n_slots), slot = uint32_t(row % c.n_slots);
+  const uint32_t b = (x * SPLIT_THREADS + threadIdx.x) >> 5;
   const uint32_t nt = c.ntiles[slot], first = c.first[slot];
   if (uint64_t(b) << SPLIT_BLOCK_LOG >= nt) return;   // whole warps
   const TileSplit sp{c.nstarts[slot], c.T, nt, mass_cum ? mass_cum + uint64_t(s) * c.n_tiles + first : nullptr,
@@ -209,10 +210,12 @@ __device__ __forceinline__ void split_block(const SeqChroms& c, uint32_t x, cons
                    pair_cnt + uint64_t(s) * c.n_tiles + first);
 }
 
-__global__ void __launch_bounds__(SPLIT_THREADS) k_tile_split(SeqChroms c, const double* __restrict__ mass_cum,
+__global__ void __launch_bounds__(SPLIT_THREADS) k_tile_split(SeqChroms c, uint64_t row0,
+                                                              const double* __restrict__ mass_cum,
                                                               const double* __restrict__ mass_tot, Key key,
                                                               uint32_t* __restrict__ pair_cnt) {
-  split_block(c, blockIdx.x, mass_cum, mass_tot, key, pair_cnt);
+  const uint32_t per = split_blocks(c);
+  split_block(c, row0 + blockIdx.x / per, blockIdx.x % per, mass_cum, mass_tot, key, pair_cnt);
 }
 
 // The steps before the read kernel that wait for nothing, each a range of
@@ -228,7 +231,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS) k_seq_prepare(SeqChroms c, SeqT
                                                                uint32_t tiles_end, Key key,
                                                                uint32_t* __restrict__ pair_cnt) {
   if (SPLIT && blockIdx.x < split_end) {
-    split_block(c, blockIdx.x, nullptr, nullptr, key, pair_cnt);
+    const uint32_t per = split_blocks(c);
+    split_block(c, blockIdx.x / per, blockIdx.x % per, nullptr, nullptr, key, pair_cnt);
   } else if (blockIdx.x < tiles_end) {
     const uint32_t t = (blockIdx.x - split_end) * SPLIT_THREADS + threadIdx.x;
     if (t >= c.n_tiles) return;
@@ -810,6 +814,7 @@ __global__ void __launch_bounds__(SEQ_THREADS, 4) k_reads(const SeqRec* __restri
             g_dep + uint64_t(s) * n_recs);
 }
 
+constexpr uint64_t MAX_GRID_X = 0x7fffffffu;
 static inline unsigned nblk(uint64_t n, int b = 256) { return unsigned((n + b - 1) / b); }
 
 // ------------------------------------------------------------ SAM reads
@@ -1181,8 +1186,13 @@ void seq_tile_mass(uint32_t n_samples, uint32_t n_slots, const uint32_t* c_first
 void seq_prepare(const SeqChroms& c, const SeqTiles& tiles, const PlaceOut& sorted, uint32_t n_recs,
                  const uint32_t* edge_tin, const uint32_t* edge_tout, uint32_t span, SeqRec* recs, uint32_t n_split,
                  uint64_t seed, uint32_t* pair_cnt, cudaStream_t st) {
-  const uint32_t split_end = n_split * c.n_slots * split_blocks(c), tiles_end = split_end + nblk(c.n_tiles, SPLIT_THREADS);
-  const uint32_t grid = tiles_end + nblk(n_recs, SPLIT_THREADS);
+  // (a split of more blocks than a grid has is launched on its own)
+  const uint64_t split = uint64_t(n_split) * c.n_slots * split_blocks(c);
+  const uint32_t rest = nblk(c.n_tiles, SPLIT_THREADS) + nblk(n_recs, SPLIT_THREADS);
+  const bool apart = split + rest > MAX_GRID_X;
+  if (apart) seq_tile_counts(c, n_split, nullptr, nullptr, seed, pair_cnt, st);
+  const uint32_t split_end = apart ? 0u : uint32_t(split), tiles_end = split_end + nblk(c.n_tiles, SPLIT_THREADS);
+  const uint32_t grid = split_end + rest;
   if (!grid) return;
   const Key key = make_key(seed);
   if (split_end)
@@ -1196,10 +1206,13 @@ void seq_prepare(const SeqChroms& c, const SeqTiles& tiles, const PlaceOut& sort
 
 void seq_tile_counts(const SeqChroms& c, uint32_t n_samples, const double* mass_cum, const double* mass_tot,
                      uint64_t seed, uint32_t* pair_cnt, cudaStream_t st) {
-  const uint32_t grid = n_samples * c.n_slots * split_blocks(c);
-  if (!grid) return;
-  k_tile_split<<<grid, SPLIT_THREADS, 0, st>>>(c, mass_cum, mass_tot, make_key(seed), pair_cnt);
-  note_launch();
+  // whole rows, as many at a time as a grid has blocks for
+  const uint64_t rows = uint64_t(n_samples) * c.n_slots, per = split_blocks(c), most = MAX_GRID_X / std::max<uint64_t>(per, 1);
+  for (uint64_t row = 0; per && row < rows; row += most) {
+    const uint32_t grid = uint32_t(std::min(most, rows - row) * per);
+    k_tile_split<<<grid, SPLIT_THREADS, 0, st>>>(c, row, mass_cum, mass_tot, make_key(seed), pair_cnt);
+    note_launch();
+  }
 }
 
 // ------------------------------------------------------------ observed rows

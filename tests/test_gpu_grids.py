@@ -37,3 +37,31 @@ def test_batch_of_many_samples(gpu_lib, orc):
         assert alt.shape == oalt.shape == ((70_002 if i == 0 else 3), b.dims(i)[0])      # and the normal sample
         np.testing.assert_array_equal(dep, odep)
         np.testing.assert_array_equal(alt, oalt)
+
+
+@pytest.mark.parametrize("cna", [False, True])
+def test_tile_split_of_many_samples_and_chromosomes(gpu_lib, orc, cna):
+    """600 samples of 60,001 chromosomes, one of them far longer than the others:
+    the tile split has more blocks (62 for each sample and chromosome) than a
+    grid (2^31 - 1)."""
+    from process_gb300 import CNA, synth
+    from process_gb300.engine import seq_cfg, sequence_counts
+    w = synth.plain_3mbp(seed=5, n_leaves=30)
+    n, samples = 60_000, 600
+    w.genome.chr_names = [str(i) for i in range(n + 1)]
+    w.genome.chr_lengths = [60] * n + [1_000_000]
+    name = w.mutants[0][0]
+    w.mutants = [(name, {"SNV": 1e-9, "indel": 0.0}, [CNA("A", str(n), 300_001, 400_000)] if cna else [])]
+    f = w.forest = synth.birth_forest(samples, samples, 3, subclone=None, mutant=name)
+    eng = synth.build_engine(w)
+    o = orc.OracleEngine.like(w)
+    sp = np.array([o.species[(m, e)] for m, e in zip(f.mutant, f.epistate)], dtype=np.uint32)
+    pf = eng.place_mutations(f, 200, 0, seed=2)
+    op = o.place(f, sp, 200, 0, 0, 0, seed=2)
+    cfg = dict(coverage=0.5, read_size=50, insert_size_mean=0, error_rate=0.0, purity=0.5, tile_size=64)
+    alt, dep = sequence_counts(pf, 4, **cfg).counts()
+    c, _ = seq_cfg(chr_index=eng._chr_index, **cfg)
+    oalt, odep, _ = op.sequence(c, 4, flavour=0)
+    assert (alt.shape[0] - 1) * (n + 1) * ((1_000_000 - 49) // 64 // 256 + 1) >= 2**31
+    np.testing.assert_array_equal(dep, odep)
+    np.testing.assert_array_equal(alt, oalt)
