@@ -41,8 +41,8 @@
 // a chunk, and the constants and the epilogues are launches of their own (in
 // k_calib they keep a CTA's slot from the next chunk).  Against three kernels
 // with a CTA per chunk, K = 4, J = 3: 2e5 sites 25.7 -> 16.5 us, 512 x 1e5 sites
-// 166 -> 155, 200 Adam steps over 64 x 5e4 sites (a graph of 600 launches) 4.98
-// -> 3.64 ms; no shape from K = J = 1 to 8 is slower at 20001 to 100 x 120001
+// 166 -> 148, 200 Adam steps over 64 x 5e4 sites (a graph of 600 launches) 4.98
+// -> 3.66 ms; no shape from K = J = 1 to 8 is slower at 20001 to 100 x 120001
 // sites.  Bound by the serial sums (64 sites a thread) while the GPU is not
 // filled, then by the instructions per site.
 #pragma once
@@ -201,7 +201,7 @@ constexpr uint32_t calib_min_blocks(uint32_t K, uint32_t J) {
 }
 
 // the Adam steps' instance, whose loop keeps more: two at most (200 steps over
-// 64 x 5e4 sites: 3.64 ms, with three CTAs 3.81, over 20 x 5e4 at K = J = 2 2.2
+// 64 x 5e4 sites: 3.66 ms, with three CTAs 3.81, over 20 x 5e4 at K = J = 2 2.2
 // against 3.3 ms: spills)
 constexpr uint32_t calib_ctas(uint32_t K, uint32_t J, bool steps) {
   return steps && calib_min_blocks(K, J) > 2 ? 2 : calib_min_blocks(K, J);
@@ -301,6 +301,12 @@ __device__ __forceinline__ float adam_update(const AdamArgs& adam, AdamBias b, f
   return adam.lr * mh / (sqrtf(vh) + adam.eps);
 }
 
+// The forms of k_calib: an evaluation with a chunk per CTA (whose threads'
+// places are their numbers: with a run-time rule, whose values spill, 512 x 1e5
+// sites took 155 us)
+// or by warps, and Adam steps
+enum CalibForm { CHUNKS_FORM, WARPS_FORM, STEPS_FORM };
+
 // one evaluation's results (and Adam step), by one CTA per replicate
 template <uint32_t K, uint32_t J>
 __device__ __forceinline__ void calib_epilogue(CalibEpilogue& sh, const CalibRow<K, J>& c, const CalibArgs& a,
@@ -321,18 +327,20 @@ __device__ __forceinline__ void calib_epilogue(CalibEpilogue& sh, const CalibRow
   }
 }
 
-// STEPS: a.steps Adam steps in a cooperative launch (an instance of its own: in
-// the other the step's state would spill).  Every CTA of a replicate keeps the
+// STEPS_FORM: a.steps Adam steps in a cooperative launch (an instance of its own: in
+// the others the step's state would spill).  Every CTA of a replicate keeps the
 // parameters and moments and makes each step itself, from the same sums in the
 // same order, so a step has one wait (the sums) where parameters
 // published by one CTA need a second: 0.4 ms of 200 steps over 64 x 5e4 sites.
 // The sums alternate between two halves of a.partial: a CTA is at
 // most one step ahead of the others.
-template <uint32_t K, uint32_t J, bool STEPS>
-__global__ void __launch_bounds__(CAL_THREADS, calib_ctas(K, J, STEPS)) k_calib(CalibArgs a, float* __restrict__ params,
+template <uint32_t K, uint32_t J, CalibForm FORM>
+__global__ void __launch_bounds__(CAL_THREADS, calib_ctas(K, J, FORM == STEPS_FORM)) k_calib(CalibArgs a, float* __restrict__ params,
                                                                                float* __restrict__ nll_out,
                                                                                float* __restrict__ grad_out,
                                                                                AdamArgs adam) {
+  constexpr bool STEPS = FORM == STEPS_FORM;
+  const bool by_warps = STEPS ? a.by_warps != 0u : FORM == WARPS_FORM;
   constexpr uint32_t JP = J > 4 ? 8 : 4;
   constexpr uint32_t NV = 1 + 3 * K + K * J;   // nll, A, B, G, H
   // The signature rows and the mixtures M_k(c) by class, eight copies of each
@@ -354,13 +362,13 @@ __global__ void __launch_bounds__(CAL_THREADS, calib_ctas(K, J, STEPS)) k_calib(
   const uint32_t seg = a.seg0 + blockIdx.x, rep = a.seg_rep[seg];
   // this thread's chunk of the replicate and its place in it
   const uint32_t part = seg - a.rep_first_seg[rep], parts = a.rep_first_seg[rep + 1] - a.rep_first_seg[rep];
-  const uint32_t unit = a.by_warps ? warp * parts + part : part * CAL_WARPS + warp, chunk = unit / CAL_WARPS;
-  const uint32_t place = unit % CAL_WARPS * 32 + lane;
+  const uint32_t unit = by_warps ? warp * parts + part : part * CAL_WARPS + warp, chunk = unit / CAL_WARPS;
+  const uint32_t place = FORM == CHUNKS_FORM ? threadIdx.x : unit % CAL_WARPS * 32 + lane;
   const uint64_t end = a.site_off[rep + 1], i0 = min(a.site_off[rep] + uint64_t(chunk) * CAL_CHUNK, end);
   const uint64_t i1 = min(i0 + CAL_CHUNK, end);
   if (lane == 0) {
     const uint32_t c0 = a.rep_first_chunk[rep];
-    s_at.row[warp] = chunk >= a.rep_first_chunk[rep + 1] - c0 ? NO_ROW : a.by_warps ? c0 * CAL_WARPS + unit : c0 + chunk;
+    s_at.row[warp] = chunk >= a.rep_first_chunk[rep + 1] - c0 ? NO_ROW : by_warps ? c0 * CAL_WARPS + unit : c0 + chunk;
     if (warp == 0) { s_at.r = rep; s_at.parts = parts; s_at.first = part == 0 ? 1u : 0u; }
   }
   if (STEPS) {
@@ -492,9 +500,11 @@ __global__ void __launch_bounds__(CAL_THREADS, calib_ctas(K, J, STEPS)) k_calib(
     const int4* d4 = reinterpret_cast<const int4*>(a.depth) + v0 / 4;
     const int4* c4 = reinterpret_cast<const int4*>(a.cls) + v0 / 4;
     const uint32_t n4 = uint32_t((v1 - v0) / 4);
-    // unrolled by two for the small shapes: 157 us for 512 x 1e5 sites (by
-    // three 166: spills)
-#pragma unroll (K * J <= 16 ? 2 : 1)
+    // unrolled for the small shapes: by three with a chunk per CTA (512 x 1e5
+    // sites 148 us, by two 150, not 169), by two otherwise (200 steps over 64 x
+    // 5e4 sites 3.66 ms, by three 4.01, not 3.94)
+    constexpr uint32_t UNROLL = K * J > 16 ? 1 : FORM == CHUNKS_FORM ? 3 : 2;
+#pragma unroll UNROLL
     for (uint32_t q = place; q < n4; q += CAL_THREADS) site4(load4(a4 + q), load4(d4 + q), load4(c4 + q));
   }
   // the warp's sums: by a fixed tree
@@ -518,10 +528,10 @@ __global__ void __launch_bounds__(CAL_THREADS, calib_ctas(K, J, STEPS)) k_calib(
     constexpr uint32_t tail = NV % 32 ? NV % 32 : 32;
     const float v = q + 32 <= NV ? warp_transpose_sum<32>(acc + q, lane) : warp_transpose_sum<tail>(acc + q, lane);
     if (q + lane >= NV) continue;
-    if (!a.by_warps) s_u.red[warp][q + lane] = v;
+    if (!by_warps) s_u.red[warp][q + lane] = v;
     else if (out_row != NO_ROW) out[q + lane] = v;
   }
-  if (!a.by_warps) {
+  if (!by_warps) {
     __syncthreads();
     for (uint32_t x = threadIdx.x; x < NV && out_row != NO_ROW; x += CAL_THREADS) {
       Neu t;
@@ -620,12 +630,13 @@ static void calib_run(const CalibArgs& a, uint32_t n_segs, uint32_t n_rep, float
   static_assert(sizeof(CalibRow<K, J>) == 4 * calib_row_floats(K, J), "a row of a.tab");
   if (a.tab) k_calib_tables<K, J><<<n_rep, CAL_THREADS, 0, st>>>(a, params);
   if (a.steps == 1) {
-    k_calib<K, J, false><<<n_segs, CAL_THREADS, 0, st>>>(a, params, nll, grad, adam);
+    if (a.by_warps) k_calib<K, J, WARPS_FORM><<<n_segs, CAL_THREADS, 0, st>>>(a, params, nll, grad, adam);
+    else k_calib<K, J, CHUNKS_FORM><<<n_segs, CAL_THREADS, 0, st>>>(a, params, nll, grad, adam);
   } else {
     CalibArgs aa = a;
     AdamArgs ad = adam;
     void* args[] = {&aa, &params, &nll, &grad, &ad};
-    cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_calib<K, J, true>), dim3(n_segs), dim3(CAL_THREADS), args, 0, st);
+    cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_calib<K, J, STEPS_FORM>), dim3(n_segs), dim3(CAL_THREADS), args, 0, st);
   }
   if (a.tab) k_calib_epilogue<K, J><<<n_rep, CAL_THREADS, 0, st>>>(a, params, nll, grad, adam);
   note_launch(a.tab ? 3 : 1);
@@ -633,12 +644,14 @@ static void calib_run(const CalibArgs& a, uint32_t n_segs, uint32_t n_rep, float
 
 template <uint32_t K, uint32_t J>
 static int calib_resident() {
-  int n = 0, m = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_calib<K, J, false>, CAL_THREADS, 0) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, k_calib<K, J, true>, CAL_THREADS, 0) != cudaSuccess)
-    return 1;
-  n = n < m ? n : m;
-  return n > 0 ? n : 1;
+  int least = 64;
+  for (const void* f : {reinterpret_cast<const void*>(k_calib<K, J, CHUNKS_FORM>), reinterpret_cast<const void*>(k_calib<K, J, WARPS_FORM>),
+                        reinterpret_cast<const void*>(k_calib<K, J, STEPS_FORM>)}) {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, CAL_THREADS, 0) != cudaSuccess) return 1;
+    least = n < least ? n : least;
+  }
+  return least > 0 ? least : 1;
 }
 
 #define PG_CALIB_J(KK, JJ) case KK * 8 + JJ - 9: PG_CALIB_DO(KK, JJ); break;
