@@ -332,11 +332,6 @@ void seq_sam_reads(const SeqRec* recs, uint32_t n_recs, const uint32_t* aux, con
                    uint64_t seed, const uint64_t* out_off, SamRead* out, char* seq, uint32_t max_len,
                    cudaStream_t st);
 
-// ---------------------------------------------------------------- batched sequencing
-// Per-instance descriptor of a batch.  The work items of instance i are its
-// (sample, tile) pairs, sample-major; every table row below is relative to
-// the instance's offsets, so each instance computes exactly what the plain
-// path computes for it alone with the same tile size and seed.
 // The copy-number draw tables of one (atom, sample), laid out for a read CTA:
 // per cell option its threshold (the last one takes what is left; unused ones
 // past any 31-bit word), its covering instances, leaves, first leaf and the
@@ -351,6 +346,10 @@ struct alignas(16) CnRow {
   uint32_t n_ids, pad[3];
 };
 
+// ---------------------------------------------------------------- batched sequencing
+// Per-instance descriptor of a batch: every table row below is relative to the
+// instance's offsets, so each instance computes exactly what the plain path
+// computes for it alone with the same tile size and seed.
 struct SeqInst {
   SeqParams prm;
   uint32_t n_samples, sample_off;   // rows of the batch's SeqSample array

@@ -353,16 +353,12 @@ __device__ __forceinline__ unsigned long long first_find(const unsigned long lon
   return FIRST_EMPTY;
 }
 
-// lost: n flags, zeroed by the caller
-__global__ void k_first_insert(const uint32_t* __restrict__ locus, uint32_t n, const uint32_t* __restrict__ drv_locus,
-                               uint32_t n_drv, unsigned long long* __restrict__ tab, uint32_t mask,
-                               uint8_t* __restrict__ lost, uint32_t* __restrict__ err) {
+// the drivers' loci (the passengers' go in with their first draw, k_place_first)
+__global__ void k_first_drivers(const uint32_t* __restrict__ drv_locus, uint32_t n_drv,
+                                unsigned long long* __restrict__ tab, uint32_t mask, uint8_t* __restrict__ lost,
+                                uint32_t* __restrict__ err) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n_drv) first_insert(tab, mask, drv_locus[i], 0u, lost, err);
-  if (i >= n) return;
-  const uint32_t k = locus[i];
-  if (k == LOCUS_INVALID) lost[i] = 1;                   // no allele at the drawn position
-  else first_insert(tab, mask, k, i + 1, lost, err);
 }
 
 // the marked slots, in no particular order (warp-aggregated appends)
@@ -387,9 +383,9 @@ __global__ void __launch_bounds__(256) k_first_collect(const uint8_t* __restrict
 
 // The first draw of every slot.  With infinite sites its insertion into the
 // first round's table is fused in: the insertion's atomics overlap the draws'
-// gathers.  The drivers go in afterwards (k_first_insert with no passenger
-// slots); the table's final state and the marks do not depend on the order of
-// the insertions.  tab (all ones) and lost (zeros) are set by the caller.
+// gathers.  The drivers go in afterwards (k_first_drivers); the table's final
+// state and the marks do not depend on the order of the insertions.  tab (all
+// ones) and lost (zeros) are set by the caller.
 // Bound by the latency of dependent loads, at full scale by random DRAM
 // accesses (list entry, table entry): the cell by a search of the warp, the
 // table's entry requested before the allele is looked up, the bases left to
@@ -820,7 +816,7 @@ void sites_first_finish(const uint32_t* drv_locus, uint32_t n_drv, unsigned long
                         uint8_t* lost, uint32_t n_slots, uint32_t* next, uint32_t* n_next, uint32_t* err,
                         cudaStream_t st) {
   if (n_drv) {
-    k_first_insert<<<nblk(n_drv), 256, 0, st>>>(nullptr, 0, drv_locus, n_drv, first, fmask, lost, err);
+    k_first_drivers<<<nblk(n_drv), 256, 0, st>>>(drv_locus, n_drv, first, fmask, lost, err);
     note_launch();
   }
   if (n_slots) { k_first_collect<<<nblk(n_slots), 256, 0, st>>>(lost, n_slots, next, n_next); note_launch(); }
