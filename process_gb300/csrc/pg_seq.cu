@@ -38,9 +38,9 @@
 // Windows with more records than shared memory holds run a per-read loop on
 // the global arrays instead.
 //
-// Bound by shared-memory wavefronts (73% of the pipe; about 90 per 32
+// Bound by shared-memory wavefronts (78% of the pipe; about 90 per 32
 // fragments: 35 for the counting sort, 35 for the visits, the draws' lookups)
-// and instruction issue (60%, 10 warp instructions per fragment) around four
+// and instruction issue (61%, 10 warp instructions per fragment) around four
 // barriers a batch, not by HBM.  At 155 Mbp, 100x paired, four samples with
 // copy-number events (2.07e8 fragments) the launch takes 2.64 ms.  The form
 // with evenly split candidate runs (a thread walks 17 or so candidates across
