@@ -306,7 +306,10 @@ __device__ __forceinline__ uint32_t mask_word(const uint32_t* __restrict__ m, in
 // classes are dealt out evenly to the lanes, each found by a search over its
 // class's partial counts.  (Ranking one class at a time over the lanes took 13
 // warp instructions per position for the 83 ID classes, 21.4 ms for 3.1 Gbp;
-// 10.7 ms this way.)
+// 10.7 ms this way.)  Where the genome has too few units to fill the GPU, 2 to
+// 16 warps take a unit, each working out all its masks and writing its share of
+// the positions: an item takes a search, a long chain at one warp per unit
+// (100 kbp, every ID position written: 0.93 ms, 72 us with 16 warps).
 // MODE 2: every position written (SBS).  The round's positions are grouped by
 // class in shared memory, then written run by run, consecutive lanes to
 // consecutive entries.  A position's slot is its lane's first slot in the
@@ -328,7 +331,7 @@ __global__ void __launch_bounds__(32 * ix_warps(MODE), MODE == 0 ? 4 : 0) k_inde
                                                                    const uint32_t* __restrict__ stride,
                                                                    const uint64_t* __restrict__ list_off,
                                                                    const uint32_t* __restrict__ list_len,
-                                                                   uint32_t* __restrict__ lists) {
+                                                                   uint32_t* __restrict__ lists, uint32_t share_log) {
   constexpr int NS = (F::NC + 31) / 32;
   constexpr uint32_t FULL = 0xffffffffu;
   constexpr int W = ix_warps(MODE);
@@ -363,7 +366,9 @@ __global__ void __launch_bounds__(32 * ix_warps(MODE), MODE == 0 ? 4 : 0) k_inde
     __syncthreads();
   }
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const uint32_t unit = blockIdx.x * W + w;
+  // MODE 1: 1 << share_log warps per unit (else one)
+  const uint32_t shares = MODE == 1 ? 1u << share_log : 1u, job = blockIdx.x * W + w;
+  const uint32_t unit = MODE == 1 ? job >> share_log : job, share = job & (shares - 1u);
   if (unit >= n_units) return;
   // MODE 0: the lane's counts, class k in byte k % 4 of word k / 4 (at most
   // 128: a unit's positions of one lane)
@@ -538,7 +543,7 @@ __global__ void __launch_bounds__(32 * ix_warps(MODE), MODE == 0 ? 4 : 0) k_inde
       }
       __syncwarp();
       // the written positions, consecutive lanes to consecutive entries of a class
-      for (uint32_t e = lane; e < total; e += 32) {
+      for (uint32_t e = share * 32 + lane; e < total; e += shares * 32) {
         uint32_t k = 0, hi = F::NC;                          // the last class with s_item <= e
         while (hi - k > 1) { const uint32_t mid = (k + hi) >> 1; if (s_item[qw][mid] <= e) k = mid; else hi = mid; }
         const uint32_t j = e - s_item[qw][k], idx = s_kidx[qw][k] + j;
@@ -600,6 +605,9 @@ void genome_pack(uint32_t* words, const uint8_t* codes, uint64_t G, cudaStream_t
   k_genome_pack<<<unsigned((nwords + 255) / 256), 256, 0, st>>>(words, codes, G, nwords); note_launch();
 }
 
+// warps of the emit pass at strides that the GPU holds at a time: 12 per SM
+constexpr uint64_t IX_SHARED_WARPS = 152 * 12;
+
 uint32_t index_num_tiles(uint64_t G) { return uint32_t((G + IX_UNIT - 1) / IX_UNIT); }
 
 template <class F>
@@ -608,7 +616,7 @@ static void index_count_t(const uint32_t* g, const uint32_t* nmask, const uint32
                           cudaStream_t st) {
   const uint32_t ntiles = index_num_tiles(G);
   k_index_scan<F, 0><<<(ntiles + IX_WARPS - 1) / IX_WARPS, 256, 0, st>>>(g, nmask, amask, G, chr_off, n_chr, ntiles,
-                                                                        cnt, nullptr, nullptr, nullptr, nullptr);
+                                                                        cnt, nullptr, nullptr, nullptr, nullptr, 0u);
   note_launch();
   scan_rows<uint32_t>(cnt, cnt, ntiles, F::NC, part, totals, st);
 }
@@ -624,14 +632,18 @@ static void index_emit_t(const uint32_t* g, const uint32_t* nmask, const uint32_
     if (every) {   // stride 1 for every context: each indexed position is written
       k_index_scan<F, 2><<<(ntiles + ix_warps(2) - 1) / ix_warps(2), 32 * ix_warps(2), 0, st>>>(
           g, nmask, amask, G, chr_off, n_chr, ntiles, const_cast<uint32_t*>(cnt_scanned), stride, list_off, list_len,
-          lists);
+          lists, 0u);
       done = true;
     }
   }
   if (!done) {
-    k_index_scan<F, 1><<<(ntiles + ix_warps(1) - 1) / ix_warps(1), 32 * ix_warps(1), 0, st>>>(
+    // warps per unit: up to 16 while all warps together stay within IX_SHARED_WARPS
+    uint32_t share_log = 0;
+    while (share_log < 4 && (uint64_t(ntiles) << (share_log + 1)) <= IX_SHARED_WARPS) ++share_log;
+    const uint64_t warps = uint64_t(ntiles) << share_log;
+    k_index_scan<F, 1><<<unsigned((warps + ix_warps(1) - 1) / ix_warps(1)), 32 * ix_warps(1), 0, st>>>(
         g, nmask, amask, G, chr_off, n_chr, ntiles, const_cast<uint32_t*>(cnt_scanned), stride, list_off, list_len,
-        lists);
+        lists, share_log);
   }
   note_launch();
 }
@@ -729,10 +741,10 @@ const char* index_counts_noalloc(int which, const uint32_t* g, uint64_t G, const
   const uint32_t blocks = (ntiles + IX_WARPS - 1) / IX_WARPS;
   if (which == 0)
     k_index_scan<SbsFamilies, 0><<<blocks, 256, 0, st>>>(g, nullptr, nullptr, G, chr_off, n_chr, ntiles, scratch,
-                                                         nullptr, nullptr, nullptr, nullptr);
+                                                         nullptr, nullptr, nullptr, nullptr, 0u);
   else
     k_index_scan<IdFamilies, 0><<<blocks, 256, 0, st>>>(g, nullptr, nullptr, G, chr_off, n_chr, ntiles, scratch,
-                                                        nullptr, nullptr, nullptr, nullptr);
+                                                        nullptr, nullptr, nullptr, nullptr, 0u);
   k_class_totals<<<nc, 256, 0, st>>>(scratch, ntiles, totals);
   note_launch(2);
   if (cudaGetLastError() != cudaSuccess) return "launch of the count kernels failed";
