@@ -9,10 +9,11 @@
 
 // A small caching pool: freed blocks are kept per engine and reused by size,
 // so repeated place/sequence calls do not pay cudaMalloc/cudaFree.  Blocks of
-// up to 2 MB are cut from slabs of 512 kB, 4 MB, then 16 MB each: an engine with
-// an index takes some 60 of them, at 3 to 10 us for each cudaMalloc (from 1 MB on
-// 30 us, whatever the size) and as much again to free them.  (A first slab of 2 MB
-// cost a small handle beside others 60 us.)  A slab can be given back only when
+// up to 2 MB are cut from slabs of 128 kB, 512 kB, 4 MB, then 16 MB each: an
+// engine with an index takes some 60 of them, at 3 to 10 us for each cudaMalloc
+// (from 1 MB on 30 us, whatever the size) and as much again to free them.  (A
+// first slab of 2 MB, which no chunk that the driver already has holds, cost a
+// small handle beside others 100 us.)  A slab can be given back only when
 // none of its blocks is in use, so the slabs take SLABS_MAX together at most; what
 // does not fit them (nor a slab the device has no room for) gets an allocation
 // of its own.
@@ -73,8 +74,8 @@ class Pool {
 
  private:
   static constexpr uint32_t OWN = 0xffffffffu;             // a block with an allocation of its own
-  static constexpr size_t SLAB_MAX_BLOCK = size_t(2) << 20, SLABS_MAX = size_t(64) << 20,
-                          FIRST_SLAB = size_t(512) << 10, NEXT_SLAB = size_t(4) << 20, LAST_SLAB = size_t(16) << 20;
+  static constexpr size_t SLAB_MAX_BLOCK = size_t(2) << 20, SLABS_MAX = size_t(64) << 20;
+  static constexpr size_t SLAB_SIZE[4] = {size_t(128) << 10, size_t(512) << 10, size_t(4) << 20, size_t(16) << 20};
   struct Slab { char* p = nullptr; size_t size = 0, used = 0; uint32_t live = 0; };
   struct Block { size_t size; uint32_t slab; };
   struct Free { void* p; uint32_t slab; };
@@ -82,7 +83,9 @@ class Pool {
   bool room(size_t bytes) {
     if (cur_ != OWN && slabs_[cur_].size - slabs_[cur_].used >= bytes) return true;
     Slab s;
-    s.size = slabs_.size() > 1 ? LAST_SLAB : slabs_.empty() && bytes <= FIRST_SLAB ? FIRST_SLAB : NEXT_SLAB;
+    size_t step = std::min<size_t>(slabs_.size(), 3);
+    while (SLAB_SIZE[step] < bytes) ++step;
+    s.size = SLAB_SIZE[step];
     if (slab_bytes_ + s.size > SLABS_MAX) return false;
     void* p = nullptr;
     if (cudaMalloc(&p, s.size) != cudaSuccess) { cudaGetLastError(); return false; }
